@@ -1,0 +1,76 @@
+"""Kernels behind a dispatch by size, at the sizes where each can go wrong: edges of tiles, remainders, the smallest and the largest of
+its range. Needs the built library and a B200."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+F32, B16 = torch.float32, torch.bfloat16
+
+
+@pytest.fixture(scope='module')
+def dev():
+    if not torch.cuda.is_available():
+        pytest.skip('needs a GPU')
+    import phi3_b200  # noqa: F401
+    return torch.device('cuda')
+
+
+def _stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
+def _gemm_any(x, w, bias=None, rows=None, seg=None, gate=None, out_dtype=F32, batch=None, N=None, K=None):
+    from phi3_b200 import _lib
+    M, n = (rows.numel() if rows is not None else x.shape[0]), (w.shape[-2] if N is None else N)
+    out = torch.full((M, n * (batch[0] if batch else 1)), float('nan'), dtype=out_dtype, device=x.device)
+    a = _lib.GemmAnyArgs()
+    a.X, a.ldx, a.x_f32, a.x_rows, a.x_row_div = x.data_ptr(), x.stride(0), int(x.dtype == F32), _lib.ptr(rows), 1
+    a.W, a.ldw, a.w_f32, a.w_group_stride = w.data_ptr(), w.stride(-2), int(w.dtype == F32), w.stride(0) if w.dim() == 3 and seg is not None else 0
+    a.bias, a.out, a.ldo, a.out_f32, a.M, a.N, a.K = _lib.ptr(bias), out.data_ptr(), out.stride(0), int(out_dtype == F32), M, n, w.shape[-1] if K is None else K
+    a.seg_offsets, a.n_groups = _lib.ptr(seg), 0 if seg is None else seg.numel() - 1
+    if batch:
+        a.n_batch, a.x_batch_stride, a.w_batch_stride, a.out_batch_stride = batch
+    if gate is not None:
+        a.gate, a.ld_gate = gate.data_ptr(), gate.stride(0)
+    _lib.call_struct('p3_gemm_any', a, _stream())
+    return out
+
+
+def _odd_pitch(t):
+    """the same matrix with a row pitch that is no multiple of 4: the kernel for any alignment takes it"""
+    out = torch.zeros(*t.shape[:-1], t.shape[-1] + 1 + t.shape[-1] % 2, dtype=t.dtype, device=t.device)
+    out[..., :t.shape[-1]] = t
+    return out[..., :t.shape[-1]]
+
+
+@pytest.mark.parametrize('M,N,K', [(1, 1, 4), (1, 33, 8), (2, 16, 128), (3, 47, 132), (5, 100, 100), (8, 17, 260), (9, 64, 640), (16, 130, 1000),
+                                   (17, 31, 16), (31, 33, 20), (33, 64, 12), (63, 129, 36), (65, 65, 260), (130, 1601, 64), (257, 200, 1000),
+                                   (700, 1700, 44), (1100, 2050, 16)])
+def test_fp32_products_of_aligned_rows_have_the_bits_of_the_general_kernel(dev, M, N, K):
+    """every tile (rows 1 .. 16, 32, 64, 128) sums one FMA chain in ascending k: the bits of the kernel that takes any alignment"""
+    g = torch.Generator(device=dev).manual_seed(M * 7 + N)
+    rn = lambda *s: torch.randn(s, generator=g, device=dev)
+    x, w, bias, gate = rn(M, K), rn(N, K), rn(N), rn(M, N)
+    for b, gt, dt in ((None, None, F32), (bias, gate, F32), (bias, None, B16)):
+        got, ref = _gemm_any(x, w, b, gate=gt, out_dtype=dt), _gemm_any(_odd_pitch(x), _odd_pitch(w), b, gate=gt, out_dtype=dt)
+        assert torch.equal(got, ref)
+    y = x.double() @ w.double().T
+    bound = 2.0 ** -24 * K * (x.double().abs() @ w.double().abs().T) + 1e-30      # rounding of a chain of K additions
+    assert ((_gemm_any(x, w).double() - y).abs() <= bound).all()
+
+
+@pytest.mark.parametrize('cuts', [[0, 0, 1, 1, 40], [0, 64, 65, 200, 200], [0, 500, 500, 501, 1200]])
+def test_fp32_grouped_gathered_and_batched_products(dev, cuts):
+    g = torch.Generator(device=dev).manual_seed(cuts[-1])
+    rn = lambda *s: torch.randn(s, generator=g, device=dev)
+    M, N, K = cuts[-1], 72, 52
+    x, w = rn(300, K), rn(4, N, K)
+    rows = torch.randint(0, 300, (M,), generator=g, device=dev, dtype=torch.int32)
+    seg = torch.tensor(cuts, dtype=torch.int32, device=dev)
+    got, ref = _gemm_any(x, w, rows=rows, seg=seg), _gemm_any(_odd_pitch(x), _odd_pitch(w), rows=rows, seg=seg)
+    assert torch.equal(got, ref) and bool(torch.isfinite(got).all())
+    for m in (1, 7, 16, 40, 200):                                   # three products over column blocks, gathered rows
+        xb, wb, r = rn(300, 3 * K), rn(3, N, K), rows[:1].repeat(m) if m > M else rows[:m].contiguous()
+        got = _gemm_any(xb, wb, rows=r, batch=(3, K, N * K, N), N=N, K=K)
+        ref = torch.cat([_gemm_any(_odd_pitch(xb[:, i * K:(i + 1) * K]), _odd_pitch(wb[i]), rows=r) for i in range(3)], 1)
+        assert torch.equal(got, ref)
