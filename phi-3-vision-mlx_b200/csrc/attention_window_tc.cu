@@ -161,16 +161,19 @@ attn_window_prefill_tc_kernel(const __grid_constant__ WinMaps tm, p3_attn_window
 
         if (warp == W_TMA) {
             if (lane == 0) {
-                for (int it = 0; it < n; it++) {
-                    const int st = it % ST;
-                    const uint32_t ph = (uint32_t)(it / ST) & 1u;
-                    const int row = (bt[page_at(it)] * a.n_kv + g) * 64;
-                    wait_lim(k_empty(st), ph ^ 1u, fail);
-                    mbar_expect_tx(k_full(st), kb * BOX);
-                    for (int b = 0; b < kb; b++) tma_load_2d(sK + (st * kb + b) * BOX, &tm.k, k_full(st), 64 * b, row);
-                    wait_lim(v_empty(st), ph ^ 1u, fail);
-                    mbar_expect_tx(v_full(st), vb * BOX);
-                    for (int b = 0; b < vb; b++) tma_load_2d(sV + (st * vb + b) * BOX, &tm.v, v_full(st), 64 * b, row);
+                for (int it = -1; it < n; it++) {            // K one page ahead of V: its stage comes free earlier
+                    if (it + 1 < n) {
+                        const int st = (it + 1) % ST, row = (bt[page_at(it + 1)] * a.n_kv + g) * 64;
+                        wait_lim(k_empty(st), ((uint32_t)((it + 1) / ST) & 1u) ^ 1u, fail);
+                        mbar_expect_tx(k_full(st), kb * BOX);
+                        for (int b = 0; b < kb; b++) tma_load_2d(sK + (st * kb + b) * BOX, &tm.k, k_full(st), 64 * b, row);
+                    }
+                    if (it >= 0) {
+                        const int st = it % ST, row = (bt[page_at(it)] * a.n_kv + g) * 64;
+                        wait_lim(v_empty(st), ((uint32_t)(it / ST) & 1u) ^ 1u, fail);
+                        mbar_expect_tx(v_full(st), vb * BOX);
+                        for (int b = 0; b < vb; b++) tma_load_2d(sV + (st * vb + b) * BOX, &tm.v, v_full(st), 64 * b, row);
+                    }
                 }
                 for (int it = max(0, n - ST); it < n; it++) {          // every release has arrived before the barriers may be set up anew
                     wait_lim(k_empty(it % ST), (uint32_t)(it / ST) & 1u, fail);
@@ -182,6 +185,8 @@ attn_window_prefill_tc_kernel(const __grid_constant__ WinMaps tm, p3_attn_window
             const int ks = d / 16;
             constexpr uint32_t ID = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);
             const uint32_t id_qk = ID | ((64u >> 3) << 17), id_pv = ID | (1u << 16) | ((uint32_t)(dv >> 3) << 17);
+            // operand descriptors; what changes is added to their address fields (16-byte units)
+            const uint64_t qd = umma_desc_sw128(sQ), kd0 = umma_desc_sw128(sK), vd0 = umma_desc_mn_sw128(sV, BOX, 1024);
             wait_lim(q_full, 0, fail);
             for (int t = 0; t < n + 2; t++) {
                 const int j = t - 2;
@@ -190,11 +195,11 @@ attn_window_prefill_tc_kernel(const __grid_constant__ WinMaps tm, p3_attn_window
                     wait_lim(sm_done(j), (uint32_t)(j >> 1) & 1u, fail);
                     tc_fence_after();
                     if (elect_one()) {
-                        const uint32_t p_col = tmem + (j & 1) * 64, vs = sV + (j % ST) * vb * BOX;
+                        const uint32_t p_col = tmem + (j & 1) * 64;
+                        const uint64_t vd = vd0 + (uint32_t)((j % ST) * vb * (BOX >> 4));
 #pragma unroll
                         for (int kk = 0; kk < 4; kk++)       // P of keys 0-31 in columns 0-15, of keys 32-63 in columns 32-47
-                            tc_mma_bf16_ts(tmem + O_COL, p_col + 32 * (kk >> 1) + 8 * (kk & 1), umma_desc_mn_sw128(vs + kk * (16 * 128), BOX, 1024), id_pv,
-                                           (j | kk) ? 1u : 0u);
+                            tc_mma_bf16_ts(tmem + O_COL, p_col + 32 * (kk >> 1) + 8 * (kk & 1), vd + kk * (16 * 128 >> 4), id_pv, kk ? 1u : (uint32_t)j);
                         tc_commit(o_done(j));
                         tc_commit(v_empty(j % ST));
                     }
@@ -204,10 +209,12 @@ attn_window_prefill_tc_kernel(const __grid_constant__ WinMaps tm, p3_attn_window
                     wait_lim(k_full(t % ST), (uint32_t)(t / ST) & 1u, fail);
                     tc_fence_after();
                     if (elect_one()) {
-                        const uint32_t ksm = sK + (t % ST) * kb * BOX, dst = tmem + (t & 1) * 64;
-                        for (int kk = 0; kk < ks; kk++)
-                            tc_mma_bf16(dst, umma_desc_sw128(sQ + (kk >> 2) * 2 * BOX) + 2 * (kk & 3), umma_desc_sw128(ksm + (kk >> 2) * BOX) + 2 * (kk & 3),
-                                        id_qk, kk ? 1u : 0u);
+                        const uint32_t dst = tmem + (t & 1) * 64;
+                        const uint64_t kd = kd0 + (uint32_t)((t % ST) * kb * (BOX >> 4));
+                        tc_mma_bf16(dst, qd, kd, id_qk, 0u);
+#pragma unroll
+                        for (int kk = 1; kk < 8; kk++)
+                            if (kk < ks) tc_mma_bf16(dst, qd + ((kk >> 2) * (2 * BOX >> 4) + 2 * (kk & 3)), kd + ((kk >> 2) * (BOX >> 4) + 2 * (kk & 3)), id_qk, 1u);
                         tc_commit(s_full(t));
                         tc_commit(k_empty(t % ST));
                     }
