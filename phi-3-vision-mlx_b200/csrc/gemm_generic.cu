@@ -450,6 +450,9 @@ __global__ void __launch_bounds__(128) gemm_any_mma_kernel(AnyP p) {
 }
 }  // namespace
 
+bool gemm_grouped_ok(const p3_gemm_any_args* a);               // gemm_tc.cu
+int launch_gemm_grouped(const p3_gemm_any_args* a, cudaStream_t st);
+
 extern "C" int p3_gemm_any(const p3_gemm_any_args* a, cudaStream_t st) {
     P3_CHECK_ARG(a && a->X && a->W && a->out, "gemm_any: null operand");
     P3_CHECK_ARG(a->M >= 0 && a->N >= 1 && a->K >= 1 && a->M < (1ll << 30), "gemm_any: bad sizes");
@@ -457,6 +460,7 @@ extern "C" int p3_gemm_any(const p3_gemm_any_args* a, cudaStream_t st) {
     P3_CHECK_ARG(!a->x_rows || a->x_row_div >= 1, "gemm_any: gather needs x_row_div >= 1");
     P3_CHECK_ARG(a->x_f32 == a->w_f32, "gemm_any: X and W must have the same element type");
     if (a->M == 0) return 0;
+    if (gemm_grouped_ok(a)) return launch_gemm_grouped(a, st);
     AnyP p{a->X, a->ldx, a->x_rows, a->x_row_div, a->W, a->ldw, a->w_group_stride, a->bias, a->bias_group_stride,
            a->out, a->ldo, a->M, a->N, a->K, a->seg_offsets, a->seg_offsets ? a->n_groups : 1,
            a->n_batch > 1 ? a->n_batch : 1, a->x_batch_stride, a->w_batch_stride, a->out_batch_stride, a->gate, a->ld_gate};

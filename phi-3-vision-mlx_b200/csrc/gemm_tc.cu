@@ -41,6 +41,8 @@ struct GemmEpi {
     // write-allocated lines do not push the resident W band / X rows out of L2 (ncu: 2.7-3.1x DRAM over-read without it)
     int stream_out;
     int band_mb;                                           // rasterisation band (MB of W kept L2-resident); 0 = default
+    // grouped product (mixture of experts): rows [seg[g], seg[g + 1]) of X multiply with the N rows of W that begin at g * w_rows
+    const int32_t* seg; int n_groups, w_rows;
 };
 __device__ __forceinline__ void st_out16(void* p, const uint4& v, int stream) {
     if (stream) __stcs(reinterpret_cast<uint4*>(p), v); else *reinterpret_cast<uint4*>(p) = v;
@@ -73,6 +75,32 @@ __host__ __device__ __forceinline__ int band_width(int K, int BN, int n_tiles, i
     long long per = (long long)BN * K * 2;
     int nb = (int)(((long long)(band_mb > 0 ? band_mb : (per <= (2ll << 20) ? 32 : 48)) << 20) / (per > 0 ? per : 1));
     return nb < 1 ? 1 : (nb > n_tiles ? n_tiles : nb);
+}
+
+// Grouped products: which rows a CTA multiplies is known on the device only. Every CTA forms the running count of row tiles of the groups (in
+// shared memory, behind the dependency wait) and finds the group of a tile by bisection; tiles of one group follow one another, column tiles
+// fastest, so that the CTAs in flight share rows of X and stream W.
+constexpr int GROUPS_MAX = 1024;
+struct GroupTable { int tiles[GROUPS_MAX + 1], row[GROUPS_MAX + 1]; };     // row tiles before group g; first row of group g
+struct GroupTile { int m, m_end, w, n; };                                  // rows [m, m_end) of X, rows of W from w + n on
+__device__ __forceinline__ void group_table(GroupTable& t, const int32_t* seg, int n_groups, int bm) {    // one warp
+    const int lane = threadIdx.x & 31;
+    int before = 0;
+    for (int g0 = 0; g0 <= n_groups; g0 += 32) {
+        const int g = g0 + lane, a = g <= n_groups ? seg[g] : 0, b = g < n_groups ? seg[g + 1] : a;
+        int c = (b - a + bm - 1) / bm;
+        const int own = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, c, o); if (lane >= o) c += v; }
+        if (g <= n_groups) { t.tiles[g] = before + c - own; t.row[g] = a; }
+        before += __shfl_sync(0xffffffffu, c, 31);
+    }
+}
+__device__ __forceinline__ GroupTile group_tile(const GroupTable& t, int n_groups, int w_rows, int tile, int n_tiles, int bm, int bn) {
+    const int mt = tile / n_tiles;
+    int lo = 0, hi = n_groups;                             // tiles[lo] <= mt < tiles[hi]
+    while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (t.tiles[mid] <= mt) lo = mid; else hi = mid; }
+    return {t.row[lo] + (mt - t.tiles[lo]) * bm, t.row[lo + 1], lo * w_rows, (tile - mt * n_tiles) * bn};
 }
 
 template <int BN>
@@ -263,9 +291,10 @@ __device__ __forceinline__ void epi_store32(const GemmEpi& ep, int64_t orow, int
     }
 }
 
-template <int BN>
+// GROUPED: tmA covers 128 rows per box, tmA32 32 (tiles of few rows: decode steps are a stream of W)
+template <int BN, bool GROUPED>
 __global__ void __launch_bounds__(384, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmEpi ep,
+gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmA32, GemmEpi ep,
                int M, int N, int K) {
     using C = TcCfg<BN>;
     extern __shared__ uint8_t smem_raw[];
@@ -282,7 +311,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m_tiles = (M + C::BM - 1) / C::BM, n_tiles = (N + BN - 1) / BN;
     const int ksplit = ep.ksplit > 1 ? ep.ksplit : 1;
-    const int total = m_tiles * n_tiles * ksplit, kb_all = (K + C::BK - 1) / C::BK;   // work item = (tile, K slice)
+    int total = m_tiles * n_tiles * ksplit; const int kb_all = (K + C::BK - 1) / C::BK;   // work item = (tile, K slice)
     const int nb = band_width(K, BN, n_tiles, ep.band_mb);
     __shared__ int s_last;
 
@@ -307,21 +336,34 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     // below (TMA loads of X, residual reads, output writes) may run before that kernel has completed
     pdl_trigger();
     pdl_wait();
+    __shared__ GroupTable groups;                              // (not part of the other kernel's shared memory)
+    if constexpr (GROUPED) {
+        if (warp == 3) group_table(groups, ep.seg, ep.n_groups, C::BM);
+        __syncthreads();
+        total = groups.tiles[ep.n_groups] * n_tiles;
+    }
 
     if (warp == 0) {
         if (lane == 0) {
             int stage = 0; uint32_t phase = 0;
             for (int item = blockIdx.x; item < total; item += gridDim.x) {
                 const int tile = item / ksplit, ks = item - tile * ksplit;
-                int mt_, nt_;
-                tile_coords(tile, m_tiles, n_tiles, nb, mt_, nt_);
-                const int m_idx = mt_ * C::BM, n_idx = nt_ * BN;
+                int m_idx, n_idx;
+                bool few = false;
+                if constexpr (GROUPED) {
+                    const GroupTile t = group_tile(groups, ep.n_groups, ep.w_rows, tile, n_tiles, C::BM, BN);
+                    m_idx = t.m; n_idx = t.w + t.n; few = t.m_end - t.m <= 32;
+                } else {
+                    int mt_, nt_;
+                    tile_coords(tile, m_tiles, n_tiles, nb, mt_, nt_);
+                    m_idx = mt_ * C::BM; n_idx = nt_ * BN;
+                }
                 const int k0 = (int)((long long)kb_all * ks / ksplit), k1 = (int)((long long)kb_all * (ks + 1) / ksplit);
                 for (int k = k0; k < k1; k++) {
                     mbar_wait(empty_bar(stage), phase ^ 1);
-                    mbar_expect_tx(full_bar(stage), C::STAGE_BYTES);
+                    mbar_expect_tx(full_bar(stage), GROUPED && few ? C::A_BYTES / 4 + C::B_BYTES : C::STAGE_BYTES);
                     const uint32_t sa = smem_base + stage * C::STAGE_BYTES;
-                    tma_load_2d(sa, &tmA, full_bar(stage), k * C::BK, m_idx);
+                    tma_load_2d(sa, GROUPED && few ? &tmA32 : &tmA, full_bar(stage), k * C::BK, m_idx);
                     tma_load_2d(sa + C::A_BYTES, &tmB, full_bar(stage), k * C::BK, n_idx);
                     if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
                 }
@@ -360,11 +402,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         int acc = 0; uint32_t acc_phase = 0;
         for (int item = blockIdx.x; item < total; item += gridDim.x) {
             const int tile = item / ksplit, ks = item - tile * ksplit;
-            int mt_, nt_;
-            tile_coords(tile, m_tiles, n_tiles, nb, mt_, nt_);
-            const int m_idx = mt_ * C::BM, n_idx = nt_ * BN;
+            int m_idx, n_idx, m_end = M;
+            if constexpr (GROUPED) {
+                const GroupTile t = group_tile(groups, ep.n_groups, ep.w_rows, tile, n_tiles, C::BM, BN);
+                m_idx = t.m; n_idx = t.n; m_end = t.m_end;
+            } else {
+                int mt_, nt_;
+                tile_coords(tile, m_tiles, n_tiles, nb, mt_, nt_);
+                m_idx = mt_ * C::BM; n_idx = nt_ * BN;
+            }
             const int row = m_idx + q * 32 + lane;
-            const bool row_ok = row < M;
+            const bool row_ok = row < m_end;
             const int64_t orow = row_ok ? (ep.row_map ? (int64_t)ep.row_map[row] : (int64_t)row) : 0;
             const float rs = epi_row_scale(ep, row, K, row_ok);  // summed while the tile's MMAs run
             RopeRow rr;                                          // likewise: page lookup + cos/sin rows pulled into L1
@@ -508,6 +556,7 @@ struct Tc2Cfg {
     static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
 };
 
+template <bool GROUPED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
 gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmEpi ep,
                 int M, int N, int K) {
@@ -528,7 +577,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const bool leader = rank == 0;
     const int m_pairs = (M + 2 * C::BM - 1) / (2 * C::BM), n_tiles = (N + BN - 1) / BN;
-    const int total = m_pairs * n_tiles, kb = (K + C::BK - 1) / C::BK;
+    int total = m_pairs * n_tiles; const int kb = (K + C::BK - 1) / C::BK;
     const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
     const int nb = band_width(K, BN, n_tiles, ep.band_mb);
 
@@ -553,15 +602,27 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     // below (TMA loads of X, residual reads, output writes) may run before that kernel has completed
     pdl_trigger();
     pdl_wait();
+    __shared__ GroupTable groups;
+    if constexpr (GROUPED) {
+        if (warp == 3) group_table(groups, ep.seg, ep.n_groups, 2 * C::BM);
+        __syncthreads();
+        total = groups.tiles[ep.n_groups] * n_tiles;
+    }
 
     if (warp == 0) {
         if (lane == 0) {
             int stage = 0; uint32_t phase = 0;
             for (int tile = cluster_id; tile < total; tile += n_clusters) {
-                int mt_, nt_;
-                tile_coords(tile, m_pairs, n_tiles, nb, mt_, nt_);
-                const int m_idx = mt_ * (2 * C::BM) + (int)rank * C::BM;
-                const int n_idx = nt_ * BN + (int)rank * (BN / 2);
+                int m_idx, n_idx;
+                if constexpr (GROUPED) {
+                    const GroupTile t = group_tile(groups, ep.n_groups, ep.w_rows, tile, n_tiles, 2 * C::BM, BN);
+                    m_idx = t.m; n_idx = t.w + t.n;
+                } else {
+                    int mt_, nt_;
+                    tile_coords(tile, m_pairs, n_tiles, nb, mt_, nt_);
+                    m_idx = mt_ * (2 * C::BM); n_idx = nt_ * BN;
+                }
+                m_idx += (int)rank * C::BM; n_idx += (int)rank * (BN / 2);
                 for (int k = 0; k < kb; k++) {
                     mbar_wait(empty_bar(stage), phase ^ 1);
                     if (leader) mbar_expect_tx(full_bar(stage), 2 * C::STAGE_BYTES);   // both CTAs' bytes land on CTA 0's barrier
@@ -603,11 +664,18 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const int q = warp & 3, half = (warp - 4) >> 2;
         int acc = 0; uint32_t acc_phase = 0;
         for (int tile = cluster_id; tile < total; tile += n_clusters) {
-            int mt_, nt_;
-            tile_coords(tile, m_pairs, n_tiles, nb, mt_, nt_);
-            const int m_idx = mt_ * (2 * C::BM) + (int)rank * C::BM, n_idx = nt_ * BN;
+            int m_idx, n_idx, m_end = M;
+            if constexpr (GROUPED) {
+                const GroupTile t = group_tile(groups, ep.n_groups, ep.w_rows, tile, n_tiles, 2 * C::BM, BN);
+                m_idx = t.m; n_idx = t.n; m_end = t.m_end;
+            } else {
+                int mt_, nt_;
+                tile_coords(tile, m_pairs, n_tiles, nb, mt_, nt_);
+                m_idx = mt_ * (2 * C::BM); n_idx = nt_ * BN;
+            }
+            m_idx += (int)rank * C::BM;
             const int row = m_idx + q * 32 + lane;
-            const bool row_ok = row < M;
+            const bool row_ok = row < m_end;
             const int64_t orow = row_ok ? (ep.row_map ? (int64_t)ep.row_map[row] : (int64_t)row) : 0;
             const float rs = epi_row_scale(ep, row, K, row_ok);  // summed while the tile's MMAs run
             RopeRow rr;                                          // likewise: page lookup + cos/sin rows pulled into L1
@@ -791,7 +859,7 @@ static int launch_tc(const void* X, int64_t ldx, const void* W, int64_t ldw, con
     else if (make_tmap(&tb, W, N, K, ldw, BN)) return -1;      // 64-row boxes are not part of the plan blob: encoded per call
     static bool attr_set[64] = {};                             // the attribute is per device
     if (!attr_set[cur_dev()]) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
         P3_CHECK_ARG(e == cudaSuccess, "gemm: cannot set %d B dynamic smem: %s", C::SMEM, cudaGetErrorString(e));
         attr_set[cur_dev()] = true;
     }
@@ -815,7 +883,7 @@ static int launch_tc(const void* X, int64_t ldx, const void* W, int64_t ldw, con
     }
     const int64_t items = tiles * e2.ksplit;
     unsigned grid = (unsigned)(items < num_sms() ? items : num_sms());
-    p3_launch_pdl(gemm_tc_kernel<BN>, dim3(grid), dim3(384), (size_t)C::SMEM, st, ta, tb, e2, (int)M, N, K);
+    p3_launch_pdl(gemm_tc_kernel<BN, false>, dim3(grid), dim3(384), (size_t)C::SMEM, st, ta, tb, ta, e2, (int)M, N, K);
     P3_CHECK_LAUNCH("gemm_tc");
     return 0;
 }
@@ -835,14 +903,51 @@ static int launch_tc2(const void* X, int64_t ldx, const void* W, int64_t ldw, co
     else if (make_tmap(&tb, W, N, K, ldw, C::BN / 2)) return -1;
     static bool attr_set[64] = {};
     if (!attr_set[cur_dev()]) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc2_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
         P3_CHECK_ARG(e == cudaSuccess, "gemm: cannot set %d B dynamic smem: %s", C::SMEM, cudaGetErrorString(e));
         attr_set[cur_dev()] = true;
     }
     int64_t tiles = ((M + 2 * C::BM - 1) / (2 * C::BM)) * ((N + C::BN - 1) / C::BN);
     int64_t clusters = tiles < num_sms() / 2 ? tiles : num_sms() / 2;
-    p3_launch_pdl(gemm_tc2_kernel, dim3((unsigned)(2 * clusters)), dim3(384), (size_t)C::SMEM, st, ta, tb, ep, (int)M, N, K);
+    p3_launch_pdl(gemm_tc2_kernel<false>, dim3((unsigned)(2 * clusters)), dim3(384), (size_t)C::SMEM, st, ta, tb, ep, (int)M, N, K);
     P3_CHECK_LAUNCH("gemm_tc2");
+    return 0;
+}
+
+// the shared memory of a grouped launch holds the group table beside the ring
+static bool grouped_attr(const void* kernel, int bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess; }
+
+// out[M, N] (fp32, or bf16) = grouped product over rows already in group order; W [n_groups][w_rows][K] with row pitch ldw
+bool gemm_grouped_ok(const p3_gemm_any_args* a) {
+    return a->seg_offsets && !a->x_rows && !a->bias && !a->gate && a->n_batch <= 1 && !a->force_fma && !a->x_f32 && a->n_groups <= GROUPS_MAX && a->K % 8 == 0 &&
+           a->ldx % 8 == 0 && a->ldw % 8 == 0 && a->ldw > 0 && a->w_group_stride % a->ldw == 0 && a->w_group_stride / a->ldw >= a->N &&
+           a->w_group_stride / a->ldw * a->n_groups < (1ll << 31) && (((uintptr_t)a->X | (uintptr_t)a->W | (uintptr_t)a->out) & 15) == 0;
+}
+int launch_gemm_grouped(const p3_gemm_any_args* a, cudaStream_t st) {
+    GemmEpi ep{};
+    ep.out = a->out; ep.ldo = a->ldo; ep.kind = a->out_f32 ? P3_EPI_F32 : P3_EPI_NONE; ep.ksplit = 1;
+    ep.seg = a->seg_offsets; ep.n_groups = a->n_groups; ep.w_rows = (int)(a->w_group_stride / a->ldw);
+    const int64_t w_all = (int64_t)ep.w_rows * (a->n_groups - 1) + a->N, mean = a->M / a->n_groups;
+    static bool attr_set[64] = {};
+    if (!attr_set[cur_dev()]) {
+        P3_CHECK_ARG(grouped_attr((const void*)gemm_tc_kernel<128, true>, TcCfg<128>::SMEM) && grouped_attr((const void*)gemm_tc2_kernel<true>, Tc2Cfg::SMEM),
+                     "gemm_any: cannot set the shared memory of the grouped product");
+        attr_set[cur_dev()] = true;
+    }
+    CUtensorMap ta, ta32, tb;
+    if (make_tmap(&ta, a->X, a->M, a->K, a->ldx, 128) || make_tmap(&tb, a->W, w_all, a->K, a->ldw, 128)) return -1;
+    if (mean >= 160) {
+        // CTA pairs on 256 x 256 tiles; more pairs than tiles only costs their launch
+        const int64_t most = (a->M / 256 + a->n_groups) * ((a->N + 255) / 256);
+        const int64_t clusters = most < num_sms() / 2 ? most : num_sms() / 2;
+        p3_launch_pdl(gemm_tc2_kernel<true>, dim3((unsigned)(2 * clusters)), dim3(384), (size_t)Tc2Cfg::SMEM, st, ta, tb, ep, (int)a->M, a->N, a->K);
+    } else {
+        if (make_tmap(&ta32, a->X, a->M, a->K, a->ldx, 32)) return -1;
+        const int64_t most = (a->M / 128 + (a->M < a->n_groups ? a->M : a->n_groups)) * ((a->N + 127) / 128);
+        p3_launch_pdl(gemm_tc_kernel<128, true>, dim3((unsigned)(most < num_sms() ? most : num_sms())), dim3(384), (size_t)TcCfg<128>::SMEM, st, ta, tb, ta32, ep,
+                      (int)a->M, a->N, a->K);
+    }
+    P3_CHECK_LAUNCH("gemm_any");
     return 0;
 }
 

@@ -45,7 +45,7 @@ class PagedLM:
     def _init_products(self):
         self.f32 = int(self.dtype == torch.float32)
         self.use_tc = os.environ.get('P3_LM_TC', '1') != '0'
-        self.moe_dense_rows = int(os.environ.get('P3_LM_MOE_DENSE_ROWS', '1024'))   # (token, choice) pairs from which experts run as dense GEMMs
+        self.moe_dense_rows = 1      # (token, choice) pairs from which the experts run on gathered rows (tcgen05)
         self.use_skinny = os.environ.get('P3_LM_SKINNY', '1') != '0' and hasattr(_lib.lib(), 'p3_gemm_skinny')
         self.profile = None      # bench.py: list of (kind, ev0, ev1, flops, bytes) when instrumenting
 
@@ -185,7 +185,7 @@ class PagedLM:
         A unit without a gate passes its up matrices alone ([E, ff, W]; the activation then gets [n, ff]). n_sorted: the router
         scores this many outputs, of which only the first f.experts have matrices (the pairs of the others are sorted behind them
         and skipped by the products); combine(dn, where) then replaces the plain weighted sum. meanwhile(): work that does not
-        depend on the choice (a shared unit); launched so that it covers the wait for the segment offsets."""
+        depend on the choice (a shared unit), launched behind the sort."""
         st, dev, n = _stream(), self.dev, T * f.top
         n_sorted = f.experts if n_sorted is None else n_sorted
         up = gu_w.shape[1]
@@ -196,41 +196,23 @@ class PagedLM:
         gu = torch.empty((n, up), dtype=torch.float32, device=dev)
         hid = torch.empty((n, f.ff), dtype=self.dtype, device=dev)
         dn = torch.empty((n, self.W), dtype=torch.float32, device=dev)
-        # Large batches (prompt portions): the segment offsets are read back (one small D2H per mixture layer, behind which the gather
-        # and `meanwhile` keep the device busy) and every expert's rows go through the tcgen05 GEMM as a dense product over the gathered,
-        # expert-ordered activations. Small batches stay on the device-side grouped kernel, which needs no host knowledge of the counts.
+        # The rows are brought into expert order and run as ONE grouped product per matrix on the tcgen05 GEMM, whose CTAs find their expert
+        # from the segment offsets on the device: nothing is read back, whatever the number of rows. What that kernel does not take (fp32,
+        # sizes that are no multiples of 8) runs on the grouped kernel for any shape, which gathers the rows itself.
         dense = self.experts_dense(f, T)
-        if dense:
-            cut = torch.empty(n_sorted + 1, dtype=torch.int32, pin_memory=True)
-            cut.copy_(seg, non_blocking=True)
-            landed = torch.cuda.Event()
-            landed.record()
         if meanwhile is not None:
             meanwhile()
         ev = self._ev()
         if dense:
             xs = torch.empty((n, self.W), dtype=self.dtype, device=dev)
             call('p3_gather_rows', ptr(xa), xa.stride(0), self.f32, ptr(order), f.top, ptr(xs), n, self.W, st)
-            landed.synchronize()
-            cut = cut.tolist()
-            for ex in range(f.experts):
-                a0, a1 = cut[ex], cut[ex + 1]
-                if a1 > a0:
-                    call('p3_gemm', ptr(xs[a0:a1]), xs.stride(0), ptr(gu_w[ex]), gu_w.stride(1), None, ptr(gu[a0:a1]), gu.stride(0),
-                         None, None, a1 - a0, up, self.W, _lib.EPI_F32, 0, st)
+            self.gemm_any(xs, gu_w, gu, seg=seg, n_groups=f.experts, M=n)
         else:
             self.gemm_any(xa, gu_w, gu, rows=order, row_div=f.top, seg=seg, n_groups=f.experts, M=n)
         self._ev(ev, 'moe_gemm', 2 * n * up * self.W, gu_w.numel() * gu_w.element_size())
         glu(gu, hid, n)
         ev = self._ev()
-        if dense:
-            for ex in range(f.experts):
-                a0, a1 = cut[ex], cut[ex + 1]
-                if a1 > a0:
-                    call('p3_gemm', ptr(hid[a0:a1]), hid.stride(0), ptr(down_w[ex]), down_w.stride(1), None, ptr(dn[a0:a1]),
-                         dn.stride(0), None, None, a1 - a0, self.W, f.ff, _lib.EPI_F32, 0, st)
-        else:
-            self.gemm_any(hid, down_w, dn, seg=seg, n_groups=f.experts, M=n)
+        self.gemm_any(hid, down_w, dn, seg=seg, n_groups=f.experts, M=n)
         self._ev(ev, 'moe_gemm', 2 * n * f.ff * self.W, down_w.numel() * down_w.element_size())
         if combine is not None:
             combine(dn, where)
@@ -239,5 +221,5 @@ class PagedLM:
                       self.W, st)
 
     def experts_dense(self, f, T):
-        """do the experts of a step with T tokens run as dense per-expert products (which reads the segment offsets back)?"""
+        """do the experts of a step with T tokens run on gathered rows (the tcgen05 GEMM)?"""
         return bool(self.use_tc and not self.f32 and T * f.top >= self.moe_dense_rows and self.W % 8 == 0 and f.ff % 8 == 0)

@@ -162,3 +162,35 @@ def test_prefill_attention_with_one_shared_row_per_token(dev):
     for H, lens in ((16, [(700, 100), (300, 0)]), (4, [(33, 0)]), (1, [(200, 64)])):
         y, ref = _attention(dev, H, 1, 128, 96, lens, window=512, shared=True, seed=H)
         assert float((y - ref).norm() / ref.norm()) < 6e-3
+
+
+@pytest.mark.parametrize('cuts', [[0, 1], [0, 0, 0, 3, 3], [0, 32, 65, 65, 200], [0, 129, 130, 258, 258], [0, 5, 300, 900, 901, 1500], [0] + [7 * i for i in range(1, 71)]])
+@pytest.mark.parametrize('N,K', [(128, 64), (200, 72), (72, 136), (384, 520)])
+def test_grouped_products_over_ordered_rows(dev, cuts, N, K):
+    """few rows per group (boxes of 32 and 128 rows) and many (CTA pairs); rows behind the last group are not written. fp32 sums of K bf16
+    products, in another order than float64: 2^-20 of the sum of magnitudes"""
+    g = torch.Generator(device=dev).manual_seed(N + cuts[-1])
+    M, E = cuts[-1] + 9, len(cuts) - 1
+    x, w = torch.randn(M, K, generator=g, device=dev).to(B16), torch.randn(E, N, K, generator=g, device=dev).to(B16)
+    seg = torch.tensor(cuts, dtype=torch.int32, device=dev)
+    for dt in (F32, B16):
+        got = _gemm_any(x, w, seg=seg, out_dtype=dt)
+        assert bool(torch.isnan(got[cuts[-1]:]).all())
+        for e in range(E):
+            a, b = cuts[e], cuts[e + 1]
+            y, bound = x[a:b].double() @ w[e].double().T, 2.0 ** -20 * (x[a:b].double().abs() @ w[e].double().abs().T)
+            if dt == B16:
+                bound = bound + 2.0 ** -8 * y.abs()
+            assert ((got[a:b].double() - y).abs() <= bound).all()
+
+
+@pytest.mark.parametrize('n,E', [(1, 1), (7, 3), (128, 8), (129, 5), (1000, 64), (8192, 8), (30001, 16)])
+def test_expert_order_is_stable(dev, n, E):
+    from phi3_b200 import _lib
+    g = torch.Generator(device=dev).manual_seed(n)
+    ids = torch.randint(0, E, (n,), generator=g, device=dev, dtype=torch.int32)
+    seg, order, where = (torch.full((k,), -1, dtype=torch.int32, device=dev) for k in (E + 1, n, n))
+    _lib.call('p3_moe_sort', ids.data_ptr(), n, E, seg.data_ptr(), order.data_ptr(), where.data_ptr(), _stream())
+    ref = torch.sort(ids.long(), stable=True).indices
+    assert torch.equal(order.long(), ref) and torch.equal(where[order.long()].long(), torch.arange(n, device=dev))
+    assert seg.tolist() == [int((ids < e).sum()) for e in range(E + 1)]
