@@ -63,7 +63,6 @@ template <typename T> __device__ __forceinline__ void stv(T* p, float v);
 template <> __device__ __forceinline__ void stv<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void stv<bf16>(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 
-constexpr int MM_TB = 32;        // tokens staged per round (16 for rows above 256 numbers, so that two rounds fit shared memory)
 constexpr int MM_MAIN = 4;       // warps that own columns of S; one more warp for the gates, one for the normaliser
 constexpr int MM_WARPS = MM_MAIN + 2;
 
@@ -72,7 +71,7 @@ __host__ __device__ inline int mm_m_copies(int vdim) { return (vdim + 31) / 32; 
 __host__ __device__ inline int64_t mm_head_floats(int dim, int vdim) { return (int64_t)dim * vdim + dim + mm_m_copies(vdim); }
 
 __device__ __forceinline__ float log_sigmoid(float z) {       // -softplus(-z), without overflow on either side
-    return z >= 0.f ? -log1pf(expf(-z)) : z - log1pf(expf(z));
+    return fminf(z, 0.f) - log1pf(expf(-fabsf(z)));          // both signs in one line: the lanes of a warp do not part
 }
 
 // 4-byte async copy global -> shared; src_bytes 0 writes zeros
@@ -80,10 +79,61 @@ __device__ __forceinline__ void cp_async4z(uint32_t dst, const void* src, int sr
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
 
+template <int VEC> __device__ __forceinline__ void ldvec(const float* p, float* v) {
+    if constexpr (VEC == 4) { const float4 u = *reinterpret_cast<const float4*>(p); v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w; }
+    else if constexpr (VEC == 2) { const float2 u = *reinterpret_cast<const float2*>(p); v[0] = u.x; v[1] = u.y; }
+    else v[0] = *p;
+}
+template <int VEC> __device__ __forceinline__ void stvec(float* p, const float* v) {
+    if constexpr (VEC == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    else if constexpr (VEC == 2) *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+    else *p = v[0];
+}
+
+template <typename K>
+int set_smem_attr(K kernel, size_t bytes) {
+    if (bytes > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        P3_CHECK_ARG(e == cudaSuccess, "matrix_memory_scan: shared memory attribute: %s", cudaGetErrorString(e));
+    }
+    return 0;
+}
+
+// The scans' launches. A scan whose CTAs fit one to an SM must get one to an SM: a launch that sets up while its predecessor (or the scan before)
+// still holds some SMs was seen to pair CTAs on others (4 x 2048 tokens of the delta rule queued one behind the other: 974 us against 580). So the
+// scans let their successor set up only at their end, and a CTA of such a launch asks for more than half of an SM's shared memory. With more CTAs
+// than SMs a round may be of `many` tokens, so that more of them share an SM (tokens per round do not change a bit of a token's numbers).
+struct ScanShape { int tb; size_t bytes; };
+inline ScanShape scan_shape(int64_t ctas, size_t floats_per_token, int dim, int many) {
+    const int tb = dim > 256 ? 16 : ctas <= 148 ? 32 : many;
+    size_t bytes = sizeof(float) * 2 * tb * floats_per_token;                            // two staged rounds
+    if (ctas <= 148 && bytes < 116 * 1024) bytes = 116 * 1024;
+    return {tb, bytes};
+}
+// a store that later shared-memory reads may be moved ahead of (the compiler cannot tell that `p` is not shared memory): with it four tokens of
+// the linear attention overlap (650 -> 550 us for 4 x 2048 tokens)
+__device__ __forceinline__ void st_out(float* p, float v) { asm volatile("st.global.f32 [%0], %1;" ::"l"(p), "f"(v)); }
+// a lane's rows d0 .. and its NC columns col, col + CW, .. of a head's state
+template <int DS, int NC, int CW>
+__device__ __forceinline__ void get_state(float (&S)[NC][DS], const float* Sg, int d, int dv, int d0, int col, bool fresh) {
+#pragma unroll
+    for (int c = 0; c < NC; c++)
+#pragma unroll
+        for (int j = 0; j < DS; j++)
+            S[c][j] = (!fresh && col + c * CW < dv && d0 + j < d) ? Sg[(size_t)(d0 + j) * dv + col + c * CW] : 0.f;
+}
+template <int DS, int NC, int CW>
+__device__ __forceinline__ void put_state(const float (&S)[NC][DS], float* Sg, int d, int dv, int d0, int col) {
+#pragma unroll
+    for (int c = 0; c < NC; c++)
+#pragma unroll
+        for (int j = 0; j < DS; j++)
+            if (col + c * CW < dv && d0 + j < d) Sg[(size_t)(d0 + j) * dv + col + c * CW] = S[c][j];
+}
+
 template <int DS, int RS, int NC, int TB>
 __global__ void __launch_bounds__(MM_WARPS * 32) matrix_memory_scan_kernel(p3_matrix_memory_args a) {
-    pdl_trigger();                                           // the next kernel may set up while this one runs ...
-    pdl_wait();                                              // ... and this one touches memory only after its predecessors are done
+    pdl_wait();                                              // memory is touched only after the predecessors are done
     // a warp = RS row slices x CW lanes, every lane with NC columns (CW apart); DP: dim rounded up; NR: n rows per lane
     constexpr int CW = 32 / RS, WCOLS = CW * NC, COLS = MM_MAIN * WCOLS, DP = DS * RS, NR = (DP + 31) / 32;
     constexpr int NT = MM_WARPS * 32;
@@ -106,11 +156,7 @@ __global__ void __launch_bounds__(MM_WARPS * 32) matrix_memory_scan_kernel(p3_ma
     float S[NC][DS], nr[NR];
     float m = 0.f;
     if (main) {
-#pragma unroll
-        for (int c = 0; c < NC; c++)
-#pragma unroll
-            for (int j = 0; j < DS; j++)
-                S[c][j] = (!fresh && col + c * CW < dv && d0 + j < d) ? Sg[(size_t)(d0 + j) * dv + col + c * CW] : 0.f;
+        get_state<DS, NC, CW>(S, Sg, d, dv, d0, col, fresh);
     } else if (gate_warp) {
         if (!fresh) m = mg[vb * (COLS / 32)];
     } else {
@@ -221,7 +267,7 @@ __global__ void __launch_bounds__(MM_WARPS * 32) matrix_memory_scan_kernel(p3_ma
                     if (RS >= 2) y += __shfl_xor_sync(0xffffffffu, y, CW);
                     if (RS >= 4) y += __shfl_xor_sync(0xffffffffu, y, 2 * CW);
                     if (lane < CW && col + c * CW < dv)
-                        a.out[(size_t)(row0 + t0 + tt) * a.ld_out + (size_t)hd * dv + col + c * CW] = y * a.q_scale;
+                        st_out(&a.out[(size_t)(row0 + t0 + tt) * a.ld_out + (size_t)hd * dv + col + c * CW], y * a.q_scale);
                 }
             }
         } else if (gate_warp) {
@@ -245,12 +291,9 @@ __global__ void __launch_bounds__(MM_WARPS * 32) matrix_memory_scan_kernel(p3_ma
             }
         }
     }
+    pdl_trigger();                                           // not before: see scan_shape
     if (main) {
-#pragma unroll
-        for (int c = 0; c < NC; c++)
-#pragma unroll
-            for (int j = 0; j < DS; j++)
-                if (col + c * CW < dv && d0 + j < d) Sg[(size_t)(d0 + j) * dv + col + c * CW] = S[c][j];
+        put_state<DS, NC, CW>(S, Sg, d, dv, d0, col);
     } else if (gate_warp) {
         if (lane == 0)
             for (int c = vb * (COLS / 32); c < min((vb + 1) * (COLS / 32), mm_m_copies(dv)); c++) mg[c] = m;
@@ -327,8 +370,7 @@ constexpr int GLA_WARPS = 4;     // every warp owns columns of S
 
 template <int DS, int RS, int NC, int TB>
 __global__ void __launch_bounds__(GLA_WARPS * 32) gla_scan_kernel(p3_gla_args a) {
-    pdl_trigger();                                           // the next kernel may set up while this one runs ...
-    pdl_wait();                                              // ... and this one touches memory only after its predecessors are done
+    pdl_wait();                                              // memory is touched only after the predecessors are done
     // a warp = RS row slices x CW lanes, every lane with NC columns (CW apart); DP: dim rounded up
     constexpr int CW = 32 / RS, WCOLS = CW * NC, COLS = GLA_WARPS * WCOLS, DP = DS * RS;
     constexpr int NT = GLA_WARPS * 32;
@@ -345,11 +387,7 @@ __global__ void __launch_bounds__(GLA_WARPS * 32) gla_scan_kernel(p3_gla_args a)
     float* Sg = a.state + ((size_t)slot * H + hd) * gla_head_floats(d, dv);
     const int col = vb * COLS + warp * WCOLS + lane % CW, d0 = (lane / CW) * DS;   // first of this lane's columns
     float S[NC][DS];
-#pragma unroll
-    for (int c = 0; c < NC; c++)
-#pragma unroll
-        for (int j = 0; j < DS; j++)
-            S[c][j] = (!fresh && col + c * CW < dv && d0 + j < d) ? Sg[(size_t)(d0 + j) * dv + col + c * CW] : 0.f;
+    get_state<DS, NC, CW>(S, Sg, d, dv, d0, col, fresh);
     const bool vec = d % 4 == 0 && a.ld_proj % 4 == 0 && a.q_off % 4 == 0 && a.k_off % 4 == 0 && ((uintptr_t)a.proj & 15) == 0 &&
                      a.ld_z % 4 == 0 && ((uintptr_t)a.z & 15) == 0;
 
@@ -395,7 +433,7 @@ __global__ void __launch_bounds__(GLA_WARPS * 32) gla_scan_kernel(p3_gla_args a)
         const float* ks = qs + TB * DPP;
         const float* as = ks + TB * DPP;
         const float* vs = as + TB * DPP;
-#pragma unroll(DS >= 128 ? 1 : 2)
+#pragma unroll(DS >= 128 ? 1 : DS <= 32 ? 4 : 2)
         for (int tt = 0; tt < nb; tt++) {
             float tv[NC], acc[NC][4];
 #pragma unroll
@@ -423,29 +461,15 @@ __global__ void __launch_bounds__(GLA_WARPS * 32) gla_scan_kernel(p3_gla_args a)
                 if (RS >= 2) y += __shfl_xor_sync(0xffffffffu, y, CW);
                 if (RS >= 4) y += __shfl_xor_sync(0xffffffffu, y, 2 * CW);
                 if (lane < CW && col + c * CW < dv)
-                    a.out[(size_t)(row0 + t0 + tt) * a.ld_out + (size_t)hd * dv + col + c * CW] = y * a.q_scale;
+                    st_out(&a.out[(size_t)(row0 + t0 + tt) * a.ld_out + (size_t)hd * dv + col + c * CW], y * a.q_scale);
             }
         }
     }
-#pragma unroll
-    for (int c = 0; c < NC; c++)
-#pragma unroll
-        for (int j = 0; j < DS; j++)
-            if (col + c * CW < dv && d0 + j < d) Sg[(size_t)(d0 + j) * dv + col + c * CW] = S[c][j];
+    pdl_trigger();                                           // not before: see scan_shape
+    put_state<DS, NC, CW>(S, Sg, d, dv, d0, col);
 }
 
 // ---------------------------------------------------------------- short convolutions, unit heads, gates of the scan behind them
-template <int VEC> __device__ __forceinline__ void ldvec(const float* p, float* v) {
-    if constexpr (VEC == 4) { const float4 u = *reinterpret_cast<const float4*>(p); v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w; }
-    else if constexpr (VEC == 2) { const float2 u = *reinterpret_cast<const float2*>(p); v[0] = u.x; v[1] = u.y; }
-    else v[0] = *p;
-}
-template <int VEC> __device__ __forceinline__ void stvec(float* p, const float* v) {
-    if constexpr (VEC == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-    else if constexpr (VEC == 2) *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
-    else *p = v[0];
-}
-
 // A lane owns NV vectors of VEC neighbouring channels, 32 VEC apart. TAPS > 0: the last TAPS - 1 inputs stay in registers from row
 // to row; TAPS 0: any number of taps, every row reads its inputs again.
 template <int VEC, int NV, int TAPS>
@@ -568,8 +592,7 @@ __host__ __device__ inline int64_t delta_head_floats(int dim, int vdim) { return
 
 template <int DS, int RS, int NC, int TB, bool DELTA>
 __global__ void __launch_bounds__(GLA_WARPS * 32) delta_scan_kernel(p3_delta_scan_args a) {
-    pdl_trigger();                                           // the next kernel may set up while this one runs ...
-    pdl_wait();                                              // ... and this one touches memory only after its predecessors are done
+    pdl_wait();                                              // memory is touched only after the predecessors are done
     // a warp = RS row slices x CW lanes, every lane with NC columns (CW apart); DP: dim rounded up
     constexpr int CW = 32 / RS, WCOLS = CW * NC, COLS = GLA_WARPS * WCOLS, DP = DS * RS;
     constexpr int NT = GLA_WARPS * 32;
@@ -633,11 +656,7 @@ __global__ void __launch_bounds__(GLA_WARPS * 32) delta_scan_kernel(p3_delta_sca
     }
     const float fixed = DELTA || a.gates ? 0.f : a.decay[hd], skip = DELTA || !a.skip ? 0.f : a.skip[hd];
     float S[NC][DS];
-#pragma unroll
-    for (int c = 0; c < NC; c++)
-#pragma unroll
-        for (int j = 0; j < DS; j++)
-            S[c][j] = (!fresh && col + c * CW < dv && d0 + j < d) ? Sg[(size_t)(d0 + j) * dv + col + c * CW] : 0.f;
+    get_state<DS, NC, CW>(S, Sg, d, dv, d0, col, fresh);
     for (int t0 = 0, r = 0; t0 < n_tok; t0 += TB, r++) {
         const int nb = min(TB, n_tok - t0), buf = r & 1;
         cp_async_wait<0>();                                  // this thread's copies of round r have landed ...
@@ -688,7 +707,7 @@ __global__ void __launch_bounds__(GLA_WARPS * 32) delta_scan_kernel(p3_delta_sca
                         r[h][c] = (sl & 1 ? p[2 * h + 1][c] : p[2 * h][c]) + __shfl_xor_sync(0xffffffffu, sl & 1 ? p[2 * h][c] : p[2 * h + 1][c], CW);
                 auto write = [&](int t, int c, float y) {
                     y = fmaf(skip, vs[t * COLS + warp * WCOLS + lane % CW + c * CW], y);
-                    if (col + c * CW < dv) a.out[(size_t)(row0 + t0 + t) * a.ld_out + (size_t)hd * dv + col + c * CW] = y;
+                    if (col + c * CW < dv) st_out(&a.out[(size_t)(row0 + t0 + t) * a.ld_out + (size_t)hd * dv + col + c * CW], y);
                 };
 #pragma unroll
                 for (int c = 0; c < NC; c++) {
@@ -697,7 +716,7 @@ __global__ void __launch_bounds__(GLA_WARPS * 32) delta_scan_kernel(p3_delta_sca
                 }
             }
         }
-#pragma unroll(DS >= (DELTA ? 64 : 128) ? 1 : 2)
+#pragma unroll(DS >= (DELTA ? 64 : 128) ? 1 : DS <= 32 ? 4 : 2)
         for (; tt < nb; tt++) {
             const float keep = DELTA || a.gates ? gs[2 * tt] : fixed, beta = DELTA || a.gates ? gs[2 * tt + 1] : 1.f;
             const float4* kq = reinterpret_cast<const float4*>(ks + tt * DPP + at_row(d0));
@@ -745,15 +764,12 @@ __global__ void __launch_bounds__(GLA_WARPS * 32) delta_scan_kernel(p3_delta_sca
                 if (RS >= 4) y += __shfl_xor_sync(0xffffffffu, y, 2 * CW);
                 if (!DELTA) y = fmaf(skip, vs[tt * COLS + warp * WCOLS + lane % CW + c * CW], y);
                 if (lane < CW && col + c * CW < dv)
-                    a.out[(size_t)(row0 + t0 + tt) * a.ld_out + (size_t)hd * dv + col + c * CW] = y;
+                    st_out(&a.out[(size_t)(row0 + t0 + tt) * a.ld_out + (size_t)hd * dv + col + c * CW], y);
             }
         }
     }
-#pragma unroll
-    for (int c = 0; c < NC; c++)
-#pragma unroll
-        for (int j = 0; j < DS; j++)
-            if (col + c * CW < dv && d0 + j < d) Sg[(size_t)(d0 + j) * dv + col + c * CW] = S[c][j];
+    pdl_trigger();                                           // not before: see scan_shape
+    put_state<DS, NC, CW>(S, Sg, d, dv, d0, col);
 }
 
 // one warp per (token, head)
@@ -856,14 +872,6 @@ __global__ void part_norm_gate_kernel(const float* __restrict__ y, int64_t ldy, 
     }
     for (int i = me + PN * nt; i < n; i += nt) stv(o + i, first(i) * r * wr[i] * (gr && !gate_first ? act(gr[i]) : 1.f));
 }
-template <typename K>
-int set_smem_attr(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        P3_CHECK_ARG(e == cudaSuccess, "matrix_memory_scan: shared memory attribute: %s", cudaGetErrorString(e));
-    }
-    return 0;
-}
 }  // namespace
 
 extern "C" int64_t p3_matrix_memory_state_floats(int n_heads, int dim, int vdim) { return (int64_t)n_heads * mm_head_floats(dim, vdim); }
@@ -882,18 +890,20 @@ extern "C" int p3_matrix_memory_scan(const p3_matrix_memory_args* a, cudaStream_
     if (a->rs_force == 8) { rs = 4; nc = 2; }
     if (a->dim > 256) { rs = 4; nc = 1; }                    // 128 rows per thread, 16 tokens per round
     const int per = (a->dim + rs - 1) / rs, ds = per <= 16 ? 16 : per <= 32 ? 32 : per <= 64 ? 64 : 128;
-    const int cols = MM_MAIN * 32 / rs * nc, tb = a->dim > 256 ? 16 : MM_TB;
+    const int cols = MM_MAIN * 32 / rs * nc;
     const dim3 grid((unsigned)a->n_seqs, (unsigned)a->n_heads, (unsigned)((a->vdim + cols - 1) / cols));
-    const size_t bytes = sizeof(float) * (size_t)2 * tb * (2 * (ds * rs + 4 * rs) + cols + 3);   // two staged rounds
+    const ScanShape sh = scan_shape((int64_t)grid.x * grid.y * grid.z, 2 * (ds * rs + 4 * rs) + cols + 3, a->dim, 32);
+#define GOT(DS, RS, NC, TB)                                                                                          \
+    do { if (set_smem_attr(matrix_memory_scan_kernel<DS, RS, NC, TB>, sh.bytes)) return -1;                           \
+         p3_launch_pdl(matrix_memory_scan_kernel<DS, RS, NC, TB>, grid, dim3(MM_WARPS * 32), sh.bytes, st, *a); } while (0)
 #define GO(DS, RS, NC)                                                                                              \
-    do { if (set_smem_attr(matrix_memory_scan_kernel<DS, RS, NC, MM_TB>, bytes)) return -1;                           \
-         p3_launch_pdl(matrix_memory_scan_kernel<DS, RS, NC, MM_TB>, dim3(grid), dim3(MM_WARPS * 32), (size_t)(bytes), st, *a); } while (0)
+    GOT(DS, RS, NC, 32)
     if (a->dim > 256) {
-        if (set_smem_attr(matrix_memory_scan_kernel<128, 4, 1, 16>, bytes)) return -1;
-        p3_launch_pdl(matrix_memory_scan_kernel<128, 4, 1, 16>, dim3(grid), dim3(MM_WARPS * 32), (size_t)(bytes), st, *a);
+        GOT(128, 4, 1, 16);
     } else if (rs == 2) { if (ds == 16) GO(16, 2, 1); else if (ds == 32) GO(32, 2, 1); else if (ds == 64) GO(64, 2, 1); else GO(128, 2, 1); }
     else if (nc == 1) { if (ds == 16) GO(16, 4, 1); else if (ds == 32) GO(32, 4, 1); else GO(64, 4, 1); }
     else { if (ds == 16) GO(16, 4, 2); else if (ds == 32) GO(32, 4, 2); else GO(64, 4, 2); }
+#undef GOT
 #undef GO
     P3_CHECK_LAUNCH("matrix_memory_scan");
     return 0;
@@ -975,18 +985,22 @@ extern "C" int p3_gla_scan(const p3_gla_args* a, cudaStream_t st) {
     if (a->rs_force == 8) { rs = 4; nc = 2; }
     if (a->dim > 256) { rs = 4; nc = 1; }                    // 128 rows per thread, 16 tokens per round
     const int per = (a->dim + rs - 1) / rs, ds = per <= 16 ? 16 : per <= 32 ? 32 : per <= 64 ? 64 : 128;
-    const int cols = GLA_WARPS * 32 / rs * nc, tb = a->dim > 256 ? 16 : MM_TB;
+    const int cols = GLA_WARPS * 32 / rs * nc;
     const dim3 grid((unsigned)a->n_seqs, (unsigned)a->n_heads, (unsigned)((a->vdim + cols - 1) / cols));
-    const size_t bytes = sizeof(float) * (size_t)2 * tb * (3 * (ds * rs + 4 * rs) + cols);   // two staged rounds
+    // 16 tokens per round for steps of few tokens per sequence (16 sequences x 1 token: 25 -> 18 us), 32 for prompts (4 x 1024 tokens of 64
+    // heads: 572 us against 630)
+    const ScanShape sh = scan_shape((int64_t)grid.x * grid.y * grid.z, 3 * (ds * rs + 4 * rs) + cols, a->dim, a->n_rows <= 4 * a->n_seqs ? 16 : 32);
+#define GOT(DS, RS, NC, TB)                                                                                          \
+    do { if (set_smem_attr(gla_scan_kernel<DS, RS, NC, TB>, sh.bytes)) return -1;                                     \
+         p3_launch_pdl(gla_scan_kernel<DS, RS, NC, TB>, grid, dim3(GLA_WARPS * 32), sh.bytes, st, *a); } while (0)
 #define GO(DS, RS, NC)                                                                                              \
-    do { if (set_smem_attr(gla_scan_kernel<DS, RS, NC, MM_TB>, bytes)) return -1;                                     \
-         p3_launch_pdl(gla_scan_kernel<DS, RS, NC, MM_TB>, dim3(grid), dim3(GLA_WARPS * 32), (size_t)(bytes), st, *a); } while (0)
+    do { if (sh.tb == 32) GOT(DS, RS, NC, 32); else GOT(DS, RS, NC, 16); } while (0)
     if (a->dim > 256) {
-        if (set_smem_attr(gla_scan_kernel<128, 4, 1, 16>, bytes)) return -1;
-        p3_launch_pdl(gla_scan_kernel<128, 4, 1, 16>, dim3(grid), dim3(GLA_WARPS * 32), (size_t)(bytes), st, *a);
+        GOT(128, 4, 1, 16);
     } else if (rs == 2) { if (ds == 16) GO(16, 2, 1); else if (ds == 32) GO(32, 2, 1); else if (ds == 64) GO(64, 2, 1); else GO(128, 2, 1); }
     else if (nc == 1) { if (ds == 16) GO(16, 4, 1); else if (ds == 32) GO(32, 4, 1); else GO(64, 4, 1); }
     else { if (ds == 16) GO(16, 4, 2); else if (ds == 32) GO(32, 4, 2); else GO(64, 4, 2); }
+#undef GOT
 #undef GO
     P3_CHECK_LAUNCH("gla_scan");
     return 0;
@@ -1042,17 +1056,19 @@ int launch_scan(const p3_delta_scan_args* a, cudaStream_t st, const char* who) {
     if (a->rs_force == 8) { rs = 4; nc = 2; }
     if (a->dim > 256) { rs = 4; nc = 1; }                    // 128 rows per thread, 16 tokens per round
     const int per = (a->dim + rs - 1) / rs, ds = per <= 16 ? 16 : per <= 32 ? 32 : per <= 64 ? 64 : 128;
-    const int cols = GLA_WARPS * 32 / rs * nc, tb = a->dim > 256 ? 16 : MM_TB;
+    const int cols = GLA_WARPS * 32 / rs * nc;
     const dim3 grid((unsigned)a->n_seqs, (unsigned)a->n_heads, (unsigned)((a->vdim + cols - 1) / cols));
-    const size_t bytes = sizeof(float) * (size_t)2 * tb * (2 * (ds * rs + 4 * rs) + cols + 2);   // two staged rounds
-#define GO(DS, RS, NC, TB)                                                                                             \
-    do { if (set_smem_attr(delta_scan_kernel<DS, RS, NC, TB, DELTA>, bytes)) return -1;                                  \
-         p3_launch_pdl(delta_scan_kernel<DS, RS, NC, TB, DELTA>, dim3(grid), dim3(GLA_WARPS * 32), (size_t)(bytes), st, *a); } while (0)
-    if (a->dim > 256) GO(128, 4, 1, 16);
-    else if (rs == 2) { if (ds == 16) GO(16, 2, 1, MM_TB); else if (ds == 32) GO(32, 2, 1, MM_TB); else if (ds == 64) GO(64, 2, 1, MM_TB); else GO(128, 2, 1, MM_TB); }
-    else if (nc == 1) { if (ds == 16) GO(16, 4, 1, MM_TB); else if (ds == 32) GO(32, 4, 1, MM_TB); else GO(64, 4, 1, MM_TB); }
-    else { if (ds == 16) GO(16, 4, 2, MM_TB); else if (ds == 32) GO(32, 4, 2, MM_TB); else GO(64, 4, 2, MM_TB); }
+    const ScanShape sh = scan_shape((int64_t)grid.x * grid.y * grid.z, 2 * (ds * rs + 4 * rs) + cols + 2, a->dim, 16);   // 16: 6 x 1000 tokens 428 -> 326 us without the correction
+#define GOT(DS, RS, NC, TB)                                                                                          \
+    do { if (set_smem_attr(delta_scan_kernel<DS, RS, NC, TB, DELTA>, sh.bytes)) return -1;                            \
+         p3_launch_pdl(delta_scan_kernel<DS, RS, NC, TB, DELTA>, grid, dim3(GLA_WARPS * 32), sh.bytes, st, *a); } while (0)
+#define GO(DS, RS, NC) do { if (sh.tb == 32) GOT(DS, RS, NC, 32); else GOT(DS, RS, NC, 16); } while (0)
+    if (a->dim > 256) GOT(128, 4, 1, 16);
+    else if (rs == 2) { if (ds == 16) GO(16, 2, 1); else if (ds == 32) GO(32, 2, 1); else if (ds == 64) GO(64, 2, 1); else GO(128, 2, 1); }
+    else if (nc == 1) { if (ds == 16) GO(16, 4, 1); else if (ds == 32) GO(32, 4, 1); else GO(64, 4, 1); }
+    else { if (ds == 16) GO(16, 4, 2); else if (ds == 32) GO(32, 4, 2); else GO(64, 4, 2); }
 #undef GO
+#undef GOT
     P3_CHECK_LAUNCH(who);
     return 0;
 }
