@@ -7,11 +7,15 @@
 //   warps 0-7:  softmax. A query row (TMEM lane) belongs to two threads, one per 32 of a page's 64 keys: sixteen such warps on an SM (two CTAs)
 //               hide one another's trips to TMEM and barriers; with a thread per row and eight warps a page of 256 rows took 2200 cycles, 1500
 //               of them arithmetic. S is double buffered in TMEM, so the scores of the next two pages are computed while this one is swept; P
-//               (bf16) goes back over the consumed S columns and is the A operand of P.V straight from TMEM. P is formed against the running
+//               goes back over the consumed S columns and is the A operand of P.V straight from TMEM. P is formed against the running
 //               reference maximum of the pages before (base-2 domain; the sink is the first reference, with a denominator of 1); the page's own
 //               maximum is found in the same sweep and shared by the row's two threads. O and l are rescaled when the reference falls 2^8
-//               behind, and the page is swept again when it falls 2^64 behind or there was none. Scores, penalties, weights before their
-//               rounding and all sums are fp32, two per instruction where that goes.
+//               behind, and the page is swept again when it falls 2^64 behind or there was none. Scores, penalties, weights and all sums are
+//               fp32, two per instruction where that goes.
+//               A weight is two bf16 numbers, its upper 16 bits and what they leave, and takes part in two products: with one rounded
+//               number the error against 64 bits was 2.4e-3 of the outputs (4 x 2048 tokens, 16 heads of 128 over 4, window 1024), above
+//               the 2.0e-3 of weights against each page's exact maximum, which took 142 us to form; with two it is 1.7e-3 in 119 us
+//               (108 with one; 298 on mma.sync).
 //   warp 8:     TMA producer, one page = 64-column SWIZZLE_128B boxes of K and of V, two mbarrier rings
 //   warp 9:     MMA issuer: O += P(j) V(j), then S(j + 2) = Q K(j + 2)^T into the columns P(j) left
 // Q rows are copied by the softmax warps (rows beyond a tile's end are not read). The penalties of a warp's 63 distances to its keys are staged
@@ -198,8 +202,9 @@ attn_window_prefill_tc_kernel(const __grid_constant__ WinMaps tm, p3_attn_window
                         const uint32_t p_col = tmem + (j & 1) * 64;
                         const uint64_t vd = vd0 + (uint32_t)((j % ST) * vb * (BOX >> 4));
 #pragma unroll
-                        for (int kk = 0; kk < 4; kk++)       // P of keys 0-31 in columns 0-15, of keys 32-63 in columns 32-47
-                            tc_mma_bf16_ts(tmem + O_COL, p_col + 32 * (kk >> 1) + 8 * (kk & 1), vd + kk * (16 * 128 >> 4), id_pv, kk ? 1u : (uint32_t)j);
+                        for (int kk = 0; kk < 8; kk++)       // P of keys 0-31 in columns 0-15, of keys 32-63 in columns 32-47; the rest 16 columns on
+                            tc_mma_bf16_ts(tmem + O_COL, p_col + 16 * (kk >> 2) + 32 * ((kk >> 1) & 1) + 8 * (kk & 1), vd + (kk & 3) * (16 * 128 >> 4), id_pv,
+                                           kk ? 1u : (uint32_t)j);
                         tc_commit(o_done(j));
                         tc_commit(v_empty(j % ST));
                     }
@@ -302,7 +307,7 @@ attn_window_prefill_tc_kernel(const __grid_constant__ WinMaps tm, p3_attn_window
                 // every key of the half page is visible to every row of the warp: behind its first row, and its last row still sees it
                 const bool full = all_rows && j0 + 31 <= warp_lo && (j0 >= lo_hi || j0 + 31 < a.keep_first);
                 const bool none = !any_rows || j0 > warp_hi;
-                uint32_t pk[16];
+                uint32_t pk[32];                             // weights: upper 16 bits, then what they leave
                 // one sweep over 32 scores of the row: maximum and / or weights against the reference mu
                 auto sweep = [&](auto do_max, auto do_exp, float mu, float& mx_out, float& ls_out) {
                     constexpr bool DM = decltype(do_max)::value, DE = decltype(do_exp)::value;
@@ -349,7 +354,10 @@ attn_window_prefill_tc_kernel(const __grid_constant__ WinMaps tm, p3_attn_window
                                     p0 = ex2f(p0); p1 = ex2f(p1);
                                     if (k & 2) add2(sA0, sA1, sA0, sA1, p0, p1); else add2(sB0, sB1, sB0, sB1, p0, p1);
                                 }
-                                pk[k / 2] = pack_bf16(p0, p1);
+                                pk[k / 2] = __byte_perm(__float_as_uint(p0), __float_as_uint(p1), 0x7632);
+                                float r0, r1;
+                                fma2(r0, r1, __uint_as_float(__float_as_uint(p0) & 0xffff0000u), __uint_as_float(__float_as_uint(p1) & 0xffff0000u), -1.f, -1.f, p0, p1);
+                                pk[16 + k / 2] = pack_bf16(r0, r1);
                             }
                         }
                     }
@@ -360,7 +368,7 @@ attn_window_prefill_tc_kernel(const __grid_constant__ WinMaps tm, p3_attn_window
                 const bool known = it > 0 || a.sink;         // there is a reference to form weights against
                 if (none) {
 #pragma unroll
-                    for (int k = 0; k < 16; k++) pk[k] = 0u;
+                    for (int k = 0; k < 32; k++) pk[k] = 0u;
                 } else if (SIG) sweep(std::false_type{}, std::true_type{}, 0.f, mx, ls);
                 else if (known) sweep(std::true_type{}, std::true_type{}, m == -INFINITY ? 0.f : m, mx, ls);
                 else sweep(std::true_type{}, std::false_type{}, 0.f, mx, ls);
@@ -382,6 +390,7 @@ attn_window_prefill_tc_kernel(const __grid_constant__ WinMaps tm, p3_attn_window
                     if (grow > 8.f) { pend = ex2f(-grow); has_pend = true; m = mx; }
                 }
                 st16(t_s, pk);
+                st16(t_s + 16, pk + 16);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(sm_done(it));
