@@ -974,13 +974,10 @@ static int launch_decode_mma(const p3_attn_window_args* a, cudaStream_t st) {
 /* rows per tile the launch accepts: 64 on the tensor-core path, 32 otherwise */
 extern "C" int p3_attn_window_tile_rows(const p3_attn_window_args* a) { return (a && prefill_mma_ok(a)) ? 64 : BQ; }
 
-bool attn_window_tc_ok(const p3_attn_window_args* a);          // attention_window_tc.cu
-int launch_attn_window_tc(const p3_attn_window_args* a, cudaStream_t st);
-
 extern "C" int p3_attn_window_prefill(const p3_attn_window_args* a, cudaStream_t st) {
     if (check_args(a, "attn_window_prefill")) return -1;
     if (a->n_tiles == 0) return 0;
-    const int rc = prefill_mma_ok(a) ? (attn_window_tc_ok(a) ? launch_attn_window_tc(a, st) : launch_prefill_mma(a, st))
+    const int rc = prefill_mma_ok(a) ? launch_prefill_mma(a, st)
                  : a->act_f32 ? launch_prefill<float, float>(a, st) : launch_prefill<bf16, bf16>(a, st);
     if (rc) return rc;
     P3_CHECK_LAUNCH("attn_window_prefill");
