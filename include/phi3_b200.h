@@ -122,6 +122,12 @@ int p3_gemm_skinny_qkv_rope_w4(const void* X, int64_t ldx, const void* norm_w, f
 int p3_gemm(const void* X, int64_t ldx, const void* W, int64_t ldw, const void* bias, void* out, int64_t ldo,
             const void* resid, const int32_t* row_map, int64_t M, int N, int K, int epi, int impl, cudaStream_t st);
 
+/* out (bf16) [M, F] = act(g) * u with [g | u] = X[M,K] . W[2F,K]^T (+ bias bf16 [2F]), gate rows of W first: the product and its gated
+ * unit in one launch on CTA pairs, fp32 up to the result. act 0 silu, 1 relu, 2 gelu (tanh form): as p3_glu_act; 3: as p3_glu_clamped
+ * with limit and alpha. F % 32 == 0, row pitches % 8 == 0, 16-byte operands. */
+int p3_gemm_glu(const void* X, int64_t ldx, const void* W, int64_t ldw, const void* bias, void* out, int64_t ldo, int64_t M, int F, int K,
+                int act, float limit, float alpha, cudaStream_t st);
+
 /* Prefill / ViT flash attention: phi:454-457 (causal + left-pad predicate instead of Mask4D
  * phi:550-563) and mx.fast.scaled_dot_product_attention phi:148 (causal=0).
  * q/k/v point into the (roped) qkv buffer; row strides in elements; head h at +h*hd.

@@ -141,6 +141,17 @@ struct P3DevFlags {
     bool& cur() { int d = 0; cudaGetDevice(&d); return set[(d < 0 || d >= 64) ? 0 : d]; }
 };
 
+// gated units y = act(g) * u; act = silu, relu or the tanh form of gelu, or the clamped unit, shared by the activation kernels and the GEMM epilogue
+#define P3_GLU_CLAMPED 3
+__device__ __forceinline__ float gelu_tanh(float z) { return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z))); }
+template <int ACT> __device__ __forceinline__ float glu_act(float g) {
+    return ACT == 0 ? g / (1.0f + expf(-g)) : ACT == 1 ? fmaxf(g, 0.f) : gelu_tanh(g);
+}
+__device__ __forceinline__ float glu_clamped(float g, float u, float limit, float alpha) {
+    const float a = fminf(g, limit), b = fminf(fmaxf(u, -limit), limit);
+    return a * (1.0f / (1.0f + expf(-alpha * a))) * (b + 1.0f);
+}
+
 // Paged KV pool addressing. One pool per layer:
 //   pool[page][kv(0=K,1=V)][head][slot(0..PAGE-1)][head_dim]   bf16
 #define P3_PAGE 64

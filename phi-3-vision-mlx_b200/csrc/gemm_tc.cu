@@ -43,6 +43,8 @@ struct GemmEpi {
     int band_mb;                                           // rasterisation band (MB of W kept L2-resident); 0 = default
     // grouped product (mixture of experts): rows [seg[g], seg[g + 1]) of X multiply with the N rows of W that begin at g * w_rows
     const int32_t* seg; int n_groups, w_rows;
+    // gated unit of [gate | up] weights, glu_f rows each (P3_EPI_GLU, pair kernel only)
+    int glu_f, glu_act; float glu_limit, glu_alpha;
 };
 __device__ __forceinline__ void st_out16(void* p, const uint4& v, int stream) {
     if (stream) __stcs(reinterpret_cast<uint4*>(p), v); else *reinterpret_cast<uint4*>(p) = v;
@@ -103,6 +105,7 @@ __device__ __forceinline__ GroupTile group_tile(const GroupTable& t, int n_group
     return {t.row[lo] + (mt - t.tiles[lo]) * bm, t.row[lo + 1], lo * w_rows, (tile - mt * n_tiles) * bn};
 }
 
+constexpr int EPI_SMEM = 8 * 2048;                           // the epilogue warps' blocks of output
 template <int BN>
 struct TcCfg {
     static constexpr int BM = 128, BK = 64;
@@ -111,22 +114,40 @@ struct TcCfg {
     static constexpr int B_BYTES = BN * BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     static constexpr int TMEM_COLS = 2 * BN;
-    static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
+    static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256 + EPI_SMEM;
     // kind::f16 instruction descriptor: D=f32 (1<<4), A=B=bf16 (1<<7, 1<<10), K-major both, N>>3 @17, M>>4 @24
     static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 };
 
-// per-row RMSNorm scale from the producer's partial sums (fixed order: deterministic); 1 when the GEMM is not normed
-__device__ __forceinline__ float epi_row_scale(const GemmEpi& ep, int row, int K, bool row_ok) {
-    if (!ep.ss_in || !row_ok) return 1.f;
-    const float* p = ep.ss_in + (size_t)row * ep.n_ss_in;
-    float s = 0.f;
-    if ((ep.n_ss_in & 3) == 0) {
-        for (int c = 0; c < ep.n_ss_in; c += 4) { const float4 f = __ldcg(reinterpret_cast<const float4*>(p + c)); s += (f.x + f.y) + (f.z + f.w); }
+// per-row RMSNorm scale from the producer's partial sums (fixed order: deterministic); 1 when the GEMM is not normed. Four lanes of the warp sum
+// a row and hand the result to the row's lane: reads of whole sectors, eight rows at a time (a lane for each row: 781 x 16384 x 3072 with 96
+// partial sums a row took 95 us, 81 without; now 91).
+__device__ __forceinline__ float epi_row_scale(const GemmEpi& ep, int row0, int m_end, int K) {
+    if (!ep.ss_in) return 1.f;
+    const int lane = threadIdx.x & 31, sub = lane >> 2, part = lane & 3, n = ep.n_ss_in;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    const float* p = ep.ss_in + (size_t)(row0 + sub) * n;
+    if ((n & 3) == 0) {
+#pragma unroll 2
+        for (int c = 4 * part; c < n; c += 16)
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (row0 + 8 * i + sub < m_end) { const float4 f = __ldcg(reinterpret_cast<const float4*>(p + (size_t)8 * i * n + c)); s[i] += (f.x + f.y) + (f.z + f.w); }
     } else {
-        for (int c = 0; c < ep.n_ss_in; c++) s += __ldcg(p + c);
+        for (int c = part; c < n; c += 4)
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (row0 + 8 * i + sub < m_end) s[i] += __ldcg(p + (size_t)8 * i * n + c);
     }
-    return rsqrtf(s / (float)K + ep.eps);
+    float own = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        s[i] += __shfl_xor_sync(0xffffffffu, s[i], 1);
+        s[i] += __shfl_xor_sync(0xffffffffu, s[i], 2);
+        const float t = __shfl_sync(0xffffffffu, s[i], 4 * (lane & 7));          // row 8 i + (lane & 7)
+        if (lane >> 3 == i) own = t;
+    }
+    return rsqrtf(own / (float)K + ep.eps);
 }
 
 // P3_EPI_ROPE_KV, per output row (token): everything that does not depend on the column chunk — computed once per tile,
@@ -207,8 +228,86 @@ __device__ __forceinline__ void epi_rope32(const GemmEpi& ep, const RopeRow& rr,
     }
 }
 
-// epilogue for 32 consecutive accumulator columns of one output row (rs: RMSNorm row scale, 1 when not normed)
-__device__ __forceinline__ void epi_store32(const GemmEpi& ep, int64_t orow, int n0, int N, const uint32_t* acc, float rs = 1.f) {
+// A warp's 32 rows x 64 bytes of output, turned in its own 2 KB of shared memory: a lane puts its row, and gets a quarter of every eighth row, so
+// that a store instruction writes 8 x 64 contiguous bytes. Straight from the accumulators' layout a lane writes 16 bytes of its own row and
+// every 32-byte sector takes two instructions (1024 x 9216 x 512, fp32 / bf16 results: 23.7 / 15.1 us, turned 16.2 / 13.3). 16-byte pieces are swizzled: no bank
+// conflicts either way.
+__device__ __forceinline__ void rows_put(uint8_t* sb, int lane, const uint4* v) {
+    __syncwarp();                                          // the block before is read
+#pragma unroll
+    for (int j = 0; j < 4; j++) *reinterpret_cast<uint4*>(sb + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = v[j];
+    __syncwarp();
+}
+__device__ __forceinline__ uint4 rows_get(const uint8_t* sb, int lane, int i) {          // of row 8 i + lane / 4
+    const int r = 8 * i + (lane >> 2);
+    return *reinterpret_cast<const uint4*>(sb + r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) << 4));
+}
+__device__ __forceinline__ int64_t epi_out_row(const GemmEpi& ep, int row) { return ep.row_map ? (int64_t)ep.row_map[row] : (int64_t)row; }
+// 32 bf16 columns of 32 rows (row0: the warp's first; rows from m_end on are not written)
+__device__ __forceinline__ void epi_put_bf16(const GemmEpi& ep, uint8_t* sb, int row0, int m_end, int n0, const uint4* v) {
+    const int lane = threadIdx.x & 31;
+    rows_put(sb, lane, v);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int row = row0 + 8 * i + (lane >> 2);
+        if (row < m_end) st_out16(reinterpret_cast<bf16*>(ep.out) + epi_out_row(ep, row) * ep.ldo + n0 + 8 * (lane & 3), rows_get(sb, lane, i), ep.stream_out);
+    }
+}
+
+// 32 outputs of a gated unit from its gate and up accumulators, in the arithmetic of the separate activation kernels
+template <int ACT> __device__ __forceinline__ void glu32(const GemmEpi& ep, const float* g, const float* u, uint32_t* o) {
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+        float y[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++)
+            y[e] = ACT == P3_GLU_CLAMPED ? glu_clamped(g[i + e], u[i + e], ep.glu_limit, ep.glu_alpha) : glu_act<ACT>(g[i + e]) * u[i + e];
+        o[i / 2] = pack_bf16(y[0], y[1]);
+    }
+}
+__device__ __forceinline__ void epi_glu32(const GemmEpi& ep, uint8_t* sb, int row0, int m_end, int n0, const uint32_t* ga, const uint32_t* ua) {
+    float g[32], u[32];
+#pragma unroll
+    for (int i = 0; i < 32; i++) { g[i] = __uint_as_float(ga[i]); u[i] = __uint_as_float(ua[i]); }
+    if (ep.bias) {
+#pragma unroll
+        for (int i = 0; i < 32; i += 8) {
+            const uint4 a = __ldg(reinterpret_cast<const uint4*>(ep.bias + n0 + i)), b = __ldg(reinterpret_cast<const uint4*>(ep.bias + ep.glu_f + n0 + i));
+            const uint32_t av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const float2 x = unpack_bf16(av[e]), y = unpack_bf16(bv[e]);
+                g[i + 2 * e] += x.x; g[i + 2 * e + 1] += x.y; u[i + 2 * e] += y.x; u[i + 2 * e + 1] += y.y;
+            }
+        }
+    }
+    uint4 o[4];
+    uint32_t* w = reinterpret_cast<uint32_t*>(o);
+    if (ep.glu_act == P3_GLU_CLAMPED) glu32<P3_GLU_CLAMPED>(ep, g, u, w);
+    else if (ep.glu_act == 0) glu32<0>(ep, g, u, w);
+    else if (ep.glu_act == 1) glu32<1>(ep, g, u, w);
+    else glu32<2>(ep, g, u, w);
+    epi_put_bf16(ep, sb, row0, m_end, n0, o);
+}
+
+// epilogue for 32 consecutive accumulator columns of a warp's 32 rows (row0: its first; rows from m_end on are not written; rs: RMSNorm scale of
+// the lane's row, 1 when not normed). Columns that end inside the 32, and row pitches that split 16-byte pieces, go element by element.
+// A residual's pieces of 64 bytes a row are read one ahead: `r` holds the first of this chunk on entry, of the chunk at n1 (none: n1 >= N) on exit.
+__device__ __forceinline__ bool epi_whole(const GemmEpi& ep, int n0, int N) {
+    return n0 + 32 <= N && (ep.ldo & (ep.kind == P3_EPI_F32 || ep.kind == P3_EPI_RESIDUAL_F32 ? 3 : 7)) == 0;
+}
+__device__ __forceinline__ void epi_resid(const GemmEpi& ep, int row0, int m_end, int n0, int N, int bytes, uint4* r) {
+    if ((ep.kind != P3_EPI_RESIDUAL && ep.kind != P3_EPI_RESIDUAL_F32) || !epi_whole(ep, n0, N)) return;
+    const int lane = threadIdx.x & 31, esz = ep.kind == P3_EPI_RESIDUAL_F32 ? 4 : 2;
+    const char* p = reinterpret_cast<const char*>(ep.resid) + (int64_t)n0 * esz + bytes + 16 * (lane & 3);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int row = row0 + 8 * i + (lane >> 2);
+        if (row < m_end) r[i] = *reinterpret_cast<const uint4*>(p + epi_out_row(ep, row) * ep.ldo * esz);
+    }
+}
+__device__ __forceinline__ void epi_rows32(const GemmEpi& ep, uint8_t* sb, int row0, int m_end, int n0, int n1, int N, const uint32_t* acc, float rs, uint4 (&r)[4]) {
+    const int lane = threadIdx.x & 31, own = row0 + lane, sub = lane >> 2, part = lane & 3;
     float v[32];
 #pragma unroll
     for (int i = 0; i < 32; i++) v[i] = __uint_as_float(acc[i]) * rs;
@@ -225,46 +324,42 @@ __device__ __forceinline__ void epi_store32(const GemmEpi& ep, int64_t orow, int
         }
     }
     if (ep.kind == P3_EPI_F32 || ep.kind == P3_EPI_RESIDUAL_F32) {
-        float* o = reinterpret_cast<float*>(ep.out) + orow * ep.ldo + n0;
-        if (ep.kind == P3_EPI_RESIDUAL_F32) {
-            const float* r = reinterpret_cast<const float*>(ep.resid) + orow * ep.ldo + n0;
-            if (n0 + 32 <= N && (ep.ldo & 3) == 0) {
+        const float* resid = ep.kind == P3_EPI_RESIDUAL_F32 ? reinterpret_cast<const float*>(ep.resid) : nullptr;
+        float* out = reinterpret_cast<float*>(ep.out);
+        if (epi_whole(ep, n0, N)) {
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    float4 f = reinterpret_cast<const float4*>(r)[i];
-                    v[4 * i] += f.x; v[4 * i + 1] += f.y; v[4 * i + 2] += f.z; v[4 * i + 3] += f.w;
+            for (int h = 0; h < 2; h++) {                      // 16 columns each
+                uint4 w[4], next[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    w[j] = make_uint4(__float_as_uint(v[16 * h + 4 * j]), __float_as_uint(v[16 * h + 4 * j + 1]), __float_as_uint(v[16 * h + 4 * j + 2]),
+                                      __float_as_uint(v[16 * h + 4 * j + 3]));
+                if (resid) epi_resid(ep, row0, m_end, h ? n1 : n0, N, h ? 0 : 64, next);
+                rows_put(sb, lane, w);
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int row = row0 + 8 * i + sub;
+                    const uint4 g = rows_get(sb, lane, i);
+                    float4 f = make_float4(__uint_as_float(g.x), __uint_as_float(g.y), __uint_as_float(g.z), __uint_as_float(g.w));
+                    if (resid) { f.x += __uint_as_float(r[i].x); f.y += __uint_as_float(r[i].y); f.z += __uint_as_float(r[i].z); f.w += __uint_as_float(r[i].w); }
+                    if (row < m_end) *reinterpret_cast<float4*>(out + epi_out_row(ep, row) * ep.ldo + n0 + 16 * h + 4 * part) = f;
                 }
-            } else {
-                for (int i = 0; i < 32; i++) if (n0 + i < N) v[i] += r[i];
-            }
-        }
-        if (n0 + 32 <= N && (ep.ldo & 3) == 0) {
+                if (resid) {
 #pragma unroll
-            for (int i = 0; i < 8; i++) reinterpret_cast<float4*>(o)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-        } else {
-            for (int i = 0; i < 32; i++) if (n0 + i < N) o[i] = v[i];
+                    for (int i = 0; i < 4; i++) r[i] = next[i];
+                }
+            }
+        } else if (own < m_end) {
+            const int64_t at = epi_out_row(ep, own) * ep.ldo + n0;
+#pragma unroll
+            for (int i = 0; i < 32; i++) if (n0 + i < N) out[at + i] = resid ? v[i] + resid[at + i] : v[i];
         }
         return;
     }
-    bf16* o = reinterpret_cast<bf16*>(ep.out) + orow * ep.ldo + n0;
-    const bool full = (n0 + 32 <= N) && ((ep.ldo & 7) == 0);
-    if (ep.kind == P3_EPI_RESIDUAL) {
-        const bf16* r = reinterpret_cast<const bf16*>(ep.resid) + orow * ep.ldo + n0;
-        if (full) {
-            uint4 rv[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) rv[i] = reinterpret_cast<const uint4*>(r)[i];
-            const uint32_t* ru = reinterpret_cast<const uint32_t*>(rv);
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                float2 f = unpack_bf16(ru[i]);
-                v[2 * i] = f.x + bf16_round(v[2 * i]);
-                v[2 * i + 1] = f.y + bf16_round(v[2 * i + 1]);
-            }
-        } else {
-            for (int i = 0; i < 32; i++) if (n0 + i < N) v[i] = __bfloat162float(r[i]) + bf16_round(v[i]);
-        }
-    } else if (ep.kind == P3_EPI_QGELU) {                     // one branch per chunk, not per element: with the kind test inside the
+    const bool full = epi_whole(ep, n0, N);
+    const bf16* resid = ep.kind == P3_EPI_RESIDUAL ? reinterpret_cast<const bf16*>(ep.resid) : nullptr;
+    bf16* out = reinterpret_cast<bf16*>(ep.out);
+    if (ep.kind == P3_EPI_QGELU) {                            // one branch per chunk, not per element: with the kind test inside the
 #pragma unroll                                                 // loop ptxas evaluates the erf polynomial for every element and selects
         for (int i = 0; i < 32; i++) v[i] = __fdividef(v[i], 1.f + __expf(-1.702f * v[i]));
     } else if (ep.kind == P3_EPI_GELU) {
@@ -276,17 +371,51 @@ __device__ __forceinline__ void epi_store32(const GemmEpi& ep, int64_t orow, int
         uint32_t* ou = reinterpret_cast<uint32_t*>(ov);
 #pragma unroll
         for (int i = 0; i < 16; i++) ou[i] = pack_bf16(v[2 * i], v[2 * i + 1]);
+        if (!resid && !ep.ss_out) { epi_put_bf16(ep, sb, row0, m_end, n0, ov); return; }
+        uint4 next[4];
+        if (resid) epi_resid(ep, row0, m_end, n1, N, 0, next);
+        rows_put(sb, lane, ov);
+        float sq[4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) st_out16(o + 8 * i, ov[i], ep.stream_out);
-        if (ep.ss_out) {                                       // sum of squares of the bf16 values just written
-            float sq = 0.f;
+        for (int i = 0; i < 4; i++) {
+            const int row = row0 + 8 * i + sub;
+            const uint4 g = rows_get(sb, lane, i);
+            uint32_t w[4] = {g.x, g.y, g.z, g.w};
+            if (resid) {
+                const uint32_t ru[4] = {r[i].x, r[i].y, r[i].z, r[i].w};
 #pragma unroll
-            for (int i = 0; i < 16; i++) { const float2 f = unpack_bf16(ou[i]); sq += f.x * f.x + f.y * f.y; }
-            ep.ss_out[(size_t)orow * (N / 32) + n0 / 32] = sq;
+                for (int e = 0; e < 4; e++) { const float2 f = unpack_bf16(ru[e]), x = unpack_bf16(w[e]); w[e] = pack_bf16(f.x + x.x, f.y + x.y); }
+            }
+            if (row < m_end) st_out16(out + epi_out_row(ep, row) * ep.ldo + n0 + 8 * part, make_uint4(w[0], w[1], w[2], w[3]), ep.stream_out);
+            sq[i] = 0.f;                                       // sum of squares of the bf16 values just written
+#pragma unroll
+            for (int e = 0; e < 4; e++) { const float2 f = unpack_bf16(w[e]); sq[i] += f.x * f.x + f.y * f.y; }
         }
-    } else {
+        if (ep.ss_out) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], 1);
+#pragma unroll
+            for (int i = 0; i < 4; i++) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], 2);
+            const int row = row0 + 8 * part + sub;
+            const float mine = part == 0 ? sq[0] : part == 1 ? sq[1] : part == 2 ? sq[2] : sq[3];
+            if (row < m_end) ep.ss_out[(size_t)epi_out_row(ep, row) * (N / 32) + n0 / 32] = mine;
+        }
+        if (resid) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) r[i] = next[i];
+        }
+    } else if (own < m_end) {
+        const int64_t orow = epi_out_row(ep, own);
+        bf16* o = out + orow * ep.ldo + n0;
+        const bf16* r = resid ? resid + orow * ep.ldo + n0 : nullptr;
         float sq = 0.f;
-        for (int i = 0; i < 32; i++) if (n0 + i < N) { o[i] = __float2bfloat16_rn(v[i]); const float f = bf16_round(v[i]); sq += f * f; }
+#pragma unroll
+        for (int i = 0; i < 32; i++) {
+            if (n0 + i >= N) continue;
+            o[i] = __float2bfloat16_rn(r ? __bfloat162float(r[i]) + bf16_round(v[i]) : v[i]);
+            const float f = __bfloat162float(o[i]);
+            sq += f * f;
+        }
         if (ep.ss_out) ep.ss_out[(size_t)orow * (N / 32) + n0 / 32] = sq;
     }
 }
@@ -399,6 +528,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     } else if (warp >= 4) {
         const int q = warp & 3, half = (warp - 4) >> 2;       // TMEM lane quarter, column half
+        uint8_t* sb = smem_raw + (bars + 256 - smem_u32(smem_raw)) + (warp - 4) * 2048;
         int acc = 0; uint32_t acc_phase = 0;
         for (int item = blockIdx.x; item < total; item += gridDim.x) {
             const int tile = item / ksplit, ks = item - tile * ksplit;
@@ -414,61 +544,72 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const int row = m_idx + q * 32 + lane;
             const bool row_ok = row < m_end;
             const int64_t orow = row_ok ? (ep.row_map ? (int64_t)ep.row_map[row] : (int64_t)row) : 0;
-            const float rs = epi_row_scale(ep, row, K, row_ok);  // summed while the tile's MMAs run
+            const float rs = epi_row_scale(ep, row - lane, m_end, K);  // summed while the tile's MMAs run
             RopeRow rr;                                          // likewise: page lookup + cos/sin rows pulled into L1
             if (ep.kind == P3_EPI_ROPE_KV && row_ok) rr = epi_rope_row(ep, (int)orow);
+            uint4 r[4];
+            epi_resid(ep, row - lane, m_end, n_idx + half * (BN / 2), N, 0, r);
             mbar_wait(tfull_bar(acc), acc_phase);
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
-            // chunk loader: 32 accumulator columns of this thread's row — straight from TMEM, or (split-K, last CTA of the
-            // tile) the sum of all K slices' partials in slice order
-            float* wsrow = ep.ws + ((size_t)tile * ksplit * C::BM + (size_t)(q * 32 + lane)) * BN;   // slice 0, this row
-            bool from_ws = false;
-            if (ksplit > 1) {
+            if (!GROUPED && ksplit > 1) {
+                float* wsrow = ep.ws + ((size_t)tile * ksplit * C::BM + (size_t)(q * 32 + lane)) * BN;   // slice 0, this row
                 float* mine = wsrow + (size_t)ks * C::BM * BN;
+#pragma unroll 1
                 for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
                     uint32_t v[32];
                     tc_ld32(taddr + c0, v);                                     // (warp-collective: every lane loads)
-                    if (!row_ok) continue;
+                    if (row_ok) {
 #pragma unroll
-                    for (int i = 0; i < 8; i++)
-                        reinterpret_cast<float4*>(mine + c0)[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
-                                                                               __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
+                        for (int i = 0; i < 8; i++)
+                            reinterpret_cast<float4*>(mine + c0)[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
+                                                                                   __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
+                    }
+                    __syncwarp();
                 }
                 tc_fence_before();
-                mbar_arrive(tempty_bar(acc));                                   // the accumulator stage is free again
-                if (++acc == 2) { acc = 0; acc_phase ^= 1; }
                 __threadfence();
                 asm volatile("bar.sync 2, 256;" ::: "memory");                  // the 8 epilogue warps
                 if (threadIdx.x == 128) s_last = (atomicAdd(ep.counters + tile, 1) == ksplit - 1);
                 asm volatile("bar.sync 2, 256;" ::: "memory");
-                if (!s_last) continue;
-                __threadfence();
-                if (threadIdx.x == 128) ep.counters[tile] = 0;                  // ready for the next launch
-                from_ws = true;
-            }
-            auto load32 = [&](int c, uint32_t* v) {
-                if (!from_ws) { tc_ld32(taddr + c, v); return; }
-                if (!row_ok) return;
-                float a[32];
-#pragma unroll
-                for (int i = 0; i < 32; i++) a[i] = 0.f;
-                for (int s2 = 0; s2 < ksplit; s2++) {
-                    const float4* src = reinterpret_cast<const float4*>(wsrow + (size_t)s2 * C::BM * BN + c);
-#pragma unroll
-                    for (int i = 0; i < 8; i++) { const float4 f = __ldcg(src + i); a[4 * i] += f.x; a[4 * i + 1] += f.y; a[4 * i + 2] += f.z; a[4 * i + 3] += f.w; }
+                if (!s_last) {
+                    mbar_arrive(tempty_bar(acc));                               // the accumulator stage is free again
+                    if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+                    continue;
                 }
+                __threadfence();
+                tc_fence_after();
+                if (threadIdx.x == 128) ep.counters[tile] = 0;                  // ready for the next launch
+                // the last CTA of the tile: all slices' partials, in slice order, back into its accumulators
+#pragma unroll 1
+                for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
+                    float4 f[8];
 #pragma unroll
-                for (int i = 0; i < 32; i++) v[i] = __float_as_uint(a[i]);
-            };
+                    for (int i = 0; i < 8; i++) f[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (row_ok) {
+#pragma unroll 1
+                        for (int s2 = 0; s2 < ksplit; s2++) {
+                            const float4* src = reinterpret_cast<const float4*>(wsrow + (size_t)s2 * C::BM * BN + c0);
+#pragma unroll
+                            for (int i = 0; i < 8; i++) { const float4 g = __ldcg(src + i); f[i].x += g.x; f[i].y += g.y; f[i].z += g.z; f[i].w += g.w; }
+                        }
+                    }
+                    __syncwarp();
+                    tc_st32(taddr + c0, reinterpret_cast<const uint32_t*>(f));
+                }
+                tc_fence_before();
+                asm volatile("bar.sync 2, 256;" ::: "memory");                  // SwiGLU reads columns that other warps summed
+                tc_fence_after();
+            }
             if (ep.kind == P3_EPI_SWIGLU) {
                 // interleaved weights: columns [0,BN/2) gate, [BN/2,BN) matching up
+#pragma unroll 1
                 for (int c0 = half * (BN / 4); c0 < (half + 1) * (BN / 4); c0 += 32) {
                     uint32_t g[32], u[32];
-                    load32(c0, g);
-                    load32(BN / 2 + c0, u);
+                    tc_ld32(taddr + c0, g);
+                    tc_ld32(taddr + BN / 2 + c0, u);
                     const int on0 = n_idx / 2 + c0;
-                    if (row_ok && on0 < N / 2) {
+                    if (on0 < N / 2) {
                         uint4 ov[4];
                         uint32_t* ou = reinterpret_cast<uint32_t*>(ov);
 #pragma unroll
@@ -478,11 +619,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             float a0 = bf16_round(g0 / (1.f + __expf(-g0))), a1 = bf16_round(g1 / (1.f + __expf(-g1)));
                             ou[i] = pack_bf16(a0 * u0, a1 * u1);
                         }
-                        bf16* o = reinterpret_cast<bf16*>(ep.out) + orow * ep.ldo + on0;
-                        if (on0 + 32 <= N / 2 && (ep.ldo & 7) == 0) {
-#pragma unroll
-                            for (int i = 0; i < 4; i++) st_out16(o + 8 * i, ov[i], ep.stream_out);
-                        } else {
+                        if (on0 + 32 <= N / 2 && (ep.ldo & 7) == 0) epi_put_bf16(ep, sb, row - lane, m_end, on0, ov);
+                        else if (row_ok) {
+                            bf16* o = reinterpret_cast<bf16*>(ep.out) + orow * ep.ldo + on0;
                             const bf16* ob = reinterpret_cast<const bf16*>(ov);
                             for (int i = 0; i < 32; i++) if (on0 + i < N / 2) o[i] = ob[i];
                         }
@@ -491,23 +630,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             } else if (ep.kind == P3_EPI_ROPE_KV) {
                 RopeRow rr;
                 if (row_ok) rr = epi_rope_row(ep, (int)orow);
+#pragma unroll 1
                 for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
                     uint32_t v[32];
-                    load32(c0, v);
+                    tc_ld32(taddr + c0, v);
                     if (row_ok && n_idx + c0 < N) epi_rope32(ep, rr, n_idx + c0, rs, v);
                 }
             } else {
+#pragma unroll 1
                 for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
                     uint32_t v[32];
-                    load32(c0, v);
-                    if (row_ok && n_idx + c0 < N) epi_store32(ep, orow, n_idx + c0, N, v, rs);
+                    tc_ld32(taddr + c0, v);
+                    if (n_idx + c0 < N) epi_rows32(ep, sb, row - lane, m_end, n_idx + c0, c0 + 32 < (half + 1) * (BN / 2) ? n_idx + c0 + 32 : N, N, v, rs, r);
                 }
             }
-            if (ksplit == 1) {
-                tc_fence_before();
-                mbar_arrive(tempty_bar(acc));
-                if (++acc == 2) { acc = 0; acc_phase ^= 1; }
-            }
+            tc_fence_before();
+            mbar_arrive(tempty_bar(acc));
+            if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         }
     }
     tc_fence_before();
@@ -548,20 +687,22 @@ __device__ __forceinline__ void cluster_sync_all() {
 }
 
 struct Tc2Cfg {
-    static constexpr int BM = 128, BN = 256, BK = 64, STAGES = 6;
-    static constexpr int A_BYTES = BM * BK * 2, B_BYTES = (BN / 2) * BK * 2;      // per CTA: own A rows + half of W rows
+    static constexpr int BM = 128, BN_MAX = 256, BK = 64, STAGES = 6;
+    static constexpr int A_BYTES = BM * BK * 2, B_BYTES = (BN_MAX / 2) * BK * 2;  // per CTA: own A rows + half of W rows
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr int TMEM_COLS = 2 * BN;
-    static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
-    static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
+    static constexpr int TMEM_COLS = 2 * BN_MAX;
+    static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256 + EPI_SMEM;
+    static constexpr __host__ __device__ uint32_t idesc(int bn) { return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24); }
 };
 
-template <bool GROUPED>
+// GLU: out = act(gate) * up in the epilogue. A tile is 128 gate columns beside the matching 128 up columns: the leader CTA loads gate rows of W,
+// its peer the up rows F further on, so the weights stay as they are and the fp32 [gate | up] rows never reach memory (5418 rows, K 2048,
+// F 8192: product 291 us + activation 110 us before, 233 us as one).
+template <bool GROUPED, bool GLU = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
 gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmEpi ep,
-                int M, int N, int K) {
+                int M, int N, int K, int BN) {
     using C = Tc2Cfg;
-    constexpr int BN = C::BN;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t bars = smem_base + C::STAGES * C::STAGE_BYTES;
@@ -576,7 +717,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const bool leader = rank == 0;
-    const int m_pairs = (M + 2 * C::BM - 1) / (2 * C::BM), n_tiles = (N + BN - 1) / BN;
+    const int m_pairs = (M + 2 * C::BM - 1) / (2 * C::BM), n_tiles = GLU ? (ep.glu_f + 127) / 128 : (N + BN - 1) / BN;
+    const uint32_t stage_tx = 2u * (C::A_BYTES + (uint32_t)BN * C::BK), idesc = Tc2Cfg::idesc(BN);   // a pair's bytes of one k block
     int total = m_pairs * n_tiles; const int kb = (K + C::BK - 1) / C::BK;
     const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
     const int nb = band_width(K, BN, n_tiles, ep.band_mb);
@@ -620,12 +762,12 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 } else {
                     int mt_, nt_;
                     tile_coords(tile, m_pairs, n_tiles, nb, mt_, nt_);
-                    m_idx = mt_ * (2 * C::BM); n_idx = nt_ * BN;
+                    m_idx = mt_ * (2 * C::BM); n_idx = nt_ * (GLU ? 128 : BN);
                 }
-                m_idx += (int)rank * C::BM; n_idx += (int)rank * (BN / 2);
+                m_idx += (int)rank * C::BM; n_idx += (int)rank * (GLU ? ep.glu_f : BN / 2);
                 for (int k = 0; k < kb; k++) {
                     mbar_wait(empty_bar(stage), phase ^ 1);
-                    if (leader) mbar_expect_tx(full_bar(stage), 2 * C::STAGE_BYTES);   // both CTAs' bytes land on CTA 0's barrier
+                    if (leader) mbar_expect_tx(full_bar(stage), stage_tx);   // both CTAs' bytes land on CTA 0's barrier
                     const uint32_t sa = smem_base + stage * C::STAGE_BYTES;
                     const uint32_t fb0 = full_bar(stage) & P3_PEER_MASK;
                     tma_load_2d_2sm(sa, &tmA, fb0, k * C::BK, m_idx);
@@ -641,7 +783,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             for (int tile = cluster_id; tile < total; tile += n_clusters) {
                 mbar_wait(tempty_bar(acc), acc_phase ^ 1);
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
+                const uint32_t d_tmem = tmem_base + (uint32_t)(acc * C::BN_MAX);
                 for (int k = 0; k < kb; k++) {
                     mbar_wait(full_bar(stage), phase);
                     tc_fence_after();
@@ -650,7 +792,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     if (elect_one()) {
 #pragma unroll
                         for (int kk = 0; kk < C::BK / 16; kk++)
-                            tc_mma_bf16_2sm(d_tmem, adesc + 2 * kk, bdesc + 2 * kk, C::IDESC, (k | kk) ? 1u : 0u);
+                            tc_mma_bf16_2sm(d_tmem, adesc + 2 * kk, bdesc + 2 * kk, idesc, (k | kk) ? 1u : 0u);
                         tc_commit_2sm_mc(empty_bar(stage));                             // frees the slot in both CTAs
                         if (k == kb - 1) tc_commit_2sm_mc(tfull_bar(acc));              // accumulators ready in both CTAs
                     }
@@ -662,6 +804,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
     } else if (warp >= 4) {
         const int q = warp & 3, half = (warp - 4) >> 2;
+        const int c_mid = (BN / 32 + 1) / 2 * 32, c_lo = half ? c_mid : 0, c_hi = half ? BN : c_mid;   // this warp's columns
+        uint8_t* sb = smem_raw + (bars + 256 - smem_u32(smem_raw)) + (warp - 4) * 2048;
         int acc = 0; uint32_t acc_phase = 0;
         for (int tile = cluster_id; tile < total; tile += n_clusters) {
             int m_idx, n_idx, m_end = M;
@@ -671,25 +815,34 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             } else {
                 int mt_, nt_;
                 tile_coords(tile, m_pairs, n_tiles, nb, mt_, nt_);
-                m_idx = mt_ * (2 * C::BM); n_idx = nt_ * BN;
+                m_idx = mt_ * (2 * C::BM); n_idx = nt_ * (GLU ? 128 : BN);
             }
             m_idx += (int)rank * C::BM;
             const int row = m_idx + q * 32 + lane;
             const bool row_ok = row < m_end;
             const int64_t orow = row_ok ? (ep.row_map ? (int64_t)ep.row_map[row] : (int64_t)row) : 0;
-            const float rs = epi_row_scale(ep, row, K, row_ok);  // summed while the tile's MMAs run
+            const float rs = epi_row_scale(ep, row - lane, m_end, K);  // summed while the tile's MMAs run
             RopeRow rr;                                          // likewise: page lookup + cos/sin rows pulled into L1
             if (ep.kind == P3_EPI_ROPE_KV && row_ok) rr = epi_rope_row(ep, (int)orow);
+            uint4 r[4];
+            if (!GLU) epi_resid(ep, row - lane, m_end, n_idx + c_lo, N, 0, r);
             mbar_wait(tfull_bar(acc), acc_phase);
             tc_fence_after();
-            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
-            if (ep.kind == P3_EPI_SWIGLU) {
-                for (int c0 = half * (BN / 4); c0 < (half + 1) * (BN / 4); c0 += 32) {
+            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * C::BN_MAX);
+            if constexpr (GLU) {
+                for (int c0 = 64 * half; c0 < 64 * half + 64; c0 += 32) {
                     uint32_t g[32], u[32];
                     tc_ld32(taddr + c0, g);
-                    tc_ld32(taddr + BN / 2 + c0, u);
+                    tc_ld32(taddr + 128 + c0, u);
+                    if (n_idx + c0 < ep.glu_f) epi_glu32(ep, sb, row - lane, m_end, n_idx + c0, g, u);
+                }
+            } else if (ep.kind == P3_EPI_SWIGLU) {
+                for (int c0 = 64 * half; c0 < 64 * half + 64; c0 += 32) {    // BN = 256
+                    uint32_t g[32], u[32];
+                    tc_ld32(taddr + c0, g);
+                    tc_ld32(taddr + 128 + c0, u);
                     const int on0 = n_idx / 2 + c0;
-                    if (row_ok && on0 < N / 2) {
+                    if (on0 < N / 2) {
                         uint4 ov[4];
                         uint32_t* ou = reinterpret_cast<uint32_t*>(ov);
 #pragma unroll
@@ -699,27 +852,25 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                             float a0 = bf16_round(g0 / (1.f + __expf(-g0))), a1 = bf16_round(g1 / (1.f + __expf(-g1)));
                             ou[i] = pack_bf16(a0 * u0, a1 * u1);
                         }
-                        bf16* o = reinterpret_cast<bf16*>(ep.out) + orow * ep.ldo + on0;
-                        if (on0 + 32 <= N / 2 && (ep.ldo & 7) == 0) {
-#pragma unroll
-                            for (int i = 0; i < 4; i++) st_out16(o + 8 * i, ov[i], ep.stream_out);
-                        } else {
+                        if (on0 + 32 <= N / 2 && (ep.ldo & 7) == 0) epi_put_bf16(ep, sb, row - lane, m_end, on0, ov);
+                        else if (row_ok) {
+                            bf16* o = reinterpret_cast<bf16*>(ep.out) + orow * ep.ldo + on0;
                             const bf16* ob = reinterpret_cast<const bf16*>(ov);
                             for (int i = 0; i < 32; i++) if (on0 + i < N / 2) o[i] = ob[i];
                         }
                     }
                 }
             } else if (ep.kind == P3_EPI_ROPE_KV) {
-                for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
+                for (int c0 = c_lo; c0 < c_hi; c0 += 32) {
                     uint32_t v[32];
                     tc_ld32(taddr + c0, v);
                     if (row_ok && n_idx + c0 < N) epi_rope32(ep, rr, n_idx + c0, rs, v);
                 }
             } else {
-                for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
+                for (int c0 = c_lo; c0 < c_hi; c0 += 32) {
                     uint32_t v[32];
                     tc_ld32(taddr + c0, v);
-                    if (row_ok && n_idx + c0 < N) epi_store32(ep, orow, n_idx + c0, N, v, rs);
+                    if (n_idx + c0 < N) epi_rows32(ep, sb, row - lane, m_end, n_idx + c0, c0 + 32 < c_hi ? n_idx + c0 + 32 : N, N, v, rs, r);
                 }
             }
             tc_fence_before();
@@ -894,28 +1045,43 @@ static int gemm_2cta_mode() {                  // P3_GEMM_2CTA=0 forces the sing
     return v;
 }
 
+// Columns of a pair's tile: the width whose waves over the CTA pairs cost least. A wave takes time in proportion to its columns (781 x 3072 x
+// 8192, one wave each: 256 53.2 us, 224 46.9, 192 41.3) plus its start and end, but narrow tiles re-read more of X per product: at equal
+// columns 224 and 192 measured 3 - 6 % behind 256 (5418 x 16384 x 2048, 19 waves of 256 and 22 of 224: 244 and 258 us), 160 15 % behind
+// (5418 x 2048 x 8192, 3 waves of 256 and 4 of 160: 136 and 143 us), and 128 takes as long as 160.
+static int tile_width(int64_t M, int N) {
+    const int64_t m = (M + 255) / 256, pairs = num_sms() / 2;
+    const int cost[4][2] = {{256, 100}, {224, 105}, {192, 105}, {160, 115}};
+    int best = 256; int64_t least = 0;
+    for (auto& c : cost) {
+        const int64_t waves = (m * ((N + c[0] - 1) / c[0]) + pairs - 1) / pairs, t = waves * (c[0] + 16) * c[1];
+        if (!least || t < least) { least = t; best = c[0]; }
+    }
+    return best;
+}
 static int launch_tc2(const void* X, int64_t ldx, const void* W, int64_t ldw, const GemmEpi& ep, int64_t M, int N, int K,
                       cudaStream_t st, const GemmWPlan* wp = nullptr) {
     using C = Tc2Cfg;
     CUtensorMap ta, tb;
     if (make_tmap(&ta, X, M, K, ldx, C::BM)) return -1;
-    if (wp) memcpy(&tb, &wp->t128, sizeof(tb));               // half of a 256-wide W tile per CTA
-    else if (make_tmap(&tb, W, N, K, ldw, C::BN / 2)) return -1;
+    const int bn = ep.kind == P3_EPI_SWIGLU ? 256 : tile_width(M, N);
+    if (wp && bn == 256) memcpy(&tb, &wp->t128, sizeof(tb));  // half of a 256-wide W tile per CTA
+    else if (make_tmap(&tb, W, N, K, ldw, bn / 2)) return -1;
     static bool attr_set[64] = {};
     if (!attr_set[cur_dev()]) {
         cudaError_t e = cudaFuncSetAttribute(gemm_tc2_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
         P3_CHECK_ARG(e == cudaSuccess, "gemm: cannot set %d B dynamic smem: %s", C::SMEM, cudaGetErrorString(e));
         attr_set[cur_dev()] = true;
     }
-    int64_t tiles = ((M + 2 * C::BM - 1) / (2 * C::BM)) * ((N + C::BN - 1) / C::BN);
+    int64_t tiles = ((M + 2 * C::BM - 1) / (2 * C::BM)) * ((N + bn - 1) / bn);
     int64_t clusters = tiles < num_sms() / 2 ? tiles : num_sms() / 2;
-    p3_launch_pdl(gemm_tc2_kernel<false>, dim3((unsigned)(2 * clusters)), dim3(384), (size_t)C::SMEM, st, ta, tb, ep, (int)M, N, K);
+    p3_launch_pdl(gemm_tc2_kernel<false>, dim3((unsigned)(2 * clusters)), dim3(384), (size_t)C::SMEM, st, ta, tb, ep, (int)M, N, K, bn);
     P3_CHECK_LAUNCH("gemm_tc2");
     return 0;
 }
 
 // the shared memory of a grouped launch holds the group table beside the ring
-static bool grouped_attr(const void* kernel, int bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess; }
+static bool smem_attr(const void* kernel, int bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess; }
 
 // out[M, N] (fp32, or bf16) = grouped product over rows already in group order; W [n_groups][w_rows][K] with row pitch ldw
 bool gemm_grouped_ok(const p3_gemm_any_args* a) {
@@ -930,17 +1096,18 @@ int launch_gemm_grouped(const p3_gemm_any_args* a, cudaStream_t st) {
     const int64_t w_all = (int64_t)ep.w_rows * (a->n_groups - 1) + a->N, mean = a->M / a->n_groups;
     static bool attr_set[64] = {};
     if (!attr_set[cur_dev()]) {
-        P3_CHECK_ARG(grouped_attr((const void*)gemm_tc_kernel<128, true>, TcCfg<128>::SMEM) && grouped_attr((const void*)gemm_tc2_kernel<true>, Tc2Cfg::SMEM),
+        P3_CHECK_ARG(smem_attr((const void*)gemm_tc_kernel<128, true>, TcCfg<128>::SMEM) && smem_attr((const void*)gemm_tc2_kernel<true>, Tc2Cfg::SMEM),
                      "gemm_any: cannot set the shared memory of the grouped product");
         attr_set[cur_dev()] = true;
     }
     CUtensorMap ta, ta32, tb;
     if (make_tmap(&ta, a->X, a->M, a->K, a->ldx, 128) || make_tmap(&tb, a->W, w_all, a->K, a->ldw, 128)) return -1;
     if (mean >= 160) {
-        // CTA pairs on 256 x 256 tiles; more pairs than tiles only costs their launch
+        // CTA pairs on 256 x 256 tiles from a mean of 160 rows a group on: below it most of a pair's 256 rows would be padding, above it the pair
+        // reads W half as often as 128 x 128 tiles do. More pairs than tiles only costs their launch.
         const int64_t most = (a->M / 256 + a->n_groups) * ((a->N + 255) / 256);
         const int64_t clusters = most < num_sms() / 2 ? most : num_sms() / 2;
-        p3_launch_pdl(gemm_tc2_kernel<true>, dim3((unsigned)(2 * clusters)), dim3(384), (size_t)Tc2Cfg::SMEM, st, ta, tb, ep, (int)a->M, a->N, a->K);
+        p3_launch_pdl(gemm_tc2_kernel<true>, dim3((unsigned)(2 * clusters)), dim3(384), (size_t)Tc2Cfg::SMEM, st, ta, tb, ep, (int)a->M, a->N, a->K, 256);
     } else {
         if (make_tmap(&ta32, a->X, a->M, a->K, a->ldx, 32)) return -1;
         const int64_t most = (a->M / 128 + (a->M < a->n_groups ? a->M : a->n_groups)) * ((a->N + 127) / 128);
@@ -999,6 +1166,31 @@ extern "C" int p3_gemm(const void* X, int64_t ldx, const void* W, int64_t ldw, c
     GemmEpi ep{};
     ep.bias = (const bf16*)bias; ep.out = out; ep.ldo = ldo; ep.resid = resid; ep.row_map = row_map; ep.kind = epi;
     return gemm_dispatch(X, ldx, W, ldw, ep, M, N, K, impl, st, nullptr);
+}
+
+extern "C" int p3_gemm_glu(const void* X, int64_t ldx, const void* W, int64_t ldw, const void* bias, void* out, int64_t ldo, int64_t M, int F, int K,
+                           int act, float limit, float alpha, cudaStream_t st) {
+    P3_CHECK_ARG(X && W && out && act >= 0 && act <= P3_GLU_CLAMPED, "gemm_glu: bad arguments");
+    P3_CHECK_ARG(ldx % 8 == 0 && ldw % 8 == 0 && ldo % 8 == 0, "gemm_glu: row pitches must be multiples of 8 elements (16 B)");
+    P3_CHECK_ARG((((uintptr_t)X | (uintptr_t)W | (uintptr_t)out | (uintptr_t)bias) & 15) == 0, "gemm_glu: operands must be 16-byte aligned");
+    P3_CHECK_ARG(M >= 0 && M < (1ll << 31) && F >= 32 && F % 32 == 0 && F < (1 << 30) && K >= 1, "gemm_glu: bad sizes");
+    if (M == 0) return 0;
+    using C = Tc2Cfg;
+    GemmEpi ep{};
+    ep.bias = (const bf16*)bias; ep.out = out; ep.ldo = ldo; ep.kind = P3_EPI_NONE; ep.ksplit = 1;
+    ep.glu_f = F; ep.glu_act = act; ep.glu_limit = limit; ep.glu_alpha = alpha;
+    ep.stream_out = M * (int64_t)F * 2 >= (64ll << 20);
+    CUtensorMap ta, tb;
+    if (make_tmap(&ta, X, M, K, ldx, C::BM) || make_tmap(&tb, W, 2 * (int64_t)F, K, ldw, C::BM)) return -1;
+    static bool attr_set[64] = {};
+    if (!attr_set[cur_dev()]) {
+        P3_CHECK_ARG(smem_attr((const void*)gemm_tc2_kernel<false, true>, C::SMEM), "gemm_glu: cannot set %d B dynamic smem", C::SMEM);
+        attr_set[cur_dev()] = true;
+    }
+    const int64_t tiles = ((M + 255) / 256) * ((F + 127) / 128), clusters = tiles < num_sms() / 2 ? tiles : num_sms() / 2;
+    p3_launch_pdl(gemm_tc2_kernel<false, true>, dim3((unsigned)(2 * clusters)), dim3(384), (size_t)C::SMEM, st, ta, tb, ep, (int)M, 2 * F, K, 256);
+    P3_CHECK_LAUNCH("gemm_glu");
+    return 0;
 }
 
 extern "C" int p3_gemm_plan_weights(const void* W, int64_t ldw, int N, int K, void* plan) {

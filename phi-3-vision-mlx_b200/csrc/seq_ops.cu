@@ -206,9 +206,8 @@ __global__ void glu_clamped_kernel(const float* __restrict__ gu, int64_t ld, AT*
     const int64_t n = R * F;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = i / F; const int c = (int)(i % F);
-        const float g = fminf(gu[(size_t)r * ld + c] + (bias ? bias[c] : 0.f), limit);
-        const float u = fminf(fmaxf(gu[(size_t)r * ld + F + c] + (bias ? bias[F + c] : 0.f), -limit), limit);
-        stv(out + (size_t)r * ldo + c, g * (1.0f / (1.0f + expf(-alpha * g))) * (u + 1.0f));
+        const float g = gu[(size_t)r * ld + c] + (bias ? bias[c] : 0.f), u = gu[(size_t)r * ld + F + c] + (bias ? bias[F + c] : 0.f);
+        stv(out + (size_t)r * ldo + c, glu_clamped(g, u, limit, alpha));
     }
 }
 
@@ -231,10 +230,7 @@ __global__ void glu_clamped_vec4_kernel(const float* __restrict__ gu, int64_t ld
         float y[4];
         const float gg[4] = {g.x, g.y, g.z, g.w}, uu[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const float a = fminf(gg[k], limit), b = fminf(fmaxf(uu[k], -limit), limit);
-            y[k] = a * (1.0f / (1.0f + expf(-alpha * a))) * (b + 1.0f);
-        }
+        for (int k = 0; k < 4; k++) y[k] = glu_clamped(gg[k], uu[k], limit, alpha);
         AT* o = out + (size_t)r * ldo + c;
         if constexpr (sizeof(AT) == 4) *reinterpret_cast<float4*>(o) = make_float4(y[0], y[1], y[2], y[3]);
         else *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]));
@@ -531,11 +527,7 @@ __global__ void latent_post_kernel(p3_latent_post_args a) {
 }
 
 // ---------------------------------------------------------------- y = act(g) * u, act = silu, relu or the tanh form of gelu
-__device__ __forceinline__ float gelu_tanh(float z) { return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z))); }
 __device__ __forceinline__ float gelu_erf(float z) { return 0.5f * z * (1.0f + erff(z * 0.7071067811865476f)); }
-template <int ACT> __device__ __forceinline__ float glu_act(float g) {
-    return ACT == 0 ? g / (1.0f + expf(-g)) : ACT == 1 ? fmaxf(g, 0.f) : gelu_tanh(g);
-}
 template <int ACT> __device__ __forceinline__ float unit_act(float z) { return ACT == 0 ? gelu_erf(z) : gelu_tanh(z); }
 
 template <typename AT, int ACT>

@@ -106,3 +106,38 @@ def test_expert_order_is_stable(dev, n, E):
     ref = torch.sort(ids.long(), stable=True).indices
     assert torch.equal(order.long(), ref) and torch.equal(where[order.long()].long(), torch.arange(n, device=dev))
     assert seg.tolist() == [int((ids < e).sum()) for e in range(E + 1)]
+
+
+@pytest.mark.parametrize('M,N,K', [(781, 3072, 200), (1030, 2056, 136), (2885, 1000, 72), (2560, 1984, 64), (5418, 3088, 128), (257, 9216, 64), (300, 19000, 72)])
+def test_products_of_cta_pairs_at_every_tile_width(dev, M, N, K):
+    """rows and columns that end inside a tile of each width; every output is the sum of the single-CTA kernel's k order, in fp32: 2^-20 of the
+    sum of magnitudes, and 2^-8 for the bf16 result"""
+    from phi3_b200 import _lib
+    g = torch.Generator(device=dev).manual_seed(N)
+    x, w, b = (torch.randn(*s, generator=g, device=dev).to(B16) for s in ((M, K), (N, K), (N,)))
+    y, bound = x.double() @ w.double().T + b.double(), 2.0 ** -20 * (x.double().abs() @ w.double().abs().T + b.double().abs())
+    for epi, dt in ((_lib.EPI_F32, F32), (_lib.EPI_NONE, B16)):
+        out = torch.full((M + 1, N + 24), float('nan'), dtype=dt, device=dev)
+        _lib.call('p3_gemm', x.data_ptr(), K, w.data_ptr(), K, b.data_ptr(), out.data_ptr(), N + 24, None, None, M, N, K, epi, 0, _stream())
+        assert ((out[:M, :N].double() - y).abs() <= bound + (2.0 ** -8 * y.abs() if dt == B16 else 0)).all()
+        assert bool(torch.isnan(out[M]).all()) and bool(torch.isnan(out[:M, N:]).all())
+
+
+@pytest.mark.parametrize('M,F,K', [(1, 32, 8), (129, 96, 72), (300, 1000 // 32 * 32, 136), (781, 2080, 64), (1030, 128, 200)])
+@pytest.mark.parametrize('act', [0, 1, 2, 3])
+@pytest.mark.parametrize('bias', [False, True])
+def test_gated_products_have_the_bits_of_product_and_activation(dev, M, F, K, act, bias):
+    """the fp32 product of the same rows through the pair kernel's plain epilogue or the single-CTA one (one k order), then the activation
+    kernel; columns end inside a tile of 128"""
+    from phi3_b200 import _lib
+    g = torch.Generator(device=dev).manual_seed(F + act)
+    x, w, b = (torch.randn(*s, generator=g, device=dev).to(B16) for s in ((M, K), (2 * F, K), (2 * F,)))
+    gu, bp = torch.empty(M, 2 * F, device=dev), b.data_ptr() if bias else None
+    want, got = torch.empty(M, F, dtype=B16, device=dev), torch.full((M + 1, F + 8), float('nan'), dtype=B16, device=dev)
+    _lib.call('p3_gemm', x.data_ptr(), K, w.data_ptr(), K, bp, gu.data_ptr(), 2 * F, None, None, M, 2 * F, K, _lib.EPI_F32, 0, _stream())
+    if act == _lib.GLU_CLAMPED:
+        _lib.call('p3_glu_clamped', gu.data_ptr(), 2 * F, want.data_ptr(), F, 0, M, F, 7.0, 1.702, None, _stream())
+    else:
+        _lib.call('p3_glu_act', gu.data_ptr(), gu[:, F:].data_ptr(), 2 * F, want.data_ptr(), F, 0, M, F, act, _stream())
+    _lib.call('p3_gemm_glu', x.data_ptr(), K, w.data_ptr(), K, bp, got.data_ptr(), F + 8, M, F, K, act, 7.0, 1.702, _stream())
+    assert torch.equal(got[:M, :F], want) and bool(torch.isnan(got[M]).all()) and bool(torch.isnan(got[:M, F:]).all())
