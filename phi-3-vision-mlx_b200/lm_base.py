@@ -106,6 +106,27 @@ class PagedLM:
         self.gemm_any(x, w, out, bias32)
         return None
 
+    def gated(self, x, w, act, hid, bias32=None, bias16=None, limit=0.0, alpha=0.0, nxt=None):
+        """hid[M,F] = act(g) * u, [g | u] = x w^T (+ bias): one launch where p3_gemm would take CTA pairs for this product (from a
+        quarter of the SMs' worth of 256 x 256 tiles on), else the product into fp32 rows and the activation kernel."""
+        (M, K), F = x.shape, w.shape[0] // 2
+        if (self.use_tc and not self.f32 and M > 128 and -(-M // 256) * -(-F // 128) >= 37 and F % 32 == 0 and w.shape[0] == 2 * F
+                and (bias32 is None or bias16 is not None) and not any(t.stride(0) % 8 or t.data_ptr() % 16 for t in (x, w, hid))
+                and (bias16 is None or bias16.data_ptr() % 16 == 0)):
+            ev = self._ev()
+            call('p3_gemm_glu', ptr(x), x.stride(0), ptr(w), w.stride(0), ptr(bias16), ptr(hid), hid.stride(0), M, F, K, act, limit, alpha, _stream())
+            self._ev(ev, 'gemm', 4 * M * F * K, w.numel() * 2 + x.numel() * 2 + hid.numel() * 2)
+            return
+        gu = torch.empty((M, w.shape[0]), dtype=torch.float32, device=self.dev)
+        left = self.linear(x, w, gu, bias32, bias16, nxt=nxt)
+        nbytes = M * F * (8 + (4 if self.f32 else 2))
+        if act == _lib.GLU_CLAMPED:
+            self.rows('activation', nbytes, 'p3_glu_clamped', ptr(gu), gu.stride(0), ptr(hid), hid.stride(0), self.f32, M, F, limit, alpha,
+                      ptr(left), _stream())
+        else:
+            self.rows('activation', nbytes, 'p3_glu_act', ptr(gu), ptr(gu[:, F:]), gu.stride(0), ptr(hid), hid.stride(0), self.f32, M, F, act,
+                      _stream())
+
     def gemm_any(self, x, w, out, bias=None, rows=None, row_div=1, seg=None, n_groups=0, M=None, N=None, K=None, ldw=None,
                  batch=None, gate=None):
         """out = x w^T on p3_gemm_any. rows / row_div: gathered activation rows; seg / n_groups: row segments that each take their

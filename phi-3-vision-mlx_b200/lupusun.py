@@ -232,11 +232,8 @@ class LupusunB200(PagedLM):
 
     def _feed_forward(self, L, h, T):
         ff = L['cfg'].ff.ff
-        gu = torch.empty((T, 2 * ff), dtype=torch.float32, device=self.dev)
         hid = torch.empty((T, ff), dtype=self.dtype, device=self.dev)
         y = torch.empty((T, self.W), dtype=torch.float32, device=self.dev)
-        self.linear(h, L['gu'], gu, nxt=L['down'])
-        self.rows('activation', T * ff * (8 + (4 if self.f32 else 2)), 'p3_glu_act', ptr(gu), ptr(gu[:, ff:]), gu.stride(0), ptr(hid),
-                  hid.stride(0), self.f32, T, ff, _lib.GLU_RELU, _stream())
+        self.gated(h, L['gu'], _lib.GLU_RELU, hid, nxt=L['down'])
         self.linear(hid, L['down'], y)
         return y

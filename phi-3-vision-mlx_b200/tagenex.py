@@ -168,10 +168,8 @@ class TagenexB200(PagedLM):
             f = L['cfg'].ff
             if f is not None:
                 if f.kind == 'dense':
-                    gu, hid = e(T, 2 * f.ff), e(T, f.ff, dt=act)
-                    left = self.linear(xa, L['gu'], gu, L['gu_b32'], L['gu_b16'], nxt=L['down'])
-                    self.rows('activation', T * f.ff * (8 + (4 if self.f32 else 2)), 'p3_glu_clamped', ptr(gu), gu.stride(0), ptr(hid),
-                              hid.stride(0), self.f32, T, f.ff, f.limit, TagenexConfig.GLU_ALPHA, ptr(left), st)
+                    hid = e(T, f.ff, dt=act)
+                    self.gated(xa, L['gu'], _lib.GLU_CLAMPED, hid, L['gu_b32'], L['gu_b16'], f.limit, TagenexConfig.GLU_ALPHA, nxt=L['down'])
                     left = self.linear(hid, L['down'], y, L['down_b32'], L['down_b16'], nxt=after)
                 else:
                     self._moe(L, f, xa, y, T)
