@@ -108,7 +108,8 @@ class PagedLM:
 
     def gated(self, x, w, act, hid, bias32=None, bias16=None, limit=0.0, alpha=0.0, nxt=None):
         """hid[M,F] = act(g) * u, [g | u] = x w^T (+ bias): one launch where p3_gemm would take CTA pairs for this product (from a
-        quarter of the SMs' worth of 256 x 256 tiles on), else the product into fp32 rows and the activation kernel."""
+        quarter of the SMs' worth of 256 x 256 tiles on: 5418 rows, 2048 -> 8192: 233 us, as two launches 401), else the product into fp32
+        rows and the activation kernel: fewer rows leave a stream of w, which the kernels of smaller tiles spread over more CTAs."""
         (M, K), F = x.shape, w.shape[0] // 2
         if (self.use_tc and not self.f32 and M > 128 and -(-M // 256) * -(-F // 128) >= 37 and F % 32 == 0 and w.shape[0] == 2 * F
                 and (bias32 is None or bias16 is not None) and not any(t.stride(0) % 8 or t.data_ptr() % 16 for t in (x, w, hid))
