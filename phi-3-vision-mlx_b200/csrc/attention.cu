@@ -288,8 +288,8 @@ __global__ void __launch_bounds__(PF_THREADS, 2) attn_prefill_kernel(AttnParams 
 // tile t is consumed, masking runs only on boundary tiles and exp2 is a single MUFU.
 // ------------------------------------------------------------------------------------------
 #define DEC_STAGES 4
-// timeline stamps (tools/chain_trace.py): compiled in only with -DP3_TRACE_ATTN — any extra uniform-register use in this kernel
-// makes ptxas 12.9 pick the [R + UR + imm] LDGSTS form with an odd policy descriptor register (see cp_async16_stream)
+// timeline stamps (tools/chain_trace.py): compiled in only with -DP3_TRACE_ATTN, because further values that are the same for the
+// whole warp bring back the illegal-instruction error of the hinted copies (see cp_async16_stream)
 #ifdef P3_TRACE_ATTN
 #define ATTN_TRACE_STAMP(tr, cta, i) trace_stamp(tr, cta, i)
 #define ATTN_TRACE_META(tr, cta, k) trace_meta(tr, cta, k)
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(128, 2) attn_decode_kernel(AttnParams p) {
             if (D == 96) {          // KV pages are read once per step: L2 evict-first
                 cp_async16_stream(sk + soff[i], kp + i * 1024, pol);
                 cp_async16_stream(sk + TILE + soff[i], kp + v_delta + i * 1024, pol);
-            } else {                // (ptxas 12.9 emits an unencodable LDGSTS descriptor pair for the D=64 instance)
+            } else {                // (the hinted copies of the D=64 instance ended with the error that cp_async16_stream tells of)
                 cp_async16(sk + soff[i], kp + i * 1024);
                 cp_async16(sk + TILE + soff[i], kp + v_delta + i * 1024);
             }

@@ -37,8 +37,7 @@
 #define QA_STAGE 8192
 #define QB_STAGES 2          // phase B: bf16 pages + the new tokens, 24 KB stages (same shared memory)
 
-// two code nibbles (bits 0-3 and 16-19) -> bf16x2 (128+n_lo, 128+n_hi), exact; ONE LOP3: the mask must live in a register
-// (two immediates do not fit one instruction; ptxas would emit AND + OR)
+// two code nibbles (bits 0-3 and 16-19) -> bf16x2 (128+n_lo, 128+n_hi), exact, as one three-input logic operation
 __device__ __forceinline__ uint32_t nib2bf(uint32_t x, uint32_t mask) {
     uint32_t d;
     asm("lop3.b32 %0, %1, %2, 0x43004300, 0xEA;" : "=r"(d) : "r"(x), "r"(mask));
