@@ -119,35 +119,42 @@ struct TcCfg {
     static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 };
 
-// per-row RMSNorm scale from the producer's partial sums (fixed order: deterministic); 1 when the GEMM is not normed. Four lanes of the warp sum
-// a row and hand the result to the row's lane: reads of whole sectors, eight rows at a time (a lane for each row: 781 x 16384 x 3072 with 96
-// partial sums a row took 95 us, 81 without; now 91).
-__device__ __forceinline__ float epi_row_scale(const GemmEpi& ep, int row0, int m_end, int K) {
+// per-row RMSNorm scale from the producer's partial sums; 1 when the GEMM is not normed. A row's lane adds the sums of its quadruples in
+// ascending order, whatever the tile: one row has one scale. Four lanes bring 64 bytes of a row, eight
+// rows at a time, and hand the quadruples over through the warp's block of shared memory: reads of whole sectors (a lane reading its own row:
+// 781 x 16384 x 3072 with 96 partial sums a row took 95 us, 81 without).
+__device__ __forceinline__ float epi_row_scale(const GemmEpi& ep, uint8_t* sb, int row0, int m_end, int K) {
     if (!ep.ss_in) return 1.f;
     const int lane = threadIdx.x & 31, sub = lane >> 2, part = lane & 3, n = ep.n_ss_in;
-    float s[4] = {0.f, 0.f, 0.f, 0.f};
-    const float* p = ep.ss_in + (size_t)(row0 + sub) * n;
+    float s = 0.f;
     if ((n & 3) == 0) {
-#pragma unroll 2
-        for (int c = 4 * part; c < n; c += 16)
+        const float* p = ep.ss_in + (size_t)(row0 + sub) * n + 4 * part;
+        float* q = reinterpret_cast<float*>(sb);               // [block of 16 numbers][row][4]
+        for (int c0 = 0; c0 < n; c0 += 32) {
+            float4 f[2][4];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-                if (row0 + 8 * i + sub < m_end) { const float4 f = __ldcg(reinterpret_cast<const float4*>(p + (size_t)8 * i * n + c)); s[i] += (f.x + f.y) + (f.z + f.w); }
-    } else {
-        for (int c = part; c < n; c += 4)
+            for (int h = 0; h < 2; h++)
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-                if (row0 + 8 * i + sub < m_end) s[i] += __ldcg(p + (size_t)8 * i * n + c);
+                for (int i = 0; i < 4; i++)
+                    f[h][i] = c0 + 16 * h + 4 * part < n && row0 + 8 * i + sub < m_end
+                                  ? __ldcg(reinterpret_cast<const float4*>(p + (size_t)8 * i * n + c0 + 16 * h)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            __syncwarp();                                      // the block before is read
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) q[h * 128 + (8 * i + sub) * 4 + part] = (f[h][i].x + f[h][i].y) + (f[h][i].z + f[h][i].w);
+            __syncwarp();
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const float4 t = *reinterpret_cast<const float4*>(q + h * 128 + lane * 4);      // zeros behind the last
+                s += t.x; s += t.y; s += t.z; s += t.w;
+            }
+        }
+    } else if (row0 + lane < m_end) {
+        const float* p = ep.ss_in + (size_t)(row0 + lane) * n;
+        for (int c = 0; c < n; c++) s += __ldcg(p + c);
     }
-    float own = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        s[i] += __shfl_xor_sync(0xffffffffu, s[i], 1);
-        s[i] += __shfl_xor_sync(0xffffffffu, s[i], 2);
-        const float t = __shfl_sync(0xffffffffu, s[i], 4 * (lane & 7));          // row 8 i + (lane & 7)
-        if (lane >> 3 == i) own = t;
-    }
-    return rsqrtf(own / (float)K + ep.eps);
+    return rsqrtf(s / (float)K + ep.eps);
 }
 
 // P3_EPI_ROPE_KV, per output row (token): everything that does not depend on the column chunk — computed once per tile,
@@ -232,16 +239,16 @@ __device__ __forceinline__ void epi_rope32(const GemmEpi& ep, const RopeRow& rr,
 // that a store instruction writes 8 x 64 contiguous bytes. Straight from the accumulators' layout a lane writes 16 bytes of its own row and
 // every 32-byte sector takes two instructions (1024 x 9216 x 512, fp32 / bf16 results: 23.7 / 15.1 us, turned 16.2 / 13.3). 16-byte pieces are swizzled: no bank
 // conflicts either way.
+template <typename T> __device__ __forceinline__ T& rows_at(uint8_t* sb, int row, int piece) {
+    return *reinterpret_cast<T*>(sb + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4));
+}
 __device__ __forceinline__ void rows_put(uint8_t* sb, int lane, const uint4* v) {
     __syncwarp();                                          // the block before is read
 #pragma unroll
-    for (int j = 0; j < 4; j++) *reinterpret_cast<uint4*>(sb + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = v[j];
+    for (int j = 0; j < 4; j++) rows_at<uint4>(sb, lane, j) = v[j];
     __syncwarp();
 }
-__device__ __forceinline__ uint4 rows_get(const uint8_t* sb, int lane, int i) {          // of row 8 i + lane / 4
-    const int r = 8 * i + (lane >> 2);
-    return *reinterpret_cast<const uint4*>(sb + r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) << 4));
-}
+__device__ __forceinline__ uint4 rows_get(uint8_t* sb, int lane, int i) { return rows_at<uint4>(sb, 8 * i + (lane >> 2), lane & 3); }   // of row 8 i + lane / 4
 __device__ __forceinline__ int64_t epi_out_row(const GemmEpi& ep, int row) { return ep.row_map ? (int64_t)ep.row_map[row] : (int64_t)row; }
 // 32 bf16 columns of 32 rows (row0: the warp's first; rows from m_end on are not written)
 __device__ __forceinline__ void epi_put_bf16(const GemmEpi& ep, uint8_t* sb, int row0, int m_end, int n0, const uint4* v) {
@@ -375,7 +382,7 @@ __device__ __forceinline__ void epi_rows32(const GemmEpi& ep, uint8_t* sb, int r
         uint4 next[4];
         if (resid) epi_resid(ep, row0, m_end, n1, N, 0, next);
         rows_put(sb, lane, ov);
-        float sq[4];
+        float4 sq[4];                                          // per row and pair of columns: squares of the bf16 values just written
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int row = row0 + 8 * i + sub;
@@ -387,18 +394,20 @@ __device__ __forceinline__ void epi_rows32(const GemmEpi& ep, uint8_t* sb, int r
                 for (int e = 0; e < 4; e++) { const float2 f = unpack_bf16(ru[e]), x = unpack_bf16(w[e]); w[e] = pack_bf16(f.x + x.x, f.y + x.y); }
             }
             if (row < m_end) st_out16(out + epi_out_row(ep, row) * ep.ldo + n0 + 8 * part, make_uint4(w[0], w[1], w[2], w[3]), ep.stream_out);
-            sq[i] = 0.f;                                       // sum of squares of the bf16 values just written
+            float t[4];
 #pragma unroll
-            for (int e = 0; e < 4; e++) { const float2 f = unpack_bf16(w[e]); sq[i] += f.x * f.x + f.y * f.y; }
+            for (int e = 0; e < 4; e++) { const float2 f = unpack_bf16(w[e]); t[e] = f.x * f.x + f.y * f.y; }
+            sq[i] = make_float4(t[0], t[1], t[2], t[3]);
         }
-        if (ep.ss_out) {
+        if (ep.ss_out) {                                       // back to the row's lane, which adds its 16 pairs from left to right
+            __syncwarp();
 #pragma unroll
-            for (int i = 0; i < 4; i++) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], 1);
+            for (int i = 0; i < 4; i++) rows_at<float4>(sb, 8 * i + sub, part) = sq[i];
+            __syncwarp();
+            float s = 0.f;
 #pragma unroll
-            for (int i = 0; i < 4; i++) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], 2);
-            const int row = row0 + 8 * part + sub;
-            const float mine = part == 0 ? sq[0] : part == 1 ? sq[1] : part == 2 ? sq[2] : sq[3];
-            if (row < m_end) ep.ss_out[(size_t)epi_out_row(ep, row) * (N / 32) + n0 / 32] = mine;
+            for (int j = 0; j < 4; j++) { const float4 t = rows_at<float4>(sb, lane, j); s += t.x; s += t.y; s += t.z; s += t.w; }
+            if (own < m_end) ep.ss_out[(size_t)epi_out_row(ep, own) * (N / 32) + n0 / 32] = s;
         }
         if (resid) {
 #pragma unroll
@@ -544,7 +553,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const int row = m_idx + q * 32 + lane;
             const bool row_ok = row < m_end;
             const int64_t orow = row_ok ? (ep.row_map ? (int64_t)ep.row_map[row] : (int64_t)row) : 0;
-            const float rs = epi_row_scale(ep, row - lane, m_end, K);  // summed while the tile's MMAs run
+            const float rs = epi_row_scale(ep, sb, row - lane, m_end, K);  // summed while the tile's MMAs run
             RopeRow rr;                                          // likewise: page lookup + cos/sin rows pulled into L1
             if (ep.kind == P3_EPI_ROPE_KV && row_ok) rr = epi_rope_row(ep, (int)orow);
             uint4 r[4];
@@ -821,7 +830,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             const int row = m_idx + q * 32 + lane;
             const bool row_ok = row < m_end;
             const int64_t orow = row_ok ? (ep.row_map ? (int64_t)ep.row_map[row] : (int64_t)row) : 0;
-            const float rs = epi_row_scale(ep, row - lane, m_end, K);  // summed while the tile's MMAs run
+            const float rs = epi_row_scale(ep, sb, row - lane, m_end, K);  // summed while the tile's MMAs run
             RopeRow rr;                                          // likewise: page lookup + cos/sin rows pulled into L1
             if (ep.kind == P3_EPI_ROPE_KV && row_ok) rr = epi_rope_row(ep, (int)orow);
             uint4 r[4];

@@ -141,3 +141,40 @@ def test_gated_products_have_the_bits_of_product_and_activation(dev, M, F, K, ac
         _lib.call('p3_glu_act', gu.data_ptr(), gu[:, F:].data_ptr(), 2 * F, want.data_ptr(), F, 0, M, F, act, _stream())
     _lib.call('p3_gemm_glu', x.data_ptr(), K, w.data_ptr(), K, bp, got.data_ptr(), F + 8, M, F, K, act, 7.0, 1.702, _stream())
     assert torch.equal(got[:M, :F], want) and bool(torch.isnan(got[M]).all()) and bool(torch.isnan(got[:M, F:]).all())
+
+
+def _fused(x, w, out, epi, **kw):
+    from phi3_b200 import _lib
+    a = _lib.GemmArgs()
+    a.X, a.ldx, a.W, a.ldw, a.out, a.ldo = x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0)
+    a.M, a.N, a.K, a.epi, a.impl = x.shape[0], w.shape[0], x.shape[1], epi, 0
+    for k, v in kw.items():
+        setattr(a, k, v.data_ptr() if isinstance(v, torch.Tensor) else v)
+    _lib.call_struct('p3_gemm_fused', a, _stream())
+    return out
+
+
+@pytest.mark.parametrize('M,N', [(1, 64), (33, 96), (130, 352), (781, 3072), (1030, 3072)])
+@pytest.mark.parametrize('n_ss', [1, 6, 12, 44, 96])
+def test_row_scales_and_sums_of_squares_have_one_order_of_additions(dev, M, N, n_ss):
+    """a row's scale adds its partial sums in quadruples (one by one where their number is no multiple of four) in ascending order, and a
+    partial sum adds its 16 pairs from left to right, whatever kernel and tile a product runs on: bit for bit, from the same product without a
+    norm and the rows that were written. (Squares of bf16 numbers are exact in fp32, so a pair has one rounding.)"""
+    from phi3_b200 import _lib
+    g = torch.Generator(device=dev).manual_seed(M + n_ss)
+    rn = lambda *s: torch.randn(s, generator=g, device=dev)
+    K = 136
+    x, w, ss = rn(M, K).to(B16), rn(N, K).to(B16), rn(M, n_ss).square() + 0.1
+    plain, normed = (_fused(x, w, torch.empty(M, N, device=dev), _lib.EPI_F32, **kw) for kw in ({}, dict(ss_in=ss, n_ss_in=n_ss, eps=1e-5)))
+    q = ss if n_ss % 4 else (ss[:, 0::4] + ss[:, 1::4]) + (ss[:, 2::4] + ss[:, 3::4])
+    s = torch.zeros(M, device=dev)
+    for c in range(q.shape[1]):
+        s = s + q[:, c]
+    assert torch.equal(normed, plain * torch.rsqrt(s / torch.tensor(float(K), device=dev) + 1e-5)[:, None])
+    h, part = rn(M, N).to(B16), torch.full((M, N // 32), float('nan'), device=dev)
+    _fused(x, w, h, _lib.EPI_RESIDUAL, resid=h, ss_out=part)
+    f = h.float().reshape(M, N // 32, 16, 2).square()
+    pairs, t = f[..., 0] + f[..., 1], torch.zeros(M, N // 32, device=dev)
+    for i in range(16):
+        t = t + pairs[..., i]
+    assert torch.equal(part, t)
