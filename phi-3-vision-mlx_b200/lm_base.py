@@ -125,6 +125,8 @@ class PagedLM:
             self.rows('activation', nbytes, 'p3_glu_clamped', ptr(gu), gu.stride(0), ptr(hid), hid.stride(0), self.f32, M, F, limit, alpha,
                       ptr(left), _stream())
         else:
+            if left is not None:                                 # p3_glu_act takes no bias
+                gu += left
             self.rows('activation', nbytes, 'p3_glu_act', ptr(gu), ptr(gu[:, F:]), gu.stride(0), ptr(hid), hid.stride(0), self.f32, M, F, act,
                       _stream())
 

@@ -178,3 +178,34 @@ def test_row_scales_and_sums_of_squares_have_one_order_of_additions(dev, M, N, n
     for i in range(16):
         t = t + pairs[..., i]
     assert torch.equal(part, t)
+
+
+def _layer(width, dtype=B16):
+    from phi3_b200.lm_base import PagedLM
+    m = PagedLM()
+    m.dev, m.dtype, m.W, m.eps = torch.device('cuda'), dtype, width, 1e-5
+    m._init_products()
+    return m
+
+
+GLU = [lambda g, u: torch.nn.functional.silu(g) * u, lambda g, u: torch.relu(g) * u, lambda g, u: torch.nn.functional.gelu(g, approximate='tanh') * u,
+       lambda g, u: g.clamp(max=7.0) * torch.sigmoid(1.702 * g.clamp(max=7.0)) * (u.clamp(-7.0, 7.0) + 1)]
+
+
+@pytest.mark.parametrize('dtype', [F32, B16])
+@pytest.mark.parametrize('M', [1, 16, 17, 700])
+@pytest.mark.parametrize('act', [0, 1, 2, 3])
+@pytest.mark.parametrize('bias', [False, True])
+def test_gated_units_with_and_without_bias(dev, dtype, M, act, bias):
+    """every unit on every route of PagedLM.gated: the weight stream of few rows (which leaves the bias to its consumer), product and activation,
+    one launch. Products of N(0, 1) rows and weights of N(0, 1 / K) are off by 2^-20 of their size; units that clamp or multiply such numbers
+    stay within 1e-4, and a bf16 result within half a unit in the last place on top"""
+    g = torch.Generator(device=dev).manual_seed(M + act)
+    K, F = 128, 1600                                                     # 3 x 13 pair tiles at 700 rows
+    x, w = torch.randn(M, K, generator=g, device=dev).to(dtype), (torch.randn(2 * F, K, generator=g, device=dev) * K ** -0.5).to(dtype)
+    b16 = torch.randn(2 * F, generator=g, device=dev).to(B16) if bias else None
+    hid = torch.empty(M, F, dtype=dtype, device=dev)
+    _layer(K, dtype).gated(x, w, act, hid, None if b16 is None else b16.float(), b16, 7.0, 1.702)
+    p = x.double() @ w.double().T + (b16.double() if bias else 0.0)
+    ref = GLU[act](p[:, :F], p[:, F:])
+    assert ((hid.double() - ref).abs() <= 1e-4 + (2.0 ** -8 * ref.abs() if dtype == B16 else 0)).all()
