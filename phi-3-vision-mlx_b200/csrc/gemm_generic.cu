@@ -331,7 +331,8 @@ int dispatch_f32(const AnyP& p, cudaStream_t st) {
         if (p.M <= 8) return launch_f32_rows<OT, 8>(p, st);
         return launch_f32_rows<OT, 16>(p, st);
     }
-    auto cost = [&](int r, int64_t alone, int64_t shared) {
+    auto cost = [&](int r, int64_t alone, int64_t shared) -> int64_t {
+        if (((int64_t)p.N + r - 1) / r > 65535) return INT64_MAX;        // more column tiles than the grid's second dimension holds
         const int64_t tiles = ((p.M + r - 1) / r + (p.seg ? p.n_groups / 2 : 0)) * ((p.N + r - 1) / r) * p.nb, per_sm = (tiles + 147) / 148;
         return alone > per_sm * shared ? alone : per_sm * shared;
     };

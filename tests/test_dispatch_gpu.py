@@ -209,3 +209,13 @@ def test_gated_units_with_and_without_bias(dev, dtype, M, act, bias):
     p = x.double() @ w.double().T + (b16.double() if bias else 0.0)
     ref = GLU[act](p[:, :F], p[:, F:])
     assert ((hid.double() - ref).abs() <= 1e-4 + (2.0 ** -8 * ref.abs() if dtype == B16 else 0)).all()
+
+
+def test_fp32_products_with_more_columns_than_small_tiles_can_number(dev):
+    """65536 tiles of 32 columns are one more than a grid holds: the next wider tile takes the product"""
+    g = torch.Generator(device=dev).manual_seed(3)
+    x, w = torch.randn(17, 4, generator=g, device=dev), torch.randn(32 * 65535 + 1, 4, generator=g, device=dev)
+    got = _gemm_any(x, w)
+    for a in range(0, w.shape[0], 1 << 19):
+        b = min(w.shape[0], a + (1 << 19))
+        assert torch.equal(got[:, a:b], _gemm_any(_odd_pitch(x), _odd_pitch(w[a:b])))
