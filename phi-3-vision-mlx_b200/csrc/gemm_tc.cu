@@ -1092,10 +1092,11 @@ static int launch_tc2(const void* X, int64_t ldx, const void* W, int64_t ldw, co
 // the shared memory of a grouped launch holds the group table beside the ring
 static bool smem_attr(const void* kernel, int bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess; }
 
-// out[M, N] (fp32, or bf16) = grouped product over rows already in group order; W [n_groups][w_rows][K] with row pitch ldw
+// out[M, N] (fp32, or bf16) = grouped product over rows already in group order; W [n_groups][w_rows][K] with row pitch ldw. Rows that overlap
+// (one row for all, say) stay with the kernel that reads them by address: a tensor map wants rows that follow one another
 bool gemm_grouped_ok(const p3_gemm_any_args* a) {
     return a->seg_offsets && !a->x_rows && !a->bias && !a->gate && a->n_batch <= 1 && !a->force_fma && !a->x_f32 && a->n_groups <= GROUPS_MAX && a->K % 8 == 0 &&
-           a->ldx % 8 == 0 && a->ldw % 8 == 0 && a->ldw > 0 && a->w_group_stride % a->ldw == 0 && a->w_group_stride / a->ldw >= a->N &&
+           a->ldx % 8 == 0 && a->ldw % 8 == 0 && a->ldx >= a->K && a->ldw >= a->K && a->w_group_stride % a->ldw == 0 && a->w_group_stride / a->ldw >= a->N &&
            a->w_group_stride / a->ldw * a->n_groups < (1ll << 31) && (((uintptr_t)a->X | (uintptr_t)a->W | (uintptr_t)a->out) & 15) == 0;
 }
 int launch_gemm_grouped(const p3_gemm_any_args* a, cudaStream_t st) {

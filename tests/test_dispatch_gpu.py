@@ -219,3 +219,17 @@ def test_fp32_products_with_more_columns_than_small_tiles_can_number(dev):
     for a in range(0, w.shape[0], 1 << 19):
         b = min(w.shape[0], a + (1 << 19))
         assert torch.equal(got[:, a:b], _gemm_any(_odd_pitch(x), _odd_pitch(w[a:b])))
+
+
+def test_grouped_products_of_overlapping_rows(dev):
+    """a pitch below the row length is no tensor map: one row of X for all rows of the groups, and rows of W that overlap"""
+    g = torch.Generator(device=dev).manual_seed(8)
+    seg, N, K = torch.tensor([0, 3, 3, 40], dtype=torch.int32, device=dev), 72, 64
+    x, w = torch.randn(1, K, generator=g, device=dev).to(B16).expand(40, K), torch.randn(3, 8 * N + K, generator=g, device=dev).to(B16)
+    windows = w.as_strided((3, N, K), (w.stride(0), 8, 1))
+    for xs, ws in ((x, windows.contiguous()), (x.contiguous(), windows), (x, windows)):
+        got = _gemm_any(xs, ws, seg=seg)
+        for e in range(3):
+            a, b = int(seg[e]), int(seg[e + 1])
+            y, mag = x[a:b].double() @ windows[e].double().T, x[a:b].double().abs() @ windows[e].double().abs().T
+            assert ((got[a:b].double() - y).abs() <= 2.0 ** -20 * mag).all()            # fp32 sums of 64 exact products
