@@ -90,11 +90,15 @@ template <int VEC> __device__ __forceinline__ void stvec(float* p, const float* 
     else *p = v[0];
 }
 
+constexpr size_t SCAN_APART = 116 * 1024;                     // more than half of an SM's shared memory
+// once per device and kernel (`set`): the most that the kernel is launched with, which is one number for each instantiation
 template <typename K>
-int set_smem_attr(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+int set_smem_attr(K kernel, size_t bytes, bool& set) {
+    if (!set) {
+        const int most = (int)(bytes > SCAN_APART ? bytes : SCAN_APART);
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         P3_CHECK_ARG(e == cudaSuccess, "matrix_memory_scan: shared memory attribute: %s", cudaGetErrorString(e));
+        set = true;
     }
     return 0;
 }
@@ -107,7 +111,7 @@ struct ScanShape { int tb; size_t bytes; };
 inline ScanShape scan_shape(int64_t ctas, size_t floats_per_token, int dim, int many) {
     const int tb = dim > 256 ? 16 : ctas <= 148 ? 32 : many;
     size_t bytes = sizeof(float) * 2 * tb * floats_per_token;                            // two staged rounds
-    if (ctas <= 148 && bytes < 116 * 1024) bytes = 116 * 1024;
+    if (ctas <= 148 && bytes < SCAN_APART) bytes = SCAN_APART;
     return {tb, bytes};
 }
 // a store that later shared-memory reads may be moved ahead of (the compiler cannot tell that `p` is not shared memory): with it four tokens of
@@ -894,7 +898,7 @@ extern "C" int p3_matrix_memory_scan(const p3_matrix_memory_args* a, cudaStream_
     const dim3 grid((unsigned)a->n_seqs, (unsigned)a->n_heads, (unsigned)((a->vdim + cols - 1) / cols));
     const ScanShape sh = scan_shape((int64_t)grid.x * grid.y * grid.z, 2 * (ds * rs + 4 * rs) + cols + 3, a->dim, 32);
 #define GOT(DS, RS, NC, TB)                                                                                          \
-    do { if (set_smem_attr(matrix_memory_scan_kernel<DS, RS, NC, TB>, sh.bytes)) return -1;                           \
+    do { static P3DevFlags set; if (set_smem_attr(matrix_memory_scan_kernel<DS, RS, NC, TB>, sh.bytes, set.cur())) return -1; \
          p3_launch_pdl(matrix_memory_scan_kernel<DS, RS, NC, TB>, grid, dim3(MM_WARPS * 32), sh.bytes, st, *a); } while (0)
 #define GO(DS, RS, NC)                                                                                              \
     GOT(DS, RS, NC, 32)
@@ -991,7 +995,7 @@ extern "C" int p3_gla_scan(const p3_gla_args* a, cudaStream_t st) {
     // heads: 572 us against 630)
     const ScanShape sh = scan_shape((int64_t)grid.x * grid.y * grid.z, 3 * (ds * rs + 4 * rs) + cols, a->dim, a->n_rows <= 4 * a->n_seqs ? 16 : 32);
 #define GOT(DS, RS, NC, TB)                                                                                          \
-    do { if (set_smem_attr(gla_scan_kernel<DS, RS, NC, TB>, sh.bytes)) return -1;                                     \
+    do { static P3DevFlags set; if (set_smem_attr(gla_scan_kernel<DS, RS, NC, TB>, sh.bytes, set.cur())) return -1;    \
          p3_launch_pdl(gla_scan_kernel<DS, RS, NC, TB>, grid, dim3(GLA_WARPS * 32), sh.bytes, st, *a); } while (0)
 #define GO(DS, RS, NC)                                                                                              \
     do { if (sh.tb == 32) GOT(DS, RS, NC, 32); else GOT(DS, RS, NC, 16); } while (0)
@@ -1060,7 +1064,7 @@ int launch_scan(const p3_delta_scan_args* a, cudaStream_t st, const char* who) {
     const dim3 grid((unsigned)a->n_seqs, (unsigned)a->n_heads, (unsigned)((a->vdim + cols - 1) / cols));
     const ScanShape sh = scan_shape((int64_t)grid.x * grid.y * grid.z, 2 * (ds * rs + 4 * rs) + cols + 2, a->dim, 16);   // 16: 6 x 1000 tokens 428 -> 326 us without the correction
 #define GOT(DS, RS, NC, TB)                                                                                          \
-    do { if (set_smem_attr(delta_scan_kernel<DS, RS, NC, TB, DELTA>, sh.bytes)) return -1;                            \
+    do { static P3DevFlags set; if (set_smem_attr(delta_scan_kernel<DS, RS, NC, TB, DELTA>, sh.bytes, set.cur())) return -1; \
          p3_launch_pdl(delta_scan_kernel<DS, RS, NC, TB, DELTA>, grid, dim3(GLA_WARPS * 32), sh.bytes, st, *a); } while (0)
 #define GO(DS, RS, NC) do { if (sh.tb == 32) GOT(DS, RS, NC, 32); else GOT(DS, RS, NC, 16); } while (0)
     if (a->dim > 256) GOT(128, 4, 1, 16);

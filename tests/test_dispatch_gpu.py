@@ -233,3 +233,49 @@ def test_grouped_products_of_overlapping_rows(dev):
             a, b = int(seg[e]), int(seg[e + 1])
             y, mag = x[a:b].double() @ windows[e].double().T, x[a:b].double().abs() @ windows[e].double().abs().T
             assert ((got[a:b].double() - y).abs() <= 2.0 ** -20 * mag).all()            # fp32 sums of 64 exact products
+
+
+@pytest.mark.parametrize('mixer', ['gla', 'delta', 'decay', 'memory'])
+@pytest.mark.parametrize('d,dv', [(24, 40), (64, 72), (128, 64), (200, 33)])
+@pytest.mark.parametrize('lens', [[1] * 40, [1, 15, 16, 17, 33, 2] * 7])
+def test_scans_of_many_ctas_have_the_bits_of_one_sequence_at_a_time(dev, mixer, d, dv, lens):
+    """more CTAs than SMs (rounds of 16 tokens: the delta and decay scans always, the linear attention at up to four rows per sequence) and at
+    most as many (rounds of 32 tokens): outputs and states of a sequence do not depend on what else the launch holds"""
+    from phi3_b200 import _lib
+    H, n = 4, len(lens)
+    g = torch.Generator(device=dev).manual_seed(d + n)
+    rn = lambda *s: torch.randn(s, generator=g, device=dev)
+    T, C = sum(lens), 2 * H * d + H * dv + 2 * H
+    proj, gates, zb, lr, a2 = rn(T, C), torch.rand(T, H, 2, generator=g, device=dev), rn(H * d), rn(T, 8), rn(H * d, 8)
+    proj[:, H * d:2 * H * d] *= d ** -0.5
+    width = d * dv + (d + -(-dv // 32) if mixer == 'memory' else 0)
+    state0 = 0.3 * rn(n, H, width)
+    if mixer == 'memory':
+        state0[..., d * dv + d:] = 0.5                               # one stabiliser per head, in a copy per 32 columns
+    first = [sum(lens[:i]) for i in range(n)]
+
+    def scan(which):
+        out, state, den, z = torch.full((T, H * dv), float('nan'), device=dev), state0.clone(), torch.zeros(T, H, device=dev), torch.empty(T, H * d, device=dev)
+        seqs = torch.tensor([(first[i], lens[i], i, 9) for i in which], dtype=torch.int32, device=dev).reshape(-1)
+        a = {'gla': _lib.GlaArgs, 'memory': _lib.MatrixMemoryArgs}.get(mixer, _lib.DeltaScanArgs)()
+        if mixer == 'gla':
+            a.proj, a.ld_proj, a.z, a.ld_z, a.z_bias, a.inv_tau, a.q_scale = proj.data_ptr(), C, z.data_ptr(), H * d, zb.data_ptr(), 0.1, 0.2
+            a.n_rows, a.lr, a.ld_lr, a.a2, a.rank = T, lr.data_ptr(), 8, a2.data_ptr(), 8
+        elif mixer == 'memory':
+            a.proj, a.ld_proj, a.i_off, a.f_off, a.i_bias, a.f_bias = proj.data_ptr(), C, C - 2 * H, C - H, zb.data_ptr(), zb.data_ptr()
+            a.q_scale, a.gate_cap, a.den = 0.2, 15.0, den.data_ptr()
+        else:
+            a.qkv, a.ld_qkv, a.n_kv, a.gates = proj.data_ptr(), C, H, gates.data_ptr()
+        a.q_off, a.k_off, a.v_off, a.n_heads, a.dim, a.vdim, a.state = 0, H * d, 2 * H * d, H, d, dv, state.data_ptr()
+        a.seqs, a.n_seqs, a.out, a.ld_out = seqs.data_ptr(), len(which), out.data_ptr(), H * dv
+        _lib.call_struct({'gla': 'p3_gla_scan', 'delta': 'p3_delta_scan', 'decay': 'p3_decay_scan', 'memory': 'p3_matrix_memory_scan'}[mixer], a, _stream())
+        torch.cuda.synchronize()
+        return out, state, den
+
+    assert n * H > 148
+    out, state, den = scan(range(n))
+    assert bool(torch.isfinite(out).all()) and bool(torch.isfinite(state).all())
+    for i in range(min(n, 12)):
+        o, s, e = scan([i])
+        rows = slice(first[i], first[i] + lens[i])
+        assert torch.equal(out[rows], o[rows]) and torch.equal(state[i], s[i]) and torch.equal(den[rows], e[rows])
