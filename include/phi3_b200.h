@@ -122,6 +122,10 @@ int p3_gemm_skinny_qkv_rope_w4(const void* X, int64_t ldx, const void* norm_w, f
 int p3_gemm(const void* X, int64_t ldx, const void* W, int64_t ldw, const void* bias, void* out, int64_t ldo,
             const void* resid, const int32_t* row_map, int64_t M, int N, int K, int epi, int impl, cudaStream_t st);
 
+/* columns of the tile when p3_gemm runs a product of M rows and N columns on CTA pairs (SwiGLU: always 256), 0 when it does not
+ * (P3_GEMM_2CTA=0: never) */
+int p3_gemm_pair_width(int64_t M, int64_t N);
+
 /* out (bf16) [M, F] = act(g) * u with [g | u] = X[M,K] . W[2F,K]^T (+ bias bf16 [2F]), gate rows of W first: the product and its gated
  * unit in one launch on CTA pairs, fp32 up to the result. act 0 silu, 1 relu, 2 gelu (tanh form): as p3_glu_act; 3: as p3_glu_clamped
  * with limit and alpha. F % 32 == 0, row pitches % 8 == 0, 16-byte operands. */
@@ -337,7 +341,7 @@ typedef struct {
     void* out; int64_t ldo; int32_t out_f32;
     int64_t M; int32_t N, K;
     const int32_t* seg_offsets; int32_t n_groups;
-    int32_t force_fma;           /* tests: bf16 operands on the FMA kernel */
+    int32_t force_fma;           /* 1: bf16 operands on the FMA kernel (tests); 2: not on tcgen05 (grouped products on mma.sync) */
     int32_t n_batch; int64_t x_batch_stride, w_batch_stride, out_batch_stride;
     const float* gate; int64_t ld_gate;
 } p3_gemm_any_args;

@@ -45,6 +45,7 @@ _SIGS = {
     'p3_gemm_skinny_w4': [_p, _l, _p, _f, _p, _p, _p, _l, _p, _i, _i, _i, _i, _p, _i, _p, _p, _l, _p],
     'p3_gemm_skinny_qkv_rope_w4': [_p, _l, _p, _f, _p, _p, _p, _p, _i, _p, _p, _l, _i, _i, _i, _i, _i, _i, _i, _p, _i, _p, _p, _i, _i, _p, _l, _p],
     'p3_gemm': [_p, _l, _p, _l, _p, _p, _l, _p, _p, _l, _i, _i, _i, _i, _p],
+    'p3_gemm_pair_width': [_l, _l],
     'p3_gemm_glu': [_p, _l, _p, _l, _p, _p, _l, _l, _i, _i, _i, _f, _f, _p],
     'p3_attention_prefill': [_p, _p, _p, _l, _l, _l, _p, _l, _i, _i, _i, _i, _i, _f, _i, _i, _p, _p, _p, _i, _i, _p],
     'p3_attention_decode': [_p, _p, _p, _l, _l, _l, _p, _l, _i, _i, _i, _i, _i, _f, _i, _p, _p, _p, _i, _i, _i, _p, _p, _p, _l, _p],
@@ -101,7 +102,8 @@ _SIGS = {
     'p3_unit_act': [_p, _l, _p, _l, _i, _l, _i, _i, _p],
 }
 UNIT_GELU, UNIT_GELU_TANH = 0, 1                                          # activations of p3_unit_act
-GLU_SILU, GLU_RELU, GLU_GELU_TANH, GLU_CLAMPED = 0, 1, 2, 3                                   # activations of p3_glu_act
+GLU_SILU, GLU_RELU, GLU_GELU_TANH = 0, 1, 2                               # activations of p3_glu_act and p3_gemm_glu
+GLU_CLAMPED = 3                                                           # of p3_gemm_glu: the unit of p3_glu_clamped
 ROUTER_SOFTMAX, ROUTER_GROUP_MAX, ROUTER_PLAIN_WEIGHTS = 1, 2, 4          # mode bits of p3_router_groups
 _STRUCT_ENTRIES = ['p3_gemm_any', 'p3_qkv_post', 'p3_attn_window_prefill', 'p3_attn_window_decode', 'p3_latent_post',
                    'p3_qkv_rope_post', 'p3_matrix_memory_scan', 'p3_gla_scan', 'p3_short_conv', 'p3_delta_scan', 'p3_decay_scan']

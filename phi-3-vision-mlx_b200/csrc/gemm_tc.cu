@@ -1112,7 +1112,7 @@ int launch_gemm_grouped(const p3_gemm_any_args* a, cudaStream_t st) {
     }
     CUtensorMap ta, ta32, tb;
     if (make_tmap(&ta, a->X, a->M, a->K, a->ldx, 128) || make_tmap(&tb, a->W, w_all, a->K, a->ldw, 128)) return -1;
-    if (mean >= 160) {
+    if (mean >= 160 && gemm_2cta_mode()) {
         // CTA pairs on 256 x 256 tiles from a mean of 160 rows a group on: below it most of a pair's 256 rows would be padding, above it the pair
         // reads W half as often as 128 x 128 tiles do. More pairs than tiles only costs their launch.
         const int64_t most = (a->M / 256 + a->n_groups) * ((a->N + 255) / 256);
@@ -1126,6 +1126,12 @@ int launch_gemm_grouped(const p3_gemm_any_args* a, cudaStream_t st) {
     }
     P3_CHECK_LAUNCH("gemm_any");
     return 0;
+}
+
+// CTA pairs from a quarter of the SMs' worth of 256 x 256 tiles on: fewer rows leave a stream of W, which the kernels of smaller tiles spread
+// over more CTAs
+extern "C" int p3_gemm_pair_width(int64_t M, int64_t N) {
+    return gemm_2cta_mode() && M > 128 && ((M + 255) / 256) * ((N + 255) / 256) >= num_sms() / 4 ? tile_width(M, (int)N) : 0;
 }
 
 static int gemm_dispatch(const void* X, int64_t ldx, const void* W, int64_t ldw, const GemmEpi& ep, int64_t M, int N, int K,
@@ -1149,7 +1155,7 @@ static int gemm_dispatch(const void* X, int64_t ldx, const void* W, int64_t ldw,
         if (band < 0) { const char* e = getenv("P3_GEMM_BAND_MB"); band = e ? atoi(e) : 0; }
         eps.band_mb = band;
     }
-    if (impl == 0 && gemm_2cta_mode() && M > 128 && ((m_tiles + 1) / 2) * ((N + 255) / 256) >= num_sms() / 4)
+    if (impl == 0 && p3_gemm_pair_width(M, N))
         return launch_tc2(X, ldx, W, ldw, eps, M, N, K, st, wp);
     bool small = m_tiles * ((N + 255) / 256) < 2 * num_sms();
     if (ep.kind == P3_EPI_SWIGLU || !small) return launch_tc<256>(X, ldx, W, ldw, eps, M, N, K, st, wp);

@@ -45,7 +45,7 @@ class PagedLM:
     def _init_products(self):
         self.f32 = int(self.dtype == torch.float32)
         self.use_tc = os.environ.get('P3_LM_TC', '1') != '0'
-        self.moe_dense_rows = 1      # (token, choice) pairs from which the experts run on gathered rows (tcgen05)
+        self.moe_dense_rows = int(os.environ.get('P3_LM_MOE_DENSE_ROWS', '1'))   # (token, choice) pairs from which the experts run on gathered rows (tcgen05)
         self.use_skinny = os.environ.get('P3_LM_SKINNY', '1') != '0' and hasattr(_lib.lib(), 'p3_gemm_skinny')
         self.profile = None      # bench.py: list of (kind, ev0, ev1, flops, bytes) when instrumenting
 
@@ -107,11 +107,10 @@ class PagedLM:
         return None
 
     def gated(self, x, w, act, hid, bias32=None, bias16=None, limit=0.0, alpha=0.0, nxt=None):
-        """hid[M,F] = act(g) * u, [g | u] = x w^T (+ bias): one launch where p3_gemm would take CTA pairs for this product (from a
-        quarter of the SMs' worth of 256 x 256 tiles on: 5418 rows, 2048 -> 8192: 233 us, as two launches 401), else the product into fp32
-        rows and the activation kernel: fewer rows leave a stream of w, which the kernels of smaller tiles spread over more CTAs."""
+        """hid[M,F] = act(g) * u, [g | u] = x w^T (+ bias): one launch where p3_gemm would take CTA pairs for this product (5418
+        rows, 2048 -> 8192: 233 us, as two launches 401), else the product into fp32 rows and the activation kernel."""
         (M, K), F = x.shape, w.shape[0] // 2
-        if (self.use_tc and not self.f32 and M > 128 and -(-M // 256) * -(-F // 128) >= 37 and F % 32 == 0 and w.shape[0] == 2 * F
+        if (self.use_tc and not self.f32 and F % 32 == 0 and w.shape[0] == 2 * F and M > 16 and _lib.lib().p3_gemm_pair_width(M, 2 * F)
                 and (bias32 is None or bias16 is not None) and not any(t.stride(0) % 8 or t.data_ptr() % 16 for t in (x, w, hid))
                 and (bias16 is None or bias16.data_ptr() % 16 == 0)):
             ev = self._ev()
@@ -144,7 +143,7 @@ class PagedLM:
         a.out, a.ldo, a.out_f32 = ptr(out), out.stride(0), int(out.dtype == torch.float32)
         a.M = x.shape[0] if M is None else M
         a.N, a.K = (w.shape[-2] if N is None else N), (w.shape[-1] if K is None else K)
-        a.seg_offsets, a.n_groups = ptr(seg), n_groups
+        a.seg_offsets, a.n_groups, a.force_fma = ptr(seg), n_groups, 2 if seg is not None and not self.use_tc else 0
         if batch is not None:
             a.n_batch, a.x_batch_stride, a.w_batch_stride, a.out_batch_stride = batch
         if gate is not None:

@@ -279,3 +279,30 @@ def test_scans_of_many_ctas_have_the_bits_of_one_sequence_at_a_time(dev, mixer, 
         o, s, e = scan([i])
         rows = slice(first[i], first[i] + lens[i])
         assert torch.equal(out[rows], o[rows]) and torch.equal(state[i], s[i]) and torch.equal(den[rows], e[rows])
+
+
+def test_switches_reach_every_product_of_a_layer(dev, monkeypatch):
+    """without tcgen05 the grouped products run on mma.sync, gathered or not, and no unit runs in one launch; without CTA pairs neither does"""
+    import os
+    import subprocess
+    import sys
+    from phi3_b200 import _lib
+    m, seen = _layer(64), []
+    whole = _lib.call
+    monkeypatch.setattr('phi3_b200.lm_base.call', lambda name, *a: (seen.append(name), whole(name, *a))[1])
+    x, w, hid = torch.randn(700, 64, device=dev).to(B16), torch.randn(3200, 64, device=dev).to(B16), torch.empty(700, 1600, dtype=B16, device=dev)
+    assert _lib.lib().p3_gemm_pair_width(700, 3200) and not _lib.lib().p3_gemm_pair_width(128, 1 << 20)
+    m.gated(x, w, 1, hid)
+    assert seen.pop() == 'p3_gemm_glu'
+    g = torch.Generator(device=dev).manual_seed(4)
+    seg, xs, ws = torch.tensor([0, 40, 200], dtype=torch.int32, device=dev), torch.randn(200, 64, generator=g, device=dev).to(B16), torch.randn(2, 72, 64, generator=g, device=dev).to(B16)
+    rows = torch.arange(200, dtype=torch.int32, device=dev)
+    outs = []
+    for m.use_tc in (True, False):
+        outs += [m.gemm_any(xs, ws, torch.empty(200, 72, device=dev), rows=r, seg=seg, n_groups=2, M=200) for r in (None, rows)]
+    assert torch.equal(outs[1], outs[3]) and torch.equal(outs[1], outs[2])      # with a gather always mma.sync; without one only then
+    m.gated(x, w, 1, hid)
+    assert 'p3_gemm_glu' not in seen
+    off = subprocess.run([sys.executable, '-c', 'import phi3_b200; from phi3_b200 import _lib; print(_lib.lib().p3_gemm_pair_width(700, 3200))'],
+                         env=dict(os.environ, P3_GEMM_2CTA='0'), capture_output=True, text=True, timeout=300)
+    assert off.stdout.strip() == '0', off.stderr
