@@ -85,11 +85,11 @@ __host__ __device__ __forceinline__ int band_width(int K, int BN, int n_tiles, i
 constexpr int GROUPS_MAX = 1024;
 struct GroupTable { int tiles[GROUPS_MAX + 1], row[GROUPS_MAX + 1]; };     // row tiles before group g; first row of group g
 struct GroupTile { int m, m_end, w, n; };                                  // rows [m, m_end) of X, rows of W from w + n on
-__device__ __forceinline__ void group_table(GroupTable& t, const int32_t* seg, int n_groups, int bm) {    // one warp
+__device__ __forceinline__ void group_table(GroupTable& t, const int32_t* seg, int n_groups, int M, int bm) {    // one warp; rows from M on are nobody's
     const int lane = threadIdx.x & 31;
     int before = 0;
     for (int g0 = 0; g0 <= n_groups; g0 += 32) {
-        const int g = g0 + lane, a = g <= n_groups ? seg[g] : 0, b = g < n_groups ? seg[g + 1] : a;
+        const int g = g0 + lane, a = g <= n_groups ? min(seg[g], M) : 0, b = g < n_groups ? min(seg[g + 1], M) : a;
         int c = (b - a + bm - 1) / bm;
         const int own = c;
 #pragma unroll
@@ -478,7 +478,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     pdl_wait();
     __shared__ GroupTable groups;                              // (not part of the other kernel's shared memory)
     if constexpr (GROUPED) {
-        if (warp == 3) group_table(groups, ep.seg, ep.n_groups, C::BM);
+        if (warp == 3) group_table(groups, ep.seg, ep.n_groups, M, C::BM);
         __syncthreads();
         total = groups.tiles[ep.n_groups] * n_tiles;
     }
@@ -760,7 +760,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     pdl_wait();
     __shared__ GroupTable groups;
     if constexpr (GROUPED) {
-        if (warp == 3) group_table(groups, ep.seg, ep.n_groups, 2 * C::BM);
+        if (warp == 3) group_table(groups, ep.seg, ep.n_groups, M, 2 * C::BM);
         __syncthreads();
         total = groups.tiles[ep.n_groups] * n_tiles;
     }
@@ -1117,7 +1117,8 @@ int launch_gemm_grouped(const p3_gemm_any_args* a, cudaStream_t st) {
         attr_set[cur_dev()] = true;
     }
     CUtensorMap ta, ta32, tb;
-    if (make_tmap(&ta, a->X, a->M, a->K, a->ldx, 128) || make_tmap(&tb, a->W, w_all, a->K, a->ldw, 128)) return -1;
+    const bool few = a->M <= 32;                               // then every tile takes the boxes of 32 rows
+    if (make_tmap(&tb, a->W, w_all, a->K, a->ldw, 128) || (!few && make_tmap(&ta, a->X, a->M, a->K, a->ldx, 128))) return -1;
     if (mean >= 160 && gemm_2cta_mode()) {
         // CTA pairs on 256 x 256 tiles from a mean of 160 rows a group on: below it most of a pair's 256 rows would be padding, above it the pair
         // reads W half as often as 128 x 128 tiles do. More pairs than tiles only costs their launch.
@@ -1126,6 +1127,7 @@ int launch_gemm_grouped(const p3_gemm_any_args* a, cudaStream_t st) {
         p3_launch_pdl(gemm_tc2_kernel<true>, dim3((unsigned)(2 * clusters)), dim3(384), (size_t)Tc2Cfg::SMEM, st, ta, tb, ep, (int)a->M, a->N, a->K, 256);
     } else {
         if (make_tmap(&ta32, a->X, a->M, a->K, a->ldx, 32)) return -1;
+        if (few) ta = ta32;
         const int64_t most = (a->M / 128 + (a->M < a->n_groups ? a->M : a->n_groups)) * ((a->N + 127) / 128);
         p3_launch_pdl(gemm_tc_kernel<128, true>, dim3((unsigned)(most < num_sms() ? most : num_sms())), dim3(384), (size_t)TcCfg<128>::SMEM, st, ta, tb, ta32, ep,
                       (int)a->M, a->N, a->K);

@@ -211,37 +211,49 @@ class PagedLM:
         depend on the choice (a shared unit), launched behind the sort."""
         st, dev, n = _stream(), self.dev, T * f.top
         n_sorted = f.experts if n_sorted is None else n_sorted
-        up = gu_w.shape[1]
-        seg = torch.empty(n_sorted + 1, dtype=torch.int32, device=dev)
-        order = torch.empty(n, dtype=torch.int32, device=dev)
-        where = torch.empty(n, dtype=torch.int32, device=dev)
-        self.rows('route', n * 12, 'p3_moe_sort', ptr(ids), n, n_sorted, ptr(seg), ptr(order), ptr(where), st)
+        up, dense, esz = gu_w.shape[1], self.experts_dense(f, T), 4 if self.f32 else 2
         gu = torch.empty((n, up), dtype=torch.float32, device=dev)
         hid = torch.empty((n, f.ff), dtype=self.dtype, device=dev)
-        dn = torch.empty((n, self.W), dtype=torch.float32, device=dev)
+        # what only the kernels here see lies in one allocation (a step of few tokens is bound by the host, and an allocation costs it as much
+        # as a launch): row outputs, rows in expert order, segment offsets, order and places, each on a 256-byte boundary
+        parts = (0 if combine is not None else n * self.W * 4, n * self.W * esz if dense else 0, 4 * (n_sorted + 1), 4 * n, 4 * n)
+        at = [0]
+        for size in parts:
+            at.append(at[-1] + (size + 255 & ~255))
+        scratch = torch.empty(at[-1], dtype=torch.uint8, device=dev)
+        base = scratch.data_ptr()
+        dn, xs, seg, order, where = (base + o for o in at[:5])
+        if combine is not None:
+            rows_out = torch.empty((n, self.W), dtype=torch.float32, device=dev)
+            places, dn = scratch[at[4]:at[4] + 4 * n].view(torch.int32), rows_out.data_ptr()
+        self.rows('route', n * 12, 'p3_moe_sort', ptr(ids), n, n_sorted, seg, order, where, st)
+        if meanwhile is not None:
+            meanwhile()
         # The rows are brought into expert order and run as ONE grouped product per matrix on the tcgen05 GEMM, whose CTAs find their expert
         # from the segment offsets on the device: nothing is read back, whatever the number of rows. What that kernel does not take (fp32,
         # sizes that are no multiples of 8) runs on the grouped kernel for any shape, which gathers the rows itself.
-        dense = self.experts_dense(f, T)
-        if meanwhile is not None:
-            meanwhile()
         ev = self._ev()
         if dense:
-            xs = torch.empty((n, self.W), dtype=self.dtype, device=dev)
-            call('p3_gather_rows', ptr(xa), xa.stride(0), self.f32, ptr(order), f.top, ptr(xs), n, self.W, st)
-            self.gemm_any(xs, gu_w, gu, seg=seg, n_groups=f.experts, M=n)
+            call('p3_gather_rows', ptr(xa), xa.stride(0), self.f32, order, f.top, xs, n, self.W, st)
+            self._grouped(xs, self.W, None, gu_w, gu.data_ptr(), up, seg, f.experts, n, st)
         else:
-            self.gemm_any(xa, gu_w, gu, rows=order, row_div=f.top, seg=seg, n_groups=f.experts, M=n)
+            self._grouped(ptr(xa), xa.stride(0), (order, f.top), gu_w, gu.data_ptr(), up, seg, f.experts, n, st)
         self._ev(ev, 'moe_gemm', 2 * n * up * self.W, gu_w.numel() * gu_w.element_size())
         glu(gu, hid, n)
         ev = self._ev()
-        self.gemm_any(hid, down_w, dn, seg=seg, n_groups=f.experts, M=n)
+        self._grouped(hid.data_ptr(), f.ff, None, down_w, dn, self.W, seg, f.experts, n, st)
         self._ev(ev, 'moe_gemm', 2 * n * f.ff * self.W, down_w.numel() * down_w.element_size())
         if combine is not None:
-            combine(dn, where)
+            combine(rows_out, places)
         else:
-            self.rows('combine', T * self.W * 4 * (f.top + 1), 'p3_moe_combine', ptr(dn), dn.stride(0), ptr(where), ptr(wts), f.top, ptr(y), T,
-                      self.W, st)
+            self.rows('combine', T * self.W * 4 * (f.top + 1), 'p3_moe_combine', dn, self.W, where, ptr(wts), f.top, ptr(y), T, self.W, st)
+
+    def _grouped(self, x, ldx, gather, w, out, ldo, seg, groups, M, st):
+        """a grouped product of the experts, by addresses: out fp32 [M, ldo] = rows of x (gather: the sorted pairs and the choices of a token,
+        else row by row), segment by segment, times w[g]^T"""
+        rows, div = (None, 1) if gather is None else gather
+        call_struct('p3_gemm_any', _lib.GemmAnyArgs(x, ldx, self.f32, rows, div, w.data_ptr(), w.stride(1), self.f32, w.stride(0), None, 0, out, ldo, 1,
+                                                    M, w.shape[1], w.shape[2], seg, groups, 0 if self.use_tc else 2), st)
 
     def experts_dense(self, f, T):
         """do the experts of a step with T tokens run on gathered rows (the tcgen05 GEMM)?"""

@@ -306,3 +306,43 @@ def test_switches_reach_every_product_of_a_layer(dev, monkeypatch):
     off = subprocess.run([sys.executable, '-c', 'import phi3_b200; from phi3_b200 import _lib; print(_lib.lib().p3_gemm_pair_width(700, 3200))'],
                          env=dict(os.environ, P3_GEMM_2CTA='0'), capture_output=True, text=True, timeout=300)
     assert off.stdout.strip() == '0', off.stderr
+
+
+def test_rows_behind_the_last_belong_to_no_group(dev):
+    """segment offsets that end behind the number of rows: nothing is read or written from there on, whatever box the rows came in"""
+    g = torch.Generator(device=dev).manual_seed(6)
+    for M, cuts in ((20, [0, 12, 40]), (150, [0, 12, 400])):
+        x, w = torch.randn(M, 72, generator=g, device=dev).to(B16), torch.randn(2, 136, 72, generator=g, device=dev).to(B16)
+        from phi3_b200 import _lib
+        seg, out = torch.tensor(cuts, dtype=torch.int32, device=dev), torch.full((cuts[-1], 136), float('nan'), device=dev)
+        a = _lib.GemmAnyArgs(x.data_ptr(), 72, 0, None, 1, w.data_ptr(), 72, 0, w.stride(0), None, 0, out.data_ptr(), 136, 1, M, 136, 72, seg.data_ptr(), 2, 0)
+        _lib.call_struct('p3_gemm_any', a, _stream())
+        ref = torch.cat([x[:12].double() @ w[0].double().T, x[12:].double() @ w[1].double().T])
+        assert (out[:M].double() - ref).abs().max() < 1e-3 and bool(torch.isnan(out[M:]).all())
+
+
+@pytest.mark.parametrize('tokens', [1, 4, 16, 17, 40])
+def test_an_expert_layer_is_its_launches_and_three_allocations(dev, tokens):
+    """at a few tokens the host sets the time of a layer: an allocation costs it as much as a launch. Result against float64: weights and rows are
+    bf16, so is the unit's result; two products of N(0, 1 / K) weights"""
+    from phi3_b200 import _lib
+    W, F, E, top = 128, 64, 8, 2
+    g = torch.Generator(device=dev).manual_seed(tokens)
+    m = _layer(W)
+    gu, down = (torch.randn(E, n, k, generator=g, device=dev).mul_(k ** -0.5).to(B16) for n, k in ((2 * F, W), (W, F)))
+    x, y = torch.randn(tokens, W, generator=g, device=dev).to(B16), torch.empty(tokens, W, device=dev)
+    ids = torch.stack([torch.randperm(E, generator=g, device=dev)[:top] for _ in range(tokens)]).to(torch.int32)
+    wts = torch.softmax(torch.randn(tokens, top, generator=g, device=dev), -1)
+    unit = type('Unit', (), dict(ff=F, experts=E, top=top))
+    glu = lambda a, hid, n: _lib.call('p3_glu_act', a.data_ptr(), a[:, F:].data_ptr(), a.stride(0), hid.data_ptr(), hid.stride(0), 0, n, F, 0, _stream())
+    m.experts(gu, down, unit, x, y, tokens, ids, wts, glu)
+    torch.cuda.synchronize()
+    allocations, launches = torch.cuda.memory_stats()['allocation.all.allocated'], _lib.launches
+    m.experts(gu, down, unit, x, y, tokens, ids, wts, glu)
+    assert torch.cuda.memory_stats()['allocation.all.allocated'] - allocations == 3 and _lib.launches - launches == 6
+    ref = torch.zeros(tokens, W, dtype=torch.float64, device=dev)
+    for t in range(tokens):
+        for j in range(top):
+            p = gu[ids[t, j]].double() @ x[t].double()
+            ref[t] += wts[t, j].double() * (down[ids[t, j]].double() @ (torch.nn.functional.silu(p[:F]) * p[F:]))
+    assert (y.double() - ref).abs().max() <= 2.0 ** -7 * ref.abs().max()
