@@ -1060,10 +1060,10 @@ static int gemm_2cta_mode() {                  // P3_GEMM_2CTA=0 forces the sing
     return v;
 }
 
-// Columns of a pair's tile: the width whose waves over the CTA pairs cost least. A wave takes time in proportion to its columns (781 x 3072 x
-// 8192, one wave each: 256 53.2 us, 224 46.9, 192 41.3) plus its start and end, but narrow tiles re-read more of X per product: at equal
-// columns 224 and 192 measured 3 - 6 % behind 256 (5418 x 16384 x 2048, 19 waves of 256 and 22 of 224: 244 and 258 us), 160 15 % behind
-// (5418 x 2048 x 8192, 3 waves of 256 and 4 of 160: 136 and 143 us), and 128 takes as long as 160.
+// Columns of a pair's tile: the width whose waves over the CTA pairs cost least. A wave takes time in proportion to its columns plus its start
+// and end (16 columns' worth), and narrow tiles re-read more of X per product: 5418 x 16384 x 3072 in 20 waves of 256 446 us, 22 of 224 447,
+// 26 of 192 469, 31 of 160 501; 781 x 3072 x 8192 in one wave of 256 57.8, 224 53.1, 192 48.2. Over 138 products (300 - 5418 rows, N 1024 -
+// 16384, K 1024 - 8192), each timed at every width, the widths chosen sum to 14.48 ms, the best ones to 14.41, 256 throughout to 14.90.
 static int tile_width(int64_t M, int N) {
     const int64_t m = (M + 255) / 256, pairs = num_sms() / 2;
     const int cost[4][2] = {{256, 100}, {224, 105}, {192, 105}, {160, 115}};
@@ -1228,7 +1228,7 @@ extern "C" int p3_gemm_plan_weights(const void* W, int64_t ldw, int N, int K, vo
     return 0;
 }
 
-// struct-argument entry (SURVEY.md par. 8b): everything p3_gemm does + the fused prefill epilogues
+// struct-argument entry: everything p3_gemm does + the fused prefill epilogues
 extern "C" int p3_gemm_fused(const p3_gemm_args* a, cudaStream_t st) {
     P3_CHECK_ARG(a, "gemm_fused: null args");
     const int epi = a->epi;
