@@ -1,6 +1,6 @@
-"""bench.py — headline benchmark of the B200 hot path (contract: see task statement / DESIGN.md §5).
+"""bench.py — headline benchmark of the B200 hot path.
 
-Workload (the batched data-parallel config the metric is quoted on,
+Workload (the batched data-parallel configuration the metric is quoted on,
 sharded 8 prompts per GPU — weak scaling; at N=8 it is exactly the 64-prompt config):
   per GPU and per step: 8 image+text prompts (one 672x672 image each, HD transform num_crops=4 ->
   5 crops, 757 image tokens) padded with random text to a 2048-token context, 256 greedy tokens.
@@ -11,7 +11,7 @@ sharded 8 prompts per GPU — weak scaling; at N=8 it is exactly the 64-prompt c
 the PUBLIC API call a user makes — parallel.dp_generate -> api.generate_batch with prompt STRINGS and
 host uint8 images (chat template, tokenizer, H2D of the images, HD transform, vision tower, prefill,
 decode, D2H of the tokens, detokenisation all inside the timed region), max over ranks.
-`vqa_prefill_ms` = BASELINE configs[1]: single-image VQA (336px HD crops, num_crops=4) time to
+`vqa_prefill_ms`: single-image VQA (336px HD crops, num_crops=4) time to
 first token at batch 1.  `--impl reference` times the CPU oracle (the reference's arithmetic,
 MLX itself is not installable here) on the host cores.
 """
@@ -30,7 +30,7 @@ sys.path.insert(0, ROOT)
 METRIC = 'batched_decode_tok_per_s'
 B_PER_GPU, CTX, NEW, IMG = 8, 2048, 256, 672
 KV_BYTES_PER_POS = 2 * 32 * 96 * 2          # per layer per sequence (K+V, bf16)
-WEIGHT_BYTES_PER_STEP = 7_445_157_888       # SURVEY.md §8 header (decoder + lm_head, bf16)
+WEIGHT_BYTES_PER_STEP = 7_445_157_888       # decoder + lm_head, bf16
 
 
 def peaks():
@@ -75,7 +75,7 @@ class ClockSampler:
 def bench_config(world):
     """the `config` object of the JSON line — identical for the b200 arm and the --impl reference arm"""
     return {'workload': 'Phi-3.5-vision batched generation: 8 image+text prompts per GPU x 2048 context x 256 '
-                        'new tokens, 672x672 image, HD transform num_crops=4 (BASELINE configs[2], 64 prompts at 8 GPUs)',
+                        'new tokens, 672x672 image, HD transform num_crops=4 (64 prompts at 8 GPUs)',
             'per_gpu_batch': B_PER_GPU, 'context': CTX, 'new_tokens': NEW, 'parallelism': f'dp{world}',
             'l2_policy': 'inputs larger than L2: 7.4 GB weights + 6.8 GB KV streamed per decode step'}
 
@@ -304,7 +304,7 @@ def run_cuda(args):
                     'layer_gemm_frac_of_hbm_peak': round(gemm_bytes / ((t_full - t_nogemm) * 1e-3) / 1e9 / peak_, 4),
                     'note': 'marginal cost inside the captured graph = step time minus step time with that kernel family skipped'}
 
-    # ---- BASELINE configs[1]: single-image VQA prefill at batch 1
+    # ---- single-image VQA prefill at batch 1
     vqa_ms = None
     if rank == 0:
         ids1 = ids_d[:1, :n_img_tok + 30].contiguous()
@@ -323,7 +323,7 @@ def run_cuda(args):
             ts.append(a.elapsed_time(b))
         vqa_ms = min(ts[2:])
 
-    # ---- BASELINE configs[4]: quantize_cache + constrained beam decoding, batch 16, beam 4 (MedQA-shaped prompts)
+    # ---- quantize_cache + constrained beam decoding, batch 16, beam 4 (MedQA-shaped prompts)
     cfg5 = None
     if rank == 0:
         try:
@@ -335,7 +335,7 @@ def run_cuda(args):
             p5 = _api._apply_chat_template(qs, None, False)[0]
             class _Cfg5Tok(ByteTokenizer):
                 """byte tokenizer for the prompts; the two constraint strings map to id lists of the lengths the Phi-3 tokenizer
-                gives them (SURVEY par. 8d: C = 2 and C = 4 after the [1:] of pv:538), not to 4 / 22 byte tokens"""
+                gives them (C = 2 and C = 4 after the [1:] of pv:538), not to 4 / 22 byte tokens"""
                 FIXED = {'\nThe': [29871, 13, 1576], ' The correct answer is': [29871, 450, 1959, 1234, 338]}
 
                 def encode(self, text, add_special_tokens=True):

@@ -1,9 +1,9 @@
 /* phi3_b200.h — C ABI of libphi3b200.so (sm_100a only).
  *
  * The reference (JosefAlbers/Phi-3-Vision-MLX) has no FFI/plugin layer: its hot path calls
- * mlx==0.15 ops from Python (SURVEY.md §2.2). Each entry below replaces one of those MLX call
- * sites; the cited lines are in /root/reference/phi.py (phi:) and
- * /root/reference/phi_3_vision_mlx.py (pv:). INTEGRATION.md shows the ctypes binding a
+ * mlx==0.15 ops from Python. Each entry below replaces one of those MLX call
+ * sites; the cited lines are in phi.py (phi:) and
+ * phi_3_vision_mlx.py (pv:). INTEGRATION.md shows the ctypes binding a
  * maintainer of the reference would add.
  *
  * Conventions: plain device pointers + sizes, caller-owned memory and workspaces, no
@@ -68,7 +68,7 @@ int p3_row_stats(const float* logits, int64_t R, int64_t ld, int V, int32_t* arg
                  float* lse_out, int n_top, int32_t* topk_ids, float* topk_lp, int n_gather,
                  const int32_t* gather_ids, float* gather_lp, cudaStream_t st);
 
-/* Nucleus (top-p) sampling — extension: the reference decodes greedily only (pv:386,392; SURVEY H13).
+/* Nucleus (top-p) sampling — extension: the reference decodes greedily only (pv:386,392).
  * tau = largest probability v with sum_{p_i>=v} p_i >= top_p (exact bisection, no sort); token drawn by
  * inverse CDF in index order over {p_i >= tau} with the caller's uniform u[R] in [0,1). tau_out may be NULL.
  * step_dev (device int32, may be NULL): u is a table and row *step_dev * u_stride is used (graph replay). */
@@ -136,7 +136,7 @@ int p3_gemm_glu(const void* X, int64_t ldx, const void* W, int64_t ldw, const vo
  * phi:550-563) and mx.fast.scaled_dot_product_attention phi:148 (causal=0).
  * q/k/v point into the (roped) qkv buffer; row strides in elements; head h at +h*hd.
  * Keys [0,past) come from the paged pool (cache row b/row_div), keys [past,past+L) from k/v.
- * kv_start int32 [B] (left-pad length; NULL = 0). Pad queries produce zeros (SURVEY H1).
+ * kv_start int32 [B] (left-pad length; NULL = 0). Pad queries produce zeros.
  * Runs the tcgen05 flash-attention kernel (S and P in TMEM, TMA operands) when past % 64 == 0, L >= 64 and
  * the pointers / strides are 16-byte aligned; otherwise (and with P3_ATTN_TC=0 in the environment, used by the
  * tests as a cross-check) the mma.sync kernel with the same contract. */
@@ -224,8 +224,8 @@ int p3_gn_assemble(const float* feats, const void* sub_GN, const void* glb_GN, v
                    cudaStream_t st);
 
 /* ------------------------------------------------------------------------------------------------
- * Struct-argument GEMM entry with the fused prefill epilogues (north_star: "SuRoPE fused into the QKV epilogue",
- * "RMSNorm and residual fused with adjacent ops"); replaces nn.RMSNorm + nn.Linear + _rotate_half + KVCache slice-assign at
+ * Struct-argument GEMM entry with the fused prefill epilogues (SuRoPE fused into the QKV epilogue, RMSNorm and
+ * residual fused with the products beside them); replaces nn.RMSNorm + nn.Linear + _rotate_half + KVCache slice-assign at
  * prefill: phi:442-453, 478-485.
  *   - ss_in / n_ss_in / eps: RMSNorm of the INPUT rows is applied as a per-row scale rsqrt(sum_c ss_in[row][c] / K + eps) on the
  *     accumulators; the gain must already be folded into W (W'[n][k] = W[n][k] * g[k]). ss_in rows hold partial sums of
@@ -273,7 +273,7 @@ int p3_row_sumsq(const void* x, int64_t ldx, float* out, int64_t T, int H, cudaS
  * e.g. o_proj(+residual) -> RMSNorm+gate_up(+SwiGLU) -> down_proj(+residual) -> RMSNorm+qkv_proj(+SuRoPE
  * +paged KV write) of the next layer, or ... -> RMSNorm+lm_head. Replaces nn.Linear / nn.RMSNorm /
  * _rotate_half / KVCache slice-assign at decode: phi:437-438, 442-453, 460, 465-471, 478-485, 604-608.
- * Arguments travel in a plain-old-data struct (device pointers + sizes), as SURVEY.md par. 8b asks. */
+ * Arguments travel in a plain-old-data struct (device pointers + sizes). */
 #define P3_MEGA_RESID 0     /* out[M,N] bf16 = bf16(out + bf16(x W^T)) in place; ss_out[tile][16] = sum of squares of the 16 new columns */
 #define P3_MEGA_SWIGLU 1    /* W = [gate rows | up rows] (phi:470); out[M,N/2] bf16 = silu(gate) * up */
 #define P3_MEGA_QKV_ROPE 2  /* out[M,N] bf16 = qkv with q,k rotated (phi:418-423) + K,V written to the page pool at `past` */

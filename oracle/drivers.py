@@ -2,7 +2,7 @@
 oracle model: _generate (phi_3_vision_mlx.py:376-409), _choose_from (pv:466-487),
 _constrain + _get_beam (pv:500-619). Dense log-softmax over the full vocabulary, exactly as the
 reference does it; token-id level only (tokenizer decode is host glue). Parity unpinned by the
-reference's own tests (SURVEY.md §4) — these follow the cited lines statement by statement.
+reference's own tests — these follow the cited lines statement by statement.
 """
 import torch
 

@@ -5,8 +5,8 @@ __graft_entry__.smoke() and bench.py's cpu_baseline / --impl reference legs.
 Nothing in the product package may import it.
 
 PARITY STATUS: *partly pinned*. The reference (MLX 0.15) cannot be executed in
-this image (no mlx wheel), and its own test.py holds no numeric goldens
-(SURVEY.md §4), so the arithmetic below is pinned two ways instead:
+this image (no mlx wheel), and its own test.py holds no numeric goldens,
+so the arithmetic below is pinned two ways instead:
   * decoder (B=1, no pad) against transformers.Phi3ForCausalLM, CLIP tower
     against transformers.CLIPVisionModel hidden_states[-2][:,1:]
     (tests/test_oracle_vs_hf.py);
@@ -15,7 +15,7 @@ this image (no mlx wheel), and its own test.py holds no numeric goldens
 MLX-internal rounding behaviour (dtype promotion, quantiser edge rule) is
 restated from mlx 0.15 semantics and marked [mlx-inferred].
 
-Each function cites the reference lines it follows (phi: = /root/reference/phi.py).
+Each function cites the reference lines it follows (phi: = phi.py).
 
 Precision modes (``prec``):
   'fp32' : every op in float32 (ideal arithmetic, HF cross-check mode)
@@ -28,7 +28,7 @@ Precision modes (``prec``):
            (phi:412-415)
   'b200' : as 'ref' but q,k,v are rounded to bf16 after rope (bf16 KV cache) and
            the attention output is rounded to bf16 — the precision delta
-           the CUDA path takes deliberately (SURVEY.md §8 H2)
+           the CUDA path takes deliberately
 """
 import math
 import torch
@@ -67,7 +67,7 @@ def quantize_q4g32(w, prec='ref', group=32, dtype=torch.float32):
     (bits=4) as called at phi:532 [mlx-inferred edge rule: the larger-magnitude edge of
     each group is exact and 0 stays representable]. Returns (q uint8 [...,G,32], scale, bias).
     In 'b200' mode scale/bias are rounded to bf16 before the codes are computed (the GPU
-    cache stores bf16 scale+bias; stated rule, see DESIGN.md). ``group`` generalises the same rule
+    cache stores bf16 scale+bias; stated rule). ``group`` generalises the same rule
     to nn.quantize(model, 64, 4) (quantize_model_weights below)."""
     shp = w.shape
     g = w.reshape(*shp[:-1], shp[-1] // group, group).to(dtype)
@@ -180,7 +180,7 @@ class KVCache:
     """phi:509-548. Dense preallocated buffer with the reference's offset bookkeeping.
     Quantised mode keeps the same read semantics as phi:528-540 (prompt part read back
     through 4-bit g32 quantise->dequantise from the second call on; later tokens exact).
-    Extensions (no working reference behaviour, SURVEY.md H10): quantised + advance_offset
+    Extensions (no working reference behaviour): quantised + advance_offset
     and quantised + n_beam behave like the dense cache with the quantised prompt image."""
 
     def __init__(self, cfg, B, L, max_tokens, prec):

@@ -1,5 +1,5 @@
 """Public inference API with the reference's signatures:
-load / generate / choose / constrain (/root/reference/phi_3_vision_mlx.py:1279, 1324, 1376, 1425)
+load / generate / choose / constrain (phi_3_vision_mlx.py:1279, 1324, 1376, 1425)
 and the decode drivers behind them (_generate pv:376-409, _choose_from pv:466-487,
 _constrain/_get_beam pv:500-619, Streamer/LogitStopper/TokenStopper pv:45-117,
 _apply_chat_template pv:341-357). Control flow lives here in Python; every tensor op is a
@@ -22,7 +22,7 @@ Differences a caller can see (all opt-in or forced by the offline environment):
   * generate_batch(prompts, images_per_prompt, ...) is an extension: the reference raises on images + a prompt list
     (pv:377-378), so its only way to run N image prompts is N sequential batch-1 calls. generate_batch runs them as ONE
     left-padded batch with per-prompt batch-1 semantics (each row keeps its own positions 0..L_i-1, pad keys masked,
-    image tokens spliced per row), which is what BASELINE config 3 (64 image+text prompts) needs;
+    image tokens spliced per row): what batches of 64 image+text prompts need;
   * load(model_path=<dir>) / load(weights=<dir>) read that directory's config.json like _get_cfg (pv:258,359-363): LM
     hyper-parameters and rope_scaling come from the checkpoint, kwargs override; `sanitized` / `quantized` keys are honoured
     (pv:262-264,371-374). The frozen PHI35_* configs are only used for random_init and weight dicts.
@@ -430,7 +430,7 @@ class LogitStopper:
 
 
 def _batch_inputs(processor, prompts, images):
-    """N image+text (or text-only) prompts -> ONE left-padded model input with per-prompt batch-1 semantics (SURVEY H11):
+    """N image+text (or text-only) prompts -> ONE left-padded model input with per-prompt batch-1 semantics:
     every prompt goes through the processor alone, exactly as the reference's batch-1 VLM path does (pv:381, phi:263-281), then
     rows are left-padded like Phi3FProcessor._tokenize (phi:236-245: ids 0, pids 1, mask 0) and the image-token positions are
     shifted by each row's pad. Row b keeps positions 0..L_b-1, so its logits equal the batch-1 call's."""
@@ -565,7 +565,7 @@ def generate(prompt, images=None, preload=None, blind_model=False, quantize_mode
 def generate_batch(prompts, images=None, preload=None, blind_model=False, quantize_model=False, quantize_cache=False,
                    use_adapter=False, max_tokens=512, verbose=False, return_tps=False, apply_chat_template=True,
                    return_tokens=False):
-    """Extension of generate() (pv:1324) for BASELINE config 3: a LIST of prompts, each with its own image(s).
+    """Extension of generate() (pv:1324): a LIST of prompts, each with its own image(s).
     `images`: None, or a list with one entry per prompt (None | image | list of images). Returns a list of strings
     (or (prompt_tps, gen_tps) / the token history). Per-prompt results equal separate batch-1 generate() calls."""
     if isinstance(prompts, str):

@@ -1,10 +1,10 @@
 """Frozen hyper-parameters for the two checkpoints the reference serves.
 
 The reference reads these at run time from the downloaded HF ``config.json``
-(/root/reference/phi_3_vision_mlx.py:258,359-363); none is in its tree, so the
+(phi_3_vision_mlx.py:258,359-363); none is in its tree, so the
 public Phi-3.5-mini-instruct / Phi-3.5-vision-instruct values are frozen here.
-LongRoPE factor vectors: /root/reference/assets/su_rope_explained.ipynb:309-310.
-CLIP constants: /root/reference/phi.py:375-384.
+LongRoPE factor vectors: assets/su_rope_explained.ipynb:309-310.
+CLIP constants: phi.py:375-384.
 """
 from types import SimpleNamespace
 import copy
@@ -29,8 +29,8 @@ LONG_FACTOR = [1.0299999713897705, 1.0499999523162842, 1.0499999523162842, 1.079
                63.48000717163086, 63.66000747680664, 63.850006103515625, 64.08000946044922, 64.760009765625,
                64.80001068115234, 64.81001281738281, 64.81001281738281]
 
-ID_EOS = 32007   # /root/reference/phi_3_vision_mlx.py:42
-ID_ASS = 32001   # /root/reference/phi_3_vision_mlx.py:43
+ID_EOS = 32007   # phi_3_vision_mlx.py:42
+ID_ASS = 32001   # phi_3_vision_mlx.py:43
 
 CLIP_VIT_L14_336 = SimpleNamespace(hidden_size=1024, image_size=336, intermediate_size=4096, layer_norm_eps=1e-5,
                                    num_attention_heads=16, num_channels=3, num_hidden_layers=24, patch_size=14)

@@ -67,7 +67,7 @@ __device__ __forceinline__ void qk_mma(const uint32_t (*qf)[4], uint32_t sk, int
 
 // One warp: O(16 x D) += P(16 x NK*8 keys) V. P is rounded to bf16 for the tensor cores (the
 // reference runs softmax.V in fp32, phi.py:454-457; a bf16 hi/lo split of P was measured to change
-// nothing: bf16 pipelines decorrelate at their noise floor regardless, DESIGN.md §4).
+// nothing: bf16 pipelines decorrelate at their noise floor regardless).
 template <int D, int NK>
 __device__ __forceinline__ void pv_mma(const float (*s)[4], uint32_t sv, int key0, float (*o)[4], int lane) {
 #pragma unroll

@@ -494,8 +494,8 @@ extern "C" int p3_decode_advance(const int32_t* tok, int32_t* history, int64_t l
 }
 
 // ------------------------------------------------------------------------------------------
-// top_p_sample: nucleus sampling (north_star "top-p kernel"; the reference is greedy only, pv:386,392 —
-// this is an extension, SURVEY.md H13, validated against a torch restatement of the same rule).
+// top_p_sample: nucleus sampling (the reference is greedy only, pv:386,392 —
+// this is an extension, validated against a torch restatement of the same rule).
 // Per row: p = softmax(logits / temperature); tau = the largest probability value v such that
 // sum_{p_i >= v} p_i >= top_p (exact: bisection over the float bit pattern, no sort); the token is
 // drawn by inverse CDF in INDEX order over the nucleus {i : p_i >= tau} with the supplied uniform u.

@@ -1,7 +1,7 @@
 // 4-bit group-32 affine quantisation of the prompt part of the paged KV cache.
 // Replaces mx.quantize(keys.reshape(B*N,-1), group_size=32) of phi.py:532 (bits=4 default).
 // Groups are 32 consecutive head-dim elements of one (token, head): 3 per 96-wide head, never
-// straddling tokens. Rule (stated in DESIGN.md, mirrors oracle.quantize_q4g32
+// straddling tokens. Rule (mirrors oracle.quantize_q4g32
 // in 'b200' mode): the larger-magnitude edge of the group is exact, 0 stays representable,
 // scale and bias are rounded to bf16 BEFORE the codes are computed, q = clamp(rint((w-b)/s),0,15).
 // Full 64-token pages get 4-bit codes + bf16 (scale,bias); every quantised position (including

@@ -170,7 +170,7 @@ extern "C" int p3_clip_embed(const float* patches, const void* cls, const void* 
     return 0;
 }
 
-// Token assembly for one image (phi.py:403-407, closed form in SURVEY.md A.3):
+// Token assembly for one image (phi.py:403-407, in closed form):
 //   [ sub tokens (plain-reshape order) with a sub_GN after every 12*wc tokens | glb_GN | global 12 rows of 12 + sub_GN ]
 // merged token (crop, r, c) channel block q=(dr*2+dc) <- feature (2r+dr, 2c+dc) of the crop (CLS dropped).
 __global__ void gn_assemble_kernel(const float* __restrict__ feats, const bf16* __restrict__ sub_GN, const bf16* __restrict__ glb_GN,

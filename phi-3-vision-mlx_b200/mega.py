@@ -2,7 +2,7 @@
 
 For <= 8 decode rows the per-layer weight stream
     o_proj(+residual) -> RMSNorm -> gate_up_proj(+SwiGLU) -> down_proj(+residual) -> RMSNorm -> qkv_proj(+SuRoPE, +KV write)
-(/root/reference/phi.py:437-438, 442-453, 460, 465-471, 478-485; the last launch ends in lm_head, phi.py:604-608) runs as ONE
+(phi.py:437-438, 442-453, 460, 465-471, 478-485; the last launch ends in lm_head, phi.py:604-608) runs as ONE
 launch of #SM persistent CTAs. This module owns
   * the stream-order copy of the decoder weights (made once at load by p3_mega_pack),
   * the tile -> CTA schedule (cumulative-byte balanced at every phase boundary),

@@ -1,6 +1,6 @@
 """Phi-3.5 (mini / vision) on B200 — host-side mirror of the reference model call protocol.
 
-`Phi3B200.__call__` keeps the signature of Phi3ForCausalLM.__call__ (/root/reference/phi.py:606):
+`Phi3B200.__call__` keeps the signature of Phi3ForCausalLM.__call__ (phi.py:606):
     model(input_ids, pixel_values=None, image_sizes=None, positions=None, cache=None, pids=None,
           mask=None, max_tokens=0, advance_offset=None, n_beam=1) -> (logits[B,L,V], cache)
 All arithmetic runs in the sm_100a kernels of libphi3b200.so through the C ABI (`_lib.call`);
@@ -234,7 +234,7 @@ class Phi3B200:
                 down=lin(w[p + 'mlp.down_proj.weight'], None, p + 'mlp.down_proj')))
         self.norm = d(w['model.norm.weight'])
         self.lm_head = lin(w['lm_head.weight'])
-        # fused prefill (north_star: SuRoPE + KV write in the QKV epilogue, RMSNorm fused with the adjacent GEMM): second copies of
+        # fused prefill (SuRoPE + KV write in the QKV epilogue, RMSNorm fused with the adjacent GEMM): second copies of
         # qkv_proj / gate_up_proj with the RMSNorm gain folded in (W' = bf16(W * g), the per-row rsqrt is applied to the
         # accumulators) and, for qkv, q/k rows permuted per head so a rotary pair meets in one 32-column accumulator chunk
         import os as _os1
@@ -505,7 +505,7 @@ class Phi3B200:
         use_long = L_all > cfg.original_max_position_embeddings if self.force_long_rope is None else self.force_long_rope
         fac = cfg.rope_scaling['long_factor'] if use_long else cfg.rope_scaling['short_factor']   # static switch (H7)
         # inv_freq: 48 values, fp32 on the host exactly as phi:498; the [Bt, L_all, 48] table itself is built by p3_rope_table on
-        # the device (a 128K-token table is 2 x 25 MB — round 1 built it with CPU torch and copied it over PCIe per call)
+        # the device (a 128K-token table is 2 x 25 MB, which a copy from the host would pay for on every call)
         inv_freq = (1.0 / (torch.tensor(fac, dtype=torch.float32)
                            * cfg.rope_theta ** (torch.arange(0, self.hd, 2, dtype=torch.float32) / self.hd))).to(self.dev)
         half = self.hd // 2
@@ -826,7 +826,7 @@ class Phi3B200:
         if write and logits_rows == 'last' and L > self.prefill_chunk:
             # chunked prefill: keys [0, past+c0) come from the paged pool, the chunk's own keys from its
             # qkv buffer; activations stay O(chunk) so a 128K prompt fits (the reference materialises
-            # L x L scores and an L x L mask and cannot run it, SURVEY.md §5)
+            # L x L scores and an L x L mask and cannot run it)
             ids2 = ids_dev.view(B, L)
             h2 = None if h is None else h.view(B, L, self.H)
             logits = None

@@ -1,7 +1,7 @@
-"""Data-parallel sharding of independent prompts over the GPUs of one box (SURVEY.md §8e).
+"""Data-parallel sharding of independent prompts over the GPUs of one box.
 
 The reference has no multi-device code; its only batching is left-padding prompts in one process
-(/root/reference/phi.py:236-245). Prompts are independent, so the B200 build shards them: one
+(phi.py:236-245). Prompts are independent, so the B200 build shards them: one
 process per GPU, weights replicated, NO collective on the data path. torch.distributed is used
 only by the harness (gathering the finished rows to rank 0, barriers around timed regions).
 

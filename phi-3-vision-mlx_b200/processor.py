@@ -1,4 +1,4 @@
-"""Processors: tokenise / left-pad (Phi3FProcessor, /root/reference/phi.py:228-250), image-token
+"""Processors: tokenise / left-pad (Phi3FProcessor, phi.py:228-250), image-token
 splice (Phi3VProcessor._merge, phi.py:263-281) and the HD transform (Phi3VImageProcessor,
 phi.py:283-372) — the latter on the GPU through p3_hd_* kernels, with the PIL resampling
 coefficient tables built on the host exactly as Pillow's Resample.c precompute_coeffs does.
@@ -173,7 +173,7 @@ def interp336_tables(in_size):
 
 def hd_geometry(w, h, num_crops):
     """Pure index math of HD_transform (phi.py:291-306): returns dict with the resize target,
-    padding and final [H, W]. Bit-exact contract (SURVEY.md B3)."""
+    padding and final [H, W]. Bit-exact contract."""
     trans = w < h
     if trans:
         w, h = h, w
@@ -190,7 +190,7 @@ def hd_geometry(w, h, num_crops):
 
 class Phi3VImageProcessor:
     """phi.py:283-372 on the GPU. `num_crops` is hard-coded 16 in the reference (phi.py:285);
-    it is a parameter here (default 16) because BASELINE config 2 names num_crops=4."""
+    it is a parameter here (default 16) because single-image prompts are also run with num_crops=4."""
 
     def __init__(self, num_crops=16, device='cuda'):
         self.num_crops = num_crops

@@ -1,4 +1,4 @@
-"""HTTP front end with request batching (SURVEY row N4; the reference's server.py, srv:1-38).
+"""HTTP front end with request batching (the reference's server.py, srv:1-38).
 
 Same wire contract as the reference: `POST /v1/completions` with `{"prompt": str | [str, ...], "max_tokens": int}` answers
 `{"model": "phi-3-vision", "responses": [str, ...]}`; any other path is a 404 (srv:9-30). The reference serves one request at a

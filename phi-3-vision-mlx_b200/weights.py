@@ -1,8 +1,8 @@
 """Seeded random-init checkpoints with the reference's parameter names.
 
-Names follow the module tree of /root/reference/phi.py (Phi3ForCausalLM phi:599-617,
+Names follow the module tree of phi.py (Phi3ForCausalLM phi:599-617,
 Phi3ImageEmbedding phi:374-391, ClipModel phi:208-221), i.e. the HF safetensors keys the
-reference loads at /root/reference/phi_3_vision_mlx.py:265,371-374 (patch_embedding weight
+reference loads at phi_3_vision_mlx.py:265,371-374 (patch_embedding weight
 already in the reference's post-transpose [O,kh,kw,I] layout).
 All tensors are bf16 (HF checkpoints are bf16); the CPU oracle and the CUDA path are fed
 the same dict. There is no network in this environment, so benchmarks and parity tests
@@ -60,7 +60,7 @@ def random_weights(cfg, seed=0, device='cpu', clip_cfg=None, vision=None, init='
     biases/pos 0.1*N, GN separators N(0,1). With the residual scaling the residual stream stays
     O(1) over 32 layers and the random network is not chaotic (a plain 0.02 init amplifies a 1e-3
     perturbation ~25x by layer 32, which says nothing about kernel accuracy); logits have O(1)
-    spread (SURVEY.md §7 hard part 1).
+    spread.
 
     init='peaked' (the parity checkpoint): identical tensors, except that lm_head is TIED to the embedding through a
     fixed seeded permutation, lm_head[t] = PEAK_ALPHA * embed[perm[t]]. The residual stream of this init keeps a cosine
