@@ -341,7 +341,7 @@ typedef struct {
     void* out; int64_t ldo; int32_t out_f32;
     int64_t M; int32_t N, K;
     const int32_t* seg_offsets; int32_t n_groups;
-    int32_t force_fma;           /* 1: bf16 operands on the FMA kernel (tests); 2: not on tcgen05 (grouped products on mma.sync) */
+    int32_t force_fma;           /* 2: not on tcgen05 (grouped products on mma.sync); else not 0: bf16 operands on the FMA kernel (tests) */
     int32_t n_batch; int64_t x_batch_stride, w_batch_stride, out_batch_stride;
     const float* gate; int64_t ld_gate;
 } p3_gemm_any_args;

@@ -481,7 +481,7 @@ extern "C" int p3_gemm_any(const p3_gemm_any_args* a, cudaStream_t st) {
     } else {
         const bool tc = a->K % 8 == 0 && a->ldx % 8 == 0 && a->ldw % 8 == 0 && a->w_group_stride % 8 == 0 &&
                         (nb == 1 || (a->x_batch_stride % 8 == 0 && a->w_batch_stride % 8 == 0)) &&
-                        ((uintptr_t)a->X & 15) == 0 && ((uintptr_t)a->W & 15) == 0 && a->force_fma != 1;
+                        ((uintptr_t)a->X & 15) == 0 && ((uintptr_t)a->W & 15) == 0 && (!a->force_fma || a->force_fma == 2);
         if (tc) {
             if (a->K <= 64) {
                 if (a->out_f32) p3_launch_pdl(gemm_any_mma_kernel<float, 64>, dim3(grid), dim3(128), (size_t)(0), st, p);
