@@ -117,7 +117,9 @@ inline ScanShape scan_shape(int64_t ctas, size_t floats_per_token, int dim, int 
 // a store that later shared-memory reads may be moved ahead of (the compiler cannot tell that `p` is not shared memory): with it four tokens of
 // the linear attention overlap (650 -> 550 us for 4 x 2048 tokens)
 __device__ __forceinline__ void st_out(float* p, float v) { asm volatile("st.global.f32 [%0], %1;" ::"l"(p), "f"(v)); }
-// a lane's rows d0 .. and its NC columns col, col + CW, .. of a head's state
+// a lane's rows d0 .. and its NC columns col, col + CW, .. of a head's state. As functions these change how far a kernel's tokens overlap: the
+// linear attention and the fixed decays read it in lines of their own (one sequence of 1500 tokens: 402 -> 303 us, 301 -> 222 with decays),
+// the matrix memory writes it so (40 single tokens 32.1 -> 30.0 us); the delta rule is level or slower (329 -> 338 us) that way.
 template <int DS, int NC, int CW>
 __device__ __forceinline__ void get_state(float (&S)[NC][DS], const float* Sg, int d, int dv, int d0, int col, bool fresh) {
 #pragma unroll
@@ -297,7 +299,11 @@ __global__ void __launch_bounds__(MM_WARPS * 32) matrix_memory_scan_kernel(p3_ma
     }
     pdl_trigger();                                           // not before: see scan_shape
     if (main) {
-        put_state<DS, NC, CW>(S, Sg, d, dv, d0, col);
+#pragma unroll
+        for (int c = 0; c < NC; c++)
+#pragma unroll
+            for (int j = 0; j < DS; j++)
+                if (col + c * CW < dv && d0 + j < d) Sg[(size_t)(d0 + j) * dv + col + c * CW] = S[c][j];
     } else if (gate_warp) {
         if (lane == 0)
             for (int c = vb * (COLS / 32); c < min((vb + 1) * (COLS / 32), mm_m_copies(dv)); c++) mg[c] = m;
@@ -391,7 +397,11 @@ __global__ void __launch_bounds__(GLA_WARPS * 32) gla_scan_kernel(p3_gla_args a)
     float* Sg = a.state + ((size_t)slot * H + hd) * gla_head_floats(d, dv);
     const int col = vb * COLS + warp * WCOLS + lane % CW, d0 = (lane / CW) * DS;   // first of this lane's columns
     float S[NC][DS];
-    get_state<DS, NC, CW>(S, Sg, d, dv, d0, col, fresh);
+#pragma unroll
+    for (int c = 0; c < NC; c++)
+#pragma unroll
+        for (int j = 0; j < DS; j++)
+            S[c][j] = (!fresh && col + c * CW < dv && d0 + j < d) ? Sg[(size_t)(d0 + j) * dv + col + c * CW] : 0.f;
     const bool vec = d % 4 == 0 && a.ld_proj % 4 == 0 && a.q_off % 4 == 0 && a.k_off % 4 == 0 && ((uintptr_t)a.proj & 15) == 0 &&
                      a.ld_z % 4 == 0 && ((uintptr_t)a.z & 15) == 0;
 
@@ -660,7 +670,14 @@ __global__ void __launch_bounds__(GLA_WARPS * 32) delta_scan_kernel(p3_delta_sca
     }
     const float fixed = DELTA || a.gates ? 0.f : a.decay[hd], skip = DELTA || !a.skip ? 0.f : a.skip[hd];
     float S[NC][DS];
-    get_state<DS, NC, CW>(S, Sg, d, dv, d0, col, fresh);
+    if constexpr (DELTA) get_state<DS, NC, CW>(S, Sg, d, dv, d0, col, fresh);
+    else {
+#pragma unroll
+        for (int c = 0; c < NC; c++)
+#pragma unroll
+            for (int j = 0; j < DS; j++)
+                S[c][j] = (!fresh && col + c * CW < dv && d0 + j < d) ? Sg[(size_t)(d0 + j) * dv + col + c * CW] : 0.f;
+    }
     for (int t0 = 0, r = 0; t0 < n_tok; t0 += TB, r++) {
         const int nb = min(TB, n_tok - t0), buf = r & 1;
         cp_async_wait<0>();                                  // this thread's copies of round r have landed ...
@@ -720,7 +737,7 @@ __global__ void __launch_bounds__(GLA_WARPS * 32) delta_scan_kernel(p3_delta_sca
                 }
             }
         }
-#pragma unroll(DS >= (DELTA ? 64 : 128) ? 1 : DS <= 32 ? 4 : 2)
+#pragma unroll(DS >= (DELTA ? 64 : 128) ? 1 : DELTA && DS <= 32 ? 4 : 2)
         for (; tt < nb; tt++) {
             const float keep = DELTA || a.gates ? gs[2 * tt] : fixed, beta = DELTA || a.gates ? gs[2 * tt + 1] : 1.f;
             const float4* kq = reinterpret_cast<const float4*>(ks + tt * DPP + at_row(d0));
