@@ -346,6 +346,8 @@ typedef struct {
     const float* gate; int64_t ld_gate;
 } p3_gemm_any_args;
 int p3_gemm_any(const p3_gemm_any_args* args, cudaStream_t st);
+/* rows of the tile that an fp32 product runs on: 16 (the stream of W for up to 16 rows), 32, 64 or 128; 0: the kernel for any alignment, or bf16 */
+int p3_gemm_any_tile(const p3_gemm_any_args* args);
 
 /* x fp32 [T,W] = table[ids] * scale (bf16 table); x_act (may be NULL; row pitch ld_act) receives the same rows in the activation
  * type */

@@ -322,23 +322,28 @@ int launch_f32_rows(const AnyP& p, cudaStream_t st) {
 // Which tile? Times of one k-step on B200 in ns, lone CTA on an SM | per CTA when several share one: 128 x 128 94 | 105, 64 x 64 47 | 29,
 // 32 x 32 41 | 11 (measured from 64 x 4096 x 3072 to 1100 x 4096 x 2048); the busiest SM decides. 64 x 128, 64 x 64 with 4 x 4 outputs per
 // thread and 32 x 64 were behind one of these three at every size tried.
-template <typename OT>
-int dispatch_f32(const AnyP& p, cudaStream_t st) {
-    if (!p.seg && p.M <= 16) {
-        if (p.M <= 1) return launch_f32_rows<OT, 1>(p, st);
-        if (p.M <= 2) return launch_f32_rows<OT, 2>(p, st);
-        if (p.M <= 4) return launch_f32_rows<OT, 4>(p, st);
-        if (p.M <= 8) return launch_f32_rows<OT, 8>(p, st);
-        return launch_f32_rows<OT, 16>(p, st);
-    }
+int f32_tile(const AnyP& p) {
+    if (!p.seg && p.M <= 16) return 16;
     auto cost = [&](int r, int64_t alone, int64_t shared) -> int64_t {
         if (((int64_t)p.N + r - 1) / r > 65535) return INT64_MAX;        // more column tiles than the grid's second dimension holds
         const int64_t tiles = ((p.M + r - 1) / r + (p.seg ? p.n_groups / 2 : 0)) * ((p.N + r - 1) / r) * p.nb, per_sm = (tiles + 147) / 148;
         return alone > per_sm * shared ? alone : per_sm * shared;
     };
     const int64_t c128 = cost(128, 94, 105), c64 = cost(64, 47, 29), c32 = cost(32, 41, 11);
-    if (c128 <= c64 && c128 <= c32) launch_f32<OT, 128, 128, 8, 8>(p, st);
-    else if (c64 <= c32) launch_f32<OT, 64, 64, 8, 4>(p, st);
+    return c128 <= c64 && c128 <= c32 ? 128 : c64 <= c32 ? 64 : 32;
+}
+template <typename OT>
+int dispatch_f32(const AnyP& p, cudaStream_t st) {
+    const int tile = f32_tile(p);
+    if (tile == 16) {
+        if (p.M <= 1) return launch_f32_rows<OT, 1>(p, st);
+        if (p.M <= 2) return launch_f32_rows<OT, 2>(p, st);
+        if (p.M <= 4) return launch_f32_rows<OT, 4>(p, st);
+        if (p.M <= 8) return launch_f32_rows<OT, 8>(p, st);
+        return launch_f32_rows<OT, 16>(p, st);
+    }
+    if (tile == 128) launch_f32<OT, 128, 128, 8, 8>(p, st);
+    else if (tile == 64) launch_f32<OT, 64, 64, 8, 4>(p, st);
     else launch_f32<OT, 32, 32, 4, 4>(p, st);
     return 0;
 }
@@ -454,6 +459,22 @@ __global__ void __launch_bounds__(128) gemm_any_mma_kernel(AnyP p) {
 bool gemm_grouped_ok(const p3_gemm_any_args* a);               // gemm_tc.cu
 int launch_gemm_grouped(const p3_gemm_any_args* a, cudaStream_t st);
 
+static AnyP any_params(const p3_gemm_any_args* a) {
+    AnyP p{a->X, a->ldx, a->x_rows, a->x_row_div, a->W, a->ldw, a->w_group_stride, a->bias, a->bias_group_stride,
+           a->out, a->ldo, a->M, a->N, a->K, a->seg_offsets, a->seg_offsets ? a->n_groups : 1,
+           a->n_batch > 1 ? a->n_batch : 1, a->x_batch_stride, a->w_batch_stride, a->out_batch_stride, a->gate, a->ld_gate};
+    if (p.nb == 1) p.x_bs = p.w_bs = p.o_bs = 0;
+    return p;
+}
+static bool aligned_f32(const p3_gemm_any_args* a, int nb) {
+    return a->x_f32 && a->K % 4 == 0 && a->ldx % 4 == 0 && a->ldw % 4 == 0 && a->w_group_stride % 4 == 0 &&
+           (nb == 1 || (a->x_batch_stride % 4 == 0 && a->w_batch_stride % 4 == 0)) && (((uintptr_t)a->X | (uintptr_t)a->W) & 15) == 0;
+}
+extern "C" int p3_gemm_any_tile(const p3_gemm_any_args* a) {
+    const AnyP p = any_params(a);
+    return aligned_f32(a, p.nb) ? f32_tile(p) : 0;
+}
+
 extern "C" int p3_gemm_any(const p3_gemm_any_args* a, cudaStream_t st) {
     P3_CHECK_ARG(a && a->X && a->W && a->out, "gemm_any: null operand");
     P3_CHECK_ARG(a->M >= 0 && a->N >= 1 && a->K >= 1 && a->M < (1ll << 30), "gemm_any: bad sizes");
@@ -462,16 +483,12 @@ extern "C" int p3_gemm_any(const p3_gemm_any_args* a, cudaStream_t st) {
     P3_CHECK_ARG(a->x_f32 == a->w_f32, "gemm_any: X and W must have the same element type");
     if (a->M == 0) return 0;
     if (gemm_grouped_ok(a)) return launch_gemm_grouped(a, st);
-    AnyP p{a->X, a->ldx, a->x_rows, a->x_row_div, a->W, a->ldw, a->w_group_stride, a->bias, a->bias_group_stride,
-           a->out, a->ldo, a->M, a->N, a->K, a->seg_offsets, a->seg_offsets ? a->n_groups : 1,
-           a->n_batch > 1 ? a->n_batch : 1, a->x_batch_stride, a->w_batch_stride, a->out_batch_stride, a->gate, a->ld_gate};
+    const AnyP p = any_params(a);
     const int nb = p.nb;
     P3_CHECK_ARG(nb <= 65535, "gemm_any: too many products in a batch");
-    if (nb == 1) p.x_bs = p.w_bs = p.o_bs = 0;
     const unsigned mt = (unsigned)((a->M + BM - 1) / BM) + (a->seg_offsets ? (unsigned)a->n_groups : 0u);
     const dim3 grid(mt * (unsigned)nb, (unsigned)((a->N + BN - 1) / BN));
-    const bool vec = a->x_f32 && a->K % 4 == 0 && a->ldx % 4 == 0 && a->ldw % 4 == 0 && a->w_group_stride % 4 == 0 &&
-                     (nb == 1 || (a->x_batch_stride % 4 == 0 && a->w_batch_stride % 4 == 0)) && (((uintptr_t)a->X | (uintptr_t)a->W) & 15) == 0;
+    const bool vec = aligned_f32(a, nb);
     if (vec) {
         const int rc = a->out_f32 ? dispatch_f32<float>(p, st) : dispatch_f32<bf16>(p, st);
         if (rc) return rc;

@@ -1,5 +1,7 @@
 """Kernels behind a dispatch by size, at the sizes where each can go wrong: edges of tiles, remainders, the smallest and the largest of
 its range. Needs the built library and a B200."""
+import ctypes
+
 import pytest
 import torch
 
@@ -19,7 +21,7 @@ def _stream():
     return torch.cuda.current_stream().cuda_stream
 
 
-def _gemm_any(x, w, bias=None, rows=None, seg=None, gate=None, out_dtype=F32, batch=None, N=None, K=None):
+def _gemm_any(x, w, bias=None, rows=None, seg=None, gate=None, out_dtype=F32, batch=None, N=None, K=None, tiles=None):
     from phi3_b200 import _lib
     M, n = (rows.numel() if rows is not None else x.shape[0]), (w.shape[-2] if N is None else N)
     out = torch.full((M, n * (batch[0] if batch else 1)), float('nan'), dtype=out_dtype, device=x.device)
@@ -32,6 +34,8 @@ def _gemm_any(x, w, bias=None, rows=None, seg=None, gate=None, out_dtype=F32, ba
         a.n_batch, a.x_batch_stride, a.w_batch_stride, a.out_batch_stride = batch
     if gate is not None:
         a.gate, a.ld_gate = gate.data_ptr(), gate.stride(0)
+    if tiles is not None:
+        tiles.append(_lib.lib().p3_gemm_any_tile(ctypes.addressof(a)))
     _lib.call_struct('p3_gemm_any', a, _stream())
     return out
 
@@ -43,11 +47,15 @@ def _odd_pitch(t):
     return out[..., :t.shape[-1]]
 
 
-@pytest.mark.parametrize('M,N,K', [(1, 1, 4), (1, 33, 8), (2, 16, 128), (3, 47, 132), (5, 100, 100), (8, 17, 260), (9, 64, 640), (16, 130, 1000),
-                                   (17, 31, 16), (31, 33, 20), (33, 64, 12), (63, 129, 36), (65, 65, 260), (130, 1601, 64), (257, 200, 1000),
-                                   (700, 1700, 44), (1100, 2050, 16)])
-def test_fp32_products_of_aligned_rows_have_the_bits_of_the_general_kernel(dev, M, N, K):
+@pytest.mark.parametrize('tile,M,N,K', [(16, 1, 1, 4), (16, 1, 33, 8), (16, 2, 16, 128), (16, 3, 47, 132), (16, 5, 100, 100), (16, 8, 17, 260), (16, 9, 64, 640),
+                                        (16, 16, 130, 1000), (32, 17, 31, 16), (32, 31, 33, 20), (32, 33, 64, 12), (32, 63, 129, 36), (32, 65, 65, 260),
+                                        (32, 130, 1601, 64), (32, 257, 200, 1000), (64, 700, 1700, 44), (64, 1100, 2050, 16), (128, 1097, 4090, 36),
+                                        (128, 1025, 4084, 16), (128, 1100, 4095, 260)])
+def test_fp32_products_of_aligned_rows_have_the_bits_of_the_general_kernel(dev, tile, M, N, K):
     """every tile (rows 1 .. 16, 32, 64, 128) sums one FMA chain in ascending k: the bits of the kernel that takes any alignment"""
+    tiles = []
+    _gemm_any(torch.zeros(M, K, device=dev), torch.zeros(N, K, device=dev), tiles=tiles)
+    assert tiles == [tile]
     g = torch.Generator(device=dev).manual_seed(M * 7 + N)
     rn = lambda *s: torch.randn(s, generator=g, device=dev)
     x, w, bias, gate = rn(M, K), rn(N, K), rn(N), rn(M, N)
@@ -59,17 +67,18 @@ def test_fp32_products_of_aligned_rows_have_the_bits_of_the_general_kernel(dev, 
     assert ((_gemm_any(x, w).double() - y).abs() <= bound).all()
 
 
-@pytest.mark.parametrize('cuts', [[0, 0, 1, 1, 40], [0, 64, 65, 200, 200], [0, 500, 500, 501, 1200]])
-def test_fp32_grouped_gathered_and_batched_products(dev, cuts):
+@pytest.mark.parametrize('cuts,N,tile', [([0, 0, 1, 1, 40], 72, 32), ([0, 64, 65, 200, 200], 72, 32), ([0, 500, 500, 501, 1200], 72, 32),
+                                         ([0, 129, 130, 257, 450], 3000, 128), ([0, 300, 300, 1200, 1450], 1100, 128)])
+def test_fp32_grouped_gathered_and_batched_products(dev, cuts, N, tile):
     g = torch.Generator(device=dev).manual_seed(cuts[-1])
     rn = lambda *s: torch.randn(s, generator=g, device=dev)
-    M, N, K = cuts[-1], 72, 52
+    M, K, tiles = cuts[-1], 52, []
     x, w = rn(300, K), rn(4, N, K)
     rows = torch.randint(0, 300, (M,), generator=g, device=dev, dtype=torch.int32)
     seg = torch.tensor(cuts, dtype=torch.int32, device=dev)
-    got, ref = _gemm_any(x, w, rows=rows, seg=seg), _gemm_any(_odd_pitch(x), _odd_pitch(w), rows=rows, seg=seg)
-    assert torch.equal(got, ref) and bool(torch.isfinite(got).all())
-    for m in (1, 7, 16, 40, 200):                                   # three products over column blocks, gathered rows
+    got, ref = _gemm_any(x, w, rows=rows, seg=seg, tiles=tiles), _gemm_any(_odd_pitch(x), _odd_pitch(w), rows=rows, seg=seg, tiles=tiles)
+    assert tiles == [tile, 0] and torch.equal(got, ref) and bool(torch.isfinite(got).all())
+    for m in (1, 7, 16, 40, 200, 520 if N > 1000 else 33):          # three products over column blocks, gathered rows
         xb, wb, r = rn(300, 3 * K), rn(3, N, K), rows[:1].repeat(m) if m > M else rows[:m].contiguous()
         got = _gemm_any(xb, wb, rows=r, batch=(3, K, N * K, N), N=N, K=K)
         ref = torch.cat([_gemm_any(_odd_pitch(xb[:, i * K:(i + 1) * K]), _odd_pitch(wb[i]), rows=r) for i in range(3)], 1)
@@ -108,11 +117,13 @@ def test_expert_order_is_stable(dev, n, E):
     assert seg.tolist() == [int((ids < e).sum()) for e in range(E + 1)]
 
 
-@pytest.mark.parametrize('M,N,K', [(781, 3072, 200), (1030, 2056, 136), (2885, 1000, 72), (2560, 1984, 64), (5418, 3088, 128), (257, 9216, 64), (300, 19000, 72)])
-def test_products_of_cta_pairs_at_every_tile_width(dev, M, N, K):
+@pytest.mark.parametrize('width,M,N,K', [(192, 781, 3072, 200), (160, 1030, 2056, 136), (192, 2885, 1000, 72), (160, 2560, 1984, 64), (256, 5418, 3088, 128),
+                                         (256, 257, 9216, 64), (192, 300, 19000, 72), (224, 1030, 3064, 136), (224, 1025, 2885, 64)])
+def test_products_of_cta_pairs_at_every_tile_width(dev, width, M, N, K):
     """rows and columns that end inside a tile of each width; every output is the sum of the single-CTA kernel's k order, in fp32: 2^-20 of the
     sum of magnitudes, and 2^-8 for the bf16 result"""
     from phi3_b200 import _lib
+    assert _lib.lib().p3_gemm_pair_width(M, N) == width
     g = torch.Generator(device=dev).manual_seed(N)
     x, w, b = (torch.randn(*s, generator=g, device=dev).to(B16) for s in ((M, K), (N, K), (N,)))
     y, bound = x.double() @ w.double().T + b.double(), 2.0 ** -20 * (x.double().abs() @ w.double().abs().T + b.double().abs())
@@ -346,3 +357,27 @@ def test_an_expert_layer_is_its_launches_and_three_allocations(dev, tokens):
             p = gu[ids[t, j]].double() @ x[t].double()
             ref[t] += wts[t, j].double() * (down[ids[t, j]].double() @ (torch.nn.functional.silu(p[:F]) * p[F:]))
     assert (y.double() - ref).abs().max() <= 2.0 ** -7 * ref.abs().max()
+
+
+@pytest.mark.parametrize('width,nh', [(192, 8), (224, 10)])
+def test_rotary_products_at_narrow_tiles(dev, width, nh):
+    """the rotated q / k / v rows and the cache pages of a product whose pair tiles are narrower than 256: bit for bit what the plain product and
+    the rotation kernel leave"""
+    from phi3_b200 import _lib
+    L, hd, K = 1030, 96, 136
+    N = 3 * nh * hd
+    assert _lib.lib().p3_gemm_pair_width(L, N) == width
+    g = torch.Generator(device=dev).manual_seed(nh)
+    rn = lambda *s: torch.randn(s, generator=g, device=dev)
+    x, w, cos, sin = rn(L, K).to(B16), (rn(N, K) * 0.05).to(B16), rn(1, L, hd // 2), rn(1, L, hd // 2)
+    pages = -(-L // 64)
+    bt = torch.randperm(pages, generator=g, device=dev).to(torch.int32)[None].contiguous()
+    ref, got = (torch.zeros(L, N, dtype=B16, device=dev) for _ in range(2))
+    pool_ref, pool = (torch.zeros(pages, 2, nh, 64, hd, dtype=B16, device=dev) for _ in range(2))
+    _lib.call('p3_gemm', x.data_ptr(), K, w.data_ptr(), K, None, ref.data_ptr(), N, None, None, L, N, K, _lib.EPI_NONE, 0, _stream())
+    _lib.call('p3_rope_kvwrite', ref.data_ptr(), cos.data_ptr(), sin.data_ptr(), cos.stride(0), 1, L, nh, nh, hd, 0, 1, pool_ref.data_ptr(), bt.data_ptr(),
+              bt.stride(0), 1, None, _stream())
+    order = [h * hd + half + 16 * j + i for h in range(2 * nh) for j in range(hd // 32) for half in (0, hd // 2) for i in range(16)] + list(range(2 * nh * hd, N))
+    _fused(x, w[torch.tensor(order, device=dev)].contiguous(), got, _lib.EPI_ROPE_KV, cosT=cos, sinT=sin, tab_bstride=cos.stride(0), L=L, n_heads=nh, n_kv=nh,
+           hd=hd, past=0, row_div=1, write_cache=1, bt_stride=bt.stride(0), pool=pool, block_table=bt)
+    assert torch.equal(got, ref) and torch.equal(pool, pool_ref)

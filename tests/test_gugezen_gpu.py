@@ -351,8 +351,8 @@ def test_stacks_of_one_kind_and_layers_that_share_tensors(lib):
 
 
 def test_large_steps_take_the_dense_expert_products_and_the_second_stream(lib):
-    """prompt steps of several hundred rows: experts as per-expert products (segment offsets read back), the two halves of a parallel mixer
-    on two streams; the same rows through the small-batch paths"""
+    """prompt steps of several hundred rows: experts as grouped tcgen05 products over rows in expert order, the two halves of a parallel mixer
+    on two streams; the same rows on one stream, with the experts on the mma.sync kernel that gathers the rows itself"""
     configs, weights, engine, gugezen, paged, O = _mods()
     width, kw, layers = OTHER['tiled']
     cfg = configs.tiny_gugezen(width=width, vocab=256, layers=layers, **kw)
@@ -371,7 +371,7 @@ def test_large_steps_take_the_dense_expert_products_and_the_second_stream(lib):
             if ref is not None:
                 assert_close(big[o:o + len(t)], ref, B16, k)
             o += len(t)
-    model.moe_dense_rows, model.SIDE_ROWS = 1 << 30, 1 << 30
+    model.use_tc, model.SIDE_ROWS = False, 1 << 30
     assert_close(big[:410], run_schedule(model, toks['a'], [410], max_tokens=512), B16)
     m32, _ = make(cfg, F32, seed=15)                          # fp32: the second stream alone
     assert rel_err(run_schedule(m32, toks['b'], [300], max_tokens=320), O.forward(cfg, w, toks['b'], torch.float64)) < TOL[F32]

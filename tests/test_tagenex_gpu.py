@@ -552,14 +552,16 @@ def test_router_sort_grouped_products_and_combine(lib, dtype):
 
 
 def test_experts_as_dense_products_equal_the_grouped_kernel(lib):
-    """large batches run every expert's rows through the tensor-core GEMM over gathered activations (segment offsets read back);
-    forced here for a small batch and compared with the device-side grouped kernel and the oracle"""
+    """the experts' rows in expert order through the grouped tcgen05 product, compared with the mma.sync kernel that gathers the rows itself
+    (both products of the layer on it: P3_LM_TC=0) and with the oracle"""
     configs, weights, engine, tagenex, paged, O = _mods()
     cfg = configs.tiny_tagenex()
     model, w = make(cfg, B16, seed=17)
     toks = tokens(150, cfg['vocab'], 18)
+    model.use_tc = False
     grouped = run_schedule(model, toks, [150])
-    model.moe_dense_rows = 1
+    model.use_tc = True
+    assert all(model.experts_dense(l.ff, 150) for l in model.cfg.layers if l.ff is not None and l.ff.kind == 'moe')
     dense = run_schedule(model, toks, [150])
     assert_close(dense, grouped, B16)
     assert_close(dense, O.forward(cfg, w, toks, torch.float64), B16)
