@@ -384,7 +384,6 @@ __device__ __forceinline__ void epi_rows32(const GemmEpi& ep, uint8_t* sb, int r
         uint4 next[4];
         if (resid) epi_resid(ep, row0, m_end, n1, N, 0, next);
         rows_put(sb, lane, ov);
-        float4 sq[4];                                          // per row and pair of columns: squares of the bf16 values just written
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int row = row0 + 8 * i + sub;
@@ -396,15 +395,14 @@ __device__ __forceinline__ void epi_rows32(const GemmEpi& ep, uint8_t* sb, int r
                 for (int e = 0; e < 4; e++) { const float2 f = unpack_bf16(ru[e]), x = unpack_bf16(w[e]); w[e] = pack_bf16(f.x + x.x, f.y + x.y); }
             }
             if (row < m_end) st_out16(out + epi_out_row(ep, row) * ep.ldo + n0 + 8 * part, make_uint4(w[0], w[1], w[2], w[3]), ep.stream_out);
-            float t[4];
+            if (ep.ss_out) {                                   // squares of the bf16 values just written, by pairs of columns, to the place just read ...
+                float t[4];
 #pragma unroll
-            for (int e = 0; e < 4; e++) { const float2 f = unpack_bf16(w[e]); t[e] = f.x * f.x + f.y * f.y; }
-            sq[i] = make_float4(t[0], t[1], t[2], t[3]);
+                for (int e = 0; e < 4; e++) { const float2 f = unpack_bf16(w[e]); t[e] = f.x * f.x + f.y * f.y; }
+                rows_at<float4>(sb, 8 * i + sub, part) = make_float4(t[0], t[1], t[2], t[3]);
+            }
         }
-        if (ep.ss_out) {                                       // back to the row's lane, which adds its 16 pairs from left to right
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 4; i++) rows_at<float4>(sb, 8 * i + sub, part) = sq[i];
+        if (ep.ss_out) {                                       // ... and so back to the row's lane, which adds its 16 pairs from left to right
             __syncwarp();
             float s = 0.f;
 #pragma unroll
@@ -625,7 +623,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     if (on0 < N / 2) {
                         uint4 ov[4];
                         uint32_t* ou = reinterpret_cast<uint32_t*>(ov);
-                        if (row_ok)                            // not for rows that do not exist, whose zeros divide slowly (297 rows: 50 us, 41 so)
+                        // rows that do not exist: their zeros would divide slowly (297 rows: 50 us, 41 so; as a branch around the units it cost
+                        // the kernel's other epilogues 2 %)
+#pragma unroll
+                        for (int i = 0; i < 32; i++) g[i] = row_ok ? g[i] : __float_as_uint(1.f);
 #pragma unroll
                         for (int i = 0; i < 16; i++) {
                             float g0 = bf16_round(__uint_as_float(g[2 * i]) * rs), g1 = bf16_round(__uint_as_float(g[2 * i + 1]) * rs);
@@ -859,7 +860,10 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     if (on0 < N / 2) {
                         uint4 ov[4];
                         uint32_t* ou = reinterpret_cast<uint32_t*>(ov);
-                        if (row_ok)                            // not for rows that do not exist, whose zeros divide slowly (297 rows: 50 us, 41 so)
+                        // rows that do not exist: their zeros would divide slowly (297 rows: 50 us, 41 so; as a branch around the units it cost
+                        // the kernel's other epilogues 2 %)
+#pragma unroll
+                        for (int i = 0; i < 32; i++) g[i] = row_ok ? g[i] : __float_as_uint(1.f);
 #pragma unroll
                         for (int i = 0; i < 16; i++) {
                             float g0 = bf16_round(__uint_as_float(g[2 * i]) * rs), g1 = bf16_round(__uint_as_float(g[2 * i + 1]) * rs);
