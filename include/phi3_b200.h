@@ -327,7 +327,8 @@ int p3_decode_mega(const p3_mega_args* args, cudaStream_t st);
  * [page][kv head][P3_PAGE_TOKENS][dim | vdim]; block_table int32 [sequence slot][bt_stride] of page ids. */
 
 /* out[M,N] = X[M,K] W[N,K]^T + bias for any sizes / strides / alignment; X and W both fp32 (FMA pipes, no TF32) or both bf16
- * (mma.sync when K, ldx, ldw are multiples of 8 and the bases 16-byte aligned, else FMA); fp32 accumulation in ascending k.
+ * (mma.sync when K, ldx, ldw are multiples of 8 and the bases 16-byte aligned, else FMA); fp32 accumulation in ascending k. Grouped bf16
+ * products of such rows without gather, bias or gate, pitches at least K, run on tcgen05 with the groups found on the device.
  * x_rows (may be NULL): row r reads X[x_rows[r] / x_row_div]. seg_offsets (device int32 [n_groups + 1], may be NULL): rows
  * [seg[g], seg[g+1]) multiply with W + g * w_group_stride and add bias + g * bias_group_stride (grouped expert product; M is
  * then the total row count = seg[n_groups]). bias fp32 or NULL.
