@@ -326,7 +326,8 @@ int p3_decode_mega(const p3_mega_args* args, cudaStream_t st);
  * norms, softmax, router and residual sums are fp32 in both. One K pool and one V pool per layer:
  * [page][kv head][P3_PAGE_TOKENS][dim | vdim]; block_table int32 [sequence slot][bt_stride] of page ids. */
 
-/* out[M,N] = X[M,K] W[N,K]^T + bias for any sizes / strides / alignment; X and W both fp32 (FMA pipes, no TF32) or both bf16
+/* out[M,N] = X[M,K] W[N,K]^T + bias for any sizes / strides / alignment; X and W both fp32 (no TF32: FMA pipes, or exact
+ * splits into bf16 parts on tcgen05 from M = 17, N = 256, K = 512 on) or both bf16
  * (mma.sync when K, ldx, ldw are multiples of 8 and the bases 16-byte aligned, else FMA); fp32 accumulation in ascending k. Grouped bf16
  * products of such rows without gather, bias or gate, pitches at least K, run on tcgen05 with the groups found on the device.
  * x_rows (may be NULL): row r reads X[x_rows[r] / x_row_div]. seg_offsets (device int32 [n_groups + 1], may be NULL): rows
@@ -342,12 +343,13 @@ typedef struct {
     void* out; int64_t ldo; int32_t out_f32;
     int64_t M; int32_t N, K;
     const int32_t* seg_offsets; int32_t n_groups;
-    int32_t force_fma;           /* 2: not on tcgen05 (grouped products on mma.sync); else not 0: bf16 operands on the FMA kernel (tests) */
+    int32_t force_fma;           /* 2: not on tcgen05 (grouped products on mma.sync, fp32 on FMA tiles); else not 0: bf16 operands on the FMA kernel too (tests) */
     int32_t n_batch; int64_t x_batch_stride, w_batch_stride, out_batch_stride;
     const float* gate; int64_t ld_gate;
 } p3_gemm_any_args;
 int p3_gemm_any(const p3_gemm_any_args* args, cudaStream_t st);
-/* rows of the tile that an fp32 product runs on: 16 (the stream of W for up to 16 rows), 32, 64 or 128; 0: the kernel for any alignment, or bf16 */
+/* rows of the tile that an fp32 product runs on: 16 (the stream of W for up to 16 rows), 32, 64 or 128; -32, -64 or -96: on tcgen05, 128 rows by so
+ * many columns; 0: the kernel for any alignment, or bf16 */
 int p3_gemm_any_tile(const p3_gemm_any_args* args);
 
 /* x fp32 [T,W] = table[ids] * scale (bf16 table); x_act (may be NULL; row pitch ld_act) receives the same rows in the activation

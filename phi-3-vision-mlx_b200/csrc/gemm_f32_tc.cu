@@ -1,0 +1,348 @@
+// fp32 products of p3_gemm_any on the 5th-gen tensor cores, without giving up fp32: an operand x is the sum of three bf16 numbers that hold its
+// 24 bits exactly (the upper 16 bits of x, of what is left, and of what is left then), and of the nine products of such parts the six that reach
+// above 2^-22 of x w are formed. The sum over 64 numbers of k is accumulated in TMEM, smallest products first, so that the accumulator is small
+// but for the last four of its 24 additions; then it is added to the output's running sum in fp32 registers. The tensor cores cut off where
+// fp32 rounds: over all of K in TMEM the error against 64 bits would be 3e-6 of the outputs at K = 3072; in pieces of 64 it is 1.4e-7 .. 1.8e-7
+// (K = 512 .. 3072), one FMA chain over K has 4.0e-7 .. 9.9e-7.
+//
+// One CTA per SM walks output tiles of 128 x BN:
+//   warps 0-15:  a block of 64 numbers of k, read one block ahead into registers, is split and goes to TMEM (X: a row is a TMEM lane) and to shared
+//                memory (W: K-major, 128B swizzle); three stages. With X in TMEM a product reads only W from shared memory: with both operands
+//                there, 24 MMAs and the split's stores ask for more than its 128 bytes a clock.
+//   warps 16-23: the sums of a block are read back (two buffers) and added in registers; epilogue
+//   warp 24:     issues the MMAs of a block. A warp that also splits cannot: 24 of them take about 1000 clocks to issue.
+// Bound by the split (five instructions a number, every CTA its own rows of X and W), then by the MMAs: a block of 128 x 96 takes 1.2 us, without
+// the split 1.1, with 4 of 24 MMAs 1.0. 512 x 3072 x 1024: 27 us (FMA kernel 100), 1200 x 4096 x 3072: 175 (723), 64 x 3072 x 1024: 15 (36).
+// Infinities have no parts: a warp that finds something else than a finite number among its sums forms them again, one FMA chain per output.
+#include <type_traits>
+#include "tc_common.cuh"
+#include "gemm_any.cuh"
+#include "../../include/phi3_b200.h"
+
+namespace {
+constexpr int TM_ROWS = 128, KB = 64, STAGES = 3;
+constexpr int SPLIT = 16, ADD = 8, W_ADD = SPLIT, W_MMA = SPLIT + ADD, THREADS = 32 * (W_MMA + 1);
+constexpr int A_COLS = 96;                                   // TMEM columns of one stage of X: three parts of 64 bf16
+constexpr int ACC_COL = STAGES * A_COLS;
+constexpr int TMEM = 512;                                    // 3 x 96 for X, 2 x BN sums
+constexpr size_t f32tc_smem(int bn) { return (size_t)STAGES * 3 * bn * KB * 2 + 1024; }
+
+__device__ __forceinline__ void wait_lim(uint32_t bar, uint32_t parity, volatile int* fail) {
+    uint32_t ok, spins = 0;
+    do {
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (!ok && (++spins & 1023u) == 0) {
+            if (*fail) return;
+            if (spins > (1u << 18)) { *fail = 1; return; }
+        }
+    } while (!ok);
+}
+// 16 TMEM lanes x 8 columns: thread t holds columns 2 (t % 4), + 1 of lane t / 4 in a and of lane t / 4 + 8 in b
+__device__ __forceinline__ void st_16x256b(uint32_t t, const uint32_t (&a)[2], const uint32_t (&b)[2]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x1.b32 [%0], {%1,%2,%3,%4};" ::"r"(t), "r"(a[0]), "r"(a[1]), "r"(b[0]), "r"(b[1]) : "memory");
+}
+__device__ __forceinline__ void ld_32x32b_x8(uint32_t t, uint32_t* v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(t));
+}
+// a - b, two at a time
+__device__ __forceinline__ void sub2(float (&d)[2], const float (&a)[2], const float (&b)[2]) {
+    asm("{\n.reg .b64 x, y, z;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nsub.rn.f32x2 z, x, y;\nmov.b64 {%0, %1}, z;\n}"
+        : "=f"(d[0]), "=f"(d[1]) : "f"(a[0]), "f"(a[1]), "f"(b[0]), "f"(b[1]));
+}
+__device__ __forceinline__ void add2(float& c0, float& c1, float a0, float a1) {
+    asm("{\n.reg .b64 x, y;\nmov.b64 x, {%0, %1};\nmov.b64 y, {%2, %3};\nadd.rn.f32x2 x, x, y;\nmov.b64 {%0, %1}, x;\n}" : "+f"(c0), "+f"(c1) : "f"(a0), "f"(a1));
+}
+__device__ __forceinline__ float upper(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
+__device__ __forceinline__ uint32_t uppers(const float (&x)[2]) { return __byte_perm(__float_as_uint(x[0]), __float_as_uint(x[1]), 0x7632); }
+// four numbers -> three parts of two words each
+__device__ __forceinline__ void split4(const float4& f, uint32_t (&p0)[2], uint32_t (&p1)[2], uint32_t (&p2)[2]) {
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const float x[2] = {i ? f.z : f.x, i ? f.w : f.y}, xh[2] = {upper(x[0]), upper(x[1])};
+        float r[2], s[2];
+        sub2(r, x, xh);
+        const float rh[2] = {upper(r[0]), upper(r[1])};
+        sub2(s, r, rh);
+        p0[i] = uppers(x); p1[i] = uppers(r); p2[i] = uppers(s);
+    }
+}
+
+template <typename OT, int BN>
+__global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_tiles, int n_tiles) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t bars_s[2 * STAGES + 4];
+    __shared__ uint32_t tmem_s;
+    __shared__ int fail_s;
+    volatile int* fail = &fail_s;
+    constexpr int PART = BN * KB * 2, STAGE = 3 * PART;
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u, bars = smem_u32(bars_s);
+    auto full = [&](uint32_t s) { return bars + 8 * s; };                            // a stage is split
+    auto empty = [&](uint32_t s) { return bars + 8 * (STAGES + s); };                // ... and multiplied
+    auto sums = [&](uint32_t s) { return bars + 8 * (2 * STAGES + s); };             // a block's sums are there
+    auto taken = [&](uint32_t s) { return bars + 8 * (2 * STAGES + 2 + s); };        // ... and read
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        fail_s = 0;
+        for (int s = 0; s < STAGES; s++) { mbar_init(full(s), SPLIT); mbar_init(empty(s), 1); }
+        for (int s = 0; s < 2; s++) { mbar_init(sums(s), 1); mbar_init(taken(s), ADD); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == W_MMA) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_s)), "n"(TMEM) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&tmem_s);
+    pdl_trigger();
+    pdl_wait();                                              // memory is touched only after the predecessors are done
+
+    const int tiles = m_tiles * n_tiles, blocks = (p.K + KB - 1) / KB;
+    // rows fastest: the CTAs in flight share columns of W
+    auto find = [&](int tile, int& bz, int& g, int& m0, int& m1) {
+        const int mt = tile % m_tiles;
+        int64_t a, b;
+        bz = mt % p.nb;
+        const bool ok = find_tile<TM_ROWS>(p, mt / p.nb, g, a, b);
+        m0 = (int)a; m1 = (int)b;
+        return ok;
+    };
+    if (warp < SPLIT) {
+        // ---- X: 16 rows and 32 of a block's numbers per warp; W: rows wr, wr + 32, ...
+        const int xr = 32 * (warp & 3) + 16 * ((warp >> 2) & 1) + (lane >> 2), xk = 32 * (warp >> 3) + 4 * (lane & 3);
+        const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3) + 16 * ((warp >> 2) & 1)) << 16) + 16 * (warp >> 3);
+        constexpr int NB = BN / 32;
+        const int wr = threadIdx.x >> 4, wk = 4 * (threadIdx.x & 15);
+        const uint32_t ws = base + wr * 128 + ((((wk >> 3) ^ (wr & 7)) << 4) | ((wk & 4) << 1));
+        const size_t w_step = (size_t)32 * p.ldw;
+        const int whole = p.K / KB;                          // blocks without an end of K inside
+        uint32_t stage = 0, phase = 1;
+        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+            int bz, g, m0, m1;
+            if (!find(tile, bz, g, m0, m1)) continue;
+            const float *xp[2], *wp;                         // rows of the tile, at this thread's numbers of the block to be read next
+            float4 fx[4], fw[NB];
+            const int n0 = tile / m_tiles * BN, n = n0 + wr < p.N ? n0 + wr : n0, w_left = p.N - n;
+            const float* X = (const float*)p.X + (size_t)bz * p.x_bs + xk;
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int m = m0 + xr + 8 * i < m1 ? m0 + xr + 8 * i : m0;
+                xp[i] = X + (size_t)(p.x_rows ? p.x_rows[m] / p.x_row_div : m) * p.ldx;
+            }
+            wp = (const float*)p.W + (size_t)g * p.w_gstride + (size_t)bz * p.w_bs + wk + (size_t)n * p.ldw;
+            // Rows that do not exist are read as the first one: their outputs are not written. Numbers behind K are zeros (`left`: numbers from
+            // the block's first on; K % 4 == 0: four are inside or outside together).
+            auto fetch_x = [&](int i, int left) {            // row xr + 8 (i & 1), numbers 16 (i >> 1) on
+                fx[i] = xk + 16 * (i >> 1) < left ? __ldg(reinterpret_cast<const float4*>(xp[i & 1] + 16 * (i >> 1))) : make_float4(0.f, 0.f, 0.f, 0.f);
+            };
+            auto fetch_w = [&](int i, int left) {
+                fw[i] = wk < left ? __ldg(reinterpret_cast<const float4*>(32 * i < w_left ? wp + i * w_step : wp)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            };
+            auto next = [&]() { xp[0] += KB; xp[1] += KB; wp += KB; };
+#pragma unroll
+            for (int i = 0; i < 4; i++) fetch_x(i, p.K);
+#pragma unroll
+            for (int i = 0; i < NB; i++) fetch_w(i, p.K);
+            next();
+            // block b is split, and block b + 1 read (mode 0: there is none, 1: whole, 2: it may end at K): what is split is read anew at once, so
+            // that the loads of a block have the time of a block
+            auto block = [&](int b, auto mode) {
+                constexpr int MODE = decltype(mode)::value;
+                const int left = MODE == 1 ? KB : p.K - (b + 1) * KB;
+                wait_lim(empty(stage), phase, fail);
+                tc_fence_after();
+#pragma unroll
+                for (int i = 0; i < 4; i += 2) {
+                    uint32_t a0[2], a1[2], a2[2], b0[2], b1[2], b2[2];
+                    split4(fx[i], a0, a1, a2);
+                    if (MODE) fetch_x(i, left);
+                    split4(fx[i + 1], b0, b1, b2);
+                    if (MODE) fetch_x(i + 1, left);
+                    const uint32_t t = ta + stage * A_COLS + 4 * i;
+                    st_16x256b(t, a0, b0); st_16x256b(t + 32, a1, b1); st_16x256b(t + 64, a2, b2);
+                }
+#pragma unroll
+                for (int i = 0; i < NB; i++) {
+                    uint32_t p0[2], p1[2], p2[2];
+                    split4(fw[i], p0, p1, p2);
+                    if (MODE) fetch_w(i, left);
+                    const uint32_t dst = ws + stage * STAGE + i * 32 * 128;
+                    asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(dst), "r"(p0[0]), "r"(p0[1]) : "memory");
+                    asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(dst + PART), "r"(p1[0]), "r"(p1[1]) : "memory");
+                    asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(dst + 2 * PART), "r"(p2[0]), "r"(p2[1]) : "memory");
+                }
+                if (MODE) next();
+                tc_wait_st();
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full(stage));
+                if (++stage == STAGES) { stage = 0; phase ^= 1; }
+            };
+            for (int b = 0; b + 1 < blocks; b++) {
+                if (b + 1 < whole) block(b, std::integral_constant<int, 1>{});
+                else block(b, std::integral_constant<int, 2>{});
+            }
+            block(blocks - 1, std::integral_constant<int, 0>{});
+        }
+    } else if (warp == W_MMA) {
+        constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TM_ROWS >> 4) << 24);
+        const uint64_t wd = umma_desc_sw128(base);
+        uint32_t it = 0, stage = 0, phase = 0;
+        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+            int bz, g, m0, m1;
+            if (!find(tile, bz, g, m0, m1)) continue;
+            for (int b = 0; b < blocks; b++, it++) {
+                wait_lim(taken(it & 1), ((it >> 1) & 1u) ^ 1u, fail);
+                wait_lim(full(stage), phase, fail);
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint32_t d = tmem + ACC_COL + (it & 1) * BN, a = tmem + stage * A_COLS;
+                    const uint64_t w = wd + stage * (STAGE >> 4);
+#pragma unroll
+                    for (int i = 0; i < 24; i++) {           // parts (of X, of W), smallest products first, in four steps of 16 numbers each
+                        constexpr int PX[6] = {2, 0, 1, 1, 0, 0}, PW[6] = {0, 2, 1, 0, 1, 0};
+                        tc_mma_bf16_ts(d, a + 32 * PX[i / 4] + 8 * (i % 4), w + (PW[i / 4] * (PART >> 4) + 2 * (i % 4)), IDESC, i ? 1u : 0u);
+                    }
+                    tc_commit(empty(stage));
+                    tc_commit(sums(it & 1));
+                }
+                __syncwarp();
+                if (++stage == STAGES) { stage = 0; phase ^= 1; }
+            }
+        }
+    } else {
+        // ---- sums: TMEM lanes 32 q .., half of the columns of a tile
+        constexpr int NC = BN / 2;
+        const int q = warp & 3, half = (warp - W_ADD) >> 2;
+        const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16) + ACC_COL + NC * half;
+        uint32_t it = 0;
+        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+            int bz, g, m0, m1;
+            if (!find(tile, bz, g, m0, m1)) continue;
+            float acc[NC];
+#pragma unroll
+            for (int c = 0; c < NC; c++) acc[c] = 0.f;
+            for (int b = 0; b < blocks; b++, it++) {
+                wait_lim(sums(it & 1), (it >> 1) & 1u, fail);
+                tc_fence_after();
+#pragma unroll
+                for (int c0 = 0; c0 < NC; c0 += 8) {
+                    uint32_t v[8];
+                    ld_32x32b_x8(tl + (it & 1) * BN + c0, v);
+                    tc_wait_ld();
+#pragma unroll
+                    for (int c = 0; c < 8; c++) asm volatile("" : "+r"(v[c]));
+#pragma unroll
+                    for (int c = 0; c < 8; c += 2) add2(acc[c0 + c], acc[c0 + c + 1], __uint_as_float(v[c]), __uint_as_float(v[c + 1]));
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(taken(it & 1));
+            }
+            const int row0 = m0 + 32 * q, n0 = tile / m_tiles * BN + NC * half;
+            // infinity less infinity is none of the parts' sums: what is not a number is summed again as one FMA chain
+            float nan = 0.f;
+#pragma unroll
+            for (int c = 0; c < NC; c++) nan = fmaf(acc[c], 0.f, nan);
+            if (__any_sync(0xffffffffu, row0 + lane < m1 && !(nan == 0.f))) {
+                const int m = min(row0 + lane, m1 - 1);
+                const float* x = (const float*)p.X + (size_t)bz * p.x_bs + (size_t)(p.x_rows ? p.x_rows[m] / p.x_row_div : m) * p.ldx;
+                const float* w = (const float*)p.W + (size_t)g * p.w_gstride + (size_t)bz * p.w_bs;
+#pragma unroll
+                for (int c = 0; c < NC; c++) acc[c] = 0.f;
+#pragma unroll 1
+                for (int k = 0; k < p.K; k++) {
+                    const float xv = __ldg(x + k);
+#pragma unroll
+                    for (int c = 0; c < NC; c++) acc[c] = fmaf(xv, __ldg(w + (size_t)min(n0 + c, p.N - 1) * p.ldw + k), acc[c]);
+                }
+            }
+            if (*fail) {
+#pragma unroll
+                for (int c = 0; c < NC; c++) acc[c] = __int_as_float(0x7fc00000);
+            }
+            const float* bias = p.bias ? p.bias + (size_t)g * p.bias_gstride : nullptr;
+            OT* out = (OT*)p.out + (size_t)bz * p.o_bs;
+            const float* gate = p.gate ? p.gate + (size_t)bz * p.o_bs : nullptr;
+            const bool quads = p.ldo % 4 == 0 && p.o_bs % 4 == 0 && ((uintptr_t)p.out) % (4 * sizeof(OT)) == 0;
+            // two neighbouring lanes trade four of eight columns: a store writes 32 bytes of each of 16 rows instead of 16 bytes of 32
+            const bool odd = lane & 1;
+#pragma unroll
+            for (int c = 0; c < NC; c += 8) {
+                float give[4], keep[2][4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) give[e] = __shfl_xor_sync(0xffffffffu, odd ? acc[c + e] : acc[c + 4 + e], 1);
+#pragma unroll
+                for (int e = 0; e < 4; e++) { keep[0][e] = odd ? give[e] : acc[c + e]; keep[1][e] = odd ? acc[c + 4 + e] : give[e]; }
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int m = row0 + (lane & ~1) + h;
+                    const int n = n0 + c + (odd ? 4 : 0);
+                    if (m >= m1 || n >= p.N) continue;
+                    float v[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        v[e] = keep[h][e];
+                        if (n + e >= p.N) continue;
+                        v[e] += bias ? bias[n + e] : 0.f;
+                        if (gate) v[e] *= 1.0f / (1.0f + expf(-gate[(size_t)m * p.ld_gate + n + e]));
+                    }
+                    OT* o = out + (size_t)m * p.ldo + n;
+                    if (quads && n + 3 < p.N) {
+                        if constexpr (sizeof(OT) == 4) *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+                        else *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; e++) if (n + e < p.N) stf(o + e, v[e]);
+                    }
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();                                         // nothing is in flight: every block's sums are read
+    tc_fence_after();
+    if (warp == W_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TMEM) : "memory");
+}
+
+template <typename OT, int BN>
+int launch(const AnyP& p, cudaStream_t st) {
+    static P3DevFlags flags; bool& set = flags.cur();
+    if (!set) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc_kernel<OT, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f32tc_smem(BN));
+        P3_CHECK_ARG(e == cudaSuccess, "gemm_any: shared memory attribute: %s", cudaGetErrorString(e));
+        set = true;
+    }
+    const int64_t m_tiles = ((p.M + TM_ROWS - 1) / TM_ROWS + (p.seg ? p.n_groups : 0)) * p.nb, n_tiles = (p.N + BN - 1) / BN;
+    const int64_t tiles = m_tiles * n_tiles;
+    p3_launch_pdl(gemm_f32_tc_kernel<OT, BN>, dim3((unsigned)(tiles < 148 ? tiles : 148)), dim3(THREADS), f32tc_smem(BN), st, p, (int)m_tiles, (int)n_tiles);
+    return 0;
+}
+template <typename OT>
+int launch_width(const AnyP& p, int bn, cudaStream_t st) {
+    return bn == 32 ? launch<OT, 32>(p, st) : bn == 64 ? launch<OT, 64>(p, st) : launch<OT, 96>(p, st);
+}
+}  // namespace
+
+// Columns of a tile: the width whose busiest SM is done first. Nanoseconds of a block of 64 numbers of k by width, and of a tile beside its blocks
+// (from 17 x 1024 x 512 to 1200 x 4096 x 3072). 128 columns took longer than 96 at every size: the sums no longer fit the registers.
+int gemm_f32_tc_width(const void* any_p) {
+    const AnyP& p = *static_cast<const AnyP*>(any_p);
+    static const int width[3] = {96, 64, 32}, block[3] = {1180, 950, 690};
+    const int64_t m_tiles = ((p.M + TM_ROWS - 1) / TM_ROWS + (p.seg ? p.n_groups / 2 : 0)) * p.nb, blocks = (p.K + KB - 1) / KB;
+    int best = 96;
+    int64_t best_cost = INT64_MAX;
+    for (int i = 0; i < 3; i++) {
+        const int64_t waves = (m_tiles * ((p.N + width[i] - 1) / width[i]) + 147) / 148, cost = waves * (blocks * block[i] + 1500);
+        if (cost < best_cost) { best = width[i]; best_cost = cost; }
+    }
+    return best;
+}
+int launch_gemm_f32_tc(const void* any_p, int out_f32, cudaStream_t st) {
+    const AnyP& p = *static_cast<const AnyP*>(any_p);
+    return out_f32 ? launch_width<float>(p, gemm_f32_tc_width(any_p), st) : launch_width<bf16>(p, gemm_f32_tc_width(any_p), st);
+}

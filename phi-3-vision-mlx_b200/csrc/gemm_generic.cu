@@ -1,52 +1,20 @@
 // p3_gemm_any: out[M,N] = X[M,K] * W[N,K]^T (+ bias) for ANY sizes, strides and alignments, operands fp32 or bf16, fp32
-// accumulation in ascending k (one FMA chain per output element, so a row's result does not depend on which other rows share
-// the launch). Two extras make it the mixture-of-experts workhorse: the rows of X can be gathered through an index list, and
+// accumulation. Two extras make it the mixture-of-experts workhorse: the rows of X can be gathered through an index list, and
 // the rows can be cut into segments that each multiply with their own weight matrix (device-side segment offsets, so the host
 // never learns how many tokens an expert received). A launch can also hold a batch of independent products over column blocks of
 // X and out (one per attention head), with an optional sigmoid gate on the result.
 //
-// fp32 operands run on the FMA pipes (this is the "true 32-bit" path: no TF32): at most 16 rows as a stream of W, more in register tiles, and a
-// plain kernel for rows that are not 16-byte aligned. bf16 operands of aligned shapes run on the
+// fp32 operands keep their 24 bits (no TF32): at most 16 rows as a stream of W, more in register tiles on the FMA pipes, each output one FMA chain
+// in ascending k whatever the tile and the other rows; from 17 rows, 256 columns and K = 512 on as exact splits on the tensor cores
+// (gemm_f32_tc.cu: closer to 64 bits than the chain, and the same bits whatever the tile and the other rows there); a plain kernel for rows
+// that are not 16-byte aligned. bf16 operands of aligned shapes run on the
 // tensor cores through mma.sync m16n8k16 (fp32 accumulators); the dense bf16 projections with K % 8 == 0 go to the tcgen05
 // kernel (p3_gemm) instead — this file is what is left: grouped expert products, fp32, and shapes p3_gemm does not take.
-#include "common.cuh"
+#include "gemm_any.cuh"
 #include "../../include/phi3_b200.h"
 
 namespace {
 constexpr int BM = 64, BN = 64, BK = 16;
-
-struct AnyP {
-    const void* X; int64_t ldx; const int32_t* x_rows; int x_row_div;
-    const void* W; int64_t ldw; int64_t w_gstride;
-    const float* bias; int64_t bias_gstride;
-    void* out; int64_t ldo;
-    int64_t M; int N, K;
-    const int32_t* seg; int n_groups;
-    // a batch of nb products over column blocks of X and out: blockIdx.x = m-tile * nb + product, so that the CTAs in flight
-    // together read whole rows of X and write whole rows of out (neighbouring column blocks) instead of one narrow column each
-    int nb; int64_t x_bs, w_bs, o_bs; const float* gate; int64_t ld_gate;
-};
-
-template <typename T> __device__ __forceinline__ float ldf(const T* p);
-template <> __device__ __forceinline__ float ldf<float>(const float* p) { return __ldg(p); }
-template <> __device__ __forceinline__ float ldf<bf16>(const bf16* p) { return __bfloat162float(*p); }
-template <typename T> __device__ __forceinline__ void stf(T* p, float v);
-template <> __device__ __forceinline__ void stf<float>(float* p, float v) { *p = v; }
-template <> __device__ __forceinline__ void stf<bf16>(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
-
-// which (group, first row, end row) does the m-tile `tile` of TM rows cover? Groups are walked in order; a launch has at most
-// ceil(M / TM) + n_groups tiles, surplus CTAs leave.
-template <int TM = BM>
-__device__ __forceinline__ bool find_tile(const AnyP& p, int tile, int& g, int64_t& m0, int64_t& m1) {
-    if (!p.seg) { g = 0; m0 = (int64_t)tile * TM; m1 = p.M; return m0 < m1; }
-    int t = tile;
-    for (int e = 0; e < p.n_groups; e++) {
-        const int a = p.seg[e], b = p.seg[e + 1], nt = (b - a + TM - 1) / TM;
-        if (t < nt) { g = e; m0 = a + (int64_t)t * TM; m1 = b; return true; }
-        t -= nt;
-    }
-    return false;
-}
 
 template <typename XT, typename WT, typename OT>
 __global__ void __launch_bounds__(256) gemm_any_fma_kernel(AnyP p) {
@@ -56,7 +24,7 @@ __global__ void __launch_bounds__(256) gemm_any_fma_kernel(AnyP p) {
     __shared__ __align__(16) float Bs[BK][BN + 4];
     int g; int64_t m0, m1;
     const int bz = blockIdx.x % p.nb;
-    if (!find_tile(p, blockIdx.x / p.nb, g, m0, m1)) return;
+    if (!find_tile<BM>(p, blockIdx.x / p.nb, g, m0, m1)) return;
     const int n0 = blockIdx.y * BN, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const XT* X = (const XT*)p.X + (size_t)bz * p.x_bs;
     const WT* W = (const WT*)p.W + (size_t)g * p.w_gstride + (size_t)bz * p.w_bs;
@@ -363,7 +331,7 @@ __global__ void __launch_bounds__(128) gemm_any_mma_kernel(AnyP p) {
     __shared__ __align__(16) bf16 Bs[BN][TK + 8];
     int g; int64_t m0, m1;
     const int bz = blockIdx.x % p.nb;
-    if (!find_tile(p, blockIdx.x / p.nb, g, m0, m1)) return;
+    if (!find_tile<BM>(p, blockIdx.x / p.nb, g, m0, m1)) return;
     const int n0 = blockIdx.y * BN, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
     const bf16* X = (const bf16*)p.X + (size_t)bz * p.x_bs;
@@ -458,6 +426,8 @@ __global__ void __launch_bounds__(128) gemm_any_mma_kernel(AnyP p) {
 
 bool gemm_grouped_ok(const p3_gemm_any_args* a);               // gemm_tc.cu
 int launch_gemm_grouped(const p3_gemm_any_args* a, cudaStream_t st);
+int gemm_f32_tc_width(const void* any_p);                      // gemm_f32_tc.cu
+int launch_gemm_f32_tc(const void* any_p, int out_f32, cudaStream_t st);
 
 static AnyP any_params(const p3_gemm_any_args* a) {
     AnyP p{a->X, a->ldx, a->x_rows, a->x_row_div, a->W, a->ldw, a->w_group_stride, a->bias, a->bias_group_stride,
@@ -470,9 +440,16 @@ static bool aligned_f32(const p3_gemm_any_args* a, int nb) {
     return a->x_f32 && a->K % 4 == 0 && a->ldx % 4 == 0 && a->ldw % 4 == 0 && a->w_group_stride % 4 == 0 &&
            (nb == 1 || (a->x_batch_stride % 4 == 0 && a->w_batch_stride % 4 == 0)) && (((uintptr_t)a->X | (uintptr_t)a->W) & 15) == 0;
 }
+// fp32 on the tensor cores (gemm_f32_tc.cu): from 17 rows on at every size timed (17 x 1024 x 512: 9 us, 17 on the FMA tiles; 512 x 3072 x 1024: 27
+// and 100). Below 512 numbers of k or 256 columns a product stays one FMA chain, the bits of the kernel for any alignment: gates, routers,
+// low ranks, products per head.
+static bool f32_tc(const p3_gemm_any_args* a, const AnyP& p) {
+    const int64_t tiles = ((a->M + 127) / 128 + (a->seg_offsets ? a->n_groups : 0)) * p.nb * (((int64_t)a->N + 31) / 32);
+    return !a->force_fma && a->M > 16 && a->N >= 256 && a->K >= 512 && tiles < (1ll << 30);
+}
 extern "C" int p3_gemm_any_tile(const p3_gemm_any_args* a) {
     const AnyP p = any_params(a);
-    return aligned_f32(a, p.nb) ? f32_tile(p) : 0;
+    return !aligned_f32(a, p.nb) ? 0 : f32_tc(a, p) ? -gemm_f32_tc_width(&p) : f32_tile(p);
 }
 
 extern "C" int p3_gemm_any(const p3_gemm_any_args* a, cudaStream_t st) {
@@ -489,7 +466,9 @@ extern "C" int p3_gemm_any(const p3_gemm_any_args* a, cudaStream_t st) {
     const unsigned mt = (unsigned)((a->M + BM - 1) / BM) + (a->seg_offsets ? (unsigned)a->n_groups : 0u);
     const dim3 grid(mt * (unsigned)nb, (unsigned)((a->N + BN - 1) / BN));
     const bool vec = aligned_f32(a, nb);
-    if (vec) {
+    if (vec && f32_tc(a, p)) {
+        if (launch_gemm_f32_tc(&p, a->out_f32, st)) return -1;
+    } else if (vec) {
         const int rc = a->out_f32 ? dispatch_f32<float>(p, st) : dispatch_f32<bf16>(p, st);
         if (rc) return rc;
     } else if (a->x_f32) {

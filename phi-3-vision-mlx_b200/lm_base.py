@@ -4,7 +4,7 @@ step and the key-slice cost model of the decode attention. A design (tagenex.py,
 gugezen.py) owns its weights and the order of its kernels; it has no cache and no loop of its own.
 
 Matrix products. Dense bf16 products with K % 8 == 0 run on the tcgen05 GEMM (p3_gemm); batches of at most 16 tokens on the
-weight-streaming kernel (p3_gemm_skinny); everything else (fp32 = true 32-bit on the FMA pipes, grouped expert products, products
+weight-streaming kernel (p3_gemm_skinny); everything else (fp32 = true 32-bit, on the FMA pipes or as exact splits on tcgen05, grouped expert products, products
 per attention head over column blocks, odd shapes) on p3_gemm_any.
 """
 import ctypes as C
@@ -41,6 +41,7 @@ class StepBatch:
 
 class PagedLM:
     """base of the engine models: subclasses set self.dev, self.dtype, self.W (width), self.eps and call _init_products()"""
+    use_tc = True                # products on tcgen05 where they can be (P3_LM_TC)
 
     def _init_products(self):
         self.f32 = int(self.dtype == torch.float32)
@@ -143,7 +144,7 @@ class PagedLM:
         a.out, a.ldo, a.out_f32 = ptr(out), out.stride(0), int(out.dtype == torch.float32)
         a.M = x.shape[0] if M is None else M
         a.N, a.K = (w.shape[-2] if N is None else N), (w.shape[-1] if K is None else K)
-        a.seg_offsets, a.n_groups, a.force_fma = ptr(seg), n_groups, 2 if seg is not None and not self.use_tc else 0
+        a.seg_offsets, a.n_groups, a.force_fma = ptr(seg), n_groups, 0 if self.use_tc else 2
         if batch is not None:
             a.n_batch, a.x_batch_stride, a.w_batch_stride, a.out_batch_stride = batch
         if gate is not None:

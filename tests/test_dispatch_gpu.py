@@ -85,6 +85,62 @@ def test_fp32_grouped_gathered_and_batched_products(dev, cuts, N, tile):
         assert torch.equal(got, ref)
 
 
+def _rel(y, ref):
+    return float((y.double() - ref).norm() / ref.norm())
+
+
+@pytest.mark.parametrize('width,M,N,K', [(32, 17, 256, 512), (32, 129, 300, 516), (64, 300, 2056, 1000), (96, 512, 3072, 1024), (96, 1000, 1601, 572), (64, 257, 2053, 1088)])
+def test_fp32_products_on_the_tensor_cores(dev, width, M, N, K):
+    """Rows, columns and numbers that end inside a tile or a block of 64. Of an operand's three parts the second is below 2^-7 and the third below
+    2^-15 of it: the products left out are below 2^-21 of |x| |w|, the additions cut off at most 2^-20 of the sum of magnitudes (24 of a block of
+    64 at 2^-23 of a partial sum that holds 2^-7 of it but for the last four, K / 64 more at 2^-24). The sums are nearer to 64 bits than one
+    FMA chain's, and a row's do not depend on the rows beside it."""
+    g = torch.Generator(device=dev).manual_seed(M + N)
+    rn = lambda *s: torch.randn(s, generator=g, device=dev)
+    x, w, bias, gate, tiles = rn(M, K) * torch.exp(2 * rn(M, K)), rn(N, K), rn(N), rn(M, N), []
+    got, chain = _gemm_any(x, w, tiles=tiles), _gemm_any(_odd_pitch(x), _odd_pitch(w))
+    assert tiles == [-width]
+    y = x.double() @ w.double().T
+    assert ((got.double() - y).abs() <= 3 * 2.0 ** -21 * (x.double().abs() @ w.double().abs().T)).all()
+    assert _rel(got, y) <= _rel(chain, y)
+    assert torch.equal(_gemm_any(x[:17].contiguous(), w), got[:17])
+    full = (got + bias) * torch.sigmoid(gate)
+    assert torch.allclose(_gemm_any(x, w, bias, gate=gate), full, rtol=1e-5, atol=1e-6)
+    assert torch.equal(_gemm_any(x, w, bias, out_dtype=B16), (got + bias).to(B16))
+
+
+def test_fp32_products_on_the_tensor_cores_gathered_grouped_and_batched(dev):
+    g = torch.Generator(device=dev).manual_seed(5)
+    rn = lambda *s: torch.randn(s, generator=g, device=dev)
+    N, K, cuts = 260, 520, [0, 130, 130, 131, 400]
+    x, w = rn(300, K), rn(4, N, K)
+    rows = torch.randint(0, 300, (400,), generator=g, device=dev, dtype=torch.int32)
+    out = _gemm_any(x, w, rows=rows, seg=torch.tensor(cuts, dtype=torch.int32, device=dev))
+    for e in range(4):
+        y = x[rows[cuts[e]:cuts[e + 1]].long()].double() @ w[e].double().T
+        assert y.numel() == 0 or _rel(out[cuts[e]:cuts[e + 1]], y) < 4e-7
+    xb, r = rn(300, 3 * K), rows[:150].contiguous()
+    got = _gemm_any(xb, rn(3, N, K).mul_(0).add_(w[:3]), rows=r, batch=(3, K, N * K, N), N=N, K=K)
+    ref = torch.cat([_gemm_any(xb[:, i * K:(i + 1) * K].contiguous(), w[i], rows=r) for i in range(3)], 1)
+    assert torch.equal(got, ref)
+
+
+def test_fp32_products_on_the_tensor_cores_of_numbers_without_parts(dev):
+    """infinities, what is not a number, the largest and the smallest numbers: as one FMA chain has them"""
+    g = torch.Generator(device=dev).manual_seed(6)
+    x, w = torch.randn(140, 512, generator=g, device=dev), torch.randn(300, 512, generator=g, device=dev)
+    x[3, 5], x[70, 511], x[71, 0], w[200, 9], w[201, 4] = float('inf'), float('-inf'), float('nan'), float('inf'), 0.0
+    w[:150, 5] = w[:150, 5].to(B16).float()                       # parts that are zeros, under an infinity
+    x[10], x[11] = 1e-38 * x[10], 3.4e38 * torch.sign(x[11])
+    w[7], w[8] = 1e-30 * w[7], 0.0
+    got, ref = _gemm_any(x, w), _gemm_any(_odd_pitch(x), _odd_pitch(w))
+    assert torch.equal(torch.isnan(got), torch.isnan(ref)) and torch.equal(torch.isinf(got), torch.isinf(ref))
+    ok = torch.isfinite(ref)
+    assert torch.equal(torch.sign(got[~ok].nan_to_num(0)), torch.sign(ref[~ok].nan_to_num(0)))
+    scale = x.abs().nan_to_num(0, 0, 0).double() @ w.abs().nan_to_num(0, 0, 0).double().T
+    assert ((got - ref).abs()[ok] <= 2.0 ** -14 * scale[ok] + 1e-44).all() and ((got - ref).abs()[12:70][ok[12:70]] <= 2.0 ** -18 * scale[12:70][ok[12:70]]).all()
+
+
 @pytest.mark.parametrize('cuts', [[0, 1], [0, 0, 0, 3, 3], [0, 32, 65, 65, 200], [0, 129, 130, 258, 258], [0, 5, 300, 900, 901, 1500], [0] + [7 * i for i in range(1, 71)]])
 @pytest.mark.parametrize('N,K', [(128, 64), (200, 72), (72, 136), (384, 520)])
 def test_grouped_products_over_ordered_rows(dev, cuts, N, K):
