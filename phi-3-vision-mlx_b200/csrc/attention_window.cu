@@ -14,7 +14,8 @@
 // needs; the sink is folded in as the INITIAL state of the online softmax (running max = sink, denominator = 1, no value).
 //   attn_window_prefill_kernel: one CTA = 32 consecutive query tokens of one sequence x one head, key tiles = whole pages, only
 //                               the pages that hold a visible key are visited
-//   attn_window_prefill_mma_kernel: the same on the tensor cores (bf16 mode, head sizes that tile), 64 query rows per CTA
+//   attn_window_prefill_mma_kernel: the same on the tensor cores (bf16 mode, head sizes that tile), 64 query rows per CTA; sizes up to 128 of
+//                               whole 16-byte pieces run on tcgen05 instead (attention_window_tc.cu)
 //   attn_window_decode_kernel:  one CTA = one single-token request x one K/V head (all of its query heads share the K/V reads)
 //                               x one slice of the visible keys, one key per lane; slices merged by attn_window_merge_kernel
 #include "common.cuh"
@@ -974,10 +975,13 @@ static int launch_decode_mma(const p3_attn_window_args* a, cudaStream_t st) {
 /* rows per tile the launch accepts: 64 on the tensor-core path, 32 otherwise */
 extern "C" int p3_attn_window_tile_rows(const p3_attn_window_args* a) { return (a && prefill_mma_ok(a)) ? 64 : BQ; }
 
+bool attn_window_tc_ok(const p3_attn_window_args* a);          // attention_window_tc.cu
+int launch_attn_window_tc(const p3_attn_window_args* a, cudaStream_t st);
+
 extern "C" int p3_attn_window_prefill(const p3_attn_window_args* a, cudaStream_t st) {
     if (check_args(a, "attn_window_prefill")) return -1;
     if (a->n_tiles == 0) return 0;
-    const int rc = prefill_mma_ok(a) ? launch_prefill_mma(a, st)
+    const int rc = prefill_mma_ok(a) ? (attn_window_tc_ok(a) ? launch_attn_window_tc(a, st) : launch_prefill_mma(a, st))
                  : a->act_f32 ? launch_prefill<float, float>(a, st) : launch_prefill<bf16, bf16>(a, st);
     if (rc) return rc;
     P3_CHECK_LAUNCH("attn_window_prefill");

@@ -1,0 +1,634 @@
+// Windowed / chunked / gated prefill attention over the page pools (the contract of attention_window.cu) on the 5th-gen tensor cores, for
+// bf16 with key sizes and value sizes that are multiples of 16 up to 128.
+//
+// A pass = 128 query rows against the pages of one sequence and K/V head, in two halves of 64 rows; a half is one tile record x one query
+// head. The halves are n_hc query heads of one group x n_tc neighbouring tile records (n_hc n_tc <= 2), so that grouped-query heads share the
+// K/V pages that a CTA stages. Records of different sequences take a pass each. Two CTAs share an SM.
+//   warps 0-3:  softmax, a query row (TMEM lane) per thread. S is double buffered in TMEM, so the scores of the next two pages are computed while
+//               this one is swept, 32 keys at a time; P goes back over the consumed S columns and is the A operand of P.V straight from TMEM.
+//               P is formed against the reference maximum of the pages before (base-2 domain; the sink is the first reference, with a
+//               denominator of 1), so that no weight waits for the page's own maximum: O and l are rescaled when the reference fell 2^8 behind,
+//               and the weights are formed again when it fell 2^64 behind or there was none. Scores, penalties, weights and all sums are fp32, two
+//               per instruction where that goes. The penalties of a warp's 95 distances to a page are staged by the warp, read one page ahead.
+//               A weight is two bf16 numbers, its upper 16 bits and what they leave, and takes part in two products: with one rounded
+//               number the error against 64 bits was 2.4e-3 of the outputs (4 x 2048 tokens, 16 heads of 128 over 4, window 1024), above
+//               the 2.0e-3 of weights against each page's exact maximum; with two it is 1.7e-3.
+//   warp 4:     finds the passes and copies queries and pages (cp.async, the addresses that the mma.sync kernel reads; as 64-column boxes swizzled
+//               for the tensor cores), two stages. No tensor maps: what a map may touch beyond the rows that exist is not asked.
+//               The grid's next CTA that has not started is taken over (cluster launch control): its first pages and scores are under way while
+//               the outputs of this one are written; as CTAs of their own they cost 17 000 clocks beside their pages.
+//   warp 5:     one thread issues the MMAs: O += P(j) V(j), then S(j + 2) = Q K(j + 2)^T into the columns P(j) left
+// Bound by the softmax warps: a page of a CTA takes 3000 clocks with two CTAs on an SM, its 64 exponentials a row alone 1000 of them; the MMAs
+// of both keep the tensor cores busy half of the time. 4 x 2048 tokens, 16 heads of 128 over 4, window 1024, penalties: 112 us (mma.sync 298);
+// 333 rows of 32 x 96 behind 704: 37 (67). With two threads a row and eight warps a CTA 125: a third more instructions.
+//
+// Every wait has a limit: when one runs out the CTA stops waiting, writes NaN and ends.
+#include "tc_common.cuh"
+#include "../../include/phi3_b200.h"
+#include <type_traits>
+
+namespace {
+constexpr float LOG2E = 1.4426950408889634f;
+constexpr int BOX = 64 * 128;                                // bytes of one 64-row x 64-column box
+
+// bounded: a try may rest for up to 10 ms, a wait of 200 of them gives up
+__device__ __forceinline__ void wait_lim(uint32_t bar, uint32_t parity, volatile int* fail) {
+    uint32_t ok, tries = 0;
+    do {
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 10000000;\nselp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (!ok) {
+            if (*fail) return;
+            if (++tries > 200) { *fail = 1; return; }
+        }
+    } while (!ok);
+}
+__device__ __forceinline__ float ex2f(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcpf(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float y;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
+}
+// Two fp32 numbers in a register pair, two operations per instruction. Pairs stay pairs from TMEM to TMEM: packed anew for every operation, a
+// page took four times the instructions.
+typedef uint64_t f2;
+__device__ __forceinline__ f2 pack2(float a, float b) { f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ float2 unpack2(f2 v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) { f2 r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+// 32 columns of the lane, as 16 pairs
+__device__ __forceinline__ void ld32(uint32_t t, f2* v) {
+    asm volatile("{\n.reg .b32 a<32>;\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x32.b32 {a0,a1,a2,a3,a4,a5,a6,a7,a8,a9,a10,a11,a12,a13,a14,a15,a16,a17,a18,a19,a20,a21,a22,a23,a24,a25,a26,"
+                 "a27,a28,a29,a30,a31}, [%16];\n"
+                 "tcgen05.wait::ld.sync.aligned;\n"
+                 "mov.b64 %0,{a0,a1};\nmov.b64 %1,{a2,a3};\nmov.b64 %2,{a4,a5};\nmov.b64 %3,{a6,a7};\nmov.b64 %4,{a8,a9};\nmov.b64 %5,{a10,a11};\n"
+                 "mov.b64 %6,{a12,a13};\nmov.b64 %7,{a14,a15};\nmov.b64 %8,{a16,a17};\nmov.b64 %9,{a18,a19};\nmov.b64 %10,{a20,a21};\n"
+                 "mov.b64 %11,{a22,a23};\nmov.b64 %12,{a24,a25};\nmov.b64 %13,{a26,a27};\nmov.b64 %14,{a28,a29};\nmov.b64 %15,{a30,a31};\n}"
+                 : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]), "=l"(v[4]), "=l"(v[5]), "=l"(v[6]), "=l"(v[7]), "=l"(v[8]), "=l"(v[9]), "=l"(v[10]),
+                   "=l"(v[11]), "=l"(v[12]), "=l"(v[13]), "=l"(v[14]), "=l"(v[15]) : "r"(t));
+}
+__device__ __forceinline__ void ld16(uint32_t t, uint32_t* v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+                   "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]) : "r"(t));
+}
+__device__ __forceinline__ void st16(uint32_t t, const uint32_t* v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n"
+                 "tcgen05.wait::st.sync.aligned;"
+                 ::"r"(t), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
+                   "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+// first position that a query at `pos` sees (kept first tokens aside), as in attention_window.cu
+__device__ __forceinline__ int first_key(const p3_attn_window_args& a, int pos) {
+    int lo = 0;
+    if (a.window > 0) lo = max(lo, pos - a.window + 1);
+    if (a.chunk > 0) lo = max(lo, pos - pos % a.chunk);
+    return lo;
+}
+
+// penalties of a warp's 32 rows against its 32 keys: entry t = distance (first row + 31 - t) to the warp's first key, so that a row's columns are
+// neighbours; four copies shifted by 0 .. 3 entries let every lane read 16-byte pieces, and their pitch keeps a quarter-warp on different banks
+constexpr int PEN_LD = 104;
+
+constexpr int ST = 2;                                        // pages in flight (as many as score buffers)
+constexpr int W_LOAD = 4, W_MMA = 5, THREADS = 192;
+constexpr int TMEM = 256, O_COL = 128;                       // S(buffer) at 64 buffer, O at O_COL
+constexpr int TURN = 2048;                                   // bytes of a warp's block of outputs: 32 rows x 64 bytes
+// Q of up to 2 boxes x 128 rows, K and V pages of up to 2 boxes, penalty slices, blocks of outputs
+size_t win_smem(int kb, int vb) { return (size_t)kb * 2 * BOX + (size_t)ST * (kb + vb) * BOX + 4 * 4 * PEN_LD * 4 + 4 * TURN + 1024; }
+
+// One pass: up to two records of one sequence, found by the loader for the other warps
+struct Pass { int4 rec[2]; int n, lo_pg, n_keep, h0, mine; };  // n: pages (0: no more work); mine: bit i: record i belongs to the pass
+
+template <bool PEN, bool SIG>
+__global__ void __launch_bounds__(THREADS, 2)
+attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(16) Pass pass_s[2];
+    __shared__ __align__(16) uint4 next_s;
+    __shared__ __align__(8) uint64_t bars_s[1 + 4 * ST + 6 + 5];
+    __shared__ int fail_s;
+    __shared__ uint32_t tmem_s;
+    volatile int* fail = &fail_s;
+    const int d = a.dim, dv = a.vdim, kb = (d + 63) / 64, vb = (dv + 63) / 64, rep = a.n_heads / a.n_kv;
+    const uint32_t raw = smem_u32(smem_raw), base = (raw + 1023u) & ~1023u;
+    const uint32_t sQ = base, sK = sQ + kb * 2 * BOX, sV = sK + ST * kb * BOX;
+    const uint32_t pen_off = sV + ST * vb * BOX - raw, turn = raw + pen_off + 4 * 4 * PEN_LD * 4, bars = smem_u32(bars_s);
+    // pages are counted through all passes of the CTA
+    const uint32_t q_full = bars;
+    auto k_full = [&](int p) { return bars + 8u * (1 + (p & 1)); };
+    auto k_empty = [&](int p) { return bars + 8u * (3 + (p & 1)); };
+    auto v_full = [&](int p) { return bars + 8u * (5 + (p & 1)); };
+    auto v_empty = [&](int p) { return bars + 8u * (7 + (p & 1)); };
+    auto s_full = [&](int p) { return bars + 8u * (9 + (p & 1)); };
+    auto sm_done = [&](int p) { return bars + 8u * (11 + (p & 1)); };
+    auto o_done = [&](int p) { return bars + 8u * (13 + (p & 1)); };
+    auto pass_full = [&](int i) { return bars + 8u * (15 + (i & 1)); };
+    auto pass_empty = [&](int i) { return bars + 8u * (17 + (i & 1)); };
+    const uint32_t next_full = bars + 8u * 19;
+    auto ph = [](int p) { return (uint32_t)(p >> 1) & 1u; };
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == W_MMA) {
+        if (lane == 0) {
+            mbar_init(q_full, 32);
+            for (int p = 0; p < 2; p++) {
+                mbar_init(k_full(p), 32); mbar_init(k_empty(p), 1); mbar_init(v_full(p), 32); mbar_init(v_empty(p), 1);
+                mbar_init(s_full(p), 1); mbar_init(o_done(p), 1); mbar_init(sm_done(p), 4);
+                mbar_init(pass_full(p), 1); mbar_init(pass_empty(p), 5);
+            }
+            mbar_init(next_full, 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            fail_s = 0;
+        }
+        __syncwarp();
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_s)), "n"(TMEM) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&tmem_s);
+    pdl_trigger();
+    pdl_wait();                                              // q, the pools, the tile records and `out` belong to earlier kernels until here
+
+    if (warp == W_LOAD) {
+        // A page of one K/V head is one block of memory: lane l of copy i brings its 16-byte piece 32 i + l. The place of a piece in the boxes
+        // (64 columns, pieces swizzled as the UMMA reads them) repeats, 8 or 16 rows on, after `per` copies: a copy costs its instruction
+        // alone (with the place formed for each one the copies of a page took 850 instructions).
+        const int v_ld = a.v_ld > 0 ? a.v_ld : dv;
+        // whole rows, also where a value is the leading part of its key (what comes in behind it is not read)
+        const bool v_whole = v_ld == dv || (a.v_pool == a.k_pool && v_ld == d && kb == vb);
+        auto period = [](int cols) { return cols % 32 == 0 ? cols / 32 : cols / 16; };
+        auto places = [&](uint32_t (&at)[8], int cols) {
+            const int pr = cols / 8, dr = 32 / pr, dc = 32 - dr * pr;        // pieces per row; rows and pieces from one copy to the next
+            int rr = lane / pr, c = lane - rr * pr;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                at[u] = (c >> 3) * BOX + rr * 128 + (((c & 7) ^ (rr & 7)) << 4);
+                rr += dr; c += dc;
+                if (c >= pr) { c -= pr; rr++; }
+            }
+        };
+        uint32_t k_at[8], v_at[8];
+        places(k_at, d);
+        places(v_at, v_whole ? v_ld : dv);
+        auto copy = [&](uint32_t dst, const bf16* src, const uint32_t (&at)[8], int cols, auto per) {
+            constexpr int P = decltype(per)::value;
+            const char* s = reinterpret_cast<const char*>(src) + 16 * lane;
+            const int n_c = cols / 4, step = 256 * P / cols * 128;
+            for (int i = 0; i < n_c; i += P, dst += step, s += 512 * P)
+#pragma unroll
+                for (int u = 0; u < P; u++) cp_async16(dst + at[u], s + 512 * u);
+        };
+        // `bar` hears from every lane when its copies have landed
+        auto stage = [&](uint32_t dst, const bf16* src, const uint32_t (&at)[8], int cols, int per, uint32_t bar) {
+            if (per == 4) copy(dst, src, at, cols, std::integral_constant<int, 4>{});
+            else if (per == 3) copy(dst, src, at, cols, std::integral_constant<int, 3>{});
+            else if (per == 2) copy(dst, src, at, cols, std::integral_constant<int, 2>{});
+            else if (per == 1) copy(dst, src, at, cols, std::integral_constant<int, 1>{});
+            else if (per == 5) copy(dst, src, at, cols, std::integral_constant<int, 5>{});
+            else copy(dst, src, at, cols, std::integral_constant<int, 7>{});
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+        };
+        const int k_per = period(d), v_cols = v_whole ? v_ld : dv, v_per = period(v_cols);
+        const int4* recs = reinterpret_cast<const int4*>(a.tiles);
+        const int hgs = a.n_heads / n_hc, groups = (a.n_tiles + n_tc - 1) / n_tc;
+        int page_0 = 0, passes = 0, taken = 0;           // pages before this pass, passes, CTAs taken over
+        for (int item = blockIdx.x; item >= 0; taken++) {
+            // the grid's next CTA that has not started is taken over after this one: its rows' pages are on the way while these outputs are written
+            if (lane == 0) {
+                mbar_expect_tx(next_full, 16);
+                asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(&next_s)), "r"(next_full) : "memory");
+            }
+            const int grp = groups - 1 - item / hgs, h0 = item % hgs * n_hc, g = h0 / rep, t_end = min(a.n_tiles, (grp + 1) * n_tc);   // later tiles (more keys) first
+            for (int ta = grp * n_tc; ta < t_end; passes++) {
+                // ---- one pass: the records [ta, tb) of one sequence
+                const int4 r0 = recs[grp * n_tc], r1 = recs[min(grp * n_tc + n_tc, t_end) - 1];
+                const int4 own = ta == grp * n_tc ? r0 : r1;
+                const bool both = ta == grp * n_tc && t_end - ta == 2 && r1.z == r0.z;
+                const int first = both ? min(first_key(a, r0.w), first_key(a, r1.w)) : first_key(a, own.w);
+                const int last = both ? max(r0.w + r0.y, r1.w + r1.y) - 1 : own.w + own.y - 1;
+                // pages: those of the kept first tokens before the window's pages, then from the first visible key to the last row's position
+                const int lo_pg = first / 64, n_keep = min((a.keep_first + 63) / 64, lo_pg), n = n_keep + last / 64 - lo_pg + 1;
+                auto page_at = [&](int it) { return it < n_keep ? it : lo_pg + it - n_keep; };
+                const int32_t* bt = a.block_table + (size_t)own.z * a.bt_stride;
+                int page = 0, page1 = bt[page_at(0)];    // ids of pages it, it + 1
+                const int mine = both ? 3 : ta == grp * n_tc ? 1 : 2;
+                if (lane == 0) {
+                    wait_lim(pass_empty(passes), ph(passes) ^ 1u, fail);
+                    Pass& ps = pass_s[passes & 1];
+                    ps.rec[0] = r0; ps.rec[1] = r1; ps.n = n; ps.lo_pg = lo_pg; ps.n_keep = n_keep; ps.h0 = h0; ps.mine = mine;
+                    mbar_arrive(pass_full(passes));
+                }
+                __syncwarp();
+                for (int it = -1; it < n; it++) {        // K one page ahead of V: its stage comes free earlier
+                    const int page2 = it + 2 < n ? bt[page_at(it + 2)] : 0, p = page_0 + it;
+                    if (it + 1 < n) {
+                        wait_lim(k_empty(p + 1), ph(p + 1) ^ 1u, fail);
+                        stage(sK + ((p + 1) & 1) * kb * BOX, (const bf16*)a.k_pool + ((size_t)page1 * a.n_kv + g) * 64 * d, k_at, d, k_per, k_full(p + 1));
+                    }
+                    if (it < 0) {                        // the queries, once the scores of the pass before are there
+                        if (p >= 0) wait_lim(k_empty(p), ph(p), fail);
+                        auto copy_q = [&](auto lanes) {  // lanes per row
+                            constexpr int LPR = decltype(lanes)::value, PER = 32 / LPR;
+                            const int c = lane % LPR, hi = lane / LPR;
+#pragma unroll 1
+                            for (int u = 0; u < 2; u++) {        // a half: one record, one head; rows that it does not have are zeros
+                                const int4 r = u / n_hc ? r1 : r0;
+                                const int left = (8 * c < d && (mine >> (u / n_hc) & 1) ? r.y : 0) - hi;
+                                const bf16* src = (const bf16*)a.q + (size_t)(r.x + hi) * a.ld_q + (size_t)(h0 + u % n_hc) * d + 8 * c;
+                                const uint32_t dst = sQ + (c >> 3) * 2 * BOX + (u * 64 + hi) * 128 + (((c & 7) ^ hi) << 4);
+#pragma unroll
+                                for (int k = 0; k < 2 * LPR; k++, src += (size_t)PER * a.ld_q)
+                                    cp_async16((dst ^ ((k * PER & 7) << 4)) + k * PER * 128, k * PER < left ? src : (const bf16*)a.q, k * PER < left ? 16 : 0);
+                            }
+                        };
+                        if (kb == 2) copy_q(std::integral_constant<int, 16>{}); else copy_q(std::integral_constant<int, 8>{});
+                        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(q_full) : "memory");
+                    } else {
+                        wait_lim(v_empty(p), ph(p) ^ 1u, fail);
+                        const uint32_t dst = sV + (p & 1) * vb * BOX;
+                        const bf16* src = (const bf16*)a.v_pool + ((size_t)page * a.n_kv + g) * 64 * v_ld;
+                        if (v_whole) stage(dst, src, v_at, v_cols, v_per, v_full(p));
+                        else {                           // the leading numbers of longer rows
+                            for (int i = lane; i < 8 * dv; i += 32) {
+                                const int rr = i / (dv / 8), c = i - rr * (dv / 8);
+                                cp_async16(dst + (c >> 3) * BOX + rr * 128 + (((c & 7) ^ (rr & 7)) << 4), src + (size_t)rr * v_ld + 8 * c);
+                            }
+                            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(v_full(p)) : "memory");
+                        }
+                    }
+                    page = page1; page1 = page2;
+                }
+                page_0 += n;
+                ta = both ? t_end : ta + 1;
+            }
+            wait_lim(next_full, taken & 1u, fail);
+            uint32_t more, x = 0;
+            asm volatile("{\n.reg .pred p;\n.reg .b128 h;\nld.shared.b128 h, [%2];\nclusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n"
+                         "selp.u32 %0, 1, 0, p;\nmov.u32 %1, 0;\n@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n}"
+                         : "=r"(more), "=r"(x) : "r"(smem_u32(&next_s)) : "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            item = more && !*fail ? (int)x : -1;
+        }
+        if (lane == 0) {
+            wait_lim(pass_empty(passes), ph(passes) ^ 1u, fail);
+            pass_s[passes & 1].n = 0;
+            mbar_arrive(pass_full(passes));
+        }
+        cp_async_wait<0>();
+        for (int p = max(0, page_0 - ST); p < page_0; p++) {       // nothing is in flight when the CTA ends
+            wait_lim(k_empty(p), ph(p), fail);
+            wait_lim(v_empty(p), ph(p), fail);
+        }
+    } else if (warp == W_MMA) {
+        // MMA issuer: one thread, its products at constant distances from what a page starts from
+        constexpr uint32_t ID = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);
+        const uint32_t id_qk = ID | ((64u >> 3) << 17), id_pv = ID | (1u << 16) | ((uint32_t)(dv >> 3) << 17);
+        // operand descriptors; what changes is added to their address fields (16-byte units)
+        const uint64_t qd = umma_desc_sw128(sQ), kd0 = umma_desc_sw128(sK), vd0 = umma_desc_mn_sw128(sV, BOX, 1024);
+        auto issue = [&](auto steps) {                   // steps of 16 numbers of a key; 0: a number that is not one of the usual
+            constexpr int KS = decltype(steps)::value;
+            const int ks = KS ? KS : d / 16;
+            for (int i = 0, page_0 = 0;; i++) {
+                wait_lim(pass_full(i), ph(i), fail);
+                const int n = *reinterpret_cast<volatile int*>(&pass_s[i & 1].n);
+                mbar_arrive(pass_empty(i));
+                if (n <= 0 || *fail) break;
+                wait_lim(q_full, i & 1, fail);
+                for (int t = 0; t < n + 2; t++) {
+                    const int p = page_0 + t, j = p - 2;
+                    if (t >= 2) wait_lim(v_full(j), ph(j), fail);
+                    if (t < n) wait_lim(k_full(p), ph(p), fail);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the copies, for the tensor cores
+                    if (t >= 2) {                        // O += P(j) V(j)
+                        wait_lim(sm_done(j), ph(j), fail);
+                        tc_fence_after();
+                        const uint32_t o = tmem + O_COL, pc = tmem + (j & 1) * 64;
+                        const uint64_t vd = vd0 + (uint32_t)((j & 1) * vb * (BOX >> 4));
+#pragma unroll
+                        for (int kk = 0; kk < 8; kk++)   // P of keys 0-31 in columns 0-15, of keys 32-63 in columns 32-47; the rest 16 columns on
+                            tc_mma_bf16_ts(o, pc + 16 * (kk >> 2) + 32 * ((kk >> 1) & 1) + 8 * (kk & 1), vd + (kk & 3) * (16 * 128 >> 4), id_pv,
+                                           kk ? 1u : (uint32_t)(t - 2));
+                        tc_commit(o_done(j));
+                        tc_commit(v_empty(j));
+                    }
+                    if (t < n) {                         // S(t) = Q K(t)^T, behind the P.V that reads the same columns
+                        tc_fence_after();
+                        const uint32_t sc = tmem + (p & 1) * 64;
+                        const uint64_t kd = kd0 + (uint32_t)((p & 1) * kb * (BOX >> 4));
+#pragma unroll
+                        for (int kk = 0; kk < 8; kk++)
+                            if (kk < ks) tc_mma_bf16(sc, qd + ((kk >> 2) * (2 * BOX >> 4) + 2 * (kk & 3)), kd + ((kk >> 2) * (BOX >> 4) + 2 * (kk & 3)), id_qk, kk ? 1u : 0u);
+                        tc_commit(s_full(p));
+                        tc_commit(k_empty(p));
+                    }
+                }
+                page_0 += n;
+            }
+        };
+        if (elect_one()) {
+            if (d == 128) issue(std::integral_constant<int, 8>{});
+            else if (d == 96) issue(std::integral_constant<int, 6>{});
+            else if (d == 64) issue(std::integral_constant<int, 4>{});
+            else issue(std::integral_constant<int, 0>{});
+        }
+        __syncwarp();
+    } else {
+        // ---- softmax: 32 rows of one half (one record, one head) per warp, a row per thread
+        const int u = warp >> 1, r0 = (warp & 1) * 32, i = r0 + lane;
+        const uint32_t t_lane = tmem + ((uint32_t)(warp * 32) << 16), t_o = t_lane + O_COL;
+        for (int pass = 0, page_0 = 0;; pass++) {
+            wait_lim(pass_full(pass), ph(pass), fail);
+            const Pass& now = pass_s[pass & 1];
+            const int n = now.n, n_keep = now.n_keep, past_keep = now.lo_pg - now.n_keep, h = now.h0 + u % n_hc;
+            const bool mine = now.mine >> (u / n_hc) & 1;
+            const int4 rec = now.rec[u / n_hc];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(pass_empty(pass));
+            if (n <= 0 || *fail) break;
+            auto page_at = [&](int it) { return it < n_keep ? it : past_keep + it; };
+            const int nq = mine ? rec.y : 0, pos = rec.w + i;
+            const bool row_ok = i < nq;
+            const float scale2 = a.scale * LOG2E, sb2 = SIG ? a.sig_bias[h] * LOG2E : 0.f;
+            const f2 scale22 = SIG && !PEN ? pack2(-scale2, -scale2) : pack2(scale2, scale2), sbias22 = pack2(-sb2, -sb2), one2 = pack2(1.f, 1.f);
+            float m = a.sink ? a.sink[h] * LOG2E : -INFINITY, l = a.sink ? 1.f : 0.f, pend = 1.f;     // pend: what O and l are to be multiplied by
+            const int lo = first_key(a, pos), warp_lo = rec.w + r0, warp_hi = rec.w + min(nq - 1, r0 + 31), lo_hi = first_key(a, max(warp_hi, 0));
+            const bool any_rows = r0 < nq, all_rows = r0 + 32 <= nq;
+            float* ps = reinterpret_cast<float*>(smem_raw + pen_off) + warp * 4 * PEN_LD;
+            const float* pl = ps + ((31 - lane) & 3) * PEN_LD + ((31 - lane) & ~3);          // this lane's copy, column 0
+            float pn[3];
+            auto pen_fetch = [&](int it) {
+                const float* p = a.penalty + (size_t)h * a.n_penalty;
+                const int dist = warp_lo + 31 - page_at(it) * 64 - lane;
+#pragma unroll
+                for (int k = 0; k < 3; k++) pn[k] = p[min(max(dist - 32 * k, 0), a.n_penalty - 1)];
+            };
+            if (PEN) pen_fetch(0);
+            for (int it = 0; it < n; it++) {
+                const int j0 = page_at(it) * 64;
+                const int p = page_0 + it;
+                const uint32_t t_s = t_lane + (p & 1) * 64;
+                if (PEN) {
+                    __syncwarp();                            // the page before is read
+#pragma unroll
+                    for (int k = 0; k < 3; k++) {
+                        const float v = -LOG2E * pn[k];
+#pragma unroll
+                        for (int c = 0; c < 4; c++)
+                            if (k || lane >= c) ps[c * PEN_LD + lane + 32 * k - c] = v;
+                    }
+                    __syncwarp();
+                    if (it + 1 < n) pen_fetch(it + 1);
+                }
+                wait_lim(s_full(p), ph(p), fail);
+                tc_fence_after();
+                auto scale_o = [&](float cf) {
+                    if (it > 0) { wait_lim(o_done(p - 1), ph(p - 1), fail); tc_fence_after(); }
+#pragma unroll 1
+                    for (int c = 0; c < dv; c += 16) {
+                        uint32_t v[16];
+                        ld16(t_o + c, v);
+#pragma unroll
+                        for (int k = 0; k < 16; k++) v[k] = __float_as_uint(__uint_as_float(v[k]) * cf);
+                        st16(t_o + c, v);
+                    }
+                };
+                auto scale_p = [&](float cf) {               // the weights of the page's first 32 keys, which are behind the older reference
+                    uint32_t w[32];
+                    tc_wait_st();
+                    tc_ld32_nowait(t_s, w);
+                    tc_wait_ld();
+                    tc_reg_fence32(w);
+#pragma unroll
+                    for (int k = 0; k < 16; k++) {
+                        const float2 a0 = unpack_bf16(w[k]), a1 = unpack_bf16(w[16 + k]);
+                        const float p0 = (a0.x + a1.x) * cf, p1 = (a0.y + a1.y) * cf;
+                        w[k] = __byte_perm(__float_as_uint(p0), __float_as_uint(p1), 0x7632);
+                        w[16 + k] = pack_bf16(p0 - __uint_as_float(__float_as_uint(p0) & 0xffff0000u), p1 - __uint_as_float(__float_as_uint(p1) & 0xffff0000u));
+                    }
+                    tc_st32_nowait(t_s, w);
+                };
+                // every key of the page is visible to every row of the warp: behind its first row, and its last row still sees it
+                const bool full = all_rows && j0 + 63 <= warp_lo && (j0 >= lo_hi || j0 + 63 < a.keep_first);
+                const bool none = !any_rows || j0 > warp_hi;
+                const bool whole = __all_sync(0xffffffffu, full);
+                float top = -INFINITY;                       // the page's maximum
+                if (!SIG && __any_sync(0xffffffffu, pend != 1.f)) { scale_o(pend); l *= pend; }
+#pragma unroll
+                for (int hf = 0; hf < 2; hf++) {             // 32 keys at a time: a page of 64 scores, penalties and weights did not fit the registers
+                    uint32_t pk[32];                         // their weights: upper 16 bits, then what they leave
+                    if (none) {
+#pragma unroll
+                        for (int k = 0; k < 32; k++) pk[k] = 0u;
+                    } else {
+                        f2 v[16];
+                        ld32(t_s + 32 * hf, v);
+                        if (PEN) {
+#pragma unroll
+                            for (int k = 0; k < 16; k += 2) {
+                                const ulonglong2 pv = *reinterpret_cast<const ulonglong2*>(pl + 32 * hf + 2 * k);
+                                v[k] = fma2(v[k], scale22, pv.x);
+                                v[k + 1] = fma2(v[k + 1], scale22, pv.y);
+                            }
+                        }
+                        if (!whole) {                        // a branch, so that whole pages do without the tests of every key
+                            auto below = [](int n) { return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u; };
+                            const int j = j0 + 32 * hf;
+                            const uint32_t seen = row_ok ? below(pos - j + 1) & (~below(lo - j) | below(a.keep_first - j)) : 0u;
+#pragma unroll
+                            for (int k = 0; k < 16; k++) {
+                                const float2 x = unpack2(v[k]);
+                                v[k] = pack2(seen >> (2 * k) & 1u ? x.x : -INFINITY, seen >> (2 * k + 1) & 1u ? x.y : -INFINITY);
+                            }
+                        }
+                        if (!SIG) {
+                            float mx[2] = {top, -INFINITY};
+#pragma unroll
+                            for (int k = 0; k < 16; k++) { const float2 x = unpack2(v[k]); mx[k & 1] = max3(mx[k & 1], PEN ? x.x : x.x * scale2, PEN ? x.y : x.y * scale2); }
+                            top = fmaxf(mx[0], mx[1]);
+                        }
+                        float ls;
+                        for (;;) {                           // a second time only for a reference that was none, or 2^64 behind
+                            const float mu = SIG || m == -INFINITY ? 0.f : m;
+                            const f2 mu2 = pack2(-mu, -mu);
+                            f2 sA = 0, sB = 0;
+#pragma unroll
+                            for (int k = 0; k < 16; k++) {
+                                const f2 x = v[k];
+                                float2 q;
+                                f2 pp;
+                                if (SIG) {                   // 1 / (1 + 2^-(score + bias)); a masked key gives 1 / inf = 0
+                                    q = unpack2(PEN ? sub2(sbias22, x) : fma2(x, scale22, sbias22));
+                                    q = unpack2(add2(pack2(ex2f(q.x), ex2f(q.y)), one2));
+                                    pp = pack2(rcpf(q.x), rcpf(q.y));
+                                } else {
+                                    q = unpack2(PEN ? add2(x, mu2) : fma2(x, scale22, mu2));
+                                    pp = pack2(ex2f(q.x), ex2f(q.y));
+                                    if (k & 1) sA = add2(sA, pp); else sB = add2(sB, pp);
+                                }
+                                q = unpack2(pp);
+                                pk[k] = __byte_perm(__float_as_uint(q.x), __float_as_uint(q.y), 0x7632);
+                                const float2 r = unpack2(sub2(pp, pp & 0xffff0000ffff0000ull));
+                                pk[16 + k] = pack_bf16(r.x, r.y);
+                            }
+                            const float2 x = unpack2(add2(sA, sB));
+                            ls = x.x + x.y;
+                            if (SIG) break;
+                            const bool redo = m == -INFINITY ? top != -INFINITY : top - m > 64.f;
+                            if (!__any_sync(0xffffffffu, redo)) break;
+                            const float corr = !redo ? 1.f : m == -INFINITY ? 0.f : ex2f(m - top);
+                            if (redo) m = top;
+                            l *= corr;
+                            if (it > 0) scale_o(corr);
+                            if (hf) scale_p(corr);
+                        }
+                        l += ls;
+                    }
+                    tc_st32_nowait(t_s + 32 * hf, pk);
+                }
+                if (!SIG) {
+                    const float grow = top - m;              // not a number (no key yet) compares false
+                    if (grow > 8.f) { pend = ex2f(-grow); m = top; } else pend = 1.f;
+                }
+                tc_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(sm_done(p));
+            }
+            // ---- epilogue: O / l, gates
+            page_0 += n;
+            if (n > 1) wait_lim(o_done(page_0 - 2), ph(page_0 - 2), fail);
+            wait_lim(o_done(page_0 - 1), ph(page_0 - 1), fail);
+            tc_fence_after();
+            if (mine && any_rows) {
+                float inv = (a.gate && row_ok ? a.gate[((size_t)rec.x + i) * a.n_heads + h] : 1.f) * (a.out_scale != 0.f ? a.out_scale : 1.f);
+                if (!SIG) inv = l > 0.f ? inv / l : 0.f;
+                if (*fail) inv = __int_as_float(0x7fc00000);
+                // row-wise out of TMEM into the warp's block, and from there in pieces of 64 bytes of a row (32 with gates: four lanes a row, eight
+                // rows an instruction) to memory; a lane writing its own row took an instruction of the load-store unit per row and 16 bytes.
+                // 16-byte pieces are swizzled: no bank conflicts either way. Without element-wise gates 32 columns go as bf16, else 16 as fp32.
+                const uint32_t tb = turn + warp * TURN;
+                const int sub = lane >> 2, part = lane & 3, left = nq - r0 - sub;        // rows from this lane's first on
+                auto piece = [&](int row, int pc) { return tb + row * 64 + ((pc ^ ((row >> 1) & 3)) << 4); };
+                const size_t row = (size_t)rec.x + r0 + sub, col = (size_t)h * dv;
+                const f2 inv2 = pack2(inv, inv);
+                auto put = [&](const uint32_t* w) {          // 16 words of the lane's row
+                    __syncwarp();
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(piece(lane, k)), "r"(w[4 * k]), "r"(w[4 * k + 1]), "r"(w[4 * k + 2]), "r"(w[4 * k + 3]) : "memory");
+                    __syncwarp();
+                };
+                auto get = [&](int k) {                      // this lane's piece of row 8 k + sub
+                    uint4 y;
+                    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(y.x), "=r"(y.y), "=r"(y.z), "=r"(y.w) : "r"(piece(8 * k + sub, part)));
+                    return y;
+                };
+                if (!a.elem_gate) {
+                    bf16* o = (bf16*)a.out + row * a.ld_out + col + 8 * part;
+#pragma unroll 1
+                    for (int c0 = 0; c0 < dv; c0 += 32) {
+                        uint32_t w[16];
+#pragma unroll
+                        for (int hf = 0; hf < 2; hf++) {
+                            if (c0 + 16 * hf >= dv) break;
+                            uint32_t v[16];
+                            ld16(t_o + c0 + 16 * hf, v);
+#pragma unroll
+                            for (int k = 0; k < 8; k++) {
+                                const float2 x = unpack2(mul2(pack2(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1])), inv2));
+                                w[8 * hf + k] = pack_bf16(x.x, x.y);
+                            }
+                        }
+                        put(w);
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const uint4 y = get(k);
+                            if (8 * k < left && c0 + 8 * part < dv) *reinterpret_cast<uint4*>(o + (size_t)(8 * k) * a.ld_out + c0) = y;
+                        }
+                    }
+                } else {
+                    bf16* o = (bf16*)a.out + row * a.ld_out + col + 4 * part;
+                    const float* eg = a.elem_gate + row * a.ld_elem_gate + col + 4 * part;
+                    const bool quads = a.ld_elem_gate % 4 == 0 && ((uintptr_t)a.elem_gate & 15) == 0;
+                    float4 t[4], t1[4];                      // gates of these 16 columns, and of the next
+                    auto gates = [&](float4* to, int c0) {
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const float* q = eg + (size_t)(8 * k) * a.ld_elem_gate + c0;
+                            to[k] = 8 * k >= left || c0 >= dv ? make_float4(0.f, 0.f, 0.f, 0.f) : quads ? *reinterpret_cast<const float4*>(q) : make_float4(q[0], q[1], q[2], q[3]);
+                        }
+                    };
+                    gates(t1, 0);
+#pragma unroll 1
+                    for (int c0 = 0; c0 < dv; c0 += 16) {
+#pragma unroll
+                        for (int k = 0; k < 4; k++) t[k] = t1[k];
+                        gates(t1, c0 + 16);
+                        uint32_t v[16];
+                        ld16(t_o + c0, v);
+#pragma unroll
+                        for (int k = 0; k < 16; k++) v[k] = __float_as_uint(__uint_as_float(v[k]) * inv);
+                        put(v);
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const uint4 y = get(k);
+                            const float y0 = __uint_as_float(y.x) * rcpf(1.0f + ex2f(-LOG2E * t[k].x)), y1 = __uint_as_float(y.y) * rcpf(1.0f + ex2f(-LOG2E * t[k].y));
+                            const float y2 = __uint_as_float(y.z) * rcpf(1.0f + ex2f(-LOG2E * t[k].z)), y3 = __uint_as_float(y.w) * rcpf(1.0f + ex2f(-LOG2E * t[k].w));
+                            if (8 * k < left) *reinterpret_cast<uint2*>(o + (size_t)(8 * k) * a.ld_out + c0) = make_uint2(pack_bf16(y0, y1), pack_bf16(y2, y3));
+                        }
+                    }
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();                                         // nothing is in flight, O is read
+    tc_fence_after();
+    if (warp == W_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TMEM) : "memory");
+}
+
+template <bool PEN, bool SIG>
+int launch(const p3_attn_window_args* a, int n_hc, int n_tc, cudaStream_t st) {
+    const size_t bytes = win_smem((a->dim + 63) / 64, (a->vdim + 63) / 64);
+    static P3DevFlags flags; bool& set = flags.cur();
+    if (!set) {
+        cudaError_t e = cudaFuncSetAttribute(attn_window_prefill_tc_kernel<PEN, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)win_smem(2, 2));
+        P3_CHECK_ARG(e == cudaSuccess, "attn_window_prefill: shared memory attribute: %s", cudaGetErrorString(e));
+        set = true;
+    }
+    const int64_t grid = (int64_t)((a->n_tiles + n_tc - 1) / n_tc) * (a->n_heads / n_hc);
+    p3_launch_pdl(attn_window_prefill_tc_kernel<PEN, SIG>, dim3((unsigned)grid), dim3(THREADS), bytes, st, *a, n_hc, n_tc);
+    return 0;
+}
+}  // namespace
+
+// whole 16-byte pieces everywhere
+bool attn_window_tc_ok(const p3_attn_window_args* a) {
+    return !a->act_f32 && a->dim % 16 == 0 && a->vdim % 16 == 0 && a->dim <= 128 && a->vdim <= 128 && a->ld_q % 8 == 0 && a->ld_out % 8 == 0 &&
+           a->v_ld % 8 == 0 && (((uintptr_t)a->q | (uintptr_t)a->out | (uintptr_t)a->k_pool | (uintptr_t)a->v_pool) & 15) == 0;
+}
+
+int launch_attn_window_tc(const p3_attn_window_args* a, cudaStream_t st) {
+    // Both halves of a CTA in use, unless that would leave half of the SMs without one (a half alone takes about as long as two): 333 rows of
+    // 32 heads of 96 on 96 CTAs 37 us, on 192 half empty ones 42.
+    int n_hc = (a->n_heads / a->n_kv) % 2 == 0 ? 2 : 1, n_tc = 2 / n_hc;
+    if ((int64_t)((a->n_tiles + n_tc - 1) / n_tc) * (a->n_heads / n_hc) < 74) n_hc = n_tc = 1;
+    if (a->sig_bias) return a->penalty ? launch<true, true>(a, n_hc, n_tc, st) : launch<false, true>(a, n_hc, n_tc, st);
+    return a->penalty ? launch<true, false>(a, n_hc, n_tc, st) : launch<false, false>(a, n_hc, n_tc, st);
+}

@@ -27,14 +27,15 @@ constexpr int ACC_COL = STAGES * A_COLS;
 constexpr int TMEM = 512;                                    // 3 x 96 for X, 2 x BN sums
 constexpr size_t f32tc_smem(int bn) { return (size_t)STAGES * 3 * bn * KB * 2 + 1024; }
 
+// bounded: a try may rest for up to 10 ms, a wait of 200 of them gives up
 __device__ __forceinline__ void wait_lim(uint32_t bar, uint32_t parity, volatile int* fail) {
-    uint32_t ok, spins = 0;
+    uint32_t ok, tries = 0;
     do {
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 10000000;\nselp.u32 %0, 1, 0, p;\n}"
                      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (!ok && (++spins & 1023u) == 0) {
+        if (!ok) {
             if (*fail) return;
-            if (spins > (1u << 18)) { *fail = 1; return; }
+            if (++tries > 200) { *fail = 1; return; }
         }
     } while (!ok);
 }

@@ -141,6 +141,94 @@ def test_fp32_products_on_the_tensor_cores_of_numbers_without_parts(dev):
     assert ((got - ref).abs()[ok] <= 2.0 ** -14 * scale[ok] + 1e-44).all() and ((got - ref).abs()[12:70][ok[12:70]] <= 2.0 ** -18 * scale[12:70][ok[12:70]]).all()
 
 
+def _attention(dev, H, G, d, dv, lens, window=0, keep=0, chunk=0, sink=True, pen=0, sig=False, gate=False, elem=False, shared=False, scale=None, seed=0,
+               offset=0, spread=1.0):
+    """ragged prompts [(tokens, position of the first)] through p3_attn_window_prefill, and the same in float64"""
+    from phi3_b200 import _lib
+    g = torch.Generator(device=dev).manual_seed(seed)
+    rn = lambda *s: torch.randn(s, generator=g, device=dev)
+    scale = d ** -0.5 if scale is None else scale
+    T = sum(n for n, _ in lens)
+    q, n_pg = (rn(T, H, d) * spread).to(B16), [-(-(n + p) // 64) for n, p in lens]
+    perm, bt = torch.randperm(sum(n_pg) + 2, generator=g, device=dev), torch.zeros(len(lens), max(n_pg), dtype=torch.int32, device=dev)
+    kp = torch.full((sum(n_pg) + 2, G, 64, d), 9.0, dtype=B16, device=dev)
+    vp = kp if shared else torch.full((sum(n_pg) + 2, G, 64, dv), 9.0, dtype=B16, device=dev)
+    sk, pe = (rn(H) if sink else None), (torch.rand(H, 1, generator=g, device=dev) * torch.log1p(torch.arange(pen, device=dev) * 0.3)[None] if pen else None)
+    sb, gt, eg = (rn(H) - 1 if sig else None), (torch.rand(T, H, generator=g, device=dev) if gate else None), (rn(T, H * dv + 3)[:, 3:] if elem else None)
+    refs, tiles, r, at = [], [], 0, 0
+    for s, ((n, p), pages) in enumerate(zip(lens, n_pg)):
+        k = rn(n + p, G, d).to(B16)
+        v = k[..., :dv] if shared else rn(n + p, G, dv).to(B16)
+        ids = perm[at:at + pages]
+        bt[s, :pages], at = ids.int(), at + pages
+        for pool, t in ((kp, k),) if shared else ((kp, k), (vp, v)):
+            full = torch.full((pages * 64, G, t.shape[-1]), 5.0, dtype=B16, device=dev)
+            full[:n + p] = t
+            pool[ids] = full.view(pages, 64, G, -1).transpose(1, 2)
+        tiles += [(r + i, min(64, n - i), s, p + i) for i in range(0, n, 64)]
+        i, j = torch.arange(p, p + n, device=dev)[:, None], torch.arange(n + p, device=dev)[None]
+        seen, dist = torch.ones(n, n + p, dtype=torch.bool, device=dev), i - j
+        if window:
+            seen &= dist < window
+        if chunk:
+            seen &= i // chunk == j // chunk
+        seen = (dist >= 0) & (seen | (j < keep))
+        sc = torch.einsum('thd,shd->hts', q[r:r + n].double(), k.double().repeat_interleave(H // G, 1)) * scale
+        if pen:
+            sc = sc - pe.double()[:, dist.clamp(0, pen - 1)]
+        if sig:
+            a = torch.sigmoid(sc + sb.double()[:, None, None]) * seen
+        else:
+            sc = sc.masked_fill(~seen, -float('inf'))
+            m = sc.amax(-1, keepdim=True)
+            m = torch.maximum(m, sk.double()[:, None, None]) if sink else m
+            e = torch.exp(sc - m)
+            a = e / (e.sum(-1, keepdim=True) + (torch.exp(sk.double()[:, None, None] - m) if sink else 0))
+        refs.append(torch.einsum('hts,shd->thd', a, v.double().repeat_interleave(H // G, 1)))
+        r += n
+    ref = torch.cat(refs)
+    if gate:
+        ref = ref * gt.double()[..., None]
+    ref = ref.reshape(T, H * dv) * (torch.sigmoid(eg.double()) if elem else 1.0)
+    td, out = torch.tensor(tiles, dtype=torch.int32, device=dev), torch.full((T, H * dv), float('nan'), dtype=B16, device=dev)
+    w = _lib.AttnWindowArgs()
+    qf = q.reshape(T, H * d)
+    w.q, w.ld_q, w.k_pool, w.v_pool, w.block_table, w.bt_stride = qf.data_ptr(), H * d, kp.data_ptr(), vp.data_ptr(), bt.data_ptr(), bt.stride(0)
+    w.sink, w.penalty, w.n_penalty, w.gate, w.out, w.ld_out = _lib.ptr(sk), _lib.ptr(pe), pen, _lib.ptr(gt), out.data_ptr(), H * dv
+    w.n_heads, w.n_kv, w.dim, w.vdim, w.scale, w.window, w.keep_first, w.chunk, w.v_ld = H, G, d, dv, scale, window, keep, chunk, d if shared else 0
+    w.sig_bias, w.elem_gate, w.ld_elem_gate, w.tiles, w.n_tiles = _lib.ptr(sb), _lib.ptr(eg), H * dv + 3, td.data_ptr(), len(tiles)
+    _lib.call_struct('p3_attn_window_prefill', w, _stream())
+    torch.cuda.synchronize()
+    return out.double(), ref
+
+
+SHAPES = [  # heads, K/V heads, key size, value size, (tokens, position of the first) of every sequence
+    (4, 4, 96, 96, [(2, 0), (64, 0), (65, 63), (130, 1)]), (8, 2, 128, 128, [(300, 0), (63, 640)]), (6, 3, 64, 64, [(129, 0), (2, 700)]),
+    (3, 1, 16, 48, [(200, 5)]), (16, 16, 112, 16, [(700, 64), (2, 0), (66, 130)]), (32, 1, 128, 128, [(70, 900)]), (2, 2, 80, 128, [(513, 0)]),
+    (64, 64, 64, 64, [(260, 0), (100, 0), (100, 0)]), (16, 4, 128, 96, [(1025, 100), (500, 0), (40, 2000)])]
+
+
+@pytest.mark.parametrize('shape', range(len(SHAPES)))
+@pytest.mark.parametrize('kind', ['plain', 'window', 'keep', 'chunk', 'sigmoid', 'gates', 'far', 'turned'])
+def test_prefill_attention_over_ragged_batches(dev, shape, kind):
+    """head groups, sizes of one and two boxes, records of several sequences in one CTA, masks, gates; weights are rounded to bf16 once
+    (relative 2^-9 each, averaging out) and so is the output (2^-9)"""
+    H, G, d, dv, lens = SHAPES[shape]
+    kw = {'plain': dict(sink=False), 'window': dict(window=100, pen=100), 'keep': dict(window=65, keep=70), 'chunk': dict(chunk=96),
+          'sigmoid': dict(sink=False, sig=True, window=200), 'gates': dict(gate=True, elem=True, pen=5000),
+          'far': dict(sink=False, spread=60.0), 'turned': dict(scale=-0.1, pen=700)}[kind]                  # scores of hundreds: the reference falls 2^64 behind and pages are swept again
+    y, ref = _attention(dev, H, G, d, dv, lens, seed=shape, **kw)
+    assert bool(torch.isfinite(y).all())
+    assert float((y - ref).norm() / ref.norm()) < 6e-3
+    assert float((y - ref).abs().max()) < 2.0 ** -6 * float(ref.abs().max())
+
+
+def test_prefill_attention_with_one_shared_row_per_token(dev):
+    for H, lens in ((16, [(700, 100), (300, 0)]), (4, [(33, 0)]), (1, [(200, 64)])):
+        y, ref = _attention(dev, H, 1, 128, 96, lens, window=512, shared=True, seed=H)
+        assert float((y - ref).norm() / ref.norm()) < 6e-3
+
+
 @pytest.mark.parametrize('cuts', [[0, 1], [0, 0, 0, 3, 3], [0, 32, 65, 65, 200], [0, 129, 130, 258, 258], [0, 5, 300, 900, 901, 1500], [0] + [7 * i for i in range(1, 71)]])
 @pytest.mark.parametrize('N,K', [(128, 64), (200, 72), (72, 136), (384, 520)])
 def test_grouped_products_over_ordered_rows(dev, cuts, N, K):
