@@ -30,7 +30,7 @@ from .lm_base import StepBatch
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())     # the current stream's handle without a Stream object
 
 
 class Engine:

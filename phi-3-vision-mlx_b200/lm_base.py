@@ -15,7 +15,7 @@ from ._lib import call, call_struct, ptr
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())     # the current stream's handle without a Stream object
 
 
 def _page_slices(pairs, pages, slots=2 * 148, merge=0.0):
