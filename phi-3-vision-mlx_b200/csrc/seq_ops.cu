@@ -17,6 +17,14 @@ template <typename T> __device__ __forceinline__ void stv(T* p, float v);
 template <> __device__ __forceinline__ void stv<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void stv<bf16>(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 
+// four numbers at once (16-byte aligned fp32, 8-byte aligned bf16)
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void st4(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void st4(bf16* p, const float4& v) { *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w)); }
+__device__ __forceinline__ float4 add4(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+__device__ __forceinline__ float sq4(const float4& a, float s) { return fmaf(a.w, a.w, fmaf(a.z, a.z, fmaf(a.y, a.y, fmaf(a.x, a.x, s)))); }
+__host__ __device__ __forceinline__ bool al16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
 // sum over a CTA of up to 1024 threads; every thread gets the total. The order of the additions is fixed by the thread
 // layout alone, so a row's statistic does not depend on the batch it is in.
 __device__ __forceinline__ float block_sum(float v, float* sh) {
@@ -67,7 +75,64 @@ __global__ void embed_rows_kernel(const bf16* __restrict__ table, const int32_t*
     }
 }
 
+// rows of a multiple of 8 numbers: 16 bytes of the table per lane (5400 rows of 2048: 17 us, one number at a time 21)
+template <typename AT>
+__global__ void embed_rows_vec_kernel(const uint4* __restrict__ table, const int32_t* __restrict__ ids, float* __restrict__ x, AT* __restrict__ xa,
+                                      int W, int vocab, float scale, int64_t ldxa) {
+    pdl_trigger();                                           // the next kernel may set up while this one runs ...
+    pdl_wait();                                              // ... and this one touches memory only after its predecessors are done
+    const int64_t t = blockIdx.x;
+    int id = ids[t];
+    if (id < 0 || id >= vocab) id = 0;
+    const uint4* src = table + (size_t)id * (W / 8);
+    for (int i0 = threadIdx.x; i0 < W / 8; i0 += 2 * blockDim.x) {
+        uint4 u[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) { const int i = i0 + k * blockDim.x; if (i < W / 8) u[k] = __ldg(src + i); }
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int i = i0 + k * blockDim.x;
+            if (i >= W / 8) continue;
+            const float2 a = unpack_bf16(u[k].x), b = unpack_bf16(u[k].y), c = unpack_bf16(u[k].z), e = unpack_bf16(u[k].w);
+            const float4 lo = make_float4(a.x * scale, a.y * scale, b.x * scale, b.y * scale), hi = make_float4(c.x * scale, c.y * scale, e.x * scale, e.y * scale);
+            float* xr = x + (size_t)t * W + 8 * i;
+            st4(xr, lo); st4(xr + 4, hi);
+            if (xa) { AT* o = xa + (size_t)t * ldxa + 8 * i; st4(o, lo); st4(o + 4, hi); }
+        }
+    }
+}
+
 // ---------------------------------------------------------------- x += rms_norm(y) * gain ; activation copy of the new x
+// aligned rows that two 16-byte pieces per thread hold (W <= 8 blockDim): 5400 rows of 2048: 23 us, one number at a time 33; 24 at the copy bandwidth
+template <typename AT>
+__global__ void postnorm_residual_vec_kernel(const float* __restrict__ y, int64_t ldy, const float* __restrict__ ybias,
+                                             const float* __restrict__ gain, float* x, AT* __restrict__ xa, int W, float eps) {
+    pdl_trigger();                                           // the next kernel may set up while this one runs ...
+    pdl_wait();                                              // ... and this one touches memory only after its predecessors are done
+    __shared__ float sh[32];
+    const int64_t t = blockIdx.x;
+    const float* yr = y + (size_t)t * ldy;
+    float* xr = x + (size_t)t * W;
+    float4 v[2], xv[2], gv[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int i = 4 * (threadIdx.x + k * blockDim.x);
+        const bool in = i < W;
+        v[k] = in ? ld4(yr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        xv[k] = in ? ld4(xr + i) : v[k];
+        gv[k] = in ? ld4(gain + i) : v[k];
+        if (in && ybias) v[k] = add4(v[k], ld4(ybias + i));
+    }
+    const float ss = block_sum(sq4(v[1], sq4(v[0], 0.f)), sh), r = 1.0f / sqrtf(ss / (float)W + eps);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int i = 4 * (threadIdx.x + k * blockDim.x);
+        if (i >= W) continue;
+        const float4 u = make_float4(xv[k].x + v[k].x * r * gv[k].x, xv[k].y + v[k].y * r * gv[k].y, xv[k].z + v[k].z * r * gv[k].z, xv[k].w + v[k].w * r * gv[k].w);
+        st4(xr + i, u);
+        if (xa) st4(xa + (size_t)t * W + i, u);
+    }
+}
 template <typename AT>
 __global__ void postnorm_residual_kernel(const float* __restrict__ y, int64_t ldy, const float* __restrict__ ybias,
                                          const float* __restrict__ gain, float* x, AT* __restrict__ xa, int W, float eps) {
@@ -189,6 +254,74 @@ __global__ void qk_norm_kv_write_kernel(p3_qkv_post_args a) {
                 if (a.v_mode == 1) vf[i] = v;
                 else if (a.v_mode == 2) v = (1.0f - a.v_lambda) * v + a.v_lambda * fv[k];
                 stv(dst + i, v);
+            }
+        }
+    }
+    if (a.gate_out && blockIdx.y == 0)
+        for (int h = threadIdx.x; h < H; h += blockDim.x)
+            a.gate_out[(size_t)t * H + h] = 1.0f / (1.0f + expf(-pr[a.g_off + h]));
+}
+
+// The same for aligned rows and head sizes that are multiples of 4: a lane holds neighbouring numbers, 16 bytes a load, and a warp has the loads of up
+// to PER heads in flight. One number at a time, a head after the other, a warp waited for memory at every head (5400 tokens of 16 + 4 + 4
+// heads of 128: 39 us, 69 that way; 15 at the copy bandwidth).
+template <typename AT, typename CT, int PER, int NE>       // NE: 1 for heads of up to 128 numbers, else 2
+__global__ void __launch_bounds__(256, NE == 1 ? 6 : 3) qk_norm_kv_write_vec_kernel(p3_qkv_post_args a) {
+    pdl_trigger();                                           // the next kernel may set up while this one runs ...
+    pdl_wait();                                              // ... and this one touches memory only after its predecessors are done
+    const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, c = 4 * lane;
+    const float* pr = a.proj + (size_t)t * a.ld_proj;
+    const int H = a.n_heads, G = a.n_kv, d = a.dim, dv = a.vdim, jobs = H + 2 * G, step = gridDim.y * nw;
+    const int slot = a.tok_slot[t], pos = a.tok_pos[t];
+    const int page = a.block_table[(size_t)slot * a.bt_stride + pos / P3_PAGE], off = pos % P3_PAGE;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j0 = blockIdx.y * nw + warp; j0 < jobs; j0 += PER * step) {
+        float4 v[PER][NE];
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            const int job = j0 + k * step;
+            if (job >= jobs) break;
+            const bool val = job >= H + G;
+            const int n = val ? dv : d, c0 = job < H ? a.q_off + job * d : !val ? a.k_off + (job - H) * d : a.v_off + (job - H - G) * dv;
+#pragma unroll
+            for (int e = 0; e < NE; e++) {
+                const int i = c + 128 * e;
+                v[k][e] = i < n ? ld4(pr + c0 + i) : zero;
+                if (a.bias && i < n) v[k][e] = add4(v[k][e], ld4(a.bias + c0 + i));
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            const int job = j0 + k * step;
+            if (job >= jobs) break;
+            if (job < H + G) {                               // query or key head: RMS norm over its d numbers, shared gain
+                const bool isq = job < H;
+                const float* gain = isq ? a.q_gain : a.k_gain;
+                float r = 1.0f / sqrtf(warp_sum(NE == 1 ? sq4(v[k][0], 0.f) : sq4(v[k][NE - 1], sq4(v[k][0], 0.f))) / (float)d + a.eps);
+                if (isq && a.q_temp_every > 0) r *= 1.0f + a.q_temp_coef * logf((float)((pos + 1) / a.q_temp_every) + 1.0f);
+#pragma unroll
+                for (int e = 0; e < NE; e++) {
+                    const int i = c + 128 * e;
+                    if (i >= d) continue;
+                    const float4 g = ld4(gain + i), x = v[k][e];
+                    const float4 y = make_float4(x.x * r * g.x, x.y * r * g.y, x.z * r * g.z, x.w * r * g.w);
+                    if (isq) st4((AT*)a.q_out + (size_t)t * a.ld_q + (size_t)job * d + i, y);
+                    else st4((CT*)a.k_pool + (((size_t)page * G + job - H) * P3_PAGE + off) * d + i, y);
+                }
+            } else {                                         // value head: v, or (1 - lam) v + lam v_first; the mixed v is cached
+                const int h = job - H - G;
+#pragma unroll
+                for (int e = 0; e < NE; e++) {
+                    const int i = c + 128 * e;
+                    if (i >= dv) continue;
+                    float4 x = v[k][e];
+                    float* first = a.v_first + (size_t)t * G * dv + (size_t)h * dv + i;
+                    const float4 m = a.v_mode == 2 ? ld4(first) : zero;
+                    const float l = a.v_lambda;
+                    if (a.v_mode == 1) st4(first, x);
+                    else if (a.v_mode == 2) x = make_float4((1.0f - l) * x.x + l * m.x, (1.0f - l) * x.y + l * m.y, (1.0f - l) * x.z + l * m.z, (1.0f - l) * x.w + l * m.w);
+                    st4((CT*)a.v_pool + (((size_t)page * G + h) * P3_PAGE + off) * dv + i, x);
+                }
             }
         }
     }
@@ -1343,7 +1476,11 @@ extern "C" int p3_embed_rows_f32(const void* table, const int32_t* ids, float* x
                                  float scale, int64_t ld_act, cudaStream_t st) {
     if (T == 0) return 0;
     if (ld_act <= 0) ld_act = W;
-    if (act_f32) p3_launch_pdl(embed_rows_kernel<float>, dim3((unsigned)T), dim3(128), (size_t)(0), st, (const bf16*)table, ids, x, (float*)x_act, W, vocab, scale, ld_act);
+    if (W % 8 == 0 && ld_act % 8 == 0 && al16(table) && al16(x) && al16(x_act)) {
+        const unsigned th = W >= 2048 ? 256 : 128;
+        if (act_f32) p3_launch_pdl(embed_rows_vec_kernel<float>, dim3((unsigned)T), dim3(th), (size_t)0, st, (const uint4*)table, ids, x, (float*)x_act, W, vocab, scale, ld_act);
+        else p3_launch_pdl(embed_rows_vec_kernel<bf16>, dim3((unsigned)T), dim3(th), (size_t)0, st, (const uint4*)table, ids, x, (bf16*)x_act, W, vocab, scale, ld_act);
+    } else if (act_f32) p3_launch_pdl(embed_rows_kernel<float>, dim3((unsigned)T), dim3(128), (size_t)(0), st, (const bf16*)table, ids, x, (float*)x_act, W, vocab, scale, ld_act);
     else p3_launch_pdl(embed_rows_kernel<bf16>, dim3((unsigned)T), dim3(128), (size_t)(0), st, (const bf16*)table, ids, x, (bf16*)x_act, W, vocab, scale, ld_act);
     P3_CHECK_LAUNCH("embed_rows_f32");
     return 0;
@@ -1353,7 +1490,10 @@ extern "C" int p3_postnorm_residual(const float* y, int64_t ldy, const float* y_
                                     int64_t T, int W, float eps, cudaStream_t st) {
     if (T == 0) return 0;
     const int th = W > 4096 ? 1024 : W > 2048 ? 512 : W >= 1024 ? 256 : 128;     // the row fits the threads' registers up to W = 8192
-    if (act_f32) p3_launch_pdl(postnorm_residual_kernel<float>, dim3((unsigned)T), dim3(th), (size_t)(0), st, y, ldy, y_bias, gain, x, (float*)x_act, W, eps);
+    if (W % 4 == 0 && W <= 8 * th && ldy % 4 == 0 && al16(y) && al16(y_bias) && al16(gain) && al16(x) && al16(x_act)) {
+        if (act_f32) p3_launch_pdl(postnorm_residual_vec_kernel<float>, dim3((unsigned)T), dim3(th), (size_t)0, st, y, ldy, y_bias, gain, x, (float*)x_act, W, eps);
+        else p3_launch_pdl(postnorm_residual_vec_kernel<bf16>, dim3((unsigned)T), dim3(th), (size_t)0, st, y, ldy, y_bias, gain, x, (bf16*)x_act, W, eps);
+    } else if (act_f32) p3_launch_pdl(postnorm_residual_kernel<float>, dim3((unsigned)T), dim3(th), (size_t)(0), st, y, ldy, y_bias, gain, x, (float*)x_act, W, eps);
     else p3_launch_pdl(postnorm_residual_kernel<bf16>, dim3((unsigned)T), dim3(th), (size_t)(0), st, y, ldy, y_bias, gain, x, (bf16*)x_act, W, eps);
     P3_CHECK_LAUNCH("postnorm_residual");
     return 0;
@@ -1379,7 +1519,18 @@ extern "C" int p3_qkv_post(const p3_qkv_post_args* a, cudaStream_t st) {
     // the jobs over more CTAs measured no faster)
     const int groups = a->T >= 1024 ? 1 : (jobs + 3) / 4;
     const dim3 grid((unsigned)a->T, (unsigned)groups);
-    if (a->act_f32 && a->cache_f32) p3_launch_pdl(qk_norm_kv_write_kernel<float, float>, dim3(grid), dim3(th), (size_t)(0), st, *a);
+    const bool vec = a->dim % 4 == 0 && a->vdim % 4 == 0 && (a->ld_proj | a->q_off | a->k_off | a->v_off | a->ld_q) % 4 == 0 && al16(a->proj) &&
+                     al16(a->q_gain) && al16(a->k_gain) && al16(a->v_first) && al16(a->bias) && al16(a->q_out) && al16(a->k_pool) && al16(a->v_pool);
+    if (vec && a->act_f32 == a->cache_f32) {
+        // many tokens: a CTA of 8 warps per token, three heads in flight each; few: a warp per head
+        const bool many = a->T >= 1024;
+        const dim3 tb(many ? 256 : th);
+#define GO(T, PER, NE) p3_launch_pdl(qk_norm_kv_write_vec_kernel<T, T, PER, NE>, grid, tb, (size_t)0, st, *a)
+        const bool small = a->dim <= 128 && a->vdim <= 128;
+        if (a->act_f32) { if (many && small) GO(float, 3, 1); else if (many) GO(float, 3, 2); else if (small) GO(float, 1, 1); else GO(float, 1, 2); }
+        else { if (many && small) GO(bf16, 3, 1); else if (many) GO(bf16, 3, 2); else if (small) GO(bf16, 1, 1); else GO(bf16, 1, 2); }
+#undef GO
+    } else if (a->act_f32 && a->cache_f32) p3_launch_pdl(qk_norm_kv_write_kernel<float, float>, dim3(grid), dim3(th), (size_t)(0), st, *a);
     else if (!a->act_f32 && !a->cache_f32) p3_launch_pdl(qk_norm_kv_write_kernel<bf16, bf16>, dim3(grid), dim3(th), (size_t)(0), st, *a);
     else P3_CHECK_ARG(false, "qkv_post: activations and cache must both be fp32 or both bf16");
     P3_CHECK_LAUNCH("qkv_post");

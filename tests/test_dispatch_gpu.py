@@ -525,3 +525,70 @@ def test_rotary_products_at_narrow_tiles(dev, width, nh):
     _fused(x, w[torch.tensor(order, device=dev)].contiguous(), got, _lib.EPI_ROPE_KV, cosT=cos, sinT=sin, tab_bstride=cos.stride(0), L=L, n_heads=nh, n_kv=nh,
            hd=hd, past=0, row_div=1, write_cache=1, bt_stride=bt.stride(0), pool=pool, block_table=bt)
     assert torch.equal(got, ref) and torch.equal(pool, pool_ref)
+
+
+@pytest.mark.parametrize('T,H,G,d,dv', [(3, 5, 1, 4, 8), (1030, 16, 4, 128, 128), (1025, 3, 3, 252, 40), (70, 2, 2, 132, 256), (1024, 1, 1, 96, 4), (9, 4, 2, 30, 33)])
+@pytest.mark.parametrize('dtype', [F32, B16])
+@pytest.mark.parametrize('mode', [0, 1, 2])
+def test_head_norms_and_cache_writes(dev, T, H, G, d, dv, dtype, mode):
+    """aligned heads of one and two pieces a lane, one head and three heads a warp, and heads of any size; fp32 arithmetic, the result rounded once"""
+    from phi3_b200 import _lib
+    g = torch.Generator(device=dev).manual_seed(T + d)
+    rn = lambda *s: torch.randn(s, generator=g, device=dev)
+    q0, k0, v0 = 4, 4 + H * d, 4 + H * d + G * d
+    ld = (v0 + G * dv + H + 11) // 4 * 4 if d % 4 == 0 else v0 + G * dv + H + 1
+    proj, qg, kg, bias, first = rn(T, ld), rn(d), rn(d), rn(ld), rn(T, G * dv)
+    slot, pos = torch.arange(T, device=dev, dtype=torch.int32) % 3, torch.arange(T, device=dev, dtype=torch.int32) // 3
+    n_pg = -(-(T // 3 + 1) // 64)
+    bt = torch.randperm(3 * n_pg, generator=g, device=dev).to(torch.int32).view(3, n_pg)
+    q = torch.full((T, H * d), float('nan'), dtype=dtype, device=dev)
+    kp, vp = (torch.full((3 * n_pg, G, 64, n), float('nan'), dtype=dtype, device=dev) for n in (d, dv))
+    gate, vf = torch.empty(T, H, device=dev), first.clone()
+    a = _lib.QkvPostArgs()
+    a.proj, a.ld_proj, a.q_off, a.k_off, a.v_off, a.g_off = proj.data_ptr(), ld, q0, k0, v0, v0 + G * dv
+    a.n_heads, a.n_kv, a.dim, a.vdim, a.q_gain, a.k_gain, a.eps = H, G, d, dv, qg.data_ptr(), kg.data_ptr(), 1e-5
+    a.v_first, a.v_mode, a.v_lambda = vf.data_ptr() if mode else None, mode, 0.375
+    a.q_out, a.ld_q, a.gate_out, a.k_pool, a.v_pool, a.block_table, a.bt_stride = q.data_ptr(), H * d, gate.data_ptr(), kp.data_ptr(), vp.data_ptr(), bt.data_ptr(), n_pg
+    a.tok_slot, a.tok_pos, a.T, a.act_f32, a.cache_f32, a.bias = slot.data_ptr(), pos.data_ptr(), T, int(dtype == F32), int(dtype == F32), bias.data_ptr()
+    a.q_temp_coef, a.q_temp_every = 0.1, 50
+    _lib.call_struct('p3_qkv_post', a, _stream())
+    x, m = proj.double() + bias.double(), proj.double().abs() + bias.double().abs()
+    rms = lambda y: torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-5)
+    norm = lambda y, gain: y / rms(y) * gain.double()
+    temp = 1 + 0.1 * torch.log(((pos + 1) // 50).double() + 1)
+    want_q = norm(x[:, q0:k0].view(T, H, d), qg) * temp[:, None, None]
+    want_k, want_v = norm(x[:, k0:v0].view(T, G, d), kg), x[:, v0:v0 + G * dv].view(T, G, dv)
+    if mode == 2:
+        want_v = 0.625 * want_v + 0.375 * first.double().view(T, G, dv)
+    pages = bt[slot.long(), (pos // 64).long()].long()
+    got_k, got_v = kp[pages, :, (pos % 64).long()], vp[pages, :, (pos % 64).long()]
+    # a few roundings at 2^-24 of the numbers that enter, however much they cancel, and of the sum of squares; 2^-8 for a bf16 result
+    size_q, size_k = (m[:, a:b].view(T, n, d) / rms(x[:, a:b].view(T, n, d)) * gain.double().abs() * 2 for a, b, n, gain in ((q0, k0, H, qg), (k0, v0, G, kg)))
+    size_v = m[:, v0:v0 + G * dv].view(T, G, dv) + first.double().abs().view(T, G, dv)
+    for got, want, size in ((q.view(T, H, d), want_q, size_q), (got_k, want_k, size_k), (got_v, want_v, size_v)):
+        assert ((got.double() - want).abs() <= 2.0 ** -20 * size + (0 if dtype == F32 else 2.0 ** -8) * want.abs()).all()
+    assert torch.allclose(gate, torch.sigmoid(proj[:, v0 + G * dv:v0 + G * dv + H]), atol=1e-6)
+    if mode == 1:
+        assert torch.equal(vf, (proj + bias)[:, v0:v0 + G * dv])
+
+
+@pytest.mark.parametrize('W', [4, 8, 1000, 1030, 2048, 2056, 8192, 8200])
+@pytest.mark.parametrize('dtype', [F32, B16])
+def test_rows_of_the_residual_stream(dev, W, dtype):
+    """embedding and output norm: rows that two pieces a thread hold, longer ones, and rows that split a piece"""
+    from phi3_b200 import _lib
+    g = torch.Generator(device=dev).manual_seed(W)
+    rn = lambda *s: torch.randn(s, generator=g, device=dev)
+    T, f32 = 37, int(dtype == F32)
+    table, ids = rn(50, W).to(B16), torch.randint(-2, 53, (T,), generator=g, device=dev, dtype=torch.int32)
+    x, xa = torch.empty(T, W, device=dev), torch.empty(T, W, dtype=dtype, device=dev)
+    _lib.call('p3_embed_rows_f32', table.data_ptr(), ids.data_ptr(), x.data_ptr(), xa.data_ptr(), f32, T, W, 50, 1.5, W, _stream())
+    want = table[torch.where((ids < 0) | (ids >= 50), 0, ids).long()].float() * 1.5
+    assert torch.equal(x, want) and torch.equal(xa, want.to(dtype))
+    for bias in (None, rn(W)):
+        y, gain, x0 = rn(T, W + 4), rn(W), x.clone()
+        _lib.call('p3_postnorm_residual', y.data_ptr(), W + 4, _lib.ptr(bias), gain.data_ptr(), x.data_ptr(), xa.data_ptr(), f32, T, W, 1e-5, _stream())
+        u = y[:, :W].double() + (0 if bias is None else bias.double())
+        want = x0.double() + u / torch.sqrt((u * u).mean(-1, keepdim=True) + 1e-5) * gain.double()
+        assert ((x.double() - want).abs() <= 3e-6 * (want.abs() + u.abs() * gain.double().abs() + 0.1)).all()
+        assert torch.equal(xa, x.to(dtype))
