@@ -229,6 +229,44 @@ def test_prefill_attention_with_one_shared_row_per_token(dev):
         assert float((y - ref).norm() / ref.norm()) < 6e-3
 
 
+@pytest.mark.parametrize('H,G,d,dv,shared', [(4, 2, 16, 128, False), (16, 4, 128, 128, False), (20, 1, 64, 48, False), (32, 1, 128, 96, True), (3, 3, 96, 40, False),
+                                             (8, 2, 192, 200, False)])
+@pytest.mark.parametrize('kind', ['plain', 'sink', 'sigmoid'])
+def test_decode_slices_of_one_cluster(dev, H, G, d, dv, shared, kind):
+    """one to eight slices of a request's pages merge inside a cluster, nine through the workspace: slices without a page, more heads than a pass
+    takes, values in two column blocks, the smallest rows under the largest states. Weights are rounded to bf16 against another maximum in
+    another slice: 2^-8 of the values that are averaged"""
+    from phi3_b200 import _lib
+    g = torch.Generator(device=dev).manual_seed(H + d)
+    rn = lambda *s: torch.randn(s, generator=g, device=dev)
+    lens = [1, 64, 65, 300, 700]
+    n, pages = len(lens), [-(-x // 64) for x in lens]
+    kp = rn(sum(pages), G, 64, d).to(B16)
+    vp = kp if shared else rn(sum(pages), G, 64, dv).to(B16)
+    bt, at = torch.zeros(n, max(pages), dtype=torch.int32, device=dev), 0
+    for i, p in enumerate(pages):
+        bt[i, :p], at = torch.arange(at, at + p, dtype=torch.int32, device=dev), at + p
+    q, sink, sig, gate = rn(n, H * d).to(B16), rn(H), rn(H) - 2, rn(n, H * dv)
+    tiles = torch.tensor([(i, 1, i, x - 1) for i, x in enumerate(lens)], dtype=torch.int32, device=dev)
+
+    def decode(ns):
+        out, ws = torch.full((n, H * dv), float('nan'), dtype=B16, device=dev), torch.full((n * H * ns * (dv + 2),), float('nan'), device=dev)
+        w = _lib.AttnWindowArgs()
+        w.q, w.ld_q, w.k_pool, w.v_pool, w.block_table, w.bt_stride = q.data_ptr(), H * d, kp.data_ptr(), vp.data_ptr(), bt.data_ptr(), bt.stride(0)
+        w.out, w.ld_out, w.n_heads, w.n_kv, w.dim, w.vdim, w.scale, w.v_ld = out.data_ptr(), H * dv, H, G, d, dv, d ** -0.5, d if shared else 0
+        w.sink, w.sig_bias = sink.data_ptr() if kind == 'sink' else None, sig.data_ptr() if kind == 'sigmoid' else None
+        w.elem_gate, w.ld_elem_gate, w.tiles, w.n_tiles, w.n_splits, w.ws = gate.data_ptr(), H * dv, tiles.data_ptr(), n, ns, ws.data_ptr()
+        _lib.call_struct('p3_attn_window_decode', w, _stream())
+        return out.double()
+
+    one = decode(1)
+    assert bool(torch.isfinite(one).all())
+    for ns in (2, 3, 7, 8, 9):
+        y = decode(ns)
+        assert float((y - one).norm() / one.norm()) < 6e-3 and float((y - one).abs().max()) < 2.0 ** -6 * float(one.abs().max())
+        assert torch.equal(y, decode(ns))
+
+
 @pytest.mark.parametrize('cuts', [[0, 1], [0, 0, 0, 3, 3], [0, 32, 65, 65, 200], [0, 129, 130, 258, 258], [0, 5, 300, 900, 901, 1500], [0] + [7 * i for i in range(1, 71)]])
 @pytest.mark.parametrize('N,K', [(128, 64), (200, 72), (72, 136), (384, 520)])
 def test_grouped_products_over_ordered_rows(dev, cuts, N, K):
