@@ -33,7 +33,7 @@ Kernels per layer (csrc/): p3_embed_pair_rows_f32 -> p3_postnorm_prenorm ->
 
 Precision. dtype=bfloat16 (serving): matrices, activations that feed a matrix product and the caches are bf16, accumulation is fp32;
 positions, angles, scores, softmax, norms, the residual sum, decays and their logarithms, the recurrent state and its sums are fp32.
-dtype=float32: everything is fp32 on the FMA pipes (no TF32).
+dtype=float32: everything is fp32 (no TF32).
 """
 import os
 

@@ -29,7 +29,7 @@ p3_moe_combine_identity (identity experts and the shared unit join the sum) -> p
 
 Precision. dtype=bfloat16 (serving): matrices, activations that feed a matrix product and the K/V cache are bf16, accumulation is
 fp32; positions, angles, scores, attention weights, norms, router, the residual sum, the token-shift state, the gates of the
-recurrence, its state and its sums are fp32. dtype=float32: everything is fp32 on the FMA pipes (no TF32).
+recurrence, its state and its sums are fp32. dtype=float32: everything is fp32 (no TF32).
 """
 import ctypes as C
 

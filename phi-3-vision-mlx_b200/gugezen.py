@@ -30,7 +30,7 @@ p3_streams_rmsnorm (behind the last layer: the final norm of the wanted rows alo
 
 Precision. dtype=bfloat16 (serving): matrices, activations that feed a matrix product and the K/V cache are bf16, accumulation is
 fp32; positions, angles, scores, softmax, norms, router, the residual streams, convolutions and their history, decays and their
-logarithms, step sizes, the recurrent states and their sums are fp32. dtype=float32: everything is fp32 on the FMA pipes (no TF32).
+logarithms, step sizes, the recurrent states and their sums are fp32. dtype=float32: everything is fp32 (no TF32).
 """
 import os
 

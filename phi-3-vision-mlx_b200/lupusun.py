@@ -25,7 +25,7 @@ norm of the wanted rows alone).
 
 Precision. dtype=bfloat16 (serving): matrices, activations that feed a matrix product and the K/V cache are bf16, accumulation is
 fp32; positions, angles, scores, softmax, norms, the residual sum, convolutions and their history, decays and their logarithms, step
-sizes, the recurrent state and its sums are fp32. dtype=float32: everything is fp32 on the FMA pipes (no TF32).
+sizes, the recurrent state and its sums are fp32. dtype=float32: everything is fp32 (no TF32).
 """
 import torch
 from . import _lib

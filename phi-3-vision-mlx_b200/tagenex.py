@@ -17,7 +17,7 @@ rows -> p3_glu_clamped -> grouped down GEMM -> p3_moe_combine.
 
 Precision. dtype=bfloat16 (serving): matrices, activations that feed a matrix product and the cache are bf16, accumulation is
 fp32; positions, penalties, scores, softmax, norms, router, gates, value mixing and the residual sum are fp32. dtype=float32:
-everything is fp32 on the FMA pipes (no TF32). Dense bf16 products with K % 8 == 0 run on the tcgen05 GEMM (p3_gemm), everything
+everything is fp32 (no TF32). Dense bf16 products with K % 8 == 0 run on the tcgen05 GEMM (p3_gemm), everything
 else on p3_gemm_any.
 """
 import torch

@@ -22,8 +22,8 @@ parts, shared expert activation) -> per-head query absorption -> p3_attn_window_
 p3_router_sigmoid_groups -> p3_moe_sort -> grouped gate|up product -> p3_glu_silu -> grouped down product -> p3_moe_combine.
 
 Precision. dtype=bfloat16 (serving): matrices, activations that feed a matrix product and the cache are bf16, accumulation is fp32;
-positions, angles, scores, softmax, norms, router, gates and the residual sum are fp32. dtype=float32: everything is fp32 on the
-FMA pipes (no TF32).
+positions, angles, scores, softmax, norms, router, gates and the residual sum are fp32. dtype=float32: everything is fp32
+(no TF32).
 """
 import ctypes as C
 
