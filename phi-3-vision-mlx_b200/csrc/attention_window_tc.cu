@@ -19,8 +19,8 @@
 //               the outputs of this one are written; as CTAs of their own they cost 17 000 clocks beside their pages.
 //   warp 5:     one thread issues the MMAs: O += P(j) V(j), then S(j + 2) = Q K(j + 2)^T into the columns P(j) left
 // Bound by the softmax warps: a page of a CTA takes 3000 clocks with two CTAs on an SM, its 64 exponentials a row alone 1000 of them; the MMAs
-// of both keep the tensor cores busy half of the time. 4 x 2048 tokens, 16 heads of 128 over 4, window 1024, penalties: 112 us (mma.sync 298);
-// 333 rows of 32 x 96 behind 704: 37 (67). With two threads a row and eight warps a CTA 125: a third more instructions.
+// of both keep the tensor cores busy half of the time. 4 x 2048 tokens, 16 heads of 128 over 4, window 1024, penalties: 115 us (mma.sync 298);
+// 333 rows of 32 x 96 behind 704: 39 (67). With two threads a row and eight warps a CTA 125: a third more instructions.
 //
 // Every wait has a limit: when one runs out the CTA stops waiting, writes NaN and ends.
 #include "tc_common.cuh"
