@@ -364,7 +364,10 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
             auto page_at = [&](int it) { return it < n_keep ? it : past_keep + it; };
             const int nq = mine ? rec.y : 0, pos = rec.w + i;
             const bool row_ok = i < nq;
-            const float scale2 = a.scale * LOG2E, sb2 = SIG ? a.sig_bias[h] * LOG2E : 0.f;
+            // without penalties a key that is not seen is `gone` before the scale is multiplied in, -infinity behind it whatever the scale's sign; a scale
+            // of zero is the smallest number instead (a score of 3e38 becomes 5e-7)
+            const float scale2 = PEN || a.scale != 0.f ? a.scale * LOG2E : __int_as_float(1), gone = PEN || scale2 > 0.f ? -INFINITY : INFINITY;
+            const float sb2 = SIG ? a.sig_bias[h] * LOG2E : 0.f;
             const f2 scale22 = SIG && !PEN ? pack2(-scale2, -scale2) : pack2(scale2, scale2), sbias22 = pack2(-sb2, -sb2), one2 = pack2(1.f, 1.f);
             float m = a.sink ? a.sink[h] * LOG2E : -INFINITY, l = a.sink ? 1.f : 0.f, pend = 1.f;     // pend: what O and l are to be multiplied by
             const int lo = first_key(a, pos), warp_lo = rec.w + r0, warp_hi = rec.w + min(nq - 1, r0 + 31), lo_hi = first_key(a, max(warp_hi, 0));
@@ -453,7 +456,7 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
 #pragma unroll
                             for (int k = 0; k < 16; k++) {
                                 const float2 x = unpack2(v[k]);
-                                v[k] = pack2(seen >> (2 * k) & 1u ? x.x : -INFINITY, seen >> (2 * k + 1) & 1u ? x.y : -INFINITY);
+                                v[k] = pack2(seen >> (2 * k) & 1u ? x.x : gone, seen >> (2 * k + 1) & 1u ? x.y : gone);
                             }
                         }
                         if (!SIG) {

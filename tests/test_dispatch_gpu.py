@@ -223,6 +223,20 @@ def test_prefill_attention_over_ragged_batches(dev, shape, kind):
     assert float((y - ref).abs().max()) < 2.0 ** -6 * float(ref.abs().max())
 
 
+@pytest.mark.parametrize('shape', [0, 1, 3, 4, 6, 8])
+@pytest.mark.parametrize('scale', [-0.1, 0.0, -2e-39])
+@pytest.mark.parametrize('kind', ['plain', 'window', 'chunk', 'sigmoid', 'penalty'])
+def test_prefill_attention_at_scales_of_zero_and_below(dev, shape, scale, kind):
+    """a masked key has no weight whatever the sign of the scale, with a penalty table and without. Bounds as for ragged batches: outputs
+    rounded to bf16, weights to two of them"""
+    H, G, d, dv, lens = SHAPES[shape]
+    kw = {'plain': dict(sink=False), 'window': dict(window=100), 'chunk': dict(chunk=96), 'sigmoid': dict(sink=False, sig=True, window=200), 'penalty': dict(pen=300)}[kind]
+    y, ref = _attention(dev, H, G, d, dv, lens, seed=shape, scale=scale, **kw)
+    assert bool(torch.isfinite(y).all())
+    assert float((y - ref).norm() / ref.norm()) < 6e-3
+    assert float((y - ref).abs().max()) < 2.0 ** -6 * float(ref.abs().max())
+
+
 def test_prefill_attention_with_one_shared_row_per_token(dev):
     for H, lens in ((16, [(700, 100), (300, 0)]), (4, [(33, 0)]), (1, [(200, 64)])):
         y, ref = _attention(dev, H, 1, 128, 96, lens, window=512, shared=True, seed=H)
