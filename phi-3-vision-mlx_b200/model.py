@@ -500,10 +500,11 @@ class Phi3B200:
     # ------------------------------------------------------------------ rope table (phi:487-507)
     def _upload(self, t, dtype=None):
         """t on the device. Host data goes through pinned memory: a copy from pageable memory would wait until the stream's earlier work is
-        done, with the device idle until the first kernel of this call (a prefill of 781 tokens behind another: 591 -> 540 us)"""
+        done, with the device idle until the first kernel of this call (a prefill of 781 tokens behind another: 591 -> 540 us). The pinned memory
+        is the copy's own: the caller's, pinned too, may be written again as soon as the call returns."""
         if t.is_cuda or self.dev.type != 'cuda':
             return t.to(self.dev) if dtype is None else t.to(self.dev, dtype)
-        return (t if dtype is None else t.to(dtype)).contiguous().pin_memory().to(self.dev, non_blocking=True)
+        return torch.empty(t.shape, dtype=dtype or t.dtype, pin_memory=True).copy_(t).to(self.dev, non_blocking=True)
 
     def _rope_table(self, L_all, pids):
         cfg = self.cfg

@@ -644,3 +644,24 @@ def test_rows_of_the_residual_stream(dev, W, dtype):
         want = x0.double() + u / torch.sqrt((u * u).mean(-1, keepdim=True) + 1e-5) * gain.double()
         assert ((x.double() - want).abs() <= 3e-6 * (want.abs() + u.abs() * gain.double().abs() + 0.1)).all()
         assert torch.equal(xa, x.to(dtype))
+
+
+@pytest.mark.parametrize('what', ['ids', 'pids', 'mask'])
+@pytest.mark.parametrize('dtype', [torch.int32, torch.int64])
+def test_a_call_keeps_no_hold_on_the_buffers_of_its_caller(dev, what, dtype):
+    """host tensors of a call, pinned ones too, may be written again as soon as it returns, however much work is queued before it on the stream"""
+    from phi3_b200 import configs, weights
+    from phi3_b200.model import Phi3B200
+    cfg = configs.tiny(layers=1)
+    m = Phi3B200(cfg, weights.random_weights(cfg, seed=0))
+    g = torch.Generator().manual_seed(1)
+    host = dict(ids=torch.randint(3, 30000, (2, 40), generator=g), pids=torch.arange(40).repeat(2, 1), mask=torch.ones(2, 40, dtype=torch.int64))
+    host['pids'][1], host['mask'][1, :7] = (torch.arange(40) - 7).clamp(min=0), 0
+    kw = lambda h: dict(pids=h['pids'], mask=h['mask'], max_tokens=4)
+    want = m(host['ids'], **kw(host))[0].float().cpu()
+    host[what] = host[what].to(dtype).pin_memory()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)                                       # a tenth of a second of work before the call
+    got = m(host['ids'], **kw(host))[0]
+    host[what].fill_(1)
+    assert torch.equal(got.float().cpu(), want)
