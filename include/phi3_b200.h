@@ -7,9 +7,12 @@
  * maintainer of the reference would add.
  *
  * Conventions: plain device pointers + sizes, caller-owned memory and workspaces, no
- * allocation and no host synchronisation inside, stream-ordered and CUDA-graph capturable.
- * Every function returns 0 on success, <0 on error; p3_last_error() gives the message
- * (thread-local). bf16 = __nv_bfloat16 storage. "Rows" are tokens (B*L flattened).
+ * allocation (but for one status word of host memory) and no host synchronisation inside,
+ * stream-ordered and CUDA-graph capturable. Every function returns 0 on success, <0 on
+ * error; p3_last_error() gives the message (thread-local). -3: a bounded wait inside a kernel
+ * launched earlier (p3_attn_window_prefill, fp32 p3_gemm_any) ran out, and outputs of that
+ * launch are not numbers; told once, by the next call that launches something, on any thread.
+ * bf16 = __nv_bfloat16 storage. "Rows" are tokens (B*L flattened).
  */
 #ifndef PHI3_B200_H
 #define PHI3_B200_H
@@ -33,6 +36,8 @@ extern "C" {
 
 const char* p3_last_error(void);
 int p3_version(void);
+/* tests: a launch whose wait runs out within some 20 ms; out32: 32 floats, NaN behind it */
+int p3_wait_selftest(float* out32, cudaStream_t st);
 /* Diagnostics (tools/chain_trace.py), not part of the reference interface: with a device buffer of n_slots x 1024 x 8 uint64 set,
  * every decode-path launch (skinny GEMMs, decode attention) takes the next slot and its CTAs store globaltimer stamps
  * {start, dependency resolved, first operands ready, main loop done, exit, smid, kind, grid}. p3_trace_set(NULL, 0) turns it off. */

@@ -47,6 +47,7 @@ _SIGS = {
     'p3_gemm': [_p, _l, _p, _l, _p, _p, _l, _p, _p, _l, _i, _i, _i, _i, _p],
     'p3_gemm_pair_width': [_l, _l],
     'p3_gemm_any_tile': [_p],
+    'p3_wait_selftest': [_p, _p],
     'p3_gemm_glu': [_p, _l, _p, _l, _p, _p, _l, _l, _i, _i, _i, _f, _f, _p],
     'p3_attention_prefill': [_p, _p, _p, _l, _l, _l, _p, _l, _i, _i, _i, _i, _i, _f, _i, _i, _p, _p, _p, _i, _i, _p],
     'p3_attention_decode': [_p, _p, _p, _l, _l, _l, _p, _l, _i, _i, _i, _i, _i, _f, _i, _p, _p, _p, _i, _i, _i, _p, _p, _p, _l, _p],

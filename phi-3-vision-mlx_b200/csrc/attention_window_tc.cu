@@ -22,7 +22,8 @@
 // of both keep the tensor cores busy half of the time. 4 x 2048 tokens, 16 heads of 128 over 4, window 1024, penalties: 115 us (mma.sync 298);
 // 333 rows of 32 x 96 behind 704: 39 (67). With two threads a row and eight warps a CTA 125: a third more instructions.
 //
-// Every wait has a limit: when one runs out the CTA stops waiting, writes NaN and ends.
+// Every wait has a limit: when one runs out no thread of the CTA waits any more, the loader takes over nothing more, and the CTA ends with its last
+// blocks of the grid (and one that it had taken over already) written as not a number and the status word set.
 #include "tc_common.cuh"
 #include "../../include/phi3_b200.h"
 #include <type_traits>
@@ -31,18 +32,6 @@ namespace {
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr int BOX = 64 * 128;                                // bytes of one 64-row x 64-column box
 
-// bounded: a try may rest for up to 10 ms, a wait of 200 of them gives up
-__device__ __forceinline__ void wait_lim(uint32_t bar, uint32_t parity, volatile int* fail) {
-    uint32_t ok, tries = 0;
-    do {
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 10000000;\nselp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (!ok) {
-            if (*fail) return;
-            if (++tries > 200) { *fail = 1; return; }
-        }
-    } while (!ok);
-}
 __device__ __forceinline__ float ex2f(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -106,6 +95,7 @@ constexpr int PEN_LD = 104;
 constexpr int ST = 2;                                        // pages in flight (as many as score buffers)
 constexpr int W_LOAD = 4, W_MMA = 5, THREADS = 192;
 constexpr int TMEM = 256, O_COL = 128;                       // S(buffer) at 64 buffer, O at O_COL
+constexpr int ITEMS = 8;                                     // grid blocks that a CTA remembers: the loader is at most four passes ahead of the outputs
 constexpr int TURN = 2048;                                   // bytes of a warp's block of outputs: 32 rows x 64 bytes
 // Q of up to 2 boxes x 128 rows, K and V pages of up to 2 boxes, penalty slices, blocks of outputs
 size_t win_smem(int kb, int vb) { return (size_t)kb * 2 * BOX + (size_t)ST * (kb + vb) * BOX + 4 * 4 * PEN_LD * 4 + 4 * TURN + 1024; }
@@ -115,12 +105,12 @@ struct Pass { int4 rec[2]; int n, lo_pg, n_keep, h0, mine; };  // n: pages (0: n
 
 template <bool PEN, bool SIG>
 __global__ void __launch_bounds__(THREADS, 2)
-attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
+attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* status) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(16) Pass pass_s[2];
     __shared__ __align__(16) uint4 next_s;
-    __shared__ __align__(8) uint64_t bars_s[1 + 4 * ST + 6 + 5];
-    __shared__ int fail_s;
+    __shared__ __align__(8) uint64_t bars_s[1 + 4 * ST + 6 + 6];
+    __shared__ int fail_s, items_s[ITEMS];
     __shared__ uint32_t tmem_s;
     volatile int* fail = &fail_s;
     const int d = a.dim, dv = a.vdim, kb = (d + 63) / 64, vb = (dv + 63) / 64, rep = a.n_heads / a.n_kv;
@@ -138,7 +128,7 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
     auto o_done = [&](int p) { return bars + 8u * (13 + (p & 1)); };
     auto pass_full = [&](int i) { return bars + 8u * (15 + (i & 1)); };
     auto pass_empty = [&](int i) { return bars + 8u * (17 + (i & 1)); };
-    const uint32_t next_full = bars + 8u * 19;
+    const uint32_t next_full = bars + 8u * 19, drained = bars + 8u * 20;
     auto ph = [](int p) { return (uint32_t)(p >> 1) & 1u; };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp == W_MMA) {
@@ -149,9 +139,10 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
                 mbar_init(s_full(p), 1); mbar_init(o_done(p), 1); mbar_init(sm_done(p), 4);
                 mbar_init(pass_full(p), 1); mbar_init(pass_empty(p), 5);
             }
-            mbar_init(next_full, 1);
+            mbar_init(next_full, 1); mbar_init(drained, 1);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             fail_s = 0;
+            for (int k = 0; k < ITEMS; k++) items_s[k] = -1;
         }
         __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_s)), "n"(TMEM) : "memory");
@@ -210,6 +201,7 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
         for (int item = blockIdx.x; item >= 0; taken++) {
             // the grid's next CTA that has not started is taken over after this one: its rows' pages are on the way while these outputs are written
             if (lane == 0) {
+                items_s[taken % ITEMS] = item;
                 mbar_expect_tx(next_full, 16);
                 asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(&next_s)), "r"(next_full) : "memory");
             }
@@ -228,20 +220,22 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
                 int page = 0, page1 = bt[page_at(0)];    // ids of pages it, it + 1
                 const int mine = both ? 3 : ta == grp * n_tc ? 1 : 2;
                 if (lane == 0) {
-                    wait_lim(pass_empty(passes), ph(passes) ^ 1u, fail);
-                    Pass& ps = pass_s[passes & 1];
-                    ps.rec[0] = r0; ps.rec[1] = r1; ps.n = n; ps.lo_pg = lo_pg; ps.n_keep = n_keep; ps.h0 = h0; ps.mine = mine;
-                    mbar_arrive(pass_full(passes));
+                    mbar_wait_lim(pass_empty(passes), ph(passes) ^ 1u, fail);
+                    if (!*fail) {                        // else the place may be in use
+                        Pass& ps = pass_s[passes & 1];
+                        ps.rec[0] = r0; ps.rec[1] = r1; ps.n = n; ps.lo_pg = lo_pg; ps.n_keep = n_keep; ps.h0 = h0; ps.mine = mine;
+                        mbar_arrive(pass_full(passes));
+                    }
                 }
                 __syncwarp();
                 for (int it = -1; it < n; it++) {        // K one page ahead of V: its stage comes free earlier
                     const int page2 = it + 2 < n ? bt[page_at(it + 2)] : 0, p = page_0 + it;
                     if (it + 1 < n) {
-                        wait_lim(k_empty(p + 1), ph(p + 1) ^ 1u, fail);
+                        mbar_wait_lim(k_empty(p + 1), ph(p + 1) ^ 1u, fail);
                         stage(sK + ((p + 1) & 1) * kb * BOX, (const bf16*)a.k_pool + ((size_t)page1 * a.n_kv + g) * 64 * d, k_at, d, k_per, k_full(p + 1));
                     }
                     if (it < 0) {                        // the queries, once the scores of the pass before are there
-                        if (p >= 0) wait_lim(k_empty(p), ph(p), fail);
+                        if (p >= 0) mbar_wait_lim(k_empty(p), ph(p), fail);
                         auto copy_q = [&](auto lanes) {  // lanes per row
                             constexpr int LPR = decltype(lanes)::value, PER = 32 / LPR;
                             const int c = lane % LPR, hi = lane / LPR;
@@ -259,7 +253,7 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
                         if (kb == 2) copy_q(std::integral_constant<int, 16>{}); else copy_q(std::integral_constant<int, 8>{});
                         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(q_full) : "memory");
                     } else {
-                        wait_lim(v_empty(p), ph(p) ^ 1u, fail);
+                        mbar_wait_lim(v_empty(p), ph(p) ^ 1u, fail);
                         const uint32_t dst = sV + (p & 1) * vb * BOX;
                         const bf16* src = (const bf16*)a.v_pool + ((size_t)page * a.n_kv + g) * 64 * v_ld;
                         if (v_whole) stage(dst, src, v_at, v_cols, v_per, v_full(p));
@@ -276,24 +270,31 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
                 page_0 += n;
                 ta = both ? t_end : ta + 1;
             }
-            wait_lim(next_full, taken & 1u, fail);
+            const bool came = __all_sync(0xffffffffu, mbar_drain(next_full, taken & 1u));       // in flight: waited for even where nothing else is
+            if (!came) *fail = 1;
             uint32_t more, x = 0;
             asm volatile("{\n.reg .pred p;\n.reg .b128 h;\nld.shared.b128 h, [%2];\nclusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n"
                          "selp.u32 %0, 1, 0, p;\nmov.u32 %1, 0;\n@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n}"
                          : "=r"(more), "=r"(x) : "r"(smem_u32(&next_s)) : "memory");
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            item = more && !*fail ? (int)x : -1;
+            item = came && more ? (int)x : -1;
+            if (__any_sync(0xffffffffu, *fail)) {
+                if (lane == 0) items_s[(taken + 1) % ITEMS] = item;
+                break;
+            }
         }
         if (lane == 0) {
-            wait_lim(pass_empty(passes), ph(passes) ^ 1u, fail);
-            pass_s[passes & 1].n = 0;
-            mbar_arrive(pass_full(passes));
+            mbar_wait_lim(pass_empty(passes), ph(passes) ^ 1u, fail);
+            if (!*fail) {
+                pass_s[passes & 1].n = 0;
+                mbar_arrive(pass_full(passes));
+            }
         }
         cp_async_wait<0>();
         for (int p = max(0, page_0 - ST); p < page_0; p++) {       // nothing is in flight when the CTA ends
-            wait_lim(k_empty(p), ph(p), fail);
-            wait_lim(v_empty(p), ph(p), fail);
+            mbar_wait_lim(k_empty(p), ph(p), fail);
+            mbar_wait_lim(v_empty(p), ph(p), fail);
         }
     } else if (warp == W_MMA) {
         // MMA issuer: one thread, its products at constant distances from what a page starts from
@@ -305,18 +306,18 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
             constexpr int KS = decltype(steps)::value;
             const int ks = KS ? KS : d / 16;
             for (int i = 0, page_0 = 0;; i++) {
-                wait_lim(pass_full(i), ph(i), fail);
+                mbar_wait_lim(pass_full(i), ph(i), fail);
                 const int n = *reinterpret_cast<volatile int*>(&pass_s[i & 1].n);
                 mbar_arrive(pass_empty(i));
                 if (n <= 0 || *fail) break;
-                wait_lim(q_full, i & 1, fail);
+                mbar_wait_lim(q_full, i & 1, fail);
                 for (int t = 0; t < n + 2; t++) {
                     const int p = page_0 + t, j = p - 2;
-                    if (t >= 2) wait_lim(v_full(j), ph(j), fail);
-                    if (t < n) wait_lim(k_full(p), ph(p), fail);
+                    if (t >= 2) mbar_wait_lim(v_full(j), ph(j), fail);
+                    if (t < n) mbar_wait_lim(k_full(p), ph(p), fail);
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the copies, for the tensor cores
                     if (t >= 2) {                        // O += P(j) V(j)
-                        wait_lim(sm_done(j), ph(j), fail);
+                        mbar_wait_lim(sm_done(j), ph(j), fail);
                         tc_fence_after();
                         const uint32_t o = tmem + O_COL, pc = tmem + (j & 1) * 64;
                         const uint64_t vd = vd0 + (uint32_t)((j & 1) * vb * (BOX >> 4));
@@ -340,6 +341,7 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
                 }
                 page_0 += n;
             }
+            if (*fail) { tc_commit(drained); mbar_drain(drained, 0); }               // products that nothing waited for
         };
         if (elect_one()) {
             if (d == 128) issue(std::integral_constant<int, 8>{});
@@ -353,14 +355,14 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
         const int u = warp >> 1, r0 = (warp & 1) * 32, i = r0 + lane;
         const uint32_t t_lane = tmem + ((uint32_t)(warp * 32) << 16), t_o = t_lane + O_COL;
         for (int pass = 0, page_0 = 0;; pass++) {
-            wait_lim(pass_full(pass), ph(pass), fail);
+            mbar_wait_lim(pass_full(pass), ph(pass), fail);
             const Pass& now = pass_s[pass & 1];
             const int n = now.n, n_keep = now.n_keep, past_keep = now.lo_pg - now.n_keep, h = now.h0 + u % n_hc;
             const bool mine = now.mine >> (u / n_hc) & 1;
             const int4 rec = now.rec[u / n_hc];
             __syncwarp();
             if (lane == 0) mbar_arrive(pass_empty(pass));
-            if (n <= 0 || *fail) break;
+            if (n <= 0 || __any_sync(0xffffffffu, *fail)) break;
             auto page_at = [&](int it) { return it < n_keep ? it : past_keep + it; };
             const int nq = mine ? rec.y : 0, pos = rec.w + i;
             const bool row_ok = i < nq;
@@ -398,10 +400,10 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
                     __syncwarp();
                     if (it + 1 < n) pen_fetch(it + 1);
                 }
-                wait_lim(s_full(p), ph(p), fail);
+                mbar_wait_lim(s_full(p), ph(p), fail);
                 tc_fence_after();
                 auto scale_o = [&](float cf) {
-                    if (it > 0) { wait_lim(o_done(p - 1), ph(p - 1), fail); tc_fence_after(); }
+                    if (it > 0) { mbar_wait_lim(o_done(p - 1), ph(p - 1), fail); tc_fence_after(); }
 #pragma unroll 1
                     for (int c = 0; c < dv; c += 16) {
                         uint32_t v[16];
@@ -515,13 +517,12 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
             }
             // ---- epilogue: O / l, gates
             page_0 += n;
-            if (n > 1) wait_lim(o_done(page_0 - 2), ph(page_0 - 2), fail);
-            wait_lim(o_done(page_0 - 1), ph(page_0 - 1), fail);
+            if (n > 1) mbar_wait_lim(o_done(page_0 - 2), ph(page_0 - 2), fail);
+            mbar_wait_lim(o_done(page_0 - 1), ph(page_0 - 1), fail);
             tc_fence_after();
             if (mine && any_rows) {
                 float inv = (a.gate && row_ok ? a.gate[((size_t)rec.x + i) * a.n_heads + h] : 1.f) * (a.out_scale != 0.f ? a.out_scale : 1.f);
                 if (!SIG) inv = l > 0.f ? inv / l : 0.f;
-                if (*fail) inv = __int_as_float(0x7fc00000);
                 // row-wise out of TMEM into the warp's block, and from there in pieces of 64 bytes of a row (32 with gates: four lanes a row, eight
                 // rows an instruction) to memory; a lane writing its own row took an instruction of the load-store unit per row and 16 bytes.
                 // 16-byte pieces are swizzled: no bank conflicts either way. Without element-wise gates 32 columns go as bf16, else 16 as fp32.
@@ -603,6 +604,18 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc) {
     tc_fence_before();
     __syncthreads();                                         // nothing is in flight, O is read
     tc_fence_after();
+    if (*fail) {                                             // which of these rows were written before is not known
+        for (int k = 0; k < ITEMS; k++) {
+            const int item = items_s[k], hgs = a.n_heads / n_hc, grp = (a.n_tiles + n_tc - 1) / n_tc - 1 - item / hgs;
+            if (item < 0) continue;
+            for (int t = grp * n_tc; t < min(a.n_tiles, (grp + 1) * n_tc); t++) {
+                const int4 r = reinterpret_cast<const int4*>(a.tiles)[t];
+                for (int i = threadIdx.x; i < r.y * n_hc * dv; i += THREADS)
+                    ((bf16*)a.out)[(size_t)(r.x + i / (n_hc * dv)) * a.ld_out + (size_t)(item % hgs * n_hc) * dv + i % (n_hc * dv)] = __float2bfloat16_rn(__int_as_float(0x7fc00000));
+            }
+        }
+        if (threadIdx.x == 0) set_status(status);
+    }
     if (warp == W_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TMEM) : "memory");
 }
 
@@ -616,7 +629,7 @@ int launch(const p3_attn_window_args* a, int n_hc, int n_tc, cudaStream_t st) {
         set = true;
     }
     const int64_t grid = (int64_t)((a->n_tiles + n_tc - 1) / n_tc) * (a->n_heads / n_hc);
-    p3_launch_pdl(attn_window_prefill_tc_kernel<PEN, SIG>, dim3((unsigned)grid), dim3(THREADS), bytes, st, *a, n_hc, n_tc);
+    p3_launch_pdl(attn_window_prefill_tc_kernel<PEN, SIG>, dim3((unsigned)grid), dim3(THREADS), bytes, st, *a, n_hc, n_tc, p3_status_word());
     return 0;
 }
 }  // namespace

@@ -17,9 +17,17 @@ extern "C" const char* p3_last_error(void);
 void p3_set_error(const char* fmt, ...);
 #define P3_CHECK_ARG(cond, ...)                                    \
     do { if (!(cond)) { p3_set_error(__VA_ARGS__); return -1; } } while (0)
+// Kernels with bounded waits that end without a fault: one whose wait runs out writes what is not a number over the outputs it owes, sets the status
+// word (host memory, read by the next entry point that launches something, which answers with an error) and ends.
+int* p3_status_word();                                     // api.cu; null where no host memory can be had
+bool p3_take_status();                                     // api.cu: was it set since the last time?
+__device__ __forceinline__ void set_status(int* word) {
+    if (word) { *reinterpret_cast<volatile int*>(word) = 1; __threadfence_system(); }
+}
 #define P3_CHECK_LAUNCH(name)                                                              \
     do { cudaError_t e_ = cudaGetLastError();                                              \
-         if (e_ != cudaSuccess) { p3_set_error("%s: %s", name, cudaGetErrorString(e_)); return -2; } } while (0)
+         if (e_ != cudaSuccess) { p3_set_error("%s: %s", name, cudaGetErrorString(e_)); return -2; } \
+         if (p3_take_status()) { p3_set_error("%s: a wait inside a kernel launched earlier ran out; outputs of that launch are not numbers", name); return -3; } } while (0)
 
 #define P3_TRACE_CTAS 1024
 unsigned long long* p3_trace_slot();                       // api.cu: next trace slot or null

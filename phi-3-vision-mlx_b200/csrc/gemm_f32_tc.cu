@@ -13,6 +13,8 @@
 //   warp 24:     issues the MMAs of a block. A warp that also splits cannot: 24 of them take about 1000 clocks to issue.
 // Bound by the split (five instructions a number, every CTA its own rows of X and W), then by the MMAs: a block of 128 x 96 takes 1.2 us, without
 // the split 1.1, with 4 of 24 MMAs 1.0. 512 x 3072 x 1024: 27 us (FMA kernel 100), 1200 x 4096 x 3072: 175 (723), 64 x 3072 x 1024: 15 (36).
+// A wait that runs out sets the status word; every tile that the CTA writes from then on is not a number (roles walk the tiles alike, so that none waits for
+// another beyond that).
 // Infinities have no parts: a warp that finds something else than a finite number among its sums forms them again, one FMA chain per output.
 #include <type_traits>
 #include "tc_common.cuh"
@@ -27,18 +29,6 @@ constexpr int ACC_COL = STAGES * A_COLS;
 constexpr int TMEM = 512;                                    // 3 x 96 for X, 2 x BN sums
 constexpr size_t f32tc_smem(int bn) { return (size_t)STAGES * 3 * bn * KB * 2 + 1024; }
 
-// bounded: a try may rest for up to 10 ms, a wait of 200 of them gives up
-__device__ __forceinline__ void wait_lim(uint32_t bar, uint32_t parity, volatile int* fail) {
-    uint32_t ok, tries = 0;
-    do {
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 10000000;\nselp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (!ok) {
-            if (*fail) return;
-            if (++tries > 200) { *fail = 1; return; }
-        }
-    } while (!ok);
-}
 // 16 TMEM lanes x 8 columns: thread t holds columns 2 (t % 4), + 1 of lane t / 4 in a and of lane t / 4 + 8 in b
 __device__ __forceinline__ void st_16x256b(uint32_t t, const uint32_t (&a)[2], const uint32_t (&b)[2]) {
     asm volatile("tcgen05.st.sync.aligned.16x256b.x1.b32 [%0], {%1,%2,%3,%4};" ::"r"(t), "r"(a[0]), "r"(a[1]), "r"(b[0]), "r"(b[1]) : "memory");
@@ -71,9 +61,9 @@ __device__ __forceinline__ void split4(const float4& f, uint32_t (&p0)[2], uint3
 }
 
 template <typename OT, int BN>
-__global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_tiles, int n_tiles) {
+__global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_tiles, int n_tiles, int* status) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bars_s[2 * STAGES + 4];
+    __shared__ __align__(8) uint64_t bars_s[2 * STAGES + 5];
     __shared__ uint32_t tmem_s;
     __shared__ int fail_s;
     volatile int* fail = &fail_s;
@@ -83,11 +73,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
     auto empty = [&](uint32_t s) { return bars + 8 * (STAGES + s); };                // ... and multiplied
     auto sums = [&](uint32_t s) { return bars + 8 * (2 * STAGES + s); };             // a block's sums are there
     auto taken = [&](uint32_t s) { return bars + 8 * (2 * STAGES + 2 + s); };        // ... and read
+    const uint32_t drained = bars + 8 * (2 * STAGES + 4);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         fail_s = 0;
         for (int s = 0; s < STAGES; s++) { mbar_init(full(s), SPLIT); mbar_init(empty(s), 1); }
         for (int s = 0; s < 2; s++) { mbar_init(sums(s), 1); mbar_init(taken(s), ADD); }
+        mbar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == W_MMA) {
@@ -153,7 +145,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
             auto block = [&](int b, auto mode) {
                 constexpr int MODE = decltype(mode)::value;
                 const int left = MODE == 1 ? KB : p.K - (b + 1) * KB;
-                wait_lim(empty(stage), phase, fail);
+                mbar_wait_lim(empty(stage), phase, fail);
                 tc_fence_after();
 #pragma unroll
                 for (int i = 0; i < 4; i += 2) {
@@ -197,8 +189,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
             int bz, g, m0, m1;
             if (!find(tile, bz, g, m0, m1)) continue;
             for (int b = 0; b < blocks; b++, it++) {
-                wait_lim(taken(it & 1), ((it >> 1) & 1u) ^ 1u, fail);
-                wait_lim(full(stage), phase, fail);
+                mbar_wait_lim(taken(it & 1), ((it >> 1) & 1u) ^ 1u, fail);
+                mbar_wait_lim(full(stage), phase, fail);
                 tc_fence_after();
                 if (elect_one()) {
                     const uint32_t d = tmem + ACC_COL + (it & 1) * BN, a = tmem + stage * A_COLS;
@@ -215,6 +207,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
                 if (++stage == STAGES) { stage = 0; phase ^= 1; }
             }
         }
+        if (__any_sync(0xffffffffu, *fail)) {                // products that nothing waited for
+            if (elect_one()) { tc_commit(drained); mbar_drain(drained, 0); }
+            __syncwarp();
+        }
     } else {
         // ---- sums: TMEM lanes 32 q .., half of the columns of a tile
         constexpr int NC = BN / 2;
@@ -228,7 +224,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
 #pragma unroll
             for (int c = 0; c < NC; c++) acc[c] = 0.f;
             for (int b = 0; b < blocks; b++, it++) {
-                wait_lim(sums(it & 1), (it >> 1) & 1u, fail);
+                mbar_wait_lim(sums(it & 1), (it >> 1) & 1u, fail);
                 tc_fence_after();
 #pragma unroll
                 for (int c0 = 0; c0 < NC; c0 += 8) {
@@ -307,6 +303,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
     tc_fence_before();
     __syncthreads();                                         // nothing is in flight: every block's sums are read
     tc_fence_after();
+    if (threadIdx.x == 0 && *fail) set_status(status);
     if (warp == W_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TMEM) : "memory");
 }
 
@@ -320,7 +317,7 @@ int launch(const AnyP& p, cudaStream_t st) {
     }
     const int64_t m_tiles = ((p.M + TM_ROWS - 1) / TM_ROWS + (p.seg ? p.n_groups : 0)) * p.nb, n_tiles = (p.N + BN - 1) / BN;
     const int64_t tiles = m_tiles * n_tiles;
-    p3_launch_pdl(gemm_f32_tc_kernel<OT, BN>, dim3((unsigned)(tiles < 148 ? tiles : 148)), dim3(THREADS), f32tc_smem(BN), st, p, (int)m_tiles, (int)n_tiles);
+    p3_launch_pdl(gemm_f32_tc_kernel<OT, BN>, dim3((unsigned)(tiles < 148 ? tiles : 148)), dim3(THREADS), f32tc_smem(BN), st, p, (int)m_tiles, (int)n_tiles, p3_status_word());
     return 0;
 }
 template <typename OT>

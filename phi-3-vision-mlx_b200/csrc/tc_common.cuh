@@ -24,6 +24,25 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
         if (!ok && ++spins > (1u << 27)) __trap();            // seconds of spinning: a protocol bug — fail loudly instead of hanging the GPU
     } while (!ok);
 }
+// Bounded wait without a fault: a try may rest for up to 10 ms; a CTA of which one wait ran out of tries has *fail set, and none of its threads waits
+// any more. What the CTA started itself is waited for all the same before it ends (mbar_drain).
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 10000000;\nselp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok;
+}
+__device__ __forceinline__ void mbar_wait_lim(uint32_t bar, uint32_t parity, volatile int* fail, uint32_t limit = 200) {
+    uint32_t tries = 0;
+    while (!mbar_try(bar, parity)) {
+        if (*fail) return;
+        if (++tries > limit) { *fail = 1; return; }
+    }
+}
+__device__ __forceinline__ bool mbar_drain(uint32_t bar, uint32_t parity) {
+    for (int tries = 0; tries < 200; tries++) if (mbar_try(bar, parity)) return true;
+    return false;
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int c0, int c1) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tm)), "r"(bar), "r"(c0), "r"(c1) : "memory");

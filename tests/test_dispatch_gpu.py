@@ -665,3 +665,15 @@ def test_a_call_keeps_no_hold_on_the_buffers_of_its_caller(dev, what, dtype):
     got = m(host['ids'], **kw(host))[0]
     host[what].fill_(1)
     assert torch.equal(got.float().cpu(), want)
+
+
+def test_a_wait_that_runs_out_is_an_error_of_the_next_call(dev):
+    """outputs that are not numbers and an error, once; the device goes on"""
+    from phi3_b200 import _lib
+    out, x = torch.zeros(32, device=dev), torch.ones(4, 8, device=dev)
+    _lib.call('p3_wait_selftest', out.data_ptr(), _stream())
+    torch.cuda.synchronize()
+    assert bool(torch.isnan(out).all())
+    with pytest.raises(RuntimeError, match='ran out'):
+        _gemm_any(x, x)
+    assert torch.equal(_gemm_any(x, x), torch.full((4, 4), 8.0, device=dev))
