@@ -15,7 +15,6 @@
 // the split 1.1, with 4 of 24 MMAs 1.0. 512 x 3072 x 1024: 27 us (FMA kernel 100), 1200 x 4096 x 3072: 175 (723), 64 x 3072 x 1024: 15 (36).
 // A wait that runs out sets the status word; every tile that the CTA writes from then on is not a number (roles walk the tiles alike, so that none waits for
 // another beyond that).
-// Infinities have no parts: a warp that finds something else than a finite number among its sums forms them again, one FMA chain per output.
 #include <type_traits>
 #include "tc_common.cuh"
 #include "gemm_any.cuh"
@@ -47,8 +46,9 @@ __device__ __forceinline__ void add2(float& c0, float& c1, float a0, float a1) {
 }
 __device__ __forceinline__ float upper(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
 __device__ __forceinline__ uint32_t uppers(const float (&x)[2]) { return __byte_perm(__float_as_uint(x[0]), __float_as_uint(x[1]), 0x7632); }
-// four numbers -> three parts of two words each
-__device__ __forceinline__ void split4(const float4& f, uint32_t (&p0)[2], uint32_t (&p1)[2], uint32_t (&p2)[2]) {
+// four numbers -> three parts of two words each. Two parts leave at most eight bits, which are the third's; numbers below 2^-110 and those
+// that are none leave more, in the lower half of their word: `more` collects these bits.
+__device__ __forceinline__ void split4(const float4& f, uint32_t (&p0)[2], uint32_t (&p1)[2], uint32_t (&p2)[2], uint32_t& more) {
 #pragma unroll
     for (int i = 0; i < 2; i++) {
         const float x[2] = {i ? f.z : f.x, i ? f.w : f.y}, xh[2] = {upper(x[0]), upper(x[1])};
@@ -57,13 +57,15 @@ __device__ __forceinline__ void split4(const float4& f, uint32_t (&p0)[2], uint3
         const float rh[2] = {upper(r[0]), upper(r[1])};
         sub2(s, r, rh);
         p0[i] = uppers(x); p1[i] = uppers(r); p2[i] = uppers(s);
+        more |= __float_as_uint(s[0]) | __float_as_uint(s[1]);
     }
 }
 
 template <typename OT, int BN>
 __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_tiles, int n_tiles, int* status) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bars_s[2 * STAGES + 5];
+    __shared__ __align__(8) uint64_t bars_s[2 * STAGES + 7];
+    __shared__ uint32_t rows_s[2][1 + TM_ROWS + BN];          // of two tiles: the last that had such a row anywhere, in row i of X, in row i of W
     __shared__ uint32_t tmem_s;
     __shared__ int fail_s;
     volatile int* fail = &fail_s;
@@ -73,15 +75,17 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
     auto empty = [&](uint32_t s) { return bars + 8 * (STAGES + s); };                // ... and multiplied
     auto sums = [&](uint32_t s) { return bars + 8 * (2 * STAGES + s); };             // a block's sums are there
     auto taken = [&](uint32_t s) { return bars + 8 * (2 * STAGES + 2 + s); };        // ... and read
-    const uint32_t drained = bars + 8 * (2 * STAGES + 4);
+    auto rows_known = [&](uint32_t s) { return bars + 8 * (2 * STAGES + 4 + s); };   // a tile is split: rows_s[s] is written
+    const uint32_t drained = bars + 8 * (2 * STAGES + 6);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         fail_s = 0;
         for (int s = 0; s < STAGES; s++) { mbar_init(full(s), SPLIT); mbar_init(empty(s), 1); }
-        for (int s = 0; s < 2; s++) { mbar_init(sums(s), 1); mbar_init(taken(s), ADD); }
+        for (int s = 0; s < 2; s++) { mbar_init(sums(s), 1); mbar_init(taken(s), ADD); mbar_init(rows_known(s), SPLIT); }
         mbar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    for (int i = threadIdx.x; i < 2 * (1 + TM_ROWS + BN); i += THREADS) (&rows_s[0][0])[i] = 0;
     if (warp == W_MMA) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_s)), "n"(TMEM) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -112,7 +116,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
         const uint32_t ws = base + wr * 128 + ((((wk >> 3) ^ (wr & 7)) << 4) | ((wk & 4) << 1));
         const size_t w_step = (size_t)32 * p.ldw;
         const int whole = p.K / KB;                          // blocks without an end of K inside
-        uint32_t stage = 0, phase = 1;
+        uint32_t stage = 0, phase = 1, count = 0;            // count: tiles of this CTA
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
             int bz, g, m0, m1;
             if (!find(tile, bz, g, m0, m1)) continue;
@@ -140,6 +144,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
 #pragma unroll
             for (int i = 0; i < NB; i++) fetch_w(i, p.K);
             next();
+            uint32_t more_x[2] = {0, 0}, more_w[NB];
+#pragma unroll
+            for (int i = 0; i < NB; i++) more_w[i] = 0;
+            count++;
             // block b is split, and block b + 1 read (mode 0: there is none, 1: whole, 2: it may end at K): what is split is read anew at once, so
             // that the loads of a block have the time of a block
             auto block = [&](int b, auto mode) {
@@ -150,9 +158,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
 #pragma unroll
                 for (int i = 0; i < 4; i += 2) {
                     uint32_t a0[2], a1[2], a2[2], b0[2], b1[2], b2[2];
-                    split4(fx[i], a0, a1, a2);
+                    split4(fx[i], a0, a1, a2, more_x[0]);
                     if (MODE) fetch_x(i, left);
-                    split4(fx[i + 1], b0, b1, b2);
+                    split4(fx[i + 1], b0, b1, b2, more_x[1]);
                     if (MODE) fetch_x(i + 1, left);
                     const uint32_t t = ta + stage * A_COLS + 4 * i;
                     st_16x256b(t, a0, b0); st_16x256b(t + 32, a1, b1); st_16x256b(t + 64, a2, b2);
@@ -160,7 +168,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
 #pragma unroll
                 for (int i = 0; i < NB; i++) {
                     uint32_t p0[2], p1[2], p2[2];
-                    split4(fw[i], p0, p1, p2);
+                    split4(fw[i], p0, p1, p2, more_w[i]);
                     if (MODE) fetch_w(i, left);
                     const uint32_t dst = ws + stage * STAGE + i * 32 * 128;
                     asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(dst), "r"(p0[0]), "r"(p0[1]) : "memory");
@@ -180,6 +188,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
                 else block(b, std::integral_constant<int, 2>{});
             }
             block(blocks - 1, std::integral_constant<int, 0>{});
+            uint32_t* mark = rows_s[count & 1];
+            uint32_t any = 0;
+#pragma unroll
+            for (int i = 0; i < 2; i++) if (more_x[i] & 0xffffu) any = mark[1 + xr + 8 * i] = count;
+#pragma unroll
+            for (int i = 0; i < NB; i++) if (more_w[i] & 0xffffu) any = mark[1 + TM_ROWS + wr + 32 * i] = count;
+            if (any) mark[0] = count;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(rows_known(count & 1));
         }
     } else if (warp == W_MMA) {
         constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TM_ROWS >> 4) << 24);
@@ -216,13 +233,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
         constexpr int NC = BN / 2;
         const int q = warp & 3, half = (warp - W_ADD) >> 2;
         const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16) + ACC_COL + NC * half;
-        uint32_t it = 0;
+        uint32_t it = 0, count = 0;
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
             int bz, g, m0, m1;
             if (!find(tile, bz, g, m0, m1)) continue;
             float acc[NC];
 #pragma unroll
             for (int c = 0; c < NC; c++) acc[c] = 0.f;
+            count++;
             for (int b = 0; b < blocks; b++, it++) {
                 mbar_wait_lim(sums(it & 1), (it >> 1) & 1u, fail);
                 tc_fence_after();
@@ -241,23 +259,24 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
                 if (lane == 0) mbar_arrive(taken(it & 1));
             }
             const int row0 = m0 + 32 * q, n0 = tile / m_tiles * BN + NC * half;
-            // infinity less infinity is none of the parts' sums: what is not a number is summed again as one FMA chain
-            float nan = 0.f;
+            // what is not a finite number, what is so small that TMEM cut off more than fp32 does, and what has a row of numbers without parts is summed
+            // again, behind the others, as one FMA chain
+            constexpr uint32_t SMALL = 15u << 23, NOT_FINITE = 255u << 23;                  // 2^-112
+            uint64_t again = 0;
 #pragma unroll
-            for (int c = 0; c < NC; c++) nan = fmaf(acc[c], 0.f, nan);
-            if (__any_sync(0xffffffffu, row0 + lane < m1 && !(nan == 0.f))) {
-                const int m = min(row0 + lane, m1 - 1);
-                const float* x = (const float*)p.X + (size_t)bz * p.x_bs + (size_t)(p.x_rows ? p.x_rows[m] / p.x_row_div : m) * p.ldx;
-                const float* w = (const float*)p.W + (size_t)g * p.w_gstride + (size_t)bz * p.w_bs;
-#pragma unroll
-                for (int c = 0; c < NC; c++) acc[c] = 0.f;
-#pragma unroll 1
-                for (int k = 0; k < p.K; k++) {
-                    const float xv = __ldg(x + k);
-#pragma unroll
-                    for (int c = 0; c < NC; c++) acc[c] = fmaf(xv, __ldg(w + (size_t)min(n0 + c, p.N - 1) * p.ldw + k), acc[c]);
-                }
+            for (int c = 0; c < NC; c++) {
+                const uint32_t u = __float_as_uint(acc[c]) & 0x7fffffffu;
+                if (u - SMALL >= NOT_FINITE - SMALL && u) again |= 1ull << c;
             }
+            mbar_wait_lim(rows_known(count & 1), ((count - 1) >> 1) & 1u, fail);
+            const volatile uint32_t* no_parts = rows_s[count & 1];
+            if (no_parts[0] == count) {
+                if (no_parts[1 + 32 * q + lane] == count) again = ~0ull;
+#pragma unroll 1
+                for (int c = 0; c < NC; c++) if (no_parts[1 + TM_ROWS + NC * half + c] == count) again |= 1ull << c;
+            }
+            again = n0 < p.N ? again & (~0ull >> (64 - min(NC, p.N - n0))) : 0;
+            if (row0 + lane >= m1 || *fail) again = 0;
             if (*fail) {
 #pragma unroll
                 for (int c = 0; c < NC; c++) acc[c] = __int_as_float(0x7fc00000);
@@ -295,6 +314,33 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
                     } else {
 #pragma unroll
                         for (int e = 0; e < 4; e++) if (n + e < p.N) stf(o + e, v[e]);
+                    }
+                }
+            }
+            if (__any_sync(0xffffffffu, again != 0)) {
+                __syncwarp();                                // the stores above are other lanes'
+                auto chain = [&](int m, int n) {
+                    const float4* x = reinterpret_cast<const float4*>((const float*)p.X + (size_t)bz * p.x_bs + (size_t)(p.x_rows ? p.x_rows[m] / p.x_row_div : m) * p.ldx);
+                    const float4* w = reinterpret_cast<const float4*>((const float*)p.W + (size_t)g * p.w_gstride + (size_t)bz * p.w_bs + (size_t)n * p.ldw);
+                    float v = 0.f;
+#pragma unroll 4
+                    for (int k = 0; k < p.K / 4; k++) {
+                        const float4 a = __ldg(x + k), b = __ldg(w + k);
+                        v = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, v))));
+                    }
+                    v += bias ? bias[n] : 0.f;
+                    if (gate) v *= 1.0f / (1.0f + expf(-gate[(size_t)m * p.ld_gate + n]));
+                    stf(out + (size_t)m * p.ldo + n, v);
+                };
+                // a lane the sums of its row, or all lanes those of a row after the other, whichever takes fewer rounds
+                const int mine = __popcll(again);
+                if (__reduce_max_sync(0xffffffffu, mine) <= __reduce_add_sync(0xffffffffu, (mine + 31) / 32)) {
+                    for (; again; again &= again - 1) chain(row0 + lane, n0 + __ffsll(again) - 1);
+                } else {
+                    for (uint32_t rows = __ballot_sync(0xffffffffu, mine > 0); rows; rows &= rows - 1) {
+                        const int src = __ffs(rows) - 1;
+                        const uint64_t cols = __shfl_sync(0xffffffffu, again, src);
+                        for (int c = lane; c < NC; c += 32) if (cols >> c & 1) chain(row0 + src, n0 + c);
                     }
                 }
             }

@@ -141,6 +141,25 @@ def test_fp32_products_on_the_tensor_cores_of_numbers_without_parts(dev):
     assert ((got - ref).abs()[ok] <= 2.0 ** -14 * scale[ok] + 1e-44).all() and ((got - ref).abs()[12:70][ok[12:70]] <= 2.0 ** -18 * scale[12:70][ok[12:70]]).all()
 
 
+@pytest.mark.parametrize('M,N,K', [(40, 300, 512), (150, 1601, 572), (512, 3072, 1024)])
+def test_fp32_sums_without_parts_are_one_chain_and_leave_the_others_as_they_are(dev, M, N, K):
+    """rows and columns of infinities, of what is not a number and of numbers whose lower bits are below every bf16 have the bits of one FMA chain, every
+    other output those of the product without them; so have sums near the smallest numbers, where TMEM cuts off more than fp32"""
+    g = torch.Generator(device=dev).manual_seed(M)
+    x, w = torch.randn(M, K, generator=g, device=dev), torch.randn(N, K, generator=g, device=dev)
+    clean, xs, ws = _gemm_any(x, w), x.clone(), w.clone()
+    xs[3, 5], xs[37, 0], ws[41, 9], ws[N - 1, K - 1] = float('inf'), float('nan'), float('-inf'), float('inf')
+    xs[11], ws[77, 8] = 1e-38 * xs[11], 1e-37
+    rows, cols = [r for r in range(M) if r not in (3, 11, 37)], [c for c in range(N) if c not in (41, 77, N - 1)]
+    for bias, dt in ((None, F32), (torch.randn(N, generator=g, device=dev), B16)):
+        got, chain, want = _gemm_any(xs, ws, bias, out_dtype=dt), _gemm_any(_odd_pitch(xs), _odd_pitch(ws), bias, out_dtype=dt), clean if bias is None else (clean + bias).to(dt)
+        assert torch.equal(got[rows][:, cols], want[rows][:, cols])
+        assert torch.equal(got[[3, 11, 37]].nan_to_num(7.0), chain[[3, 11, 37]].nan_to_num(7.0))
+        assert torch.equal(got[:, [41, 77, N - 1]].nan_to_num(7.0), chain[:, [41, 77, N - 1]].nan_to_num(7.0))
+    small, chain = (f(x * 2.0 ** -65, w * 2.0 ** -65) for f in (_gemm_any, lambda a, b: _gemm_any(_odd_pitch(a), _odd_pitch(b))))
+    assert torch.equal(small, chain) and bool((small != 0).any())
+
+
 def _attention(dev, H, G, d, dv, lens, window=0, keep=0, chunk=0, sink=True, pen=0, sig=False, gate=False, elem=False, shared=False, scale=None, seed=0,
                offset=0, spread=1.0):
     """ragged prompts [(tokens, position of the first)] through p3_attn_window_prefill, and the same in float64"""
