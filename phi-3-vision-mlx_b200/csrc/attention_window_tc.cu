@@ -18,6 +18,8 @@
 //               The grid's next CTA that has not started is taken over (cluster launch control): its first pages and scores are under way while
 //               the outputs of this one are written; as CTAs of their own they cost 17 000 clocks beside their pages.
 //   warp 5:     one thread issues the MMAs: O += P(j) V(j), then S(j + 2) = Q K(j + 2)^T into the columns P(j) left
+// Two records that share a pass see each other's pages with weights of zero, which a value that is not finite would make something else: the warps of
+// the half that a page does not belong to have nothing to do there but to look its values over, and where one is found they hold O across the page.
 // Bound by the softmax warps: a page of a CTA takes 3000 clocks with two CTAs on an SM, its 64 exponentials a row alone 1000 of them; the MMAs
 // of both keep the tensor cores busy half of the time. 4 x 2048 tokens, 16 heads of 128 over 4, window 1024, penalties: 115 us (mma.sync 298);
 // 333 rows of 32 x 96 behind 704: 39 (67). With two threads a row and eight warps a CTA 125: a third more instructions.
@@ -88,6 +90,45 @@ __device__ __forceinline__ int first_key(const p3_attn_window_args& a, int pos) 
     return lo;
 }
 
+// Are all values of a staged page finite? (two rows a lane; the exponent's bits are all ones where one is not)
+__device__ __noinline__ bool finite_page(uint32_t sv, int dv) {
+    const int lane = threadIdx.x & 31;
+    uint32_t odd = 0;
+#pragma unroll 1
+    for (int k = 0; k < dv / 8; k++)
+#pragma unroll
+        for (int r = lane; r < 64; r += 32) {
+            uint4 x;
+            asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "r"(sv + (k >> 3) * BOX + r * 128 + (((k & 7) ^ (r & 7)) << 4)) : "memory");
+            odd |= ((x.x & 0x7f807f80u) + 0x00800080u) | ((x.y & 0x7f807f80u) + 0x00800080u) | ((x.z & 0x7f807f80u) + 0x00800080u) | ((x.w & 0x7f807f80u) + 0x00800080u);
+        }
+    return !__any_sync(0xffffffffu, odd & 0x80008000u);
+}
+// A page of the other record with such values: O (zero before the pass's first page) is held while the page is multiplied, and put back
+__device__ __noinline__ void hold_o(uint32_t t_o, int dv, bool first, uint32_t done_before, uint32_t ph_before, uint32_t done, uint32_t ph, uint32_t ready, volatile int* fail) {
+    uint32_t held[128];
+    if (!first) { mbar_wait_lim(done_before, ph_before, fail); tc_fence_after(); }
+#pragma unroll 1
+    for (int c = 0; c < dv; c += 16) {
+        uint32_t v[16];
+        ld16(t_o + c, v);
+#pragma unroll
+        for (int k = 0; k < 16; k++) held[c + k] = first ? 0u : v[k];
+    }
+    tc_fence_before();
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(ready);
+    mbar_wait_lim(done, ph, fail);
+    tc_fence_after();
+#pragma unroll 1
+    for (int c = 0; c < dv; c += 16) {
+        uint32_t v[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) v[k] = held[c + k];
+        st16(t_o + c, v);
+    }
+}
+
 // penalties of a warp's 32 rows against its 32 keys: entry t = distance (first row + 31 - t) to the warp's first key, so that a row's columns are
 // neighbours; four copies shifted by 0 .. 3 entries let every lane read 16-byte pieces, and their pitch keeps a quarter-warp on different banks
 constexpr int PEN_LD = 104;
@@ -103,7 +144,8 @@ size_t win_smem(int kb, int vb) { return (size_t)kb * 2 * BOX + (size_t)ST * (kb
 // One pass: up to two records of one sequence, found by the loader for the other warps
 struct Pass { int4 rec[2]; int n, lo_pg, n_keep, h0, mine; };  // n: pages (0: no more work); mine: bit i: record i belongs to the pass
 
-template <bool PEN, bool SIG>
+// PAIR: a pass may hold two records
+template <bool PEN, bool SIG, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 2)
 attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* status) {
     extern __shared__ uint8_t smem_raw[];
@@ -210,7 +252,7 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* st
                 // ---- one pass: the records [ta, tb) of one sequence
                 const int4 r0 = recs[grp * n_tc], r1 = recs[min(grp * n_tc + n_tc, t_end) - 1];
                 const int4 own = ta == grp * n_tc ? r0 : r1;
-                const bool both = ta == grp * n_tc && t_end - ta == 2 && r1.z == r0.z;
+                const bool both = PAIR && ta == grp * n_tc && t_end - ta == 2 && r1.z == r0.z;
                 const int first = both ? min(first_key(a, r0.w), first_key(a, r1.w)) : first_key(a, own.w);
                 const int last = both ? max(r0.w + r0.y, r1.w + r1.y) - 1 : own.w + own.y - 1;
                 // pages: those of the kept first tokens before the window's pages, then from the first visible key to the last row's position
@@ -358,7 +400,7 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* st
             mbar_wait_lim(pass_full(pass), ph(pass), fail);
             const Pass& now = pass_s[pass & 1];
             const int n = now.n, n_keep = now.n_keep, past_keep = now.lo_pg - now.n_keep, h = now.h0 + u % n_hc;
-            const bool mine = now.mine >> (u / n_hc) & 1;
+            const bool mine = now.mine >> (u / n_hc) & 1, shared = PAIR && now.mine == 3;
             const int4 rec = now.rec[u / n_hc];
             __syncwarp();
             if (lane == 0) mbar_arrive(pass_empty(pass));
@@ -374,6 +416,8 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* st
             float m = a.sink ? a.sink[h] * LOG2E : -INFINITY, l = a.sink ? 1.f : 0.f, pend = 1.f;     // pend: what O and l are to be multiplied by
             const int lo = first_key(a, pos), warp_lo = rec.w + r0, warp_hi = rec.w + min(nq - 1, r0 + 31), lo_hi = first_key(a, max(warp_hi, 0));
             const bool any_rows = r0 < nq, all_rows = r0 + 32 <= nq;
+            // this record's own pages, where another shares the pass
+            const int lo_own = first_key(a, rec.w) >> 6, hi_own = (rec.w + nq - 1) >> 6, keep_own = min((a.keep_first + 63) >> 6, lo_own);
             float* ps = reinterpret_cast<float*>(smem_raw + pen_off) + warp * 4 * PEN_LD;
             const float* pl = ps + ((31 - lane) & 3) * PEN_LD + ((31 - lane) & ~3);          // this lane's copy, column 0
             float pn[3];
@@ -513,7 +557,18 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* st
                 tc_wait_st();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(sm_done(p));
+                bool arrive = true;
+                if (shared) {
+                    const int pg = j0 >> 6;
+                    if (pg >= keep_own && (pg < lo_own || pg > hi_own)) {
+                        mbar_wait_lim(v_full(p), ph(p), fail);
+                        if (!finite_page(sV + (p & 1) * vb * BOX, dv)) {
+                            hold_o(t_o, dv, it == 0, o_done(p - 1), ph(p - 1), o_done(p), ph(p), sm_done(p), fail);
+                            arrive = false;
+                        }
+                    }
+                }
+                if (arrive && lane == 0) mbar_arrive(sm_done(p));
             }
             // ---- epilogue: O / l, gates
             page_0 += n;
@@ -619,17 +674,17 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* st
     if (warp == W_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TMEM) : "memory");
 }
 
-template <bool PEN, bool SIG>
+template <bool PEN, bool SIG, bool PAIR>
 int launch(const p3_attn_window_args* a, int n_hc, int n_tc, cudaStream_t st) {
     const size_t bytes = win_smem((a->dim + 63) / 64, (a->vdim + 63) / 64);
     static P3DevFlags flags; bool& set = flags.cur();
     if (!set) {
-        cudaError_t e = cudaFuncSetAttribute(attn_window_prefill_tc_kernel<PEN, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)win_smem(2, 2));
+        cudaError_t e = cudaFuncSetAttribute(attn_window_prefill_tc_kernel<PEN, SIG, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)win_smem(2, 2));
         P3_CHECK_ARG(e == cudaSuccess, "attn_window_prefill: shared memory attribute: %s", cudaGetErrorString(e));
         set = true;
     }
     const int64_t grid = (int64_t)((a->n_tiles + n_tc - 1) / n_tc) * (a->n_heads / n_hc);
-    p3_launch_pdl(attn_window_prefill_tc_kernel<PEN, SIG>, dim3((unsigned)grid), dim3(THREADS), bytes, st, *a, n_hc, n_tc, p3_status_word());
+    p3_launch_pdl(attn_window_prefill_tc_kernel<PEN, SIG, PAIR>, dim3((unsigned)grid), dim3(THREADS), bytes, st, *a, n_hc, n_tc, p3_status_word());
     return 0;
 }
 }  // namespace
@@ -645,6 +700,10 @@ int launch_attn_window_tc(const p3_attn_window_args* a, cudaStream_t st) {
     // 32 heads of 96 on 96 CTAs 37 us, on 192 half empty ones 42.
     int n_hc = (a->n_heads / a->n_kv) % 2 == 0 ? 2 : 1, n_tc = 2 / n_hc;
     if ((int64_t)((a->n_tiles + n_tc - 1) / n_tc) * (a->n_heads / n_hc) < 74) n_hc = n_tc = 1;
-    if (a->sig_bias) return a->penalty ? launch<true, true>(a, n_hc, n_tc, st) : launch<false, true>(a, n_hc, n_tc, st);
-    return a->penalty ? launch<true, false>(a, n_hc, n_tc, st) : launch<false, false>(a, n_hc, n_tc, st);
+    if (n_tc == 2) {
+        if (a->sig_bias) return a->penalty ? launch<true, true, true>(a, n_hc, n_tc, st) : launch<false, true, true>(a, n_hc, n_tc, st);
+        return a->penalty ? launch<true, false, true>(a, n_hc, n_tc, st) : launch<false, false, true>(a, n_hc, n_tc, st);
+    }
+    if (a->sig_bias) return a->penalty ? launch<true, true, false>(a, n_hc, n_tc, st) : launch<false, true, false>(a, n_hc, n_tc, st);
+    return a->penalty ? launch<true, false, false>(a, n_hc, n_tc, st) : launch<false, false, false>(a, n_hc, n_tc, st);
 }

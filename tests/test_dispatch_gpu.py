@@ -161,8 +161,9 @@ def test_fp32_sums_without_parts_are_one_chain_and_leave_the_others_as_they_are(
 
 
 def _attention(dev, H, G, d, dv, lens, window=0, keep=0, chunk=0, sink=True, pen=0, sig=False, gate=False, elem=False, shared=False, scale=None, seed=0,
-               offset=0, spread=1.0):
-    """ragged prompts [(tokens, position of the first)] through p3_attn_window_prefill, and the same in float64"""
+               offset=0, spread=1.0, poison=None):
+    """ragged prompts [(tokens, position of the first)] through p3_attn_window_prefill, and the same in float64. poison: a position whose values are
+    infinite in the pool, and not in the float64 result"""
     from phi3_b200 import _lib
     g = torch.Generator(device=dev).manual_seed(seed)
     rn = lambda *s: torch.randn(s, generator=g, device=dev)
@@ -183,6 +184,8 @@ def _attention(dev, H, G, d, dv, lens, window=0, keep=0, chunk=0, sink=True, pen
         for pool, t in ((kp, k),) if shared else ((kp, k), (vp, v)):
             full = torch.full((pages * 64, G, t.shape[-1]), 5.0, dtype=B16, device=dev)
             full[:n + p] = t
+            if poison is not None and pool is vp and poison < n + p:
+                full[poison] = float('inf')
             pool[ids] = full.view(pages, 64, G, -1).transpose(1, 2)
         tiles += [(r + i, min(64, n - i), s, p + i) for i in range(0, n, 64)]
         i, j = torch.arange(p, p + n, device=dev)[:, None], torch.arange(n + p, device=dev)[None]
@@ -254,6 +257,32 @@ def test_prefill_attention_at_scales_of_zero_and_below(dev, shape, scale, kind):
     assert bool(torch.isfinite(y).all())
     assert float((y - ref).norm() / ref.norm()) < 6e-3
     assert float((y - ref).abs().max()) < 2.0 ** -6 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize('H,G,d,dv', [(48, 48, 96, 96), (60, 20, 64, 128), (80, 40, 128, 64)])
+@pytest.mark.parametrize('kind', ['plain', 'window', 'keep', 'kept pages', 'sigmoid', 'chunk'])
+@pytest.mark.parametrize('lens', [[(200, 0)], [(300, 100), (130, 30)], [(64, 64), (129, 191)]])
+def test_values_that_are_not_finite_stay_with_the_records_whose_pages_hold_them(dev, H, G, d, dv, kind, lens):
+    """a record of up to 64 rows is multiplied by the pages from the first key of its first row to its last row (and those of the kept tokens), and by
+    no page beside them, although two neighbouring records of a sequence may share a pass: all other rows keep their bits"""
+    kw = {'plain': dict(), 'window': dict(window=70, pen=70), 'keep': dict(window=40, keep=10), 'kept pages': dict(window=65, keep=130),
+          'sigmoid': dict(sink=False, sig=True, window=90), 'chunk': dict(chunk=80)}[kind]
+    window, keep, chunk = kw.get('window', 0), kw.get('keep', 0), kw.get('chunk', 0)
+    clean, _ = _attention(dev, H, G, d, dv, lens, seed=d, **kw)
+    hit = 0
+    for poison in range(3, max(n + p for n, p in lens), 61):
+        y, _ = _attention(dev, H, G, d, dv, lens, seed=d, poison=poison, **kw)
+        r = 0
+        for n, p in lens:
+            for i in range(0, n, 64):
+                rows, at, last = min(64, n - i), p + i, p + min(n, i + 64) - 1
+                lo = max(max(0, at - window + 1) if window else 0, at - at % chunk if chunk else 0) // 64
+                own = poison < n + p and (poison // 64 < min((keep + 63) // 64, lo) or lo <= poison // 64 <= last // 64)
+                if not own:
+                    assert torch.equal(y[r + i:r + i + rows], clean[r + i:r + i + rows]), (poison, at)
+                    hit += 1
+            r += n
+    assert hit
 
 
 def test_prefill_attention_with_one_shared_row_per_token(dev):
