@@ -2,8 +2,9 @@
 // bf16 with key sizes and value sizes that are multiples of 16 up to 128.
 //
 // A pass = 128 query rows against the pages of one sequence and K/V head, in two halves of 64 rows; a half is one tile record x one query
-// head. The halves are n_hc query heads of one group x n_tc neighbouring tile records (n_hc n_tc <= 2), so that grouped-query heads share the
-// K/V pages that a CTA stages. Records of different sequences take a pass each. Two CTAs share an SM.
+// head. The halves are two query heads of one group, so that grouped-query heads share the K/V pages that a CTA stages, or, in groups of odd
+// size, two neighbouring tile records of a sequence (the block of the second takes both; records whose neighbour is another sequence's take a
+// pass each, with one half idle). Two CTAs share an SM.
 //   warps 0-3:  softmax, a query row (TMEM lane) per thread. S is double buffered in TMEM, so the scores of the next two pages are computed while
 //               this one is swept, 32 keys at a time; P goes back over the consumed S columns and is the A operand of P.V straight from TMEM.
 //               P is formed against the reference maximum of the pages before (base-2 domain; the sink is the first reference, with a
@@ -18,11 +19,12 @@
 //               The grid's next CTA that has not started is taken over (cluster launch control): its first pages and scores are under way while
 //               the outputs of this one are written; as CTAs of their own they cost 17 000 clocks beside their pages.
 //   warp 5:     one thread issues the MMAs: O += P(j) V(j), then S(j + 2) = Q K(j + 2)^T into the columns P(j) left
-// Two records that share a pass see each other's pages with weights of zero, which a value that is not finite would make something else: the warps of
-// the half that a page does not belong to have nothing to do there but to look its values over, and where one is found they hold O across the page.
+// A page that belongs to one record of a pass only is multiplied by weights of zero for the other, which a value that is not finite would make something
+// else: the idle half's warps look the page's values over, and where there is one they hold O across the page.
 // Bound by the softmax warps: a page of a CTA takes 3000 clocks with two CTAs on an SM, its 64 exponentials a row alone 1000 of them; the MMAs
-// of both keep the tensor cores busy half of the time. 4 x 2048 tokens, 16 heads of 128 over 4, window 1024, penalties: 115 us (mma.sync 298);
-// 333 rows of 32 x 96 behind 704: 39 (67). With two threads a row and eight warps a CTA 125: a third more instructions.
+// of both keep the tensor cores busy half of the time. 4 x 2048 tokens, 16 heads of 128 over 4, window 1024, penalties: 114 us (mma.sync 298);
+// 333 rows of 32 x 96 behind 704: 39 (67); 16 prompts of 60 tokens behind 500, 16 heads of 96: 0.6 of mma.sync. With two threads a row and eight
+// warps a CTA 125 instead of 115: a third more instructions.
 //
 // Every wait has a limit: when one runs out no thread of the CTA waits any more, the loader takes over nothing more, and the CTA ends with its last
 // blocks of the grid (and one that it had taken over already) written as not a number and the status word set.
@@ -90,45 +92,6 @@ __device__ __forceinline__ int first_key(const p3_attn_window_args& a, int pos) 
     return lo;
 }
 
-// Are all values of a staged page finite? (two rows a lane; the exponent's bits are all ones where one is not)
-__device__ __noinline__ bool finite_page(uint32_t sv, int dv) {
-    const int lane = threadIdx.x & 31;
-    uint32_t odd = 0;
-#pragma unroll 1
-    for (int k = 0; k < dv / 8; k++)
-#pragma unroll
-        for (int r = lane; r < 64; r += 32) {
-            uint4 x;
-            asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "r"(sv + (k >> 3) * BOX + r * 128 + (((k & 7) ^ (r & 7)) << 4)) : "memory");
-            odd |= ((x.x & 0x7f807f80u) + 0x00800080u) | ((x.y & 0x7f807f80u) + 0x00800080u) | ((x.z & 0x7f807f80u) + 0x00800080u) | ((x.w & 0x7f807f80u) + 0x00800080u);
-        }
-    return !__any_sync(0xffffffffu, odd & 0x80008000u);
-}
-// A page of the other record with such values: O (zero before the pass's first page) is held while the page is multiplied, and put back
-__device__ __noinline__ void hold_o(uint32_t t_o, int dv, bool first, uint32_t done_before, uint32_t ph_before, uint32_t done, uint32_t ph, uint32_t ready, volatile int* fail) {
-    uint32_t held[128];
-    if (!first) { mbar_wait_lim(done_before, ph_before, fail); tc_fence_after(); }
-#pragma unroll 1
-    for (int c = 0; c < dv; c += 16) {
-        uint32_t v[16];
-        ld16(t_o + c, v);
-#pragma unroll
-        for (int k = 0; k < 16; k++) held[c + k] = first ? 0u : v[k];
-    }
-    tc_fence_before();
-    __syncwarp();
-    if ((threadIdx.x & 31) == 0) mbar_arrive(ready);
-    mbar_wait_lim(done, ph, fail);
-    tc_fence_after();
-#pragma unroll 1
-    for (int c = 0; c < dv; c += 16) {
-        uint32_t v[16];
-#pragma unroll
-        for (int k = 0; k < 16; k++) v[k] = held[c + k];
-        st16(t_o + c, v);
-    }
-}
-
 // penalties of a warp's 32 rows against its 32 keys: entry t = distance (first row + 31 - t) to the warp's first key, so that a row's columns are
 // neighbours; four copies shifted by 0 .. 3 entries let every lane read 16-byte pieces, and their pitch keeps a quarter-warp on different banks
 constexpr int PEN_LD = 104;
@@ -136,22 +99,88 @@ constexpr int PEN_LD = 104;
 constexpr int ST = 2;                                        // pages in flight (as many as score buffers)
 constexpr int W_LOAD = 4, W_MMA = 5, THREADS = 192;
 constexpr int TMEM = 256, O_COL = 128;                       // S(buffer) at 64 buffer, O at O_COL
-constexpr int ITEMS = 8;                                     // grid blocks that a CTA remembers: the loader is at most four passes ahead of the outputs
+constexpr int ITEMS = 8;                                     // passes whose grid blocks a CTA remembers: the loader is at most four ahead of the outputs
 constexpr int TURN = 2048;                                   // bytes of a warp's block of outputs: 32 rows x 64 bytes
 // Q of up to 2 boxes x 128 rows, K and V pages of up to 2 boxes, penalty slices, blocks of outputs
 size_t win_smem(int kb, int vb) { return (size_t)kb * 2 * BOX + (size_t)ST * (kb + vb) * BOX + 4 * 4 * PEN_LD * 4 + 4 * TURN + 1024; }
 
+// barriers: index of the first of two (by page or pass), but for Q_FULL, NEXT_FULL and DRAINED
+enum { Q_FULL = 0, K_FULL = 1, K_EMPTY = 3, V_FULL = 5, V_EMPTY = 7, S_FULL = 9, SM_DONE = 11, O_DONE = 13, PASS_FULL = 15, PASS_EMPTY = 17, NEXT_FULL = 19, DRAINED = 20, BARS = 21 };
+__device__ __forceinline__ uint32_t ph(int p) { return (uint32_t)(p >> 1) & 1u; }
+
 // One pass: up to two records of one sequence, found by the loader for the other warps
 struct Pass { int4 rec[2]; int n, lo_pg, n_keep, h0, mine; };  // n: pages (0: no more work); mine: bit i: record i belongs to the pass
 
-// PAIR: a pass may hold two records
+// A page of the other record (softmax warps): weights of zero, and O, zero before the pass's first page, held across the page if a value of it is not finite
+// (two rows a lane; a number times zero, added up, stays zero)
+__device__ __noinline__ void other_page(uint32_t bars, int p, bool first, uint32_t t_lane, uint32_t sv, int dv, volatile int* fail) {
+    const int lane = threadIdx.x & 31;
+    auto bar = [&](int first_of_two, int q) { return bars + 8u * (first_of_two + (q & 1)); };
+    uint32_t w[32], z[2] = {0u, 0u};
+#pragma unroll
+    for (int k = 0; k < 32; k++) w[k] = 0u;
+    mbar_wait_lim(bar(S_FULL, p), ph(p), fail);
+    tc_fence_after();
+    tc_st32_nowait(t_lane + (p & 1) * 64, w);
+    tc_st32_nowait(t_lane + (p & 1) * 64 + 32, w);
+    mbar_wait_lim(bar(V_FULL, p), ph(p), fail);
+#pragma unroll 2
+    for (int k = 0; k < dv / 8; k++)
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            uint4 x;
+            asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w)
+                         : "r"(sv + (k >> 3) * BOX + (lane + 32 * r) * 128 + (((k & 7) ^ (lane & 7)) << 4)) : "memory");
+            asm("{\n.reg .b32 t;\nfma.rn.bf16x2 t, %1, %5, %0;\nfma.rn.bf16x2 t, %2, %5, t;\nfma.rn.bf16x2 t, %3, %5, t;\nfma.rn.bf16x2 %0, %4, %5, t;\n}"
+                : "+r"(z[r]) : "r"(x.x), "r"(x.y), "r"(x.z), "r"(x.w), "r"(0));
+        }
+    const bool hold = __any_sync(0xffffffffu, ((z[0] | z[1]) & 0x7fff7fffu) != 0u);
+    uint32_t held[128];
+    if (hold) {
+        if (!first) { mbar_wait_lim(bar(O_DONE, p - 1), ph(p - 1), fail); tc_fence_after(); }
+#pragma unroll 1
+        for (int c = 0; c < dv; c += 16) {
+            uint32_t v[16];
+            ld16(t_lane + O_COL + c, v);
+#pragma unroll
+            for (int k = 0; k < 16; k++) held[c + k] = first ? 0u : v[k];
+        }
+    }
+    tc_wait_st();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar(SM_DONE, p));
+    if (hold) {
+        mbar_wait_lim(bar(O_DONE, p), ph(p), fail);
+        tc_fence_after();
+#pragma unroll 1
+        for (int c = 0; c < dv; c += 16) {
+            uint32_t v[16];
+#pragma unroll
+            for (int k = 0; k < 16; k++) v[k] = held[c + k];
+            st16(t_lane + O_COL + c, v);
+        }
+    }
+}
+
+// Tile record of the i-th blocks of the grid: later ones (more keys) first. With pairs those that always have a pass, the second records and the last if it has
+// no partner, before the first records, most of which went with their partners.
+template <bool PAIR>
+__device__ __forceinline__ int tile_of(int i, int n) {
+    if (!PAIR) return n - 1 - i;
+    const int early = (n + 1) / 2;
+    if (i < early) return n - 2 * i - ((n & 1) == 0 || i == 0 ? 1 : 0);
+    return (n & ~1) - 2 - 2 * (i - early);
+}
+
+// PAIR: neighbouring records of a sequence share a pass
 template <bool PEN, bool SIG, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 2)
-attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* status) {
+attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int* status) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(16) Pass pass_s[2];
     __shared__ __align__(16) uint4 next_s;
-    __shared__ __align__(8) uint64_t bars_s[1 + 4 * ST + 6 + 6];
+    __shared__ __align__(8) uint64_t bars_s[BARS];
     __shared__ int fail_s, items_s[ITEMS];
     __shared__ uint32_t tmem_s;
     volatile int* fail = &fail_s;
@@ -160,18 +189,17 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* st
     const uint32_t sQ = base, sK = sQ + kb * 2 * BOX, sV = sK + ST * kb * BOX;
     const uint32_t pen_off = sV + ST * vb * BOX - raw, turn = raw + pen_off + 4 * 4 * PEN_LD * 4, bars = smem_u32(bars_s);
     // pages are counted through all passes of the CTA
-    const uint32_t q_full = bars;
-    auto k_full = [&](int p) { return bars + 8u * (1 + (p & 1)); };
-    auto k_empty = [&](int p) { return bars + 8u * (3 + (p & 1)); };
-    auto v_full = [&](int p) { return bars + 8u * (5 + (p & 1)); };
-    auto v_empty = [&](int p) { return bars + 8u * (7 + (p & 1)); };
-    auto s_full = [&](int p) { return bars + 8u * (9 + (p & 1)); };
-    auto sm_done = [&](int p) { return bars + 8u * (11 + (p & 1)); };
-    auto o_done = [&](int p) { return bars + 8u * (13 + (p & 1)); };
-    auto pass_full = [&](int i) { return bars + 8u * (15 + (i & 1)); };
-    auto pass_empty = [&](int i) { return bars + 8u * (17 + (i & 1)); };
-    const uint32_t next_full = bars + 8u * 19, drained = bars + 8u * 20;
-    auto ph = [](int p) { return (uint32_t)(p >> 1) & 1u; };
+    const uint32_t q_full = bars + 8u * Q_FULL;
+    auto k_full = [&](int p) { return bars + 8u * (K_FULL + (p & 1)); };
+    auto k_empty = [&](int p) { return bars + 8u * (K_EMPTY + (p & 1)); };
+    auto v_full = [&](int p) { return bars + 8u * (V_FULL + (p & 1)); };
+    auto v_empty = [&](int p) { return bars + 8u * (V_EMPTY + (p & 1)); };
+    auto s_full = [&](int p) { return bars + 8u * (S_FULL + (p & 1)); };
+    auto sm_done = [&](int p) { return bars + 8u * (SM_DONE + (p & 1)); };
+    auto o_done = [&](int p) { return bars + 8u * (O_DONE + (p & 1)); };
+    auto pass_full = [&](int i) { return bars + 8u * (PASS_FULL + (i & 1)); };
+    auto pass_empty = [&](int i) { return bars + 8u * (PASS_EMPTY + (i & 1)); };
+    const uint32_t next_full = bars + 8u * NEXT_FULL, drained = bars + 8u * DRAINED;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp == W_MMA) {
         if (lane == 0) {
@@ -238,30 +266,33 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* st
         };
         const int k_per = period(d), v_cols = v_whole ? v_ld : dv, v_per = period(v_cols);
         const int4* recs = reinterpret_cast<const int4*>(a.tiles);
-        const int hgs = a.n_heads / n_hc, groups = (a.n_tiles + n_tc - 1) / n_tc;
+        const int hgs = a.n_heads / n_hc, keep_pg = (a.keep_first + 63) / 64;
         int page_0 = 0, passes = 0, taken = 0;           // pages before this pass, passes, CTAs taken over
         for (int item = blockIdx.x; item >= 0; taken++) {
-            // the grid's next CTA that has not started is taken over after this one: its rows' pages are on the way while these outputs are written
-            if (lane == 0) {
-                items_s[taken % ITEMS] = item;
-                mbar_expect_tx(next_full, 16);
-                asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(&next_s)), "r"(next_full) : "memory");
-            }
-            const int grp = groups - 1 - item / hgs, h0 = item % hgs * n_hc, g = h0 / rep, t_end = min(a.n_tiles, (grp + 1) * n_tc);   // later tiles (more keys) first
-            for (int ta = grp * n_tc; ta < t_end; passes++) {
-                // ---- one pass: the records [ta, tb) of one sequence
-                const int4 r0 = recs[grp * n_tc], r1 = recs[min(grp * n_tc + n_tc, t_end) - 1];
-                const int4 own = ta == grp * n_tc ? r0 : r1;
-                const bool both = PAIR && ta == grp * n_tc && t_end - ta == 2 && r1.z == r0.z;
+            // The grid's next CTA that has not started is taken over after this one: its rows' pages are on the way while these outputs are written. Where
+            // blocks may turn out to be without a pass it is asked for once the pages of this one are on the way, so that none waits behind a
+            // long pass while other CTAs find nothing to do.
+            auto take_over = [&]() {
+                if (lane == 0) {
+                    mbar_expect_tx(next_full, 16);
+                    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(&next_s)), "r"(next_full) : "memory");
+                }
+            };
+            if (!PAIR) take_over();
+            const int t = tile_of<PAIR>(item / hgs, a.n_tiles), h0 = item % hgs * n_hc, g = h0 / rep;
+            const int4 r0 = recs[PAIR ? t & ~1 : t], r1 = PAIR ? recs[min(t | 1, a.n_tiles - 1)] : r0, own = PAIR && (t & 1) ? r1 : r0;
+            const bool both = PAIR && (t | 1) < a.n_tiles && r1.z == r0.z && r0.y > 0 && r1.y > 0;
+            if (both ? (t & 1) != 0 : own.y > 0) {       // a pass, unless the block of the next record takes this one too, or there are no rows
                 const int first = both ? min(first_key(a, r0.w), first_key(a, r1.w)) : first_key(a, own.w);
                 const int last = both ? max(r0.w + r0.y, r1.w + r1.y) - 1 : own.w + own.y - 1;
                 // pages: those of the kept first tokens before the window's pages, then from the first visible key to the last row's position
-                const int lo_pg = first / 64, n_keep = min((a.keep_first + 63) / 64, lo_pg), n = n_keep + last / 64 - lo_pg + 1;
+                const int lo_pg = first / 64, n_keep = min(keep_pg, lo_pg), n = n_keep + last / 64 - lo_pg + 1;
                 auto page_at = [&](int it) { return it < n_keep ? it : lo_pg + it - n_keep; };
                 const int32_t* bt = a.block_table + (size_t)own.z * a.bt_stride;
                 int page = 0, page1 = bt[page_at(0)];    // ids of pages it, it + 1
-                const int mine = both ? 3 : ta == grp * n_tc ? 1 : 2;
+                const int mine = both ? 3 : PAIR && (t & 1) ? 2 : 1;
                 if (lane == 0) {
+                    items_s[passes % ITEMS] = item;
                     mbar_wait_lim(pass_empty(passes), ph(passes) ^ 1u, fail);
                     if (!*fail) {                        // else the place may be in use
                         Pass& ps = pass_s[passes & 1];
@@ -310,8 +341,9 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* st
                     page = page1; page1 = page2;
                 }
                 page_0 += n;
-                ta = both ? t_end : ta + 1;
+                passes++;
             }
+            if (PAIR) take_over();
             const bool came = __all_sync(0xffffffffu, mbar_drain(next_full, taken & 1u));       // in flight: waited for even where nothing else is
             if (!came) *fail = 1;
             uint32_t more, x = 0;
@@ -322,7 +354,7 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* st
             __syncwarp();
             item = came && more ? (int)x : -1;
             if (__any_sync(0xffffffffu, *fail)) {
-                if (lane == 0) items_s[(taken + 1) % ITEMS] = item;
+                if (lane == 0) items_s[passes % ITEMS] = item;
                 break;
             }
         }
@@ -402,6 +434,7 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* st
             const int n = now.n, n_keep = now.n_keep, past_keep = now.lo_pg - now.n_keep, h = now.h0 + u % n_hc;
             const bool mine = now.mine >> (u / n_hc) & 1, shared = PAIR && now.mine == 3;
             const int4 rec = now.rec[u / n_hc];
+            const int lo_pg = now.lo_pg;
             __syncwarp();
             if (lane == 0) mbar_arrive(pass_empty(pass));
             if (n <= 0 || __any_sync(0xffffffffu, *fail)) break;
@@ -416,8 +449,6 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* st
             float m = a.sink ? a.sink[h] * LOG2E : -INFINITY, l = a.sink ? 1.f : 0.f, pend = 1.f;     // pend: what O and l are to be multiplied by
             const int lo = first_key(a, pos), warp_lo = rec.w + r0, warp_hi = rec.w + min(nq - 1, r0 + 31), lo_hi = first_key(a, max(warp_hi, 0));
             const bool any_rows = r0 < nq, all_rows = r0 + 32 <= nq;
-            // this record's own pages, where another shares the pass
-            const int lo_own = first_key(a, rec.w) >> 6, hi_own = (rec.w + nq - 1) >> 6, keep_own = min((a.keep_first + 63) >> 6, lo_own);
             float* ps = reinterpret_cast<float*>(smem_raw + pen_off) + warp * 4 * PEN_LD;
             const float* pl = ps + ((31 - lane) & 3) * PEN_LD + ((31 - lane) & ~3);          // this lane's copy, column 0
             float pn[3];
@@ -427,148 +458,151 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* st
 #pragma unroll
                 for (int k = 0; k < 3; k++) pn[k] = p[min(max(dist - 32 * k, 0), a.n_penalty - 1)];
             };
-            if (PEN) pen_fetch(0);
-            for (int it = 0; it < n; it++) {
-                const int j0 = page_at(it) * 64;
-                const int p = page_0 + it;
-                const uint32_t t_s = t_lane + (p & 1) * 64;
-                if (PEN) {
-                    __syncwarp();                            // the page before is read
+            // a record's own pages are two runs of the pass's: kept ones from 0 to x, and from y to `end`
+            int x = 0, y = 0, end = n;
+            if (shared) {
+                const int lo_own = first_key(a, rec.w) / 64, keep_own = min((a.keep_first + 63) / 64, lo_own);
+                if (lo_own > lo_pg) { x = n_keep + max(0, keep_own - lo_pg); y = n_keep + lo_own - lo_pg; }
+                end = n_keep + (rec.w + nq - 1) / 64 - lo_pg + 1;
+            }
+            for (int run = PAIR ? 0 : 1; run < 2; run++) {
+                int it = run ? y : 0;
+                const int stop = run ? end : x;
+                if (PEN && it < stop) pen_fetch(it);
+                for (; it < stop; it++) {
+                    const int j0 = page_at(it) * 64;
+                    const int p = page_0 + it;
+                    const uint32_t t_s = t_lane + (p & 1) * 64;
+                    if (PEN) {
+                        __syncwarp();                            // the page before is read
 #pragma unroll
-                    for (int k = 0; k < 3; k++) {
-                        const float v = -LOG2E * pn[k];
+                        for (int k = 0; k < 3; k++) {
+                            const float v = -LOG2E * pn[k];
 #pragma unroll
-                        for (int c = 0; c < 4; c++)
-                            if (k || lane >= c) ps[c * PEN_LD + lane + 32 * k - c] = v;
+                            for (int c = 0; c < 4; c++)
+                                if (k || lane >= c) ps[c * PEN_LD + lane + 32 * k - c] = v;
+                        }
+                        __syncwarp();
+                        if (it + 1 < stop) pen_fetch(it + 1);
                     }
-                    __syncwarp();
-                    if (it + 1 < n) pen_fetch(it + 1);
-                }
-                mbar_wait_lim(s_full(p), ph(p), fail);
-                tc_fence_after();
-                auto scale_o = [&](float cf) {
-                    if (it > 0) { mbar_wait_lim(o_done(p - 1), ph(p - 1), fail); tc_fence_after(); }
+                    mbar_wait_lim(s_full(p), ph(p), fail);
+                    tc_fence_after();
+                    auto scale_o = [&](float cf) {
+                        if (it > 0) { mbar_wait_lim(o_done(p - 1), ph(p - 1), fail); tc_fence_after(); }
 #pragma unroll 1
-                    for (int c = 0; c < dv; c += 16) {
-                        uint32_t v[16];
-                        ld16(t_o + c, v);
+                        for (int c = 0; c < dv; c += 16) {
+                            uint32_t v[16];
+                            ld16(t_o + c, v);
 #pragma unroll
-                        for (int k = 0; k < 16; k++) v[k] = __float_as_uint(__uint_as_float(v[k]) * cf);
-                        st16(t_o + c, v);
-                    }
-                };
-                auto scale_p = [&](float cf) {               // the weights of the page's first 32 keys, which are behind the older reference
-                    uint32_t w[32];
-                    tc_wait_st();
-                    tc_ld32_nowait(t_s, w);
-                    tc_wait_ld();
-                    tc_reg_fence32(w);
-#pragma unroll
-                    for (int k = 0; k < 16; k++) {
-                        const float2 a0 = unpack_bf16(w[k]), a1 = unpack_bf16(w[16 + k]);
-                        const float p0 = (a0.x + a1.x) * cf, p1 = (a0.y + a1.y) * cf;
-                        w[k] = __byte_perm(__float_as_uint(p0), __float_as_uint(p1), 0x7632);
-                        w[16 + k] = pack_bf16(p0 - __uint_as_float(__float_as_uint(p0) & 0xffff0000u), p1 - __uint_as_float(__float_as_uint(p1) & 0xffff0000u));
-                    }
-                    tc_st32_nowait(t_s, w);
-                };
-                // every key of the page is visible to every row of the warp: behind its first row, and its last row still sees it
-                const bool full = all_rows && j0 + 63 <= warp_lo && (j0 >= lo_hi || j0 + 63 < a.keep_first);
-                const bool none = !any_rows || j0 > warp_hi;
-                const bool whole = __all_sync(0xffffffffu, full);
-                float top = -INFINITY;                       // the page's maximum
-                if (!SIG && __any_sync(0xffffffffu, pend != 1.f)) { scale_o(pend); l *= pend; }
-#pragma unroll
-                for (int hf = 0; hf < 2; hf++) {             // 32 keys at a time: a page of 64 scores, penalties and weights did not fit the registers
-                    uint32_t pk[32];                         // their weights: upper 16 bits, then what they leave
-                    if (none) {
-#pragma unroll
-                        for (int k = 0; k < 32; k++) pk[k] = 0u;
-                    } else {
-                        f2 v[16];
-                        ld32(t_s + 32 * hf, v);
-                        if (PEN) {
-#pragma unroll
-                            for (int k = 0; k < 16; k += 2) {
-                                const ulonglong2 pv = *reinterpret_cast<const ulonglong2*>(pl + 32 * hf + 2 * k);
-                                v[k] = fma2(v[k], scale22, pv.x);
-                                v[k + 1] = fma2(v[k + 1], scale22, pv.y);
-                            }
+                            for (int k = 0; k < 16; k++) v[k] = __float_as_uint(__uint_as_float(v[k]) * cf);
+                            st16(t_o + c, v);
                         }
-                        if (!whole) {                        // a branch, so that whole pages do without the tests of every key
-                            auto below = [](int n) { return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u; };
-                            const int j = j0 + 32 * hf;
-                            const uint32_t seen = row_ok ? below(pos - j + 1) & (~below(lo - j) | below(a.keep_first - j)) : 0u;
+                    };
+                    auto scale_p = [&](float cf) {               // the weights of the page's first 32 keys, which are behind the older reference
+                        uint32_t w[32];
+                        tc_wait_st();
+                        tc_ld32_nowait(t_s, w);
+                        tc_wait_ld();
+                        tc_reg_fence32(w);
 #pragma unroll
-                            for (int k = 0; k < 16; k++) {
-                                const float2 x = unpack2(v[k]);
-                                v[k] = pack2(seen >> (2 * k) & 1u ? x.x : gone, seen >> (2 * k + 1) & 1u ? x.y : gone);
-                            }
+                        for (int k = 0; k < 16; k++) {
+                            const float2 a0 = unpack_bf16(w[k]), a1 = unpack_bf16(w[16 + k]);
+                            const float p0 = (a0.x + a1.x) * cf, p1 = (a0.y + a1.y) * cf;
+                            w[k] = __byte_perm(__float_as_uint(p0), __float_as_uint(p1), 0x7632);
+                            w[16 + k] = pack_bf16(p0 - __uint_as_float(__float_as_uint(p0) & 0xffff0000u), p1 - __uint_as_float(__float_as_uint(p1) & 0xffff0000u));
                         }
-                        if (!SIG) {
-                            float mx[2] = {top, -INFINITY};
+                        tc_st32_nowait(t_s, w);
+                    };
+                    // every key of the page is visible to every row of the warp: behind its first row, and its last row still sees it
+                    const bool full = all_rows && j0 + 63 <= warp_lo && (j0 >= lo_hi || j0 + 63 < a.keep_first);
+                    const bool none = !any_rows || j0 > warp_hi;
+                    const bool whole = __all_sync(0xffffffffu, full);
+                    float top = -INFINITY;                       // the page's maximum
+                    if (!SIG && __any_sync(0xffffffffu, pend != 1.f)) { scale_o(pend); l *= pend; }
 #pragma unroll
-                            for (int k = 0; k < 16; k++) { const float2 x = unpack2(v[k]); mx[k & 1] = max3(mx[k & 1], PEN ? x.x : x.x * scale2, PEN ? x.y : x.y * scale2); }
-                            top = fmaxf(mx[0], mx[1]);
-                        }
-                        float ls;
-                        for (;;) {                           // a second time only for a reference that was none, or 2^64 behind
-                            const float mu = SIG || m == -INFINITY ? 0.f : m;
-                            const f2 mu2 = pack2(-mu, -mu);
-                            f2 sA = 0, sB = 0;
+                    for (int hf = 0; hf < 2; hf++) {             // 32 keys at a time: a page of 64 scores, penalties and weights did not fit the registers
+                        uint32_t pk[32];                         // their weights: upper 16 bits, then what they leave
+                        if (none) {
 #pragma unroll
-                            for (int k = 0; k < 16; k++) {
-                                const f2 x = v[k];
-                                float2 q;
-                                f2 pp;
-                                if (SIG) {                   // 1 / (1 + 2^-(score + bias)); a masked key gives 1 / inf = 0
-                                    q = unpack2(PEN ? sub2(sbias22, x) : fma2(x, scale22, sbias22));
-                                    q = unpack2(add2(pack2(ex2f(q.x), ex2f(q.y)), one2));
-                                    pp = pack2(rcpf(q.x), rcpf(q.y));
-                                } else {
-                                    q = unpack2(PEN ? add2(x, mu2) : fma2(x, scale22, mu2));
-                                    pp = pack2(ex2f(q.x), ex2f(q.y));
-                                    if (k & 1) sA = add2(sA, pp); else sB = add2(sB, pp);
+                            for (int k = 0; k < 32; k++) pk[k] = 0u;
+                        } else {
+                            f2 v[16];
+                            ld32(t_s + 32 * hf, v);
+                            if (PEN) {
+#pragma unroll
+                                for (int k = 0; k < 16; k += 2) {
+                                    const ulonglong2 pv = *reinterpret_cast<const ulonglong2*>(pl + 32 * hf + 2 * k);
+                                    v[k] = fma2(v[k], scale22, pv.x);
+                                    v[k + 1] = fma2(v[k + 1], scale22, pv.y);
                                 }
-                                q = unpack2(pp);
-                                pk[k] = __byte_perm(__float_as_uint(q.x), __float_as_uint(q.y), 0x7632);
-                                const float2 r = unpack2(sub2(pp, pp & 0xffff0000ffff0000ull));
-                                pk[16 + k] = pack_bf16(r.x, r.y);
                             }
-                            const float2 x = unpack2(add2(sA, sB));
-                            ls = x.x + x.y;
-                            if (SIG) break;
-                            const bool redo = m == -INFINITY ? top != -INFINITY : top - m > 64.f;
-                            if (!__any_sync(0xffffffffu, redo)) break;
-                            const float corr = !redo ? 1.f : m == -INFINITY ? 0.f : ex2f(m - top);
-                            if (redo) m = top;
-                            l *= corr;
-                            if (it > 0) scale_o(corr);
-                            if (hf) scale_p(corr);
+                            if (!whole) {                        // a branch, so that whole pages do without the tests of every key
+                                auto below = [](int n) { return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u; };
+                                const int j = j0 + 32 * hf;
+                                const uint32_t seen = row_ok ? below(pos - j + 1) & (~below(lo - j) | below(a.keep_first - j)) : 0u;
+#pragma unroll
+                                for (int k = 0; k < 16; k++) {
+                                    const float2 x = unpack2(v[k]);
+                                    v[k] = pack2(seen >> (2 * k) & 1u ? x.x : gone, seen >> (2 * k + 1) & 1u ? x.y : gone);
+                                }
+                            }
+                            if (!SIG) {
+                                float mx[2] = {top, -INFINITY};
+#pragma unroll
+                                for (int k = 0; k < 16; k++) { const float2 x = unpack2(v[k]); mx[k & 1] = max3(mx[k & 1], PEN ? x.x : x.x * scale2, PEN ? x.y : x.y * scale2); }
+                                top = fmaxf(mx[0], mx[1]);
+                            }
+                            float ls;
+                            for (;;) {                           // a second time only for a reference that was none, or 2^64 behind
+                                const float mu = SIG || m == -INFINITY ? 0.f : m;
+                                const f2 mu2 = pack2(-mu, -mu);
+                                f2 sA = 0, sB = 0;
+#pragma unroll
+                                for (int k = 0; k < 16; k++) {
+                                    const f2 x = v[k];
+                                    float2 q;
+                                    f2 pp;
+                                    if (SIG) {                   // 1 / (1 + 2^-(score + bias)); a masked key gives 1 / inf = 0
+                                        q = unpack2(PEN ? sub2(sbias22, x) : fma2(x, scale22, sbias22));
+                                        q = unpack2(add2(pack2(ex2f(q.x), ex2f(q.y)), one2));
+                                        pp = pack2(rcpf(q.x), rcpf(q.y));
+                                    } else {
+                                        q = unpack2(PEN ? add2(x, mu2) : fma2(x, scale22, mu2));
+                                        pp = pack2(ex2f(q.x), ex2f(q.y));
+                                        if (k & 1) sA = add2(sA, pp); else sB = add2(sB, pp);
+                                    }
+                                    q = unpack2(pp);
+                                    pk[k] = __byte_perm(__float_as_uint(q.x), __float_as_uint(q.y), 0x7632);
+                                    const float2 r = unpack2(sub2(pp, pp & 0xffff0000ffff0000ull));
+                                    pk[16 + k] = pack_bf16(r.x, r.y);
+                                }
+                                const float2 x = unpack2(add2(sA, sB));
+                                ls = x.x + x.y;
+                                if (SIG) break;
+                                const bool redo = m == -INFINITY ? top != -INFINITY : top - m > 64.f;
+                                if (!__any_sync(0xffffffffu, redo)) break;
+                                const float corr = !redo ? 1.f : m == -INFINITY ? 0.f : ex2f(m - top);
+                                if (redo) m = top;
+                                l *= corr;
+                                if (it > 0) scale_o(corr);
+                                if (hf) scale_p(corr);
+                            }
+                            l += ls;
                         }
-                        l += ls;
+                        tc_st32_nowait(t_s + 32 * hf, pk);
                     }
-                    tc_st32_nowait(t_s + 32 * hf, pk);
-                }
-                if (!SIG) {
-                    const float grow = top - m;              // not a number (no key yet) compares false
-                    if (grow > 8.f) { pend = ex2f(-grow); m = top; } else pend = 1.f;
-                }
-                tc_wait_st();
-                tc_fence_before();
-                __syncwarp();
-                bool arrive = true;
-                if (shared) {
-                    const int pg = j0 >> 6;
-                    if (pg >= keep_own && (pg < lo_own || pg > hi_own)) {
-                        mbar_wait_lim(v_full(p), ph(p), fail);
-                        if (!finite_page(sV + (p & 1) * vb * BOX, dv)) {
-                            hold_o(t_o, dv, it == 0, o_done(p - 1), ph(p - 1), o_done(p), ph(p), sm_done(p), fail);
-                            arrive = false;
-                        }
+                    if (!SIG) {
+                        const float grow = top - m;              // not a number (no key yet) compares false
+                        if (grow > 8.f) { pend = ex2f(-grow); m = top; } else pend = 1.f;
                     }
+                    tc_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(sm_done(p));
                 }
-                if (arrive && lane == 0) mbar_arrive(sm_done(p));
+                if (PAIR)
+#pragma unroll 1
+                    for (; it < (run ? n : y); it++) other_page(bars, page_0 + it, it == 0, t_lane, sV + ((page_0 + it) & 1) * vb * BOX, dv, fail);
             }
             // ---- epilogue: O / l, gates
             page_0 += n;
@@ -661,9 +695,9 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* st
     tc_fence_after();
     if (*fail) {                                             // which of these rows were written before is not known
         for (int k = 0; k < ITEMS; k++) {
-            const int item = items_s[k], hgs = a.n_heads / n_hc, grp = (a.n_tiles + n_tc - 1) / n_tc - 1 - item / hgs;
+            const int item = items_s[k], hgs = a.n_heads / n_hc, last = tile_of<PAIR>(item / hgs, a.n_tiles);
             if (item < 0) continue;
-            for (int t = grp * n_tc; t < min(a.n_tiles, (grp + 1) * n_tc); t++) {
+            for (int t = PAIR ? last & ~1 : last; t <= last; t++) {
                 const int4 r = reinterpret_cast<const int4*>(a.tiles)[t];
                 for (int i = threadIdx.x; i < r.y * n_hc * dv; i += THREADS)
                     ((bf16*)a.out)[(size_t)(r.x + i / (n_hc * dv)) * a.ld_out + (size_t)(item % hgs * n_hc) * dv + i % (n_hc * dv)] = __float2bfloat16_rn(__int_as_float(0x7fc00000));
@@ -675,7 +709,7 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_tc, int* st
 }
 
 template <bool PEN, bool SIG, bool PAIR>
-int launch(const p3_attn_window_args* a, int n_hc, int n_tc, cudaStream_t st) {
+int launch(const p3_attn_window_args* a, int n_hc, cudaStream_t st) {
     const size_t bytes = win_smem((a->dim + 63) / 64, (a->vdim + 63) / 64);
     static P3DevFlags flags; bool& set = flags.cur();
     if (!set) {
@@ -683,8 +717,8 @@ int launch(const p3_attn_window_args* a, int n_hc, int n_tc, cudaStream_t st) {
         P3_CHECK_ARG(e == cudaSuccess, "attn_window_prefill: shared memory attribute: %s", cudaGetErrorString(e));
         set = true;
     }
-    const int64_t grid = (int64_t)((a->n_tiles + n_tc - 1) / n_tc) * (a->n_heads / n_hc);
-    p3_launch_pdl(attn_window_prefill_tc_kernel<PEN, SIG, PAIR>, dim3((unsigned)grid), dim3(THREADS), bytes, st, *a, n_hc, n_tc, p3_status_word());
+    const int64_t grid = (int64_t)a->n_tiles * (a->n_heads / n_hc);
+    p3_launch_pdl(attn_window_prefill_tc_kernel<PEN, SIG, PAIR>, dim3((unsigned)grid), dim3(THREADS), bytes, st, *a, n_hc, p3_status_word());
     return 0;
 }
 }  // namespace
@@ -697,13 +731,14 @@ bool attn_window_tc_ok(const p3_attn_window_args* a) {
 
 int launch_attn_window_tc(const p3_attn_window_args* a, cudaStream_t st) {
     // Both halves of a CTA in use, unless that would leave half of the SMs without one (a half alone takes about as long as two): 333 rows of
-    // 32 heads of 96 on 96 CTAs 37 us, on 192 half empty ones 42.
-    int n_hc = (a->n_heads / a->n_kv) % 2 == 0 ? 2 : 1, n_tc = 2 / n_hc;
-    if ((int64_t)((a->n_tiles + n_tc - 1) / n_tc) * (a->n_heads / n_hc) < 74) n_hc = n_tc = 1;
-    if (n_tc == 2) {
-        if (a->sig_bias) return a->penalty ? launch<true, true, true>(a, n_hc, n_tc, st) : launch<false, true, true>(a, n_hc, n_tc, st);
-        return a->penalty ? launch<true, false, true>(a, n_hc, n_tc, st) : launch<false, false, true>(a, n_hc, n_tc, st);
+    // 32 heads of 96 on 96 CTAs 39 us, on 192 half empty ones 42.
+    const bool even = (a->n_heads / a->n_kv) % 2 == 0;
+    const bool two = (even ? (int64_t)a->n_tiles * (a->n_heads / 2) : (int64_t)((a->n_tiles + 1) / 2) * a->n_heads) >= 74;
+    if (two && !even) {
+        if (a->sig_bias) return a->penalty ? launch<true, true, true>(a, 1, st) : launch<false, true, true>(a, 1, st);
+        return a->penalty ? launch<true, false, true>(a, 1, st) : launch<false, false, true>(a, 1, st);
     }
-    if (a->sig_bias) return a->penalty ? launch<true, true, false>(a, n_hc, n_tc, st) : launch<false, true, false>(a, n_hc, n_tc, st);
-    return a->penalty ? launch<true, false, false>(a, n_hc, n_tc, st) : launch<false, false, false>(a, n_hc, n_tc, st);
+    const int n_hc = two ? 2 : 1;
+    if (a->sig_bias) return a->penalty ? launch<true, true, false>(a, n_hc, st) : launch<false, true, false>(a, n_hc, st);
+    return a->penalty ? launch<true, false, false>(a, n_hc, st) : launch<false, false, false>(a, n_hc, st);
 }

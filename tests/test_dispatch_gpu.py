@@ -161,9 +161,9 @@ def test_fp32_sums_without_parts_are_one_chain_and_leave_the_others_as_they_are(
 
 
 def _attention(dev, H, G, d, dv, lens, window=0, keep=0, chunk=0, sink=True, pen=0, sig=False, gate=False, elem=False, shared=False, scale=None, seed=0,
-               offset=0, spread=1.0, poison=None):
+               offset=0, spread=1.0, poison=None, shift=0):
     """ragged prompts [(tokens, position of the first)] through p3_attn_window_prefill, and the same in float64. poison: a position whose values are
-    infinite in the pool, and not in the float64 result"""
+    infinite in the pool, and not in the float64 result. shift: records without rows before the others (1) and between them (2)"""
     from phi3_b200 import _lib
     g = torch.Generator(device=dev).manual_seed(seed)
     rn = lambda *s: torch.randn(s, generator=g, device=dev)
@@ -187,7 +187,7 @@ def _attention(dev, H, G, d, dv, lens, window=0, keep=0, chunk=0, sink=True, pen
             if poison is not None and pool is vp and poison < n + p:
                 full[poison] = float('inf')
             pool[ids] = full.view(pages, 64, G, -1).transpose(1, 2)
-        tiles += [(r + i, min(64, n - i), s, p + i) for i in range(0, n, 64)]
+        tiles += [t for i in range(0, n, 64) for t in [(r + i, 0, s, p + i)] * (shift == 2) + [(r + i, min(64, n - i), s, p + i)]]
         i, j = torch.arange(p, p + n, device=dev)[:, None], torch.arange(n + p, device=dev)[None]
         seen, dist = torch.ones(n, n + p, dtype=torch.bool, device=dev), i - j
         if window:
@@ -212,6 +212,7 @@ def _attention(dev, H, G, d, dv, lens, window=0, keep=0, chunk=0, sink=True, pen
     if gate:
         ref = ref * gt.double()[..., None]
     ref = ref.reshape(T, H * dv) * (torch.sigmoid(eg.double()) if elem else 1.0)
+    tiles = [(0, 0, 0, 0)] * (shift == 1) + tiles
     td, out = torch.tensor(tiles, dtype=torch.int32, device=dev), torch.full((T, H * dv), float('nan'), dtype=B16, device=dev)
     w = _lib.AttnWindowArgs()
     qf = q.reshape(T, H * d)
@@ -283,6 +284,19 @@ def test_values_that_are_not_finite_stay_with_the_records_whose_pages_hold_them(
                     hit += 1
             r += n
     assert hit
+
+
+@pytest.mark.parametrize('H,G,d,dv', [(40, 40, 96, 96), (75, 25, 80, 128)])
+@pytest.mark.parametrize('lens', [[(60, 100)] * 7, [(130, 0), (60, 7), (64, 64), (1, 300), (193, 5)], [(64, 0)], [(320, 64)]])
+@pytest.mark.parametrize('kind', ['plain', 'window', 'keep', 'chunk', 'sigmoid'])
+def test_prefill_attention_of_odd_groups_in_any_order_of_records(dev, H, G, d, dv, lens, kind):
+    """records with a partner in their sequence and without, an odd and an even number of them, and records without rows between them (as the first and the
+    second of a pair, at the start of a chunk too): every row is written, and the bits do not depend on who shares a pass"""
+    kw = {'plain': dict(), 'window': dict(window=70, pen=70), 'keep': dict(window=65, keep=130), 'chunk': dict(chunk=64), 'sigmoid': dict(sink=False, sig=True, window=90)}[kind]
+    y, ref = _attention(dev, H, G, d, dv, lens, seed=d, **kw)
+    assert bool(torch.isfinite(y).all()) and float((y - ref).norm() / ref.norm()) < 6e-3 and float((y - ref).abs().max()) < 2.0 ** -6 * float(ref.abs().max())
+    for shift in (1, 2):
+        assert torch.equal(_attention(dev, H, G, d, dv, lens, seed=d, shift=shift, **kw)[0], y)
 
 
 def test_prefill_attention_with_one_shared_row_per_token(dev):
