@@ -331,9 +331,11 @@ int p3_decode_mega(const p3_mega_args* args, cudaStream_t st);
  * norms, softmax, router and residual sums are fp32 in both. One K pool and one V pool per layer:
  * [page][kv head][P3_PAGE_TOKENS][dim | vdim]; block_table int32 [sequence slot][bt_stride] of page ids. */
 
-/* out[M,N] = X[M,K] W[N,K]^T + bias for any sizes / strides / alignment; X and W both fp32 (no TF32: FMA pipes, or exact
- * splits into bf16 parts on tcgen05 from M = 17, N = 256, K = 512 on) or both bf16
- * (mma.sync when K, ldx, ldw are multiples of 8 and the bases 16-byte aligned, else FMA); fp32 accumulation in ascending k. Grouped bf16
+/* out[M,N] = X[M,K] W[N,K]^T + bias for any sizes / strides / alignment; X and W both fp32 (no TF32) or both bf16 (mma.sync when K, ldx, ldw
+ * are multiples of 8 and the bases 16-byte aligned, else FMA); fp32 accumulation in ascending k. fp32 of aligned rows runs on tcgen05 from M = 17,
+ * N = 256, K = 512 on (few rows a segment excepted): operands as three bf16 numbers that hold their 24 bits, products to 2^-32, sums over 64 numbers
+ * that are added in ascending k; the error against 64 bits is that of one fp32 FMA chain or below it but for rows of a few products (1.4 times at
+ * most where measured). A row has the same bits whatever the other rows are, up to 16 rows and from 17 rows on, but not the same in both. Grouped bf16
  * products of such rows without gather, bias or gate, pitches at least K, run on tcgen05 with the groups found on the device.
  * x_rows (may be NULL): row r reads X[x_rows[r] / x_row_div]. seg_offsets (device int32 [n_groups + 1], may be NULL): rows
  * [seg[g], seg[g+1]) multiply with W + g * w_group_stride and add bias + g * bias_group_stride (grouped expert product; M is

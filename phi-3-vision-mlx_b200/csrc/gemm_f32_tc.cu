@@ -1,18 +1,25 @@
 // fp32 products of p3_gemm_any on the 5th-gen tensor cores, without giving up fp32: an operand x is the sum of three bf16 numbers that hold its
-// 24 bits exactly (the upper 16 bits of x, of what is left, and of what is left then), and of the nine products of such parts the six that reach
-// above 2^-22 of x w are formed. The sum over 64 numbers of k is accumulated in TMEM, smallest products first, so that the accumulator is small
-// but for the last four of its 24 additions; then it is added to the output's running sum in fp32 registers. The tensor cores cut off where
-// fp32 rounds: over all of K in TMEM the error against 64 bits would be 3e-6 of the outputs at K = 3072; in pieces of 64 it is 1.4e-7 .. 1.8e-7
-// (K = 512 .. 3072), one FMA chain over K has 4.0e-7 .. 9.9e-7.
+// 24 bits exactly (the nearest to x, to what that leaves, and the rest), and of the nine products of such parts all but that of the third parts are
+// formed: a product is exact to 2^-32 of itself. The tensor cores cut off where fp32 rounds, so TMEM does not sum all of K: the products of first parts
+// (16 bits each) are summed over 64 numbers of k and then added to the output's running sum in fp32 registers; the others, below 2^-7 of
+// them, have a sum of their own over up to 2048 numbers, smallest products of a block first.
+// Relative error against 64 bits, and that of one FMA chain over K = 512 | 3072 | 8192: dense rows of N(0, 1) 9e-8 | 1.5e-7 | 2.2e-7 (chain 4.1e-7 |
+// 9.9e-7 | 1.6e-6), all positive 1.0e-7 | 1.2e-7 | 2.0e-7 (3.5e-7 | 7.4e-7 | 1.4e-6), one number a row 2.5e-8 (2.5e-8), four 2.6e-8 | 3.8e-8 | 4.5e-8
+// (4.0e-8). Above the chain's only where a few products are all there is: 1.1 times with two or four among 8192 numbers, 1.4 times with four of very
+// different size side by side (5e-8: four cut off a block).
 //
 // One CTA per SM walks output tiles of 128 x BN:
 //   warps 0-15:  a block of 64 numbers of k, read one block ahead into registers, is split and goes to TMEM (X: a row is a TMEM lane) and to shared
 //                memory (W: K-major, 128B swizzle); three stages. With X in TMEM a product reads only W from shared memory: with both operands
-//                there, 24 MMAs and the split's stores ask for more than its 128 bytes a clock.
-//   warps 16-23: the sums of a block are read back (two buffers) and added in registers; epilogue
-//   warp 24:     issues the MMAs of a block. A warp that also splits cannot: 24 of them take about 1000 clocks to issue.
-// Bound by the split (five instructions a number, every CTA its own rows of X and W), then by the MMAs: a block of 128 x 96 takes 1.2 us, without
-// the split 1.1, with 4 of 24 MMAs 1.0. 512 x 3072 x 1024: 27 us (FMA kernel 100), 1200 x 4096 x 3072: 175 (723), 64 x 3072 x 1024: 15 (36).
+//                there, the MMAs and the split's stores ask for more than its 128 bytes a clock.
+//   warps 16-23: the sums of first parts are read back while the other products of the block are formed (one buffer), the others' every 32 blocks, and
+//                added in registers; epilogue
+//   warp 24:     issues the 32 MMAs of a block. A warp that also splits cannot: that takes some 1300 clocks.
+// Bound by the split (five instructions a number, every CTA its own rows of X and W) and the MMAs, about 40 clocks each. With six products
+// (24 MMAs, exact to 2^-24 at worst) 512 x 3072 x 1024 (rows, columns, K) took 27.2 us instead of 29.7 (FMA kernel 102). 1200 x 4096 x 3072: 238 us
+// (725), 64 x 1024 x 3072: 41 (86), 17 x 1024 x 512: 10.9 (16.4).
+// What has no parts is one FMA chain, as on the FMA pipes: rows of X and W with numbers below 2^-110 (their lower parts are below every bf16), above the
+// largest bf16 or not finite, sums that are not finite, and sums below 2^-112, where TMEM cuts off more than fp32 does.
 // A wait that runs out sets the status word; every tile that the CTA writes from then on is not a number (roles walk the tiles alike, so that none waits for
 // another beyond that).
 #include <type_traits>
@@ -21,11 +28,11 @@
 #include "../../include/phi3_b200.h"
 
 namespace {
-constexpr int TM_ROWS = 128, KB = 64, STAGES = 3;
+constexpr int TM_ROWS = 128, KB = 64, STAGES = 3, FLUSH = 32;   // FLUSH: blocks whose small products are summed in TMEM
 constexpr int SPLIT = 16, ADD = 8, W_ADD = SPLIT, W_MMA = SPLIT + ADD, THREADS = 32 * (W_MMA + 1);
 constexpr int A_COLS = 96;                                   // TMEM columns of one stage of X: three parts of 64 bf16
 constexpr int ACC_COL = STAGES * A_COLS;
-constexpr int TMEM = 512;                                    // 3 x 96 for X, 2 x BN sums
+constexpr int TMEM = 512;                                    // 3 x 96 for X, BN sums of products of first parts, BN of the others
 constexpr size_t f32tc_smem(int bn) { return (size_t)STAGES * 3 * bn * KB * 2 + 1024; }
 
 // 16 TMEM lanes x 8 columns: thread t holds columns 2 (t % 4), + 1 of lane t / 4 in a and of lane t / 4 + 8 in b
@@ -44,20 +51,25 @@ __device__ __forceinline__ void sub2(float (&d)[2], const float (&a)[2], const f
 __device__ __forceinline__ void add2(float& c0, float& c1, float a0, float a1) {
     asm("{\n.reg .b64 x, y;\nmov.b64 x, {%0, %1};\nmov.b64 y, {%2, %3};\nadd.rn.f32x2 x, x, y;\nmov.b64 {%0, %1}, x;\n}" : "+f"(c0), "+f"(c1) : "f"(a0), "f"(a1));
 }
-__device__ __forceinline__ float upper(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
-__device__ __forceinline__ uint32_t uppers(const float (&x)[2]) { return __byte_perm(__float_as_uint(x[0]), __float_as_uint(x[1]), 0x7632); }
-// four numbers -> three parts of two words each. Two parts leave at most eight bits, which are the third's; numbers below 2^-110 and those
-// that are none leave more, in the lower half of their word: `more` collects these bits.
+// the nearest bf16 numbers, packed, and what they leave
+__device__ __forceinline__ uint32_t part(const float (&x)[2], float (&rest)[2]) {
+    const uint32_t p = pack_bf16(x[0], x[1]);
+    const float h[2] = {__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u)};
+    sub2(rest, x, h);
+    return p;
+}
+// four numbers -> three parts of two words each. Two parts leave at most eight bits, which are the third's; numbers below 2^-110, above the largest
+// bf16 and those that are none leave more, in the lower half of their word: `more` collects these bits.
 __device__ __forceinline__ void split4(const float4& f, uint32_t (&p0)[2], uint32_t (&p1)[2], uint32_t (&p2)[2], uint32_t& more) {
 #pragma unroll
     for (int i = 0; i < 2; i++) {
-        const float x[2] = {i ? f.z : f.x, i ? f.w : f.y}, xh[2] = {upper(x[0]), upper(x[1])};
+        const float x[2] = {i ? f.z : f.x, i ? f.w : f.y};
         float r[2], s[2];
-        sub2(r, x, xh);
-        const float rh[2] = {upper(r[0]), upper(r[1])};
-        sub2(s, r, rh);
-        p0[i] = uppers(x); p1[i] = uppers(r); p2[i] = uppers(s);
-        more |= __float_as_uint(s[0]) | __float_as_uint(s[1]);
+        p0[i] = part(x, r);
+        p1[i] = part(r, s);
+        const uint32_t s0 = __float_as_uint(s[0]), s1 = __float_as_uint(s[1]);
+        p2[i] = __byte_perm(s0, s1, 0x7632);
+        more |= s0 | s1;
     }
 }
 
@@ -73,7 +85,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u, bars = smem_u32(bars_s);
     auto full = [&](uint32_t s) { return bars + 8 * s; };                            // a stage is split
     auto empty = [&](uint32_t s) { return bars + 8 * (STAGES + s); };                // ... and multiplied
-    auto sums = [&](uint32_t s) { return bars + 8 * (2 * STAGES + s); };             // a block's sums are there
+    auto sums = [&](uint32_t s) { return bars + 8 * (2 * STAGES + s); };             // sums are there (0: of a block's first parts, 1: of the others)
     auto taken = [&](uint32_t s) { return bars + 8 * (2 * STAGES + 2 + s); };        // ... and read
     auto rows_known = [&](uint32_t s) { return bars + 8 * (2 * STAGES + 4 + s); };   // a tile is split: rows_s[s] is written
     const uint32_t drained = bars + 8 * (2 * STAGES + 6);
@@ -201,24 +213,34 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
     } else if (warp == W_MMA) {
         constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TM_ROWS >> 4) << 24);
         const uint64_t wd = umma_desc_sw128(base);
-        uint32_t it = 0, stage = 0, phase = 0;
+        uint32_t it = 0, stage = 0, phase = 0, flush = 0;
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
             int bz, g, m0, m1;
             if (!find(tile, bz, g, m0, m1)) continue;
             for (int b = 0; b < blocks; b++, it++) {
-                mbar_wait_lim(taken(it & 1), ((it >> 1) & 1u) ^ 1u, fail);
+                mbar_wait_lim(taken(0), (it & 1u) ^ 1u, fail);
                 mbar_wait_lim(full(stage), phase, fail);
                 tc_fence_after();
+                const uint32_t a = tmem + stage * A_COLS, hi = tmem + ACC_COL, lo = hi + BN;
+                const uint64_t w = wd + stage * (STAGE >> 4);
                 if (elect_one()) {
-                    const uint32_t d = tmem + ACC_COL + (it & 1) * BN, a = tmem + stage * A_COLS;
-                    const uint64_t w = wd + stage * (STAGE >> 4);
 #pragma unroll
-                    for (int i = 0; i < 24; i++) {           // parts (of X, of W), smallest products first, in four steps of 16 numbers each
-                        constexpr int PX[6] = {2, 0, 1, 1, 0, 0}, PW[6] = {0, 2, 1, 0, 1, 0};
-                        tc_mma_bf16_ts(d, a + 32 * PX[i / 4] + 8 * (i % 4), w + (PW[i / 4] * (PART >> 4) + 2 * (i % 4)), IDESC, i ? 1u : 0u);
+                    for (int i = 0; i < 4; i++) tc_mma_bf16_ts(hi, a + 8 * i, w + 2 * i, IDESC, i ? 1u : 0u);
+                    tc_commit(sums(0));                      // read back while the other products are formed: one buffer is enough
+                }
+                __syncwarp();
+                if (b % FLUSH == 0) {
+                    mbar_wait_lim(taken(1), (flush++ & 1u) ^ 1u, fail);
+                    tc_fence_after();
+                }
+                if (elect_one()) {
+#pragma unroll
+                    for (int i = 0; i < 28; i++) {           // parts (of X, of W), smallest products first, in four steps of 16 numbers each
+                        constexpr int PX[7] = {2, 1, 2, 0, 1, 1, 0}, PW[7] = {1, 2, 0, 2, 1, 0, 1};
+                        tc_mma_bf16_ts(lo, a + 32 * PX[i / 4] + 8 * (i % 4), w + (PW[i / 4] * (PART >> 4) + 2 * (i % 4)), IDESC, i ? 1u : (uint32_t)(b % FLUSH));
                     }
                     tc_commit(empty(stage));
-                    tc_commit(sums(it & 1));
+                    if (b % FLUSH == FLUSH - 1 || b == blocks - 1) tc_commit(sums(1));
                 }
                 __syncwarp();
                 if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -233,7 +255,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
         constexpr int NC = BN / 2;
         const int q = warp & 3, half = (warp - W_ADD) >> 2;
         const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16) + ACC_COL + NC * half;
-        uint32_t it = 0, count = 0;
+        uint32_t it = 0, flush = 0, count = 0;
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
             int bz, g, m0, m1;
             if (!find(tile, bz, g, m0, m1)) continue;
@@ -241,13 +263,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
 #pragma unroll
             for (int c = 0; c < NC; c++) acc[c] = 0.f;
             count++;
-            for (int b = 0; b < blocks; b++, it++) {
-                mbar_wait_lim(sums(it & 1), (it >> 1) & 1u, fail);
+            auto add = [&](int which) {
                 tc_fence_after();
 #pragma unroll
                 for (int c0 = 0; c0 < NC; c0 += 8) {
                     uint32_t v[8];
-                    ld_32x32b_x8(tl + (it & 1) * BN + c0, v);
+                    ld_32x32b_x8(tl + which * BN + c0, v);
                     tc_wait_ld();
 #pragma unroll
                     for (int c = 0; c < 8; c++) asm volatile("" : "+r"(v[c]));
@@ -256,7 +277,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(AnyP p, int m_t
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(taken(it & 1));
+                if (lane == 0) mbar_arrive(taken(which));
+            };
+            for (int b = 0; b < blocks; b++, it++) {
+                mbar_wait_lim(sums(0), it & 1u, fail);
+                add(0);
+                if (b % FLUSH == FLUSH - 1 || b == blocks - 1) {
+                    mbar_wait_lim(sums(1), flush++ & 1u, fail);
+                    add(1);
+                }
             }
             const int row0 = m0 + 32 * q, n0 = tile / m_tiles * BN + NC * half;
             // what is not a finite number, what is so small that TMEM cut off more than fp32 does, and what has a row of numbers without parts is summed
@@ -372,11 +401,12 @@ int launch_width(const AnyP& p, int bn, cudaStream_t st) {
 }
 }  // namespace
 
-// Columns of a tile: the width whose busiest SM is done first. Nanoseconds of a block of 64 numbers of k by width, and of a tile beside its blocks
-// (from 17 x 1024 x 512 to 1200 x 4096 x 3072). 128 columns took longer than 96 at every size: the sums no longer fit the registers.
+// Columns of a tile: the width whose busiest SM is done first. Nanoseconds of a block of 64 numbers of k by width (128 rows, a tile an SM, K from 4096 to
+// 8192), and about those of a tile beside its blocks. 128 columns took longer than 96 at every size: of 72 registers a thread the 96-wide
+// kernel spills 128 bytes already.
 int gemm_f32_tc_width(const void* any_p) {
     const AnyP& p = *static_cast<const AnyP*>(any_p);
-    static const int width[3] = {96, 64, 32}, block[3] = {1180, 950, 690};
+    static const int width[3] = {96, 64, 32}, block[3] = {1450, 1090, 790};
     const int64_t m_tiles = ((p.M + TM_ROWS - 1) / TM_ROWS + (p.seg ? p.n_groups / 2 : 0)) * p.nb, blocks = (p.K + KB - 1) / KB;
     int best = 96;
     int64_t best_cost = INT64_MAX;

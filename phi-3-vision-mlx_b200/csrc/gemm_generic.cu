@@ -5,9 +5,9 @@
 // X and out (one per attention head), with an optional sigmoid gate on the result.
 //
 // fp32 operands keep their 24 bits (no TF32): at most 16 rows as a stream of W, more in register tiles on the FMA pipes, each output one FMA chain
-// in ascending k whatever the tile and the other rows; from 17 rows, 256 columns and K = 512 on as exact splits on the tensor cores
-// (gemm_f32_tc.cu: closer to 64 bits than the chain, and the same bits whatever the tile and the other rows there); a plain kernel for rows
-// that are not 16-byte aligned. bf16 operands of aligned shapes run on the
+// in ascending k whatever the tile and the other rows; from 17 rows, 256 columns and K = 512 on as splits into bf16 parts on the tensor cores
+// (gemm_f32_tc.cu: sums as near to 64 bits as the chain's or nearer, and one row's bits whatever the tile and the other rows there, but not the
+// chain's: a row of a launch of 16 and of 17 rows differs in the last bits); a plain kernel for rows that are not 16-byte aligned. bf16 operands of aligned shapes run on the
 // tensor cores through mma.sync m16n8k16 (fp32 accumulators); the dense bf16 projections with K % 8 == 0 go to the tcgen05
 // kernel (p3_gemm) instead — this file is what is left: grouped expert products, fp32, and shapes p3_gemm does not take.
 #include "gemm_any.cuh"

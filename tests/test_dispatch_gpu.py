@@ -91,10 +91,10 @@ def _rel(y, ref):
 
 @pytest.mark.parametrize('width,M,N,K', [(32, 17, 256, 512), (32, 129, 300, 516), (64, 300, 2056, 1000), (96, 512, 3072, 1024), (96, 1000, 1601, 572), (64, 257, 2053, 1088)])
 def test_fp32_products_on_the_tensor_cores(dev, width, M, N, K):
-    """Rows, columns and numbers that end inside a tile or a block of 64. Of an operand's three parts the second is below 2^-7 and the third below
-    2^-15 of it: the products left out are below 2^-21 of |x| |w|, the additions cut off at most 2^-20 of the sum of magnitudes (24 of a block of
-    64 at 2^-23 of a partial sum that holds 2^-7 of it but for the last four, K / 64 more at 2^-24). The sums are nearer to 64 bits than one
-    FMA chain's, and a row's do not depend on the rows beside it."""
+    """Rows, columns and numbers that end inside a tile or a block of 64. Products are exact to 2^-32; of the sum of magnitudes the additions cut off at
+    most 2^-21 (four a block of 64, at 2^-23 of a partial sum) and 2^-21 (28 a block, 17 blocks, at 2^-23 of the 2^-7 of it that the smaller products
+    are), and K / 64 are rounded, either way, at 2^-24. The sums are nearer to 64 bits than one FMA chain's, and a row's do not depend on the
+    rows beside it."""
     g = torch.Generator(device=dev).manual_seed(M + N)
     rn = lambda *s: torch.randn(s, generator=g, device=dev)
     x, w, bias, gate, tiles = rn(M, K) * torch.exp(2 * rn(M, K)), rn(N, K), rn(N), rn(M, N), []
@@ -158,6 +158,21 @@ def test_fp32_sums_without_parts_are_one_chain_and_leave_the_others_as_they_are(
         assert torch.equal(got[:, [41, 77, N - 1]].nan_to_num(7.0), chain[:, [41, 77, N - 1]].nan_to_num(7.0))
     small, chain = (f(x * 2.0 ** -65, w * 2.0 ** -65) for f in (_gemm_any, lambda a, b: _gemm_any(_odd_pitch(a), _odd_pitch(b))))
     assert torch.equal(small, chain) and bool((small != 0).any())
+
+
+@pytest.mark.parametrize('M,N,K', [(20, 300, 512), (130, 1601, 1088), (512, 3072, 3072)])
+def test_fp32_products_of_few_numbers_are_as_near_to_64_bits_as_one_chain(dev, M, N, K):
+    """rows with 1, 2, 4 or 64 numbers that are not zero, where a product's own rounding is the error: an output of one product is its nearest fp32
+    number (products are exact to 2^-32), sums round no more often than the chain that adds the same numbers one by one (a twentieth for the spread)"""
+    g = torch.Generator(device=dev).manual_seed(M)
+    rn = lambda *s: torch.randn(s, generator=g, device=dev)
+    w, tiles = rn(N, K), []
+    for n in (1, 2, 4, 64):
+        x = torch.zeros(M, K, device=dev).scatter_(1, torch.rand(M, K, generator=g, device=dev).topk(n, dim=1).indices, rn(M, n))
+        y, got, chain = x.double() @ w.double().T, _gemm_any(x, w, tiles=tiles), _gemm_any(_odd_pitch(x), _odd_pitch(w))
+        assert tiles.pop() < 0 and _rel(got, y) <= 1.05 * _rel(chain, y)
+        if n == 1:
+            assert ((got.double() - y).abs() <= (2.0 ** -24 + 2.0 ** -30) * y.abs()).all()
 
 
 def _attention(dev, H, G, d, dv, lens, window=0, keep=0, chunk=0, sink=True, pen=0, sig=False, gate=False, elem=False, shared=False, scale=None, seed=0,
