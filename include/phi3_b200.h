@@ -419,6 +419,8 @@ typedef struct {
 } p3_attn_window_args;
 /* query rows per tile that p3_attn_window_prefill takes for these sizes: 64 on its tensor-core path, else 32 */
 int p3_attn_window_tile_rows(const p3_attn_window_args* args);
+/* 1 where p3_attn_window_prefill runs these arguments on tcgen05, 0 where on mma.sync or the FMA pipes */
+int p3_attn_window_tcgen05(const p3_attn_window_args* args);
 int p3_attn_window_prefill(const p3_attn_window_args* args, cudaStream_t st);
 int p3_attn_window_decode(const p3_attn_window_args* args, cudaStream_t st);
 

@@ -118,7 +118,7 @@ launches = 0          # number of p3_* kernel-launching calls issued (bench.py r
 def exported_symbols():
     return sorted(list(_SIGS) + ['p3_last_error', 'p3_version', 'p3_attention_decode_workspace', 'p3_decode_mega',
                                  'p3_decode_mega_ctas', 'p3_gemm_fused', 'p3_gemm_plan_weights', 'p3_gemm_skinny_x', 'p3_trace_set', 'p3_trace_count',
-                                 'p3_attn_window_tile_rows', 'p3_matrix_memory_state_floats', 'p3_gla_state_floats',
+                                 'p3_attn_window_tile_rows', 'p3_attn_window_tcgen05', 'p3_matrix_memory_state_floats', 'p3_gla_state_floats',
                                  'p3_delta_state_floats']
                   + _STRUCT_ENTRIES)
 
@@ -141,6 +141,7 @@ def lib():
             for name in _STRUCT_ENTRIES:
                 getattr(L, name).argtypes, getattr(L, name).restype = [_p, _p], C.c_int
             L.p3_attn_window_tile_rows.argtypes, L.p3_attn_window_tile_rows.restype = [_p], C.c_int
+            L.p3_attn_window_tcgen05.argtypes, L.p3_attn_window_tcgen05.restype = [_p], C.c_int
             L.p3_matrix_memory_state_floats.argtypes, L.p3_matrix_memory_state_floats.restype = [_i, _i, _i], C.c_int64
             L.p3_gla_state_floats.argtypes, L.p3_gla_state_floats.restype = [_i, _i, _i], C.c_int64
             L.p3_delta_state_floats.argtypes, L.p3_delta_state_floats.restype = [_i, _i, _i], C.c_int64
@@ -157,11 +158,12 @@ def lib():
         L.p3_gemm_fused.argtypes, L.p3_gemm_fused.restype = [_p, _p], C.c_int        # (const p3_gemm_args*, stream)
         L.p3_gemm_plan_weights.argtypes, L.p3_gemm_plan_weights.restype = [_p, _l, _i, _i, _p], C.c_int
         L.p3_gemm_skinny_x.argtypes, L.p3_gemm_skinny_x.restype = [_p, _p], C.c_int        # (const p3_skinny_args*, stream)
-        L.p3_trace_set.argtypes, L.p3_trace_set.restype = [_p, C.c_int], C.c_int           # diagnostics (tools/chain_trace.py)
+        L.p3_trace_set.argtypes, L.p3_trace_set.restype = [_p, C.c_int], C.c_int           # diagnostics
         L.p3_trace_count.argtypes, L.p3_trace_count.restype = [], C.c_int
         for name in _STRUCT_ENTRIES:                                                        # (const args*, stream)
             getattr(L, name).argtypes, getattr(L, name).restype = [_p, _p], C.c_int
         L.p3_attn_window_tile_rows.argtypes, L.p3_attn_window_tile_rows.restype = [_p], C.c_int
+        L.p3_attn_window_tcgen05.argtypes, L.p3_attn_window_tcgen05.restype = [_p], C.c_int
         L.p3_matrix_memory_state_floats.argtypes, L.p3_matrix_memory_state_floats.restype = [_i, _i, _i], C.c_int64
         L.p3_gla_state_floats.argtypes, L.p3_gla_state_floats.restype = [_i, _i, _i], C.c_int64
         L.p3_delta_state_floats.argtypes, L.p3_delta_state_floats.restype = [_i, _i, _i], C.c_int64

@@ -15,7 +15,7 @@
 //   attn_window_prefill_kernel: one CTA = 32 consecutive query tokens of one sequence x one head, key tiles = whole pages, only
 //                               the pages that hold a visible key are visited
 //   attn_window_prefill_mma_kernel: the same on the tensor cores (bf16 mode, head sizes that tile), 64 query rows per CTA; sizes up to 128 of
-//                               whole 16-byte pieces run on tcgen05 instead (attention_window_tc.cu)
+//                               whole 16-byte pieces run on tcgen05 where that is faster (attention_window_tc.cu)
 //   attn_window_decode_kernel:  one CTA = one single-token request x one K/V head (all of its query heads share the K/V reads)
 //                               x one slice of the visible keys, one key per lane; slices merged by attn_window_merge_kernel (on the tensor
 //                               cores up to eight slices inside a cluster)
@@ -1029,6 +1029,9 @@ extern "C" int p3_attn_window_tile_rows(const p3_attn_window_args* a) { return (
 
 bool attn_window_tc_ok(const p3_attn_window_args* a);          // attention_window_tc.cu
 int launch_attn_window_tc(const p3_attn_window_args* a, cudaStream_t st);
+
+/* does p3_attn_window_prefill run on tcgen05 for these arguments? */
+extern "C" int p3_attn_window_tcgen05(const p3_attn_window_args* a) { return a && prefill_mma_ok(a) && attn_window_tc_ok(a); }
 
 extern "C" int p3_attn_window_prefill(const p3_attn_window_args* a, cudaStream_t st) {
     if (check_args(a, "attn_window_prefill")) return -1;

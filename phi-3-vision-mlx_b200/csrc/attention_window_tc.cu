@@ -723,9 +723,25 @@ int launch(const p3_attn_window_args* a, int n_hc, cudaStream_t st) {
 }
 }  // namespace
 
+// Where this kernel is the faster one, measured both ways at 8 to 32 heads and 1 to 128 tiles of rows (us, here and mma.sync). A CTA takes longer until
+// its first outputs, a page less. Above 64 numbers nearly always (1 x 40 tokens, 16 heads of 96: 8.9 and 9.0; 1 x 130: 11.5 and 15.1; 4 x 2048: 143 and
+// 343). mma.sync has three CTAs an SM up to 64 numbers: there with sigmoid weights (two sums a key, no maximum) from the second tile of rows on (16
+// heads of 64, 1 x 64 tokens: 7.1 and 6.8; 1 x 130: 9.8 and 12.7); else once the work, in tiles x heads, fills the SMs well: for 64 numbers from 192 on
+// with two heads of a group a CTA (32 heads over 8, 1 x 333 tokens behind 704: 27.9 and 32.3), from 448 with penalties (192: 15.1 and 14.2, 704: 24.7
+// and 27.4) or two records a CTA (16 heads, 256: 21.7 and 21.8, 480: 30.7 and 33.6, 2048: 112 and 182); not with both (480: 23.3 and 19.9, 2048: 74 and
+// 66); below 64 numbers from 1536 on (48 numbers, 48: 10.7 and 7.0, 960: 52.7 and 50.2, 1536: 91 and 104, 4096: 265 and 307).
+static bool tc_wins(const p3_attn_window_args* a) {
+    const int size = a->dim > a->vdim ? a->dim : a->vdim;
+    const int64_t work = (int64_t)a->n_tiles * a->n_heads;
+    const bool even = (a->n_heads / a->n_kv) % 2 == 0;
+    if (size > 64) return true;
+    if (a->sig_bias) return a->n_tiles > 1;
+    if (a->penalty && !even) return false;
+    return work >= (size <= 48 ? 1536 : even && !a->penalty ? 192 : 448);
+}
 // whole 16-byte pieces everywhere
 bool attn_window_tc_ok(const p3_attn_window_args* a) {
-    return !a->act_f32 && a->dim % 16 == 0 && a->vdim % 16 == 0 && a->dim <= 128 && a->vdim <= 128 && a->ld_q % 8 == 0 && a->ld_out % 8 == 0 &&
+    return tc_wins(a) && !a->act_f32 && a->dim % 16 == 0 && a->vdim % 16 == 0 && a->dim <= 128 && a->vdim <= 128 && a->ld_q % 8 == 0 && a->ld_out % 8 == 0 &&
            a->v_ld % 8 == 0 && (((uintptr_t)a->q | (uintptr_t)a->out | (uintptr_t)a->k_pool | (uintptr_t)a->v_pool) & 15) == 0;
 }
 

@@ -314,6 +314,39 @@ def test_prefill_attention_of_odd_groups_in_any_order_of_records(dev, H, G, d, d
         assert torch.equal(_attention(dev, H, G, d, dv, lens, seed=d, shift=shift, **kw)[0], y)
 
 
+def test_prefill_attention_runs_where_it_is_faster(dev):
+    """above 64 numbers on tcgen05, up to 64 where the work fills the GPU, sigmoid weights from two tiles on"""
+    from phi3_b200 import _lib
+
+    def tc(H, G, d, dv, n_tiles, sig=False, pen=False):
+        a = _lib.AttnWindowArgs()
+        a.q = a.k_pool = a.v_pool = a.out = 4096
+        a.n_heads, a.n_kv, a.dim, a.vdim, a.ld_q, a.ld_out, a.n_tiles = H, G, d, dv, H * d, H * dv, n_tiles
+        a.sig_bias, a.penalty, a.n_penalty = 4096 if sig else None, 4096 if pen else None, 9
+        return _lib.lib().p3_attn_window_tcgen05(ctypes.addressof(a))
+
+    for args, want in (((16, 16, 96, 96, 1), 1), ((16, 16, 64, 80, 1), 1), ((16, 16, 64, 64, 27), 0), ((16, 16, 64, 64, 28), 1), ((16, 8, 64, 64, 11), 0), ((16, 8, 64, 64, 12), 1),
+                       ((16, 8, 64, 64, 27, False, True), 0), ((16, 8, 64, 64, 28, False, True), 1), ((16, 16, 64, 64, 900, False, True), 0), ((16, 8, 48, 48, 95), 0),
+                       ((16, 16, 48, 16, 96), 1), ((8, 8, 64, 64, 1, True), 0), ((8, 8, 64, 16, 2, True), 1), ((16, 16, 132, 96, 9), 0), ((16, 16, 96, 136, 9), 0)):
+        assert tc(*args) == want, args
+
+
+MANY = [(1 + 37 * i % 97, 11 * i % 90) for i in range(66)]       # sequences of one or two records each
+
+
+@pytest.mark.parametrize('H,G,d,dv', [(64, 32, 48, 48), (64, 64, 16, 64), (64, 1, 32, 16), (8, 8, 64, 64), (6, 3, 64, 48), (7, 1, 64, 32)])
+@pytest.mark.parametrize('kind', ['plain', 'window', 'keep', 'chunk', 'sigmoid', 'gates'])
+def test_prefill_attention_of_small_heads_on_both_kernels(dev, H, G, d, dv, kind):
+    """enough records for tcgen05, and one record less of the work on mma.sync: weights of eight bits there, outputs of eight bits in both"""
+    kw = {'plain': dict(sink=False), 'window': dict(window=40, pen=40), 'keep': dict(window=30, keep=70), 'chunk': dict(chunk=50), 'sigmoid': dict(sink=False, sig=True, window=60),
+          'gates': dict(gate=True, elem=True, pen=200)}[kind]
+    for lens in (MANY, MANY[:3]):
+        y, ref = _attention(dev, H, G, d, dv, lens, seed=d, **kw)
+        assert bool(torch.isfinite(y).all())
+        assert float((y - ref).norm() / ref.norm()) < 6e-3
+        assert float((y - ref).abs().max()) < 2.0 ** -6 * float(ref.abs().max())
+
+
 def test_prefill_attention_with_one_shared_row_per_token(dev):
     for H, lens in ((16, [(700, 100), (300, 0)]), (4, [(33, 0)]), (1, [(200, 64)])):
         y, ref = _attention(dev, H, 1, 128, 96, lens, window=512, shared=True, seed=H)
