@@ -440,12 +440,20 @@ static bool aligned_f32(const p3_gemm_any_args* a, int nb) {
     return a->x_f32 && a->K % 4 == 0 && a->ldx % 4 == 0 && a->ldw % 4 == 0 && a->w_group_stride % 4 == 0 &&
            (nb == 1 || (a->x_batch_stride % 4 == 0 && a->w_batch_stride % 4 == 0)) && (((uintptr_t)a->X | (uintptr_t)a->W) & 15) == 0;
 }
-// fp32 on the tensor cores (gemm_f32_tc.cu): from 17 rows on at every size timed (17 x 1024 x 512: 9 us, 17 on the FMA tiles; 512 x 3072 x 1024: 27
-// and 100). Below 512 numbers of k or 256 columns a product stays one FMA chain, the bits of the kernel for any alignment: gates, routers,
+// fp32 on the tensor cores (gemm_f32_tc.cu): dense products from 17 rows on at every size timed (rows, columns, K: 17 x 1024 x 512 10.9 us, 16.4 on the
+// FMA tiles; 17 x 256 x 3072 41 and 86; 512 x 3072 x 1024 29.7 and 102). Below 512 numbers of k or 256 columns a product stays one FMA chain, the bits of the kernel for any alignment: gates, routers,
 // low ranks, products per head.
+// Segments of few rows fill a small part of 128-row tiles: where that makes more tiles than the SMs take at once, FMA tiles of 32 rows are faster for short
+// products (64 segments, 512 columns, FMA and tensor cores: K = 512, 16 rows a segment 51 and 63 us, 64 rows 78 and 76; K = 768, 16 rows 77 and 77;
+// K = 1024, 4 rows 87 and 93, 16 rows 101 and 89; K = 2048, 4 rows 167 and 156). With few tiles the tensor cores were faster at every size (8
+// segments of 512 columns, K = 1024, 17 to 512 rows: 31 .. 41 and 18 .. 33).
+static bool few_rows_a_segment(const p3_gemm_any_args* a) {
+    const int64_t rows = a->K < 768 ? 32 : a->K < 1024 ? 16 : a->K < 1536 ? 8 : 0;
+    return a->seg_offsets && (int64_t)a->n_groups * (((int64_t)a->N + 63) / 64) > 96 && a->M <= a->n_groups * rows;
+}
 static bool f32_tc(const p3_gemm_any_args* a, const AnyP& p) {
     const int64_t tiles = ((a->M + 127) / 128 + (a->seg_offsets ? a->n_groups : 0)) * p.nb * (((int64_t)a->N + 31) / 32);
-    return !a->force_fma && a->M > 16 && a->N >= 256 && a->K >= 512 && tiles < (1ll << 30);
+    return !a->force_fma && a->M > 16 && a->N >= 256 && a->K >= 512 && tiles < (1ll << 30) && !few_rows_a_segment(a);
 }
 extern "C" int p3_gemm_any_tile(const p3_gemm_any_args* a) {
     const AnyP p = any_params(a);

@@ -175,6 +175,20 @@ def test_fp32_products_of_few_numbers_are_as_near_to_64_bits_as_one_chain(dev, M
             assert ((got.double() - y).abs() <= (2.0 ** -24 + 2.0 ** -30) * y.abs()).all()
 
 
+@pytest.mark.parametrize('E,N,K,rows,tc', [(4, 260, 512, 9, True), (32, 256, 512, 32, False), (32, 256, 512, 33, True), (25, 256, 768, 16, False), (25, 256, 768, 17, True), (24, 256, 512, 1, True),
+                                           (13, 512, 1024, 8, False), (13, 512, 1024, 9, True), (13, 512, 1536, 2, True)])
+def test_fp32_grouped_products_of_few_rows_a_segment(dev, E, N, K, rows, tc):
+    """FMA tiles (the bits of the general kernel) where 128-row tiles would be many and nearly empty, the tensor cores else (the bound of their test)"""
+    g = torch.Generator(device=dev).manual_seed(E + rows)
+    x, w, tiles = torch.randn(E * rows, K, generator=g, device=dev), torch.randn(E, N, K, generator=g, device=dev), []
+    cuts = [0] + [i * rows + (min(3, rows // 2) if i % 2 else 0) for i in range(1, E + 1)]             # segments of unequal lengths
+    cuts[-1] = E * rows
+    seg = torch.tensor(cuts, dtype=torch.int32, device=dev)
+    got, ref = _gemm_any(x, w, seg=seg, tiles=tiles), _gemm_any(_odd_pitch(x), _odd_pitch(w), seg=seg)
+    assert (tiles[0] < 0) == tc
+    assert bool(torch.isfinite(ref).all()) and (float((got - ref).norm() / ref.norm()) < 2e-6 if tc else torch.equal(got, ref))
+
+
 def _attention(dev, H, G, d, dv, lens, window=0, keep=0, chunk=0, sink=True, pen=0, sig=False, gate=False, elem=False, shared=False, scale=None, seed=0,
                offset=0, spread=1.0, poison=None, shift=0):
     """ragged prompts [(tokens, position of the first)] through p3_attn_window_prefill, and the same in float64. poison: a position whose values are
