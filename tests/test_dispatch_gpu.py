@@ -190,9 +190,9 @@ def test_fp32_grouped_products_of_few_rows_a_segment(dev, E, N, K, rows, tc):
 
 
 def _attention(dev, H, G, d, dv, lens, window=0, keep=0, chunk=0, sink=True, pen=0, sig=False, gate=False, elem=False, shared=False, scale=None, seed=0,
-               offset=0, spread=1.0, poison=None, shift=0):
+               offset=0, spread=1.0, poison=None, shift=0, turns=False):
     """ragged prompts [(tokens, position of the first)] through p3_attn_window_prefill, and the same in float64. poison: a position whose values are
-    infinite in the pool, and not in the float64 result. shift: records without rows before the others (1) and between them (2)"""
+    infinite in the pool, and not in the float64 result. shift: records without rows before the others (1) and between them (2). turns: values of +1 and -1 in turn, and a third result, of weights rounded to bf16 once"""
     from phi3_b200 import _lib
     g = torch.Generator(device=dev).manual_seed(seed)
     rn = lambda *s: torch.randn(s, generator=g, device=dev)
@@ -204,10 +204,12 @@ def _attention(dev, H, G, d, dv, lens, window=0, keep=0, chunk=0, sink=True, pen
     vp = kp if shared else torch.full((sum(n_pg) + 2, G, 64, dv), 9.0, dtype=B16, device=dev)
     sk, pe = (rn(H) if sink else None), (torch.rand(H, 1, generator=g, device=dev) * torch.log1p(torch.arange(pen, device=dev) * 0.3)[None] if pen else None)
     sb, gt, eg = (rn(H) - 1 if sig else None), (torch.rand(T, H, generator=g, device=dev) if gate else None), (rn(T, H * dv + 3)[:, 3:] if elem else None)
-    refs, tiles, r, at = [], [], 0, 0
+    refs, once, tiles, r, at = [], [], [], 0, 0
     for s, ((n, p), pages) in enumerate(zip(lens, n_pg)):
         k = rn(n + p, G, d).to(B16)
         v = k[..., :dv] if shared else rn(n + p, G, dv).to(B16)
+        if turns:
+            v = (1.0 - 2.0 * (torch.arange(n + p, device=dev) % 2)).to(B16)[:, None, None].expand(n + p, G, dv)
         ids = perm[at:at + pages]
         bt[s, :pages], at = ids.int(), at + pages
         for pool, t in ((kp, k),) if shared else ((kp, k), (vp, v)):
@@ -236,6 +238,8 @@ def _attention(dev, H, G, d, dv, lens, window=0, keep=0, chunk=0, sink=True, pen
             e = torch.exp(sc - m)
             a = e / (e.sum(-1, keepdim=True) + (torch.exp(sk.double()[:, None, None] - m) if sink else 0))
         refs.append(torch.einsum('hts,shd->thd', a, v.double().repeat_interleave(H // G, 1)))
+        if turns:
+            once.append(torch.einsum('hts,shd->thd', e.to(B16).double(), v.double().repeat_interleave(H // G, 1)) / e.sum(-1).T[..., None])
         r += n
     ref = torch.cat(refs)
     if gate:
@@ -251,7 +255,7 @@ def _attention(dev, H, G, d, dv, lens, window=0, keep=0, chunk=0, sink=True, pen
     w.sig_bias, w.elem_gate, w.ld_elem_gate, w.tiles, w.n_tiles = _lib.ptr(sb), _lib.ptr(eg), H * dv + 3, td.data_ptr(), len(tiles)
     _lib.call_struct('p3_attn_window_prefill', w, _stream())
     torch.cuda.synchronize()
-    return out.double(), ref
+    return (out.double(), ref, torch.cat(once).reshape(T, H * dv)) if turns else (out.double(), ref)
 
 
 SHAPES = [  # heads, K/V heads, key size, value size, (tokens, position of the first) of every sequence
@@ -263,8 +267,8 @@ SHAPES = [  # heads, K/V heads, key size, value size, (tokens, position of the f
 @pytest.mark.parametrize('shape', range(len(SHAPES)))
 @pytest.mark.parametrize('kind', ['plain', 'window', 'keep', 'chunk', 'sigmoid', 'gates', 'far', 'turned'])
 def test_prefill_attention_over_ragged_batches(dev, shape, kind):
-    """head groups, sizes of one and two boxes, records of several sequences in one CTA, masks, gates; weights are rounded to bf16 once
-    (relative 2^-9 each, averaging out) and so is the output (2^-9)"""
+    """head groups, sizes of one and two boxes, records of several sequences in one CTA, masks, gates; weights are two bf16 numbers on tcgen05 and one on
+    mma.sync (relative 2^-9 each, averaging out), outputs one (2^-9)"""
     H, G, d, dv, lens = SHAPES[shape]
     kw = {'plain': dict(sink=False), 'window': dict(window=100, pen=100), 'keep': dict(window=65, keep=70), 'chunk': dict(chunk=96),
           'sigmoid': dict(sink=False, sig=True, window=200), 'gates': dict(gate=True, elem=True, pen=5000),
@@ -359,6 +363,18 @@ def test_prefill_attention_of_small_heads_on_both_kernels(dev, H, G, d, dv, kind
         assert bool(torch.isfinite(y).all())
         assert float((y - ref).norm() / ref.norm()) < 6e-3
         assert float((y - ref).abs().max()) < 2.0 ** -6 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize('shape', [0, 1, 4, 8])
+def test_prefill_attention_weights_have_more_than_eight_bits(dev, shape):
+    """values of +1 and -1 in turn under nearly equal weights: what is left of a row with as many of either is the weights' differences, a twentieth of
+    what it is made of, and shows their rounding. Two bf16 numbers a weight leave the rounding of the output (2^-9 at most, 1.7e-3 in the mean
+    square); weights rounded once are off by several times the bound"""
+    H, G, d, dv, lens = SHAPES[shape]
+    y, ref, once = _attention(dev, H, G, d, dv, lens, seed=shape, sink=False, spread=0.05, turns=True)
+    rows = torch.cat([torch.arange(p, p + n, device=dev) for n, p in lens]) % 2 == 1
+    rel = lambda t: float((t - ref)[rows].norm() / ref[rows].norm())
+    assert rel(y) < 3e-3 < 0.5 * rel(once)
 
 
 def test_prefill_attention_with_one_shared_row_per_token(dev):
