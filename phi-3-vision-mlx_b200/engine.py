@@ -25,12 +25,7 @@ import torch
 from . import _lib
 from ._lib import call, ptr
 from .paged import PagePool, PoolExhausted, PAGE
-from .lm_base import StepBatch
-
-
-
-def _stream():
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())     # the current stream's handle without a Stream object
+from .lm_base import StepBatch, _stream
 
 
 class Engine:

@@ -4,8 +4,8 @@ step and the key-slice cost model of the decode attention. A design (tagenex.py,
 gugezen.py) owns its weights and the order of its kernels; it has no cache and no loop of its own.
 
 Matrix products. Dense bf16 products with K % 8 == 0 run on the tcgen05 GEMM (p3_gemm); batches of at most 16 tokens on the
-weight-streaming kernel (p3_gemm_skinny); everything else (fp32 = true 32-bit, on the FMA pipes or as exact splits on tcgen05, grouped expert products, products
-per attention head over column blocks, odd shapes) on p3_gemm_any.
+weight-streaming kernel (p3_gemm_skinny); everything else (fp32 = true 32-bit, on the FMA pipes or in three bf16 parts
+on tcgen05; grouped expert products, products per attention head over column blocks, odd shapes) on p3_gemm_any.
 """
 import ctypes as C
 import os
@@ -15,7 +15,8 @@ from ._lib import call, call_struct, ptr
 
 
 def _stream():
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())     # the current stream's handle without a Stream object
+    """handle of the current stream, without the Stream object that torch.cuda.current_stream() makes for every launch"""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _page_slices(pairs, pages, slots=2 * 148, merge=0.0):

@@ -15,19 +15,14 @@ HBM layout
                  indices and carry kv_start[b] = pad length (replaces Mask4D, phi:550-563)
   quantised KV   full prompt pages as 4-bit codes + bf16 (scale,bias) per 32 values (phi:528-540)
 """
+import contextlib
 import math
 import torch
 from . import _lib
 from ._lib import call, ptr, PAGE
+from .lm_base import _stream
 from .quant import W4, fake_quant
 from .configs import CLIP_VIT_L14_336
-
-
-def _stream():
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())     # the current stream's handle without a Stream object
-
-
-import contextlib
 
 
 @contextlib.contextmanager
@@ -48,7 +43,7 @@ def capture_graph(graph):
 
 
 def pick_splits(n_bh, tiles, slots=2 * 148, max_splits=32):
-    """Split-KV factor for decode attention from a cost model fitted to tools/microbench.py on B200:
+    """Split-KV factor for decode attention from a cost model fitted to the kernel's times on B200:
         T(s) = 2 us + 2.5 us * waves + bytes / min(5.95 TB/s, concurrent_CTAs * 34 GB/s)
     (waves = ceil(n_bh*s / 296 resident CTAs); one CTA alone sustains ~34 GB/s from its 72 KB in
     flight). Long streams per CTA beat full waves: 256 CTAs x 34 pages reach 91 % of the measured
@@ -256,7 +251,7 @@ class Phi3B200:
         self._raw_src = w             # names only looked up for adapter targets (set_adapter); the dict stays the caller's
         # persistent decode-layer kernel (mega.py / decode_mega.cu): a second, stream-order copy of the decoder weights
         # (7.4 GB at Phi-3.5 sizes; HBM has 180 GB). bf16 weights only. Opt-in (P3_MEGA=1) while it is slower than the chain
-        # of per-matrix skinny kernels it replaces (profiles/r02_decode_mega.md).
+        # of per-matrix skinny kernels it replaces.
         self.mega = None
         import os as _os0
         if not self.quantize_model and _os0.environ.get('P3_MEGA', '0') == '1':
@@ -286,7 +281,7 @@ class Phi3B200:
         # bf16(h * gain_of_next_norm), the consumer applies rstd to its reduced accumulators -> no norm kernel, no per-warp
         # re-normalisation inside the K loop, no statistics reduction in front of it. Built for the 4-bit stream (7 -> 5 launches
         # per layer); on bf16 weights it replaces the fused-norm prologue and measured -3.8 % (8 x 2048), -5.3 % (16 x 448), -5.9 %
-        # (4 x 128) per decode step (profiles/r02_split_norm_bf16_ab.log). P3_XG=0 restores the fused / separate norm.
+        # (4 x 128) per decode step. P3_XG=0 restores the fused / separate norm.
         self.xg = _os.environ.get('P3_XG', '1') != '0'
         self.profile = None      # bench.py: list of (kind, ev0, ev1, algorithmic_bytes) when instrumenting
 
