@@ -19,8 +19,7 @@
 //   attn_window_decode_kernel:  one CTA = one single-token request x one K/V head (all of its query heads share the K/V reads)
 //                               x one slice of the visible keys, one key per lane; slices merged by attn_window_merge_kernel (on the tensor
 //                               cores up to eight slices inside a cluster)
-#include "common.cuh"
-#include "../../include/phi3_b200.h"
+#include "attention_window.cuh"
 #include <cfloat>
 #include <cstdlib>
 
@@ -39,15 +38,6 @@ __device__ __forceinline__ float elem_gate(const p3_attn_window_args& a, size_t 
 
 constexpr int BQ = 32, WARPS = 4, RPW = BQ / WARPS;          // prefill: query rows per CTA / per warp
 constexpr int WIDE = 256;                                    // fp32 kernels: key numbers per chunk, value columns per CTA
-
-// first position that a query at `pos` sees (kept first tokens aside): the start of its window, the start of its chunk, or 0. It
-// never falls as pos grows.
-__device__ __forceinline__ int first_key(const p3_attn_window_args& a, int pos) {
-    int lo = 0;
-    if (a.window > 0) lo = max(lo, pos - a.window + 1);
-    if (a.chunk > 0) lo = max(lo, pos - pos % a.chunk);
-    return lo;
-}
 
 // The pages a tile of queries visits: those of the kept first tokens that lie before the window's pages, then the pages from
 // the first key the first row sees to the last row's own position.

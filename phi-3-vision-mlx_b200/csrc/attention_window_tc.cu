@@ -29,7 +29,7 @@
 // Every wait has a limit: when one runs out no thread of the CTA waits any more, the loader takes over nothing more, and the CTA ends with its last
 // blocks of the grid (and one that it had taken over already) written as not a number and the status word set.
 #include "tc_common.cuh"
-#include "../../include/phi3_b200.h"
+#include "attention_window.cuh"
 #include <type_traits>
 
 namespace {
@@ -83,13 +83,6 @@ __device__ __forceinline__ void st16(uint32_t t, const uint32_t* v) {
                  "tcgen05.wait::st.sync.aligned;"
                  ::"r"(t), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
                    "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
-}
-// first position that a query at `pos` sees (kept first tokens aside), as in attention_window.cu
-__device__ __forceinline__ int first_key(const p3_attn_window_args& a, int pos) {
-    int lo = 0;
-    if (a.window > 0) lo = max(lo, pos - a.window + 1);
-    if (a.chunk > 0) lo = max(lo, pos - pos % a.chunk);
-    return lo;
 }
 
 // penalties of a warp's 32 rows against its 32 keys: entry t = distance (first row + 31 - t) to the warp's first key, so that a row's columns are
