@@ -38,7 +38,7 @@ const char* p3_last_error(void);
 int p3_version(void);
 /* tests: a launch whose wait runs out within some 20 ms; out32: 32 floats, NaN behind it */
 int p3_wait_selftest(float* out32, cudaStream_t st);
-/* Diagnostics (tools/chain_trace.py), not part of the reference interface: with a device buffer of n_slots x 1024 x 8 uint64 set,
+/* Diagnostics, not part of the reference interface: with a device buffer of n_slots x 1024 x 8 uint64 set,
  * every decode-path launch (skinny GEMMs, decode attention) takes the next slot and its CTAs store globaltimer stamps
  * {start, dependency resolved, first operands ready, main loop done, exit, smid, kind, grid}. p3_trace_set(NULL, 0) turns it off. */
 int p3_trace_set(void* buf, int n_slots);
@@ -316,7 +316,7 @@ typedef struct {
     void* pool;                 /* this layer's page pool [page][2][n_kv][64][hd] bf16 */
     const int32_t* block_table; /* int32 [M, bt_stride] */
     int32_t bt_stride, _pad2;
-    long long* dbg;             /* NULL, or int64 [n_ctas][4][8]: per-CTA / per-phase SM-clock stamps (tools/mega_trace.py) */
+    long long* dbg;             /* NULL, or int64 [n_ctas][4][8]: per-CTA / per-phase SM-clock stamps */
 } p3_mega_args;
 
 /* W [N,K] bf16 (nn.Linear layout; SWIGLU: the checkpoint's [gate | up] row order) -> stream order for `kind` */

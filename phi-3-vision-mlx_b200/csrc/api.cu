@@ -59,7 +59,7 @@ extern "C" int p3_wait_selftest(float* out32, cudaStream_t st) {
     return 0;
 }
 
-// ---- in-kernel timeline (tools/chain_trace.py; off unless a buffer is set): every traced launch takes the next slot of
+// ---- in-kernel timeline (off unless a buffer is set): every traced launch takes the next slot of
 // P3_TRACE_CTAS x 8 u64 and its CTAs' thread 0 store {globaltimer at start, after the dependency wait, first operands ready,
 // main loop done, exit, smid, kind}. Diagnostic only; costs one null test per launch when off.
 static unsigned long long* g_trace = nullptr;

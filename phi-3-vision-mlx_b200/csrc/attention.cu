@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2) attn_prefill_kernel(AttnParams 
 // tile t is consumed, masking runs only on boundary tiles and exp2 is a single MUFU.
 // ------------------------------------------------------------------------------------------
 #define DEC_STAGES 4
-// timeline stamps (tools/chain_trace.py): compiled in only with -DP3_TRACE_ATTN, because further values that are the same for the
+// timeline stamps: compiled in only with -DP3_TRACE_ATTN, because further values that are the same for the
 // whole warp bring back the illegal-instruction error of the hinted copies (see cp_async16_stream)
 #ifdef P3_TRACE_ATTN
 #define ATTN_TRACE_STAMP(tr, cta, i) trace_stamp(tr, cta, i)

@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
 
     unsigned n_bar = 0;
     int red_buf = 0;
-    // optional instrumentation (P.dbg, tools/mega_trace.py): per CTA and phase, SM-clock stamps
+    // optional instrumentation (P.dbg): per CTA and phase, SM-clock stamps
     //   [0] phase start (barrier arrive)  [1] barrier released  [2] warp 0 has its X fragments  [3] last item done
     //   [4] cycles warp 0 spent waiting for weight data   [5] same, warp 7
     long long* dbg = P.dbg ? P.dbg + (size_t)cta * (P3_MEGA_MAX_PHASES * 8) : nullptr;

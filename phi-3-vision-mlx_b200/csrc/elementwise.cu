@@ -168,7 +168,7 @@ __global__ void rmsnorm_kernel(const bf16* __restrict__ x, const bf16* __restric
 
 // Decode-time variant (T <= 16 rows): one CTA per row, programmatic dependent launch on both sides, so that the
 // skinny GEMMs that follow stream weights only (normalising X inside every 32-row GEMM CTA costs more
-// instructions than its weight tile: tools/microbench.py, qkv 14.9 -> 11.1 us without the fused norm).
+// instructions than its weight tile: qkv 14.9 -> 11.1 us without the fused norm).
 __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
                                                           bf16* __restrict__ y, int H, float eps) {
     __shared__ float s_part[8];

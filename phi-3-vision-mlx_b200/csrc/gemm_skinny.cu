@@ -44,10 +44,10 @@ struct SkParams {
     // xg_out[m][n] = bf16(h[m][n] * xg_gain[n]) (gain of the NEXT norm); a consumer with rs_epi = 1 reads that as X and applies
     // rsqrt(mean(h^2) + eps) from ss_in to its reduced accumulators (norm_w must be null then).
     const bf16* xg_gain; bf16* xg_out; int64_t ldxg; int rs_epi;
-    unsigned long long* trace;                   // tools/chain_trace.py (null in production)
+    unsigned long long* trace;                   // in-kernel timeline (null in production)
     // 16-row tiles of W stored in stream order [tile][64-k chunk][row half][k half][lane][16 B] (model.pack_rows16): a stage is one
     // contiguous 2 KB block and a CTA reads one contiguous 16 x K block, instead of 8 rows x 64 B per instruction at a stride of
-    // K x 2 bytes. Same bytes, same arithmetic; the memory round trip of a contiguous stream is about half (tools/sm_ingest_bench.cu),
+    // K x 2 bytes. Same bytes, same arithmetic; the memory round trip of a contiguous stream is about half,
     // which is what bounds the 192-CTA kernels (o_proj, down_proj: a CTA streams ring / round-trip bytes per us).
     int packed;
     int n_tiles;                                 // output tiles; the grid may be smaller (persistent CTAs, tile = blockIdx.x + i * gridDim.x)
@@ -630,9 +630,9 @@ static int sk_pair_mt1() {
     if (v < 0) { const char* e = getenv("P3_SK_MT1"); v = e ? atoi(e) : 0; }
     return v;
 }
-// Persistent grid: at most one wave of CTAs (2 per SM) walks the output tiles. In-kernel stamps (profiles/r02_chain_trace_*.log):
+// Persistent grid: at most one wave of CTAs (2 per SM) walks the output tiles. In-kernel stamps:
 // with one CTA per tile gate_up (512 tiles) ran a second, partly filled wave whose CTAs all started with an empty ring: 20.1 us
-// for a 15.6 us stream; one wave with a continuous ring: 19.4 us, decode step -2 % (profiles/r02_skinny_persistent_ab.log).
+// for a 15.6 us stream; one wave with a continuous ring: 19.4 us, decode step -2 %.
 // P3_SK_GRID=0 restores one CTA per tile, any other value is the cap (1 CTA/SM = 148 measured 25 % slower: half the bytes in flight).
 static int sk_grid_cap() {
     static int v = -1;
@@ -661,7 +661,7 @@ static int launch_skinny(const SkParams& p_, unsigned grid, cudaStream_t st) {
     if (p.Wq) return launch_skinny_d<NT, MT, (MT == 2 ? 3 : 4), true>(p, grid, st);
     int d = sk_depth_override();
     { static int d1 = -1; if (d1 < 0) { const char* e = getenv("P3_SK_DEPTH1"); d1 = e ? atoi(e) : 0; } if (MT == 1 && d1) d = d1; }
-    if (d == 0) d = (MT == 1) ? 4 : 2;                       // measured best (tools/microbench.py): deeper rings do not pay, residency does
+    if (d == 0) d = (MT == 1) ? 4 : 2;                       // measured best: deeper rings do not pay, residency does
     switch (d) {
         case 2: return launch_skinny_d<NT, MT, 2>(p, grid, st);
         case 3: return launch_skinny_d<NT, MT, 3>(p, grid, st);

@@ -372,7 +372,7 @@ def test_dp_generate_with_images_single_process(dev):
 
 
 def test_short_left_padded_first_call_masks_pad_keys(dev):
-    """ADVICE r1: a left-padded batch with L <= 16 takes the decode-attention kernel on its FIRST call (past == 0); the
+    """a left-padded batch with L <= 16 takes the decode-attention kernel on its FIRST call (past == 0); the
     present tile must mask the pad keys like Mask4D does (phi:557-559)."""
     api, model, proc, ora = _setup()
     lens, n = [5, 9, 12], 12

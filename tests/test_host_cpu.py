@@ -235,7 +235,7 @@ def test_mega_args_layout_matches_header():
     assert ctypes.sizeof(_lib.GemmArgs) == 224
 
 
-# ------------------------------------------------------------------ round 2 host logic: batching, checkpoint directories
+# ------------------------------------------------------------------ batching, checkpoint directories
 def _fake_vproc():
     import torch
     import phi3_b200  # noqa

@@ -750,7 +750,7 @@ def test_top_p_sample_matches_torch_restatement(dev, top_p, temp):
             assert abs(idx.index(got) - idx.index(min(want, idx[-1]))) <= 1
 
 
-# ------------------------------------------------------------------ round 2: fused prefill epilogues of the tensor-core GEMM
+# ------------------------------------------------------------------ fused prefill epilogues of the tensor-core GEMM
 def _gemm_fused(dev, x, w, out, epi, **kw):
     import ctypes
     import phi3_b200  # noqa

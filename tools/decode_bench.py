@@ -1,6 +1,6 @@
 """Decode-step time of the graph-replayed loop at the bench shape (8 rows x 2048 context), text-only Phi-3.5-mini weights:
     [P3_PF_CHAIN=0] [P3_PF_CAP_MB=..] [P3_SK_DEPTH=..] [P3_MEGA=1] python tools/decode_bench.py [--B 8] [--ctx 2048]
-Prints ms per decode step (mean over 200 replays). For A/B of decode-path knobs inside ONE gpurun call."""
+Prints ms per decode step (mean over 200 replays). For A/B of decode-path knobs in one session."""
 import argparse
 import os
 import sys

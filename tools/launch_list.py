@@ -1,5 +1,5 @@
 """Summarise an ncu launch list (`ncu --metrics gpu__time_duration.sum --clock-control none --csv --log-file X.csv <cmd>`) into a
-markdown table: python tools/launch_list.py gpurun_out/X.csv profiles/rNN_launches.md "<command that was profiled>" """
+markdown table: python tools/launch_list.py LAUNCHES.csv SUMMARY.md "<command that was profiled>" """
 import csv
 import sys
 from collections import defaultdict

@@ -1,5 +1,5 @@
 """Summarise an .ncu-rep (read with `ncu -i ... --page raw --csv`) into a markdown table for profiles/.
-    python tools/ncu_summary.py gpurun_out/prof_r01_final.ncu-rep profiles/r01_ncu_final.md"""
+    python tools/ncu_summary.py CAPTURE.ncu-rep SUMMARY.md"""
 import csv
 import io
 import json

@@ -1,5 +1,5 @@
 """Parity report at BASELINE config-1 shapes (run on the GPU box):
-    python tools/parity_report.py [--layers N] > gpurun_out/parity.json
+    python tools/parity_report.py [--layers N] > parity.json
 Phi-3.5-mini (random-init, seed 0), 4 prompts x 32 tokens; the CUDA path vs the CPU oracle in its
 three precision modes. Reports logits error (max-abs/max-abs and rms/rms) and teacher-forced
 greedy agreement over all positions, plus step-wise decode agreement through the skinny kernels."""

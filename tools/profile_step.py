@@ -1,5 +1,5 @@
 """Small driver for ncu captures (never used for bench numbers):
-    ncu --metrics gpu__time_duration.sum --clock-control none --csv --log-file gpurun_out/launches.csv \
+    ncu --metrics gpu__time_duration.sum --clock-control none --csv --log-file launches.csv \
         python tools/profile_step.py --decode-steps 2
 One pass of the bench workload per GPU (8 x 2048-token image+text prompts) with eager decode steps."""
 import argparse
