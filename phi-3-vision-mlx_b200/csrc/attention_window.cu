@@ -637,7 +637,6 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
 // CL: the slices of a request and K/V head are the CTAs of one cluster. They leave their maximum, sum and vector in shared memory and each
 // merges a part of the output columns from all of them, in the order of attn_window_merge_kernel (the same bits), without the trip
 // through the workspace and the launch (16 requests of 2048 tokens, 16 heads over 4: 26.2 -> 22.7 us).
-__device__ __forceinline__ void cluster_sync() { asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory"); }
 __device__ __forceinline__ float ld_cluster(uint32_t addr, uint32_t cta) {
     uint32_t r; float v;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta));

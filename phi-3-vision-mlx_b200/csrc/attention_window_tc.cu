@@ -208,10 +208,6 @@ __device__ __noinline__ void mark_rows(bf16* out, int64_t ld_out, const int4* ti
     if (threadIdx.x == 0) set_status(status);
 }
 
-__device__ __forceinline__ void cluster_sync() {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
-}
 __device__ __forceinline__ uint32_t at_cta(uint32_t addr, int cta) {
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta));
@@ -250,7 +246,8 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_split, int*
     // split: every CTA's rows' {reference maximum, sum}, where the blocks of outputs are otherwise
     auto state = [&](int cta, int row) -> float2& { return reinterpret_cast<float2*>(smem_raw + (turn - raw))[cta * 128 + row]; };
     const int rank = SPLIT ? (int)(blockIdx.x % n_split) : 0;
-    auto tell = [&](int row, float m, float l) {             // to all CTAs
+    float run_at = -INFINITY, run_l = 0.f;                   // those of this thread's row, of a CTA with pages
+    auto tell = [&](int row, float m, float l) {             // to all CTAs, of which it is known that they run
 #pragma unroll 1
         for (int c = 0; c < n_split; c++)
             asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(at_cta(turn + 8 * (rank * 128 + row), c)), "f"(m), "f"(l) : "memory");
@@ -275,6 +272,7 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_split, int*
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (SPLIT) cluster_arrive();                             // this CTA runs: the others may write to its shared memory once all have said so
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&tmem_s);
     pdl_trigger();
     pdl_wait();                                              // q, the pools, the tile records and `out` belong to earlier kernels until here
@@ -653,7 +651,7 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_split, int*
             mbar_wait_lim<false>(o_done(page_0 - 1), ph(page_0 - 1), fail);
             tc_fence_after();
             if constexpr (SPLIT) {
-                tell(warp * 32 + lane, row_ok ? at : -INFINITY, row_ok ? l : 0.f);
+                if (row_ok) { run_at = at; run_l = l; }
                 continue;
             }
             if (mine && any_rows) {
@@ -746,9 +744,11 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_split, int*
         const bool work = now.n_all > 0 && now.mine;
         auto pages = [&](int c) { return now.n_all * (c + 1) / n_split - now.n_all * c / n_split; };
         auto rows = [&](int r) { return work && now.mine >> (r / 64 / n_hc) & 1 ? now.rec[r / 64 / n_hc].y - r % 64 : 0; };     // above 0: the row exists
+        cluster_wait();                                      // every CTA runs; this one said so at its start
         if (row < 128) {
             if (*fail) tell(row, __int_as_float(0x7fc00000), 0.f);         // every CTA's rows become what is not a number
-            else if (pages(rank) == 0) {                     // no page of the CTA's own: the sink, which the first one counts, or nothing
+            else if (pages(rank) > 0) tell(row, run_at, run_l);
+            else {                                           // no page of the CTA's own: the sink, which the first one counts, or nothing
                 const bool sink = !SIG && a.sink && rank == 0 && rows(row) > 0;
                 tell(row, sink ? a.sink[now.h0 + row / 64 % n_hc] * LOG2E : -INFINITY, sink ? 1.f : 0.f);
             }
