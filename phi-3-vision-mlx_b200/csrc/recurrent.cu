@@ -493,31 +493,28 @@ __device__ __forceinline__ void row_token(f2 (&S)[NC][DS / 2], const RowToken<DS
     for (int c = 0; c < NC; c++) { const float2 s = unpack2(acc[c]); y[c] = s.x + s.y; }
 }
 
-// a lane's slice and columns col .. of a head's state
-template <int DS, int RS, int NC> __device__ __forceinline__ void get_tile(f2 (&S)[NC][DS / 2], const float* Sg, int d, int dv, int slice, int col, bool fresh, bool vec) {
+// A lane's slice and columns col .. of a head's state: all reads in a row, without a look at what they bring, so that a step of single tokens waits for memory
+// once (read and paired two rows at a time a tile took DS / 2 trips one behind the other; single tokens of cold states, decays: 4 sequences of 8 heads of
+// 128 x 256 6.3 -> 4.4 us, 24 14.9 -> 13.0, 40 of 64 heads of 64 x 128 37.9 -> 29.3; delta rule, 40 of 128 x 256 28.6 -> 18.1).
+template <int DS, int RS, int NC> __device__ __forceinline__ void read_tile(float (&r)[DS][NC], const float* Sg, int d, int dv, int slice, int col, bool fresh, bool vec) {
     constexpr int V = NC < 4 ? NC : 4;
+    auto at = [&](int j) { return 4 * (j / 4 * RS + slice) + j % 4; };
 #pragma unroll
-    for (int j = 0; j < DS; j += 2) {
-        float r[2][NC];
+    for (int j = 0; j < DS; j++)
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const int row = 4 * (j / 4 * RS + slice) + j % 4 + i;
-            const float* p = Sg + (size_t)row * dv + col;
+        for (int c = 0; c < NC; c++) r[j][c] = 0.f;
+    if (!fresh && vec) {
 #pragma unroll
-            for (int c = 0; c < NC; c += V) {
+        for (int j = 0; j < DS; j++)
 #pragma unroll
-                for (int e = 0; e < V; e++) r[i][c + e] = 0.f;
-                if (!fresh && row < d) {
-                    if (vec) { if (col + c < dv) ldvec<V>(p + c, r[i] + c); }
-                    else {
+            for (int c = 0; c < NC; c += V)
+                if (at(j) < d && col + c < dv) ldvec<V>(Sg + (size_t)at(j) * dv + col + c, r[j] + c);
+    } else if (!fresh) {
 #pragma unroll
-                        for (int e = 0; e < V; e++) if (col + c + e < dv) r[i][c + e] = p[c + e];
-                    }
-                }
-            }
-        }
+        for (int j = 0; j < DS; j++)
 #pragma unroll
-        for (int c = 0; c < NC; c++) S[c][j / 2] = pack2(r[0][c], r[1][c]);
+            for (int c = 0; c < NC; c++)
+                if (at(j) < d && col + c < dv) r[j][c] = Sg[(size_t)at(j) * dv + col + c];
     }
 }
 template <int DS, int RS, int NC> __device__ __forceinline__ void put_tile(const f2 (&S)[NC][DS / 2], float* Sg, int d, int dv, int slice, int col, bool vec) {
@@ -576,8 +573,7 @@ __global__ void __launch_bounds__(GLA_WARPS * 32, STEP == SINGLE ? (DS * NC <= 3
     // two rounds in flight, a token as q [DP] (zeros beyond dim) | k alike | decays alike (DIAG) | v [COLS] | {decay, factor of v} (not DIAG)
     // The CTAs of a sequence follow one another, so that those of a prompt among decodes start on different SMs (one of 500 tokens and 15 of one, 8 heads
     // of 128 x 256: 147 -> 76 us). Single tokens take the sequences in turn (16 of 8 heads of 128 x 128, delta rule: 9.3 us, the other way 11).
-    const int nvb = (dv + COLS - 1) / COLS, parts = H * nvb, seq = ONE ? blockIdx.x % a.n_seqs : blockIdx.x / parts,
-              part = ONE ? blockIdx.x / a.n_seqs : blockIdx.x - seq * parts, hd = ONE ? part % H : part / nvb, vb = ONE ? part / H : part - hd * nvb;
+    const int nvb = ONE ? gridDim.z : gridDim.x, seq = ONE ? blockIdx.x : blockIdx.z, hd = blockIdx.y, vb = ONE ? blockIdx.z : blockIdx.x;
     const int4 rec = reinterpret_cast<const int4*>(a.seqs)[seq];
     const int row0 = rec.x, n_tok = rec.y, slot = rec.z, pos0 = rec.w;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -633,16 +629,21 @@ __global__ void __launch_bounds__(GLA_WARPS * 32, STEP == SINGLE ? (DS * NC <= 3
         }
     };
 
+    float r[DS][NC];                                         // on the way before anything else is asked for
+    read_tile<DS, RS, NC>(r, Sg, d, dv, slice, col, pos0 == 0, vecs);
     stage(0, 0);
     cp_async_commit();
     float fixed = 0.f, skip = 0.f;
     bool gated = false;
     if constexpr (!DIAG) {
-        if (a.taps > 1) move_history(a, row0, n_tok, slot, pos0, part, parts);
+        if (a.taps > 1) move_history(a, row0, n_tok, slot, pos0, hd * nvb + vb, H * nvb);
         gated = a.gates; fixed = gated ? 0.f : a.decay[hd]; skip = !DELTA && a.skip ? a.skip[hd] : 0.f;
     }
     f2 S[NC][DS / 2];
-    get_tile<DS, RS, NC>(S, Sg, d, dv, slice, col, pos0 == 0, vecs);
+#pragma unroll
+    for (int j = 0; j < DS; j += 2)
+#pragma unroll
+        for (int c = 0; c < NC; c++) S[c][j / 2] = pack2(r[j][c], r[j + 1][c]);
     typedef ColumnSums<RS, NC, 4> Four;                      // of four tokens, behind two stages that halve the tokens
     typedef ColumnSums<RS, NC, 16> One;
     const int mine = (lane & 16 ? 1 : 0) + (lane & 8 ? 2 : 0), c4 = Four::first(lane), c1 = One::first(lane), vcol = DELTA ? wcol + One::column(lane) : wcol;
@@ -1018,8 +1019,10 @@ int launch_row_scan(const A& a, int step, int tb, cudaStream_t st) {
         const int64_t ctas = (int64_t)a.n_seqs * a.n_heads * ((a.vdim + w - 1) / w), m = (ctas + 147) / 148, cost = step == SINGLE ? (n == 8 && ctas > 3 * 148 && ctas <= 4 * 148) || (n == 1 && ctas <= 10 * 148) ? 0 : n == 4 ? 1 : 2 : a.n_seqs > MANY_SEQS ? n != 4 : m * (w + 16);
         if (!nc || (a.rs_force ? n >= a.rs_force : cost < best)) { nc = n; cols = w; best = cost; }
     }
-    const dim3 grid((unsigned)((int64_t)a.n_seqs * a.n_heads * ((a.vdim + cols - 1) / cols)));
-    const ScanShape sh = scan_shape(grid.x, row_token_floats(DIAG, ds * rs, cols), a.dim, tb);
+    const unsigned nvb = (a.vdim + cols - 1) / cols;
+    if (a.n_seqs > 65535) step = SINGLE;                     // (numbers them along x)
+    const dim3 grid = step == SINGLE ? dim3(a.n_seqs, a.n_heads, nvb) : dim3(nvb, a.n_heads, a.n_seqs);
+    const ScanShape sh = scan_shape((int64_t)nvb * a.n_heads * a.n_seqs, row_token_floats(DIAG, ds * rs, cols), a.dim, tb);
     const size_t most = sizeof(float) * 2 * (ds > 16 ? 16 : 32) * row_token_floats(DIAG, ds * rs, cols);   // with the longest rounds
 #define GOM(DS, RS, NC, STEP)                                                                                           \
     do { static P3DevFlags set; if (set_smem_attr(row_scan_kernel<MODE, A, DS, RS, NC, STEP>, most, set.cur())) return -1;  \
