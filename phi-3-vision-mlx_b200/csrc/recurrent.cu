@@ -493,8 +493,8 @@ __device__ __forceinline__ void row_token(f2 (&S)[NC][DS / 2], const RowToken<DS
     for (int c = 0; c < NC; c++) { const float2 s = unpack2(acc[c]); y[c] = s.x + s.y; }
 }
 
-// A lane's slice and columns col .. of a head's state: all reads in a row, without a look at what they bring, so that a step of single tokens waits for memory
-// once (read and paired two rows at a time a tile took DS / 2 trips one behind the other; single tokens of cold states, decays: 4 sequences of 8 heads of
+// A lane's slice and columns col .. of a head's state: all reads in a row, without a look at what they bring, so that a step of single tokens waits for
+// memory once (get_tile: two rows at a time, for RUNS; read and paired two rows at a time a tile took DS / 2 trips one behind the other; single tokens of cold states, decays: 4 sequences of 8 heads of
 // 128 x 256 6.3 -> 4.4 us, 24 14.9 -> 13.0, 40 of 64 heads of 64 x 128 37.9 -> 29.3; delta rule, 40 of 128 x 256 28.6 -> 18.1).
 template <int DS, int RS, int NC> __device__ __forceinline__ void read_tile(float (&r)[DS][NC], const float* Sg, int d, int dv, int slice, int col, bool fresh, bool vec) {
     constexpr int V = NC < 4 ? NC : 4;
@@ -515,6 +515,32 @@ template <int DS, int RS, int NC> __device__ __forceinline__ void read_tile(floa
 #pragma unroll
             for (int c = 0; c < NC; c++)
                 if (at(j) < d && col + c < dv) r[j][c] = Sg[(size_t)at(j) * dv + col + c];
+    }
+}
+template <int DS, int RS, int NC> __device__ __forceinline__ void get_tile(f2 (&S)[NC][DS / 2], const float* Sg, int d, int dv, int slice, int col, bool fresh, bool vec) {
+    constexpr int V = NC < 4 ? NC : 4;
+#pragma unroll
+    for (int j = 0; j < DS; j += 2) {
+        float r[2][NC];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int row = 4 * (j / 4 * RS + slice) + j % 4 + i;
+            const float* p = Sg + (size_t)row * dv + col;
+#pragma unroll
+            for (int c = 0; c < NC; c += V) {
+#pragma unroll
+                for (int e = 0; e < V; e++) r[i][c + e] = 0.f;
+                if (!fresh && row < d) {
+                    if (vec) { if (col + c < dv) ldvec<V>(p + c, r[i] + c); }
+                    else {
+#pragma unroll
+                        for (int e = 0; e < V; e++) if (col + c + e < dv) r[i][c + e] = p[c + e];
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < NC; c++) S[c][j / 2] = pack2(r[0][c], r[1][c]);
     }
 }
 template <int DS, int RS, int NC> __device__ __forceinline__ void put_tile(const f2 (&S)[NC][DS / 2], float* Sg, int d, int dv, int slice, int col, bool vec) {
@@ -556,16 +582,21 @@ __device__ __forceinline__ void move_history(const p3_delta_scan_args& a, int ro
 }
 
 // the linear attention (A = p3_gla_args), the memory with one decay per head and the delta rule (A = p3_delta_scan_args), in rounds of tb tokens. STEP:
-//   RUNS    tokens that follow one another, taken by fours, each read ahead of its turn
+//   RUNS    prompts: tokens that follow one another, taken by fours, each read ahead of its turn. States are read two rows at a time, beside the tokens on
+//           their way: with all of a tile's reads in a row ptxas gives the loop other registers (one sequence of 1500 tokens, 8 heads of 128 x 256, decays:
+//           148 us, 159 so; 4 x 2048 tokens of the linear attention 418 and 452)
+//   ANY     the same for drafts, and where the caller does not say, with all reads in a row (16 x 3 tokens, delta rule: 19.9 us as RUNS, 11.1)
+//   EITHER  ANY within the registers of five or four CTAs an SM, for more CTAs than that holds two of an SM
 //   SINGLE  a token or two per sequence: reads and writes of states, which want to be in flight from many CTAs, six or four an SM, at up to 80 or 128
-//           registers; tokens one by one (states that come from DRAM, 24 sequences of 64 heads of 64 x 128, decays: 25.0 us, 6.4 TB/s, as RUNS 30;
-//           prompts would take up to twice their time)
-//   EITHER  not known which: RUNS within the registers of five CTAs an SM (28.2 us)
-enum { RUNS, SINGLE, EITHER };
+//           registers; tokens one by one (states that come from DRAM, 24 sequences of 64 heads of 64 x 128, decays: 19.1 us, 5.2 TB/s, EITHER 19.5)
+//   FEW     the same where four or three CTAs an SM hold all: no number leaves the registers (6 sequences of 8 heads of 128 x 256: 5.5 us as SINGLE, 5.1)
+enum { RUNS, SINGLE, FEW, EITHER, ANY };
 template <int MODE, typename A, int DS, int RS, int NC, int STEP>
-__global__ void __launch_bounds__(GLA_WARPS * 32, STEP == SINGLE ? (DS * NC <= 32 ? 6 : 4) : STEP == EITHER ? (DS * NC <= 32 ? 5 : 4) : MODE == SCAN_DELTA && DS * NC <= 16 ? 1 : 0) row_scan_kernel(A a, int tb) {
+__global__ void __launch_bounds__(GLA_WARPS * 32, STEP == SINGLE ? (DS * NC <= 32 ? 6 : 4) : STEP == FEW ? (DS * NC <= 32 ? 4 : 3) : STEP == EITHER ? (DS * NC <= 32 ? 5 : 4)
+                                                                                                          : MODE == SCAN_DELTA && DS * NC <= 16 ? 1 : 0)
+row_scan_kernel(A a, int tb) {
     pdl_wait();                                              // memory is touched only after the predecessors are done
-    constexpr bool DIAG = MODE == SCAN_DIAG, DELTA = MODE == SCAN_DELTA, ONE = STEP == SINGLE;
+    constexpr bool DIAG = MODE == SCAN_DIAG, DELTA = MODE == SCAN_DELTA, ONE = STEP == SINGLE || STEP == FEW;
     constexpr int CW = 32 / RS, WCOLS = CW * NC, COLS = GLA_WARPS * WCOLS, DP = DS * RS, NT = GLA_WARPS * 32;
     constexpr int VO = (DIAG ? 3 : 2) * DP, GO = VO + COLS, TOK = row_token_floats(DIAG, DP, COLS);
     extern __shared__ __align__(16) float sm[];
@@ -573,7 +604,15 @@ __global__ void __launch_bounds__(GLA_WARPS * 32, STEP == SINGLE ? (DS * NC <= 3
     // two rounds in flight, a token as q [DP] (zeros beyond dim) | k alike | decays alike (DIAG) | v [COLS] | {decay, factor of v} (not DIAG)
     // The CTAs of a sequence follow one another, so that those of a prompt among decodes start on different SMs (one of 500 tokens and 15 of one, 8 heads
     // of 128 x 256: 147 -> 76 us). Single tokens take the sequences in turn (16 of 8 heads of 128 x 128, delta rule: 9.3 us, the other way 11).
-    const int nvb = ONE ? gridDim.z : gridDim.x, seq = ONE ? blockIdx.x : blockIdx.z, hd = blockIdx.y, vb = ONE ? blockIdx.z : blockIdx.x;
+    int seq, hd, vb, part, parts;
+    if constexpr (STEP == RUNS) {
+        const int nvb = (dv + COLS - 1) / COLS;
+        parts = H * nvb; seq = blockIdx.x / parts; part = blockIdx.x - seq * parts; hd = part / nvb; vb = part - hd * nvb;
+    } else if constexpr (ONE) {
+        seq = blockIdx.x; hd = blockIdx.y; vb = blockIdx.z; part = hd * gridDim.z + vb; parts = H * gridDim.z;
+    } else {
+        seq = blockIdx.z; hd = blockIdx.y; vb = blockIdx.x; part = hd * gridDim.x + vb; parts = H * gridDim.x;
+    }
     const int4 rec = reinterpret_cast<const int4*>(a.seqs)[seq];
     const int row0 = rec.x, n_tok = rec.y, slot = rec.z, pos0 = rec.w;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -630,20 +669,23 @@ __global__ void __launch_bounds__(GLA_WARPS * 32, STEP == SINGLE ? (DS * NC <= 3
     };
 
     float r[DS][NC];                                         // on the way before anything else is asked for
-    read_tile<DS, RS, NC>(r, Sg, d, dv, slice, col, pos0 == 0, vecs);
+    if constexpr (STEP != RUNS) read_tile<DS, RS, NC>(r, Sg, d, dv, slice, col, pos0 == 0, vecs);
     stage(0, 0);
     cp_async_commit();
     float fixed = 0.f, skip = 0.f;
     bool gated = false;
     if constexpr (!DIAG) {
-        if (a.taps > 1) move_history(a, row0, n_tok, slot, pos0, hd * nvb + vb, H * nvb);
+        if (a.taps > 1) move_history(a, row0, n_tok, slot, pos0, part, parts);
         gated = a.gates; fixed = gated ? 0.f : a.decay[hd]; skip = !DELTA && a.skip ? a.skip[hd] : 0.f;
     }
     f2 S[NC][DS / 2];
+    if constexpr (STEP == RUNS) get_tile<DS, RS, NC>(S, Sg, d, dv, slice, col, pos0 == 0, vecs);
+    else {
 #pragma unroll
-    for (int j = 0; j < DS; j += 2)
+        for (int j = 0; j < DS; j += 2)
 #pragma unroll
-        for (int c = 0; c < NC; c++) S[c][j / 2] = pack2(r[j][c], r[j + 1][c]);
+            for (int c = 0; c < NC; c++) S[c][j / 2] = pack2(r[j][c], r[j + 1][c]);
+    }
     typedef ColumnSums<RS, NC, 4> Four;                      // of four tokens, behind two stages that halve the tokens
     typedef ColumnSums<RS, NC, 16> One;
     const int mine = (lane & 16 ? 1 : 0) + (lane & 8 ? 2 : 0), c4 = Four::first(lane), c1 = One::first(lane), vcol = DELTA ? wcol + One::column(lane) : wcol;
@@ -1001,37 +1043,59 @@ extern "C" int p3_part_norm_gate(const float* y, int64_t ldy, int parts, int n, 
 
 namespace {
 constexpr int MANY_SEQS = 8;
+// Kernel, columns of a lane and tokens of a round for a step of n_rows tokens (0: not known). Row slices by the size of a key alone, so that a sum has one
+// order whatever is chosen (the delta rule closes a sum before every update: fewer slices, 4 x 2048 tokens of 128 x 256 529 us against 626). Over 1430 steps
+// (eight shapes of heads, 1 to 64 sequences, single tokens of states in DRAM, drafts, prompts, one prompt among single tokens) this takes 0.78 of the time of
+// tiles of 16 to 128 rows by one or two columns a lane, 1.12 at the most (0.3 us of 5). Columns, each number of them timed:
+//   a token or two   four: states in 16-byte pieces. The delta rule over long keys (its sum S^T k is on the way) fewer while CTAs are few: one up to two CTAs
+//                    an SM (2 sequences of 8 heads of 128 x 256 3.2 us, 3.7 with four), two up to four (6 sequences 5.0 and 5.6; 16: 10.0 and 8.4)
+//   else             by what the busiest SM has to do for a token while CTAs of four columns are two an SM or fewer (2 x 700 tokens of the linear attention 102
+//                    us with four, 107 with two, 153 with eight), four with more of them; eight only without MANY_SEQS sequences, of which one may be much
+//                    longer than the others (16, one with 500 tokens, decays: 76 us with four, 120 with eight). The delta rule over long keys one or
+//                    two (4 x 1000 tokens 255 us, with four 302; 12 x 300 of 2 heads of 128 x 128 62 and 90), four behind MANY_SEQS that fill the SMs
+//                    (9 x 500 of 8 heads of 128 x 256 235 us, with two 254)
+// Rounds: four tokens for one or two a sequence; eight for drafts of the linear attention (16 x 3 tokens 26.2 -> 19.5 us: 32 leave two CTAs an SM), 32 for
+// its prompts; else 16, or eight where 16 of long keys would keep EITHER's fourth CTA off an SM (9 single tokens of 8 heads of 256 x 256 15.8 -> 10.2).
 template <int MODE, typename A>
-int launch_row_scan(const A& a, int step, int tb, cudaStream_t st) {
+int launch_row_scan(const A& a, int64_t n_rows, cudaStream_t st) {
     constexpr bool DIAG = MODE == SCAN_DIAG, DELTA = MODE == SCAN_DELTA;
-    // Row slices by the size of a key alone, so that a sum has one order (the delta rule closes a sum before every update: fewer slices, 4 x 2048 tokens
-    // of 128 x 256 529 us against 626). Columns of a lane, for tokens that follow one another: by what the busiest SM has to do for a token, and 4 behind
-    // more than MANY_SEQS sequences, of which one may be much longer than the others (10 of 8 heads of 128 x 256, one with 500 tokens: 154 -> 114 us with
-    // 4 for the 8 of the sum). For single tokens 4 (states in pieces of 16 bytes; with 2 up to twice the time); 8 where only they make it one wave at four
-    // CTAs an SM (16 sequences of that size, decays: 13.6 -> 11.7 us); the delta rule over long keys 1 while there are few CTAs (6: 9.5 -> 7.3 us, 12:
-    // 11.4 -> 10.9; 16 would take 13.2 for 11.8).
     const int ds = a.dim <= 32 ? 4 : a.dim <= 64 || (!DELTA && a.dim <= 128) ? 8 : a.dim <= 256 ? 16 : 32, rs = a.dim <= (DELTA ? 128 : 64) ? 8 : 16;
-    int nc = 0, cols = 0;
-    int64_t best = 0;
-    for (int n = 8; n >= 1; n /= 2) {
-        const int w = GLA_WARPS * 32 / rs * n;
-        if (n * ds > 64 || (n == 1 && !(DELTA && ds == 16 && rs == 8))) continue;
-        const int64_t ctas = (int64_t)a.n_seqs * a.n_heads * ((a.vdim + w - 1) / w), m = (ctas + 147) / 148, cost = step == SINGLE ? (n == 8 && ctas > 3 * 148 && ctas <= 4 * 148) || (n == 1 && ctas <= 10 * 148) ? 0 : n == 4 ? 1 : 2 : a.n_seqs > MANY_SEQS ? n != 4 : m * (w + 16);
-        if (!nc || (a.rs_force ? n >= a.rs_force : cost < best)) { nc = n; cols = w; best = cost; }
+    const bool tall = DELTA && ds == 16 && rs == 8, layers = a.n_seqs <= 65535;          // (what a grid's z can number)
+    const bool few = n_rows && n_rows <= 8 * (int64_t)a.n_seqs, single = layers && n_rows && n_rows <= 2 * (int64_t)a.n_seqs;
+    const int least = tall ? 1 : 2, most = 64 / ds < 8 ? 64 / ds : 8;
+    auto ctas = [&](int n) { const int w = GLA_WARPS * 32 / rs * n; return (int64_t)a.n_seqs * a.n_heads * ((a.vdim + w - 1) / w); };
+    const int wide = most < 4 ? most : 4;
+    int nc = wide;
+    if (a.rs_force) for (nc = least; nc < a.rs_force && nc < most;) nc *= 2;
+    else if (single) { if (tall) nc = ctas(1) <= 2 * 148 ? 1 : ctas(2) <= 4 * 148 ? 2 : 4; }
+    else if (tall ? a.n_seqs <= MANY_SEQS || ctas(4) <= 148 : ctas(wide) <= 2 * 148 || a.n_seqs <= MANY_SEQS) {
+        int64_t best = 0;
+        for (int n = tall ? 2 : most; n >= least; n /= 2) {
+            if (n > 4 && (a.n_seqs > MANY_SEQS || ctas(n) > (DIAG ? 1 : 2) * 148 || (!n_rows && ctas(4) > 2 * 148))) continue;
+            if (!tall && n < wide && ctas(wide) > 2 * 148) continue;
+            const int64_t cost = (ctas(n) + 147) / 148 * (GLA_WARPS * 32 / rs * n + (DIAG ? 16 : 8));
+            if (!best || cost < best) { nc = n; best = cost; }
+        }
     }
+    const int step = single ? ctas(nc) <= (nc * ds <= 32 ? 4 : 3) * 148 ? FEW : SINGLE : (n_rows && !few) || !layers ? RUNS : !DIAG && !n_rows && nc == 4 && ctas(4) > 2 * 148 ? EITHER : ANY;
+    const int many = single ? 4 : DIAG ? few ? 8 : 32 : step == EITHER && a.dim > 128 ? 8 : 16;
+    const int cols = GLA_WARPS * 32 / rs * nc;
     const unsigned nvb = (a.vdim + cols - 1) / cols;
-    if (a.n_seqs > 65535) step = SINGLE;                     // (numbers them along x)
-    const dim3 grid = step == SINGLE ? dim3(a.n_seqs, a.n_heads, nvb) : dim3(nvb, a.n_heads, a.n_seqs);
-    const ScanShape sh = scan_shape((int64_t)nvb * a.n_heads * a.n_seqs, row_token_floats(DIAG, ds * rs, cols), a.dim, tb);
-    const size_t most = sizeof(float) * 2 * (ds > 16 ? 16 : 32) * row_token_floats(DIAG, ds * rs, cols);   // with the longest rounds
-#define GOM(DS, RS, NC, STEP)                                                                                           \
-    do { static P3DevFlags set; if (set_smem_attr(row_scan_kernel<MODE, A, DS, RS, NC, STEP>, most, set.cur())) return -1;  \
-         p3_launch_pdl(row_scan_kernel<MODE, A, DS, RS, NC, STEP>, grid, dim3(GLA_WARPS * 32), sh.bytes, st, a, sh.tb); } while (0)
-#define GO(DS, RS, NC)                                                                                               \
-    if constexpr (DELTA ? DS != 8 || RS != 16 : DS != 16 || RS != 8) if (ds == DS && rs == RS && nc == NC) {          \
-        if (step == SINGLE) GOM(DS, RS, NC, SINGLE);                                                                  \
-        else if (!DIAG && NC == 4 && step == EITHER) GOM(DS, RS, NC, !DIAG && NC == 4 ? EITHER : RUNS);               \
-        else GOM(DS, RS, NC, RUNS);                                                                                   \
+    const dim3 grids[3] = {dim3((unsigned)ctas(nc)), dim3(a.n_seqs, a.n_heads, nvb), dim3(nvb, a.n_heads, a.n_seqs)};
+    const ScanShape sh = scan_shape(ctas(nc), row_token_floats(DIAG, ds * rs, cols), a.dim, many);
+    const size_t bytes = sizeof(float) * 2 * (ds > 16 ? 16 : 32) * row_token_floats(DIAG, ds * rs, cols);   // with the longest rounds
+#define GOM(DS, RS, NC, STEP)                                                                                            \
+    do { static P3DevFlags set; if (set_smem_attr(row_scan_kernel<MODE, A, DS, RS, NC, STEP>, bytes, set.cur())) return -1; \
+         p3_launch_pdl(row_scan_kernel<MODE, A, DS, RS, NC, STEP>, grids[STEP == RUNS ? 0 : STEP == SINGLE || STEP == FEW ? 1 : 2], dim3(GLA_WARPS * 32), sh.bytes, st, a, sh.tb); } while (0)
+    // numbers of columns that the rules above do not choose but are asked for run as ANY
+#define GO(DS, RS, NC)                                                                                                   \
+    if constexpr (DELTA ? DS != 8 || RS != 16 : DS != 16 || RS != 8) if (ds == DS && rs == RS && nc == NC) {              \
+        constexpr int S = NC == 4 || DS == 32 ? SINGLE : ANY, F = S == SINGLE || (DELTA && DS == 16 && RS == 8) ? FEW : ANY, E = !DIAG && NC == 4 && (DS != 16 || RS != 8) ? EITHER : ANY; \
+        if (step == SINGLE) GOM(DS, RS, NC, S);                                                                           \
+        else if (step == FEW) GOM(DS, RS, NC, F);                                                                         \
+        else if (step == EITHER) GOM(DS, RS, NC, E);                                                                      \
+        else if (step == ANY) GOM(DS, RS, NC, ANY);                                                                       \
+        else GOM(DS, RS, NC, RUNS);                                                                                       \
     }
     GO(4, 8, 2) GO(4, 8, 4) GO(4, 8, 8) GO(8, 8, 2) GO(8, 8, 4) GO(8, 8, 8) GO(8, 16, 2) GO(8, 16, 4) GO(8, 16, 8) GO(16, 8, 1) GO(16, 8, 2) GO(16, 8, 4) GO(16, 16, 2) GO(16, 16, 4) GO(32, 16, 2)
 #undef GO
@@ -1068,10 +1132,7 @@ extern "C" int p3_gla_scan(const p3_gla_args* a, cudaStream_t st) {
         const unsigned blocks = (unsigned)(work + 255) / 256 < 148u * 8 ? (unsigned)((work + 255) / 256) : 148u * 8;
         p3_launch_pdl(gla_decay_kernel, dim3(blocks ? blocks : 1), dim3(256), (size_t)(0), st, a->z, a->ld_z, a->z_bias, (int64_t)a->n_rows, n, a->inv_tau, vec);
     }
-    // Rounds of 4 tokens for steps of few tokens per sequence (less shared memory: more CTAs an SM), 32 for prompts (4 x 1024 tokens of 64 heads: 572 us,
-    // with 16 630). Few are two a sequence: drafts are longer, and with read-ahead faster.
-    const bool few = a->n_rows <= 2 * a->n_seqs;
-    if (launch_row_scan<SCAN_DIAG>(*a, few ? SINGLE : RUNS, few ? 4 : 32, st)) return -1;
+    if (launch_row_scan<SCAN_DIAG>(*a, a->n_rows, st)) return -1;
     P3_CHECK_LAUNCH("gla_scan");
     return 0;
 }
@@ -1119,15 +1180,13 @@ int check_scan(const p3_delta_scan_args* a, const char* who) {
     P3_CHECK_ARG(a->n_rows >= 0, "%s: the number of rows must not be negative", who);
     return 0;
 }
-
-int step_of(const p3_delta_scan_args& a) { return !a.n_rows ? a.n_seqs > MANY_SEQS ? EITHER : RUNS : a.n_rows <= 2 * a.n_seqs ? SINGLE : RUNS; }
 }  // namespace
 
 extern "C" int p3_delta_scan(const p3_delta_scan_args* a, cudaStream_t st) {
     P3_CHECK_ARG(a && a->gates, "delta_scan: null argument");
     if (check_scan(a, "delta_scan")) return -1;
     if (a->n_seqs == 0) return 0;
-    if (launch_row_scan<SCAN_DELTA>(*a, step_of(*a), step_of(*a) == SINGLE ? 4 : 16, st)) return -1;
+    if (launch_row_scan<SCAN_DELTA>(*a, a->n_rows, st)) return -1;
     P3_CHECK_LAUNCH("delta_scan");
     return 0;
 }
@@ -1136,8 +1195,7 @@ extern "C" int p3_decay_scan(const p3_delta_scan_args* a, cudaStream_t st) {
     P3_CHECK_ARG(a && (a->gates || a->decay), "decay_scan: needs gates, or one decay per head");
     if (check_scan(a, "decay_scan")) return -1;
     if (a->n_seqs == 0) return 0;
-    // rounds of 16 tokens where CTAs share an SM (6 x 1000 tokens 428 -> 326 us)
-    if (launch_row_scan<SCAN_DECAY>(*a, step_of(*a), step_of(*a) == SINGLE ? 4 : 16, st)) return -1;
+    if (launch_row_scan<SCAN_DECAY>(*a, a->n_rows, st)) return -1;
     P3_CHECK_LAUNCH("decay_scan");
     return 0;
 }
