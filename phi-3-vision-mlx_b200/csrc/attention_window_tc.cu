@@ -30,8 +30,9 @@
 // 96: 0.6 of mma.sync. Not kept: two threads a row and eight warps a CTA (125 for 115: a third more instructions), a loader in warps of its own with
 // the softmax warps' registers raised (130), runs of 16 keys (116).
 //
-// Every wait has a limit: when one runs out no thread of the CTA waits any more, the loader takes over nothing more, and the CTA ends with its last
-// blocks of the grid (and one that it had taken over already) written as not a number and the status word set.
+// Every wait of a CTA has a limit: when one runs out no thread of the CTA waits any more, the loader takes over nothing more, and the CTA ends with its last
+// blocks of the grid (and one that it had taken over already) written as not a number and the status word set. A cluster's barriers have none of their
+// own: every CTA comes to them, as its waits end, and one whose waits ran out tells the others, which write the rows of the pass as not a number.
 #include "tc_common.cuh"
 #include "attention_window.cuh"
 #include <type_traits>
@@ -348,7 +349,7 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_split, int*
                 if (lane == 0) {
                     items_s[passes % ITEMS] = item;
                     mbar_wait_lim<false>(pass_empty(passes), ph(passes) ^ 1u, fail);
-                    if (!*fail) {                        // else the place may be in use
+                    if (SPLIT || !*fail) {               // else the place may be in use (split: the only pass, which the CTA's end goes by whatever ran out)
                         Pass& ps = pass_s[passes & 1];
                         ps.rec[0] = r0; ps.rec[1] = r1; ps.n = n; ps.lo_pg = lo_pg; ps.n_keep = n_keep; ps.h0 = h0; ps.mine = mine; ps.first = from; ps.n_all = n_all;
                         mbar_arrive(pass_full(passes));
@@ -416,8 +417,8 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_split, int*
         }
         if (lane == 0 && !all_done) {
             mbar_wait_lim<false>(pass_empty(passes), ph(passes) ^ 1u, fail);
+            if (SPLIT && passes == 0) pass_s[0].mine = pass_s[0].n_all = 0;
             if (!*fail) {
-                if (SPLIT && passes == 0) pass_s[0].mine = pass_s[0].n_all = 0;
                 pass_s[passes & 1].n = 0;
                 mbar_arrive(pass_full(passes));
             }
