@@ -36,7 +36,7 @@ extern "C" {
 
 const char* p3_last_error(void);
 int p3_version(void);
-/* tests: a launch whose wait runs out within some 20 ms; out32: 32 floats, NaN behind it */
+/* tests: a launch with a wait of either kind that runs out within some 20 ms; out32: 32 floats, NaN behind the first and the second (16 each) */
 int p3_wait_selftest(float* out32, cudaStream_t st);
 /* Diagnostics, not part of the reference interface: with a device buffer of n_slots x 1024 x 8 uint64 set,
  * every decode-path launch (skinny GEMMs, decode attention) takes the next slot and its CTAs store globaltimer stamps

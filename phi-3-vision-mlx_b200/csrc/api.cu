@@ -38,19 +38,27 @@ bool p3_take_status() {
     return w && __atomic_load_n(w, __ATOMIC_RELAXED) && __atomic_exchange_n(w, 0, __ATOMIC_ACQ_REL);
 }
 
-// One warp waits, for a few milliseconds, at a barrier that nothing arrives at, and gives up as the kernels above do
+// One warp waits, for a few milliseconds, at a barrier that nothing arrives at, and gives up as the kernels above do: numbers 0 .. 15 behind a wait whose
+// tries rest for long, 16 .. 31 behind one whose tries rest as the hardware sees fit
+template <bool HINT> __device__ void wait_runs_out(uint32_t bar, volatile int* fail, float* out16, int* status) {
+    if (threadIdx.x == 0) *fail = 0;
+    __syncwarp();
+    mbar_wait_lim<HINT>(bar, 0, fail, 1000000);
+    __syncwarp();
+    if (*fail) {
+        if (threadIdx.x < 16) out16[threadIdx.x] = __int_as_float(0x7fc00000);
+        if (threadIdx.x == 0) set_status(status);
+    }
+    __syncwarp();
+}
 __global__ void wait_runs_out_kernel(float* out, int* status) {
     __shared__ __align__(8) uint64_t bar_s;
     __shared__ int fail_s;
     const uint32_t bar = smem_u32(&bar_s);
-    if (threadIdx.x == 0) { fail_s = 0; mbar_init(bar, 1); }
+    if (threadIdx.x == 0) mbar_init(bar, 1);
     __syncwarp();
-    mbar_wait_lim(bar, 0, &fail_s, 1);
-    __syncwarp();
-    if (fail_s) {
-        out[threadIdx.x] = __int_as_float(0x7fc00000);
-        if (threadIdx.x == 0) set_status(status);
-    }
+    wait_runs_out<true>(bar, &fail_s, out, status);
+    wait_runs_out<false>(bar, &fail_s, out + 16, status);
 }
 extern "C" int p3_wait_selftest(float* out32, cudaStream_t st) {
     P3_CHECK_ARG(out32, "wait_selftest: null argument");

@@ -24,14 +24,16 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
         if (!ok && ++spins > (1u << 27)) __trap();            // seconds of spinning: a protocol bug — fail loudly instead of hanging the GPU
     } while (!ok);
 }
-// Bounded wait without a fault: a CTA of which one wait ran out of tries has *fail set, and none of its threads waits any more. What the CTA started
-// itself is waited for all the same before it ends (mbar_drain). LONG: a try may rest for up to 10 ms, as the fp32 products have it (512 x 3072 x 1024:
-// 30.0 us, 30.4 without the hint); else for as long as the hardware sees fit, after which threads were seen to go on sooner (prefill attention of 4 x 2048
-// tokens, 16 heads of 128 over 4: 111 -> 109 us).
-constexpr uint32_t LONG_TRIES = 200, SHORT_TRIES = 1u << 22;
-template <bool LONG = true> __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+// Bounded wait without a fault: a CTA of which one wait ran out has *fail set, and none of its threads waits any more. What the CTA started itself is
+// waited for all the same before it ends (mbar_drain). HINT: a try may rest for up to 10 ms, as the fp32 products have it (512 x 3072 x 1024: 30.0 us,
+// 30.4 without the hint); else for as long as the hardware sees fit, after which threads were seen to go on sooner (prefill attention of 4 x 2048
+// tokens, 16 heads of 128 over 4: 111 -> 109 us). How long that is nobody says, so the limit is a time, two seconds, looked at only behind a try that
+// brought nothing.
+constexpr uint64_t WAIT_NS = 2000000000ull;
+__device__ __forceinline__ uint64_t now_ns() { uint64_t t; asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t)); return t; }
+template <bool HINT = true> __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    if constexpr (!LONG) {
+    if constexpr (!HINT) {
         asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
         return ok;
     }
@@ -39,17 +41,21 @@ template <bool LONG = true> __device__ __forceinline__ bool mbar_try(uint32_t ba
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
-template <bool LONG = true>
-__device__ __forceinline__ void mbar_wait_lim(uint32_t bar, uint32_t parity, volatile int* fail, uint32_t limit = LONG ? LONG_TRIES : SHORT_TRIES) {
-    uint32_t tries = 0;
-    while (!mbar_try<LONG>(bar, parity)) {
+template <bool HINT = true>
+__device__ __forceinline__ void mbar_wait_lim(uint32_t bar, uint32_t parity, volatile int* fail, uint64_t limit_ns = WAIT_NS) {
+    if (mbar_try<HINT>(bar, parity)) return;
+    const uint64_t from = now_ns();
+    while (!mbar_try<HINT>(bar, parity)) {
         if (*fail) return;
-        if (++tries > limit) { *fail = 1; return; }
+        if (now_ns() - from > limit_ns) { *fail = 1; return; }
     }
 }
-template <bool LONG = true> __device__ __forceinline__ bool mbar_drain(uint32_t bar, uint32_t parity) {
-    for (uint32_t tries = 0; tries < (LONG ? LONG_TRIES : SHORT_TRIES); tries++) if (mbar_try<LONG>(bar, parity)) return true;
-    return false;
+template <bool HINT = true> __device__ __forceinline__ bool mbar_drain(uint32_t bar, uint32_t parity) {
+    if (mbar_try<HINT>(bar, parity)) return true;
+    const uint64_t from = now_ns();
+    while (!mbar_try<HINT>(bar, parity))
+        if (now_ns() - from > WAIT_NS) return false;
+    return true;
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int c0, int c1) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
