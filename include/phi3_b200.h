@@ -127,8 +127,8 @@ int p3_gemm_skinny_qkv_rope_w4(const void* X, int64_t ldx, const void* norm_w, f
 int p3_gemm(const void* X, int64_t ldx, const void* W, int64_t ldw, const void* bias, void* out, int64_t ldo,
             const void* resid, const int32_t* row_map, int64_t M, int N, int K, int epi, int impl, cudaStream_t st);
 
-/* columns of the tile when p3_gemm runs a product of M rows and N columns on CTA pairs (SwiGLU: always 256), 0 when it does not
- * (P3_GEMM_2CTA=0: never) */
+/* 0 when p3_gemm does not run a product of M rows and N columns on CTA pairs (P3_GEMM_2CTA=0: never); else the columns of a pair's tile where X is its
+ * 256-row side: products with row scales or a rotation, and plain ones where p3_gemm_turned_rows is 0 (SwiGLU: always 256) */
 int p3_gemm_pair_width(int64_t M, int64_t N);
 /* rows of X per tile where a plain product of such a size takes W as the 256-row side of its tiles; 0: X is that side */
 int p3_gemm_turned_rows(int64_t M, int64_t N);

@@ -1133,9 +1133,11 @@ static int tile_width(int64_t M, int N) {
 // Rows of X of a tile where W is its 256-row side; 0: X is. A wave on that side takes its rows plus 64 rows' worth (start, end and the turned epilogue).
 // Over 79 products (200 - 5418 rows, N 2048 - 16384, K 1024 - 8192), each timed at nine widths, what this chooses takes 0.83 to 1.007 of the time of X as
 // the 256-row side, 0.983 in the mean, the best of all widths 0.972: 300 x 9216 x 3072 25.4 -> 21.1 us with 160 rows, 781 rows 42.2 -> 38.7 with 208, 1100 x
-// 3072 x 8192 46.9 -> 43.9 with 192.
+// 3072 x 8192 46.9 -> 43.9 with 192. (From 224 rows on no choice of it: X as the 256-row side always costs less.) On 240 products of other sizes (130 - 6200 rows,
+// N 1024 - 16384, K 1024 - 8192, fp32 and bf16 outputs) it takes 0.947, the best of all widths 0.934, and more than X as that side at two
+// (1.002 and 1.04: 3407 x 3000 x 1024, 21.7 -> 22.6).
 static int turned_rows(int64_t M, int N) {
-    const int cost[9][2] = {{256, 96}, {240, 108}, {224, 108}, {208, 99}, {192, 97}, {176, 97}, {160, 101}, {144, 106}, {128, 104}};
+    const int cost[6][2] = {{208, 99}, {192, 97}, {176, 97}, {160, 101}, {144, 106}, {128, 104}};
     int64_t least = INT64_MAX;
     for (const auto& c : plain_widths) {
         const int64_t t = tile_cost((M + 255) / 256 * ((N + c[0] - 1) / c[0]), c[0], 16, c[1]);
