@@ -62,7 +62,7 @@ struct FaMaps {                                         // [0]: 64-column SW128 
 
 template <int D>
 __global__ void __launch_bounds__(FA_THREADS, 1)
-attn_prefill_tc_kernel(const __grid_constant__ FaMaps tm, AttnParams p, long long* dbg) {
+attn_prefill_tc_kernel(const __grid_constant__ FaMaps tm, AttnParams p) {
     using C = FaCfg<D>;
     constexpr int ST = C::STAGES, KT = C::KT;
     extern __shared__ uint8_t smem_raw[];
@@ -106,14 +106,7 @@ attn_prefill_tc_kernel(const __grid_constant__ FaMaps tm, AttnParams p, long lon
     }
     if (!act_b) n_x[1] = 0;
     const int n_max = max(n_x[0], n_x[1]);
-#ifdef P3_FA_TIMING   // clock64 stamps of CTA 0's pipeline (slot: 0/1 softmax a/b, 2/3 MMA issue for a/b); printed by the launcher
-    const bool dbg_on = dbg && blockIdx.x == 0;
-#define FA_T(slot, it, k) do { if (dbg_on && (it) < 64 && (threadIdx.x & 31) == 0) dbg[((slot) * 64 + (it)) * 8 + (k)] = clock64(); } while (0)
-#else
-#define FA_T(slot, it, k) do { } while (0)
-#endif
 
-    FA_T(3, 0, 5);
     if (warp == FA_W_TMA && lane == 0) {
 #pragma unroll
         for (int i = 0; i < (C::TWO ? 2 : 1); i++) {
@@ -143,7 +136,6 @@ attn_prefill_tc_kernel(const __grid_constant__ FaMaps tm, AttnParams p, long lon
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot_ptr;
-    FA_T(3, 0, 6);
     pdl_trigger();                                               // setup above overlaps the previous kernel's tail
     pdl_wait();                                                  // q/k/v, the pool and `out` belong to earlier kernels until here
 
@@ -218,7 +210,6 @@ attn_prefill_tc_kernel(const __grid_constant__ FaMaps tm, AttnParams p, long lon
                 if (j + 2 < n_max) mbar_wait(k_full((j + 2) % ST), (uint32_t)((j + 2) / ST) & 1u);
                 if (j < nx) mbar_wait(sm_done(x, j), (uint32_t)(j >> 1) & 1u);   // P_x(j) is in TMEM (exactly one wait per tile, in order)
                 tc_fence_after();
-                FA_T(2 + x, j, 0);
                 if (elect_one()) {
                     if (j < nx) {
                         // O_x += P_x(j) V(j): A from TMEM (lane = row, two bf16 keys per column), V in place as MN-major B
@@ -236,7 +227,6 @@ attn_prefill_tc_kernel(const __grid_constant__ FaMaps tm, AttnParams p, long lon
                     if (j + 2 < n_max) tc_commit(k_empty((j + 2) % ST));
                 }
                 __syncwarp();
-                FA_T(2 + x, j, 1);
             }
         }
     } else {
@@ -256,7 +246,6 @@ attn_prefill_tc_kernel(const __grid_constant__ FaMaps tm, AttnParams p, long lon
             const uint32_t t_s = t_lane + C::S_COL + x * 128 + (it & 1) * 64;
             mbar_wait(s_full(x, it), (uint32_t)(it >> 1) & 1u); // S_x(it) ready (issued two tiles ago: normally no wait)
             tc_fence_after();
-            if (wq == 0) FA_T(x, it, 0);
             auto scale_o = [&](float cf) {                       // warp-collective: every lane runs the TMEM round trip
                 // O_x must be complete up to tile it-1 and PV_x(it) waits for our P: rare path, so the barrier is only
                 // waited here (two alternating barriers keep the parity unambiguous)
@@ -337,7 +326,6 @@ attn_prefill_tc_kernel(const __grid_constant__ FaMaps tm, AttnParams p, long lon
                 sweep(std::false_type{}, std::true_type{}, (m == -INFINITY) ? 0.f : m * sl, mx, ls);
             }
             l += ls;
-            if (wq == 0) FA_T(x, it, 2);
             const float grow = (mx - m) * sl;                    // NaN (no keys yet) compares false
             if (grow > FA_RESCALE_LOG2) { pend = ex2_approx(-grow); has_pend = true; m = mx; }
             // P_x(it) over the first 32 columns of its own S buffer (the row is fully consumed; S_x(it+2) is issued after PV_x(it))
@@ -345,7 +333,6 @@ attn_prefill_tc_kernel(const __grid_constant__ FaMaps tm, AttnParams p, long lon
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(sm_done(x, it));
-            if (wq == 0) FA_T(x, it, 3);
         }
         // ---- epilogue: O / l
         if (x == 0 || act_b) {
@@ -376,10 +363,8 @@ attn_prefill_tc_kernel(const __grid_constant__ FaMaps tm, AttnParams p, long lon
             }
         }
     }
-    if (warp < 4) FA_T(3, 1 + warp, 5);
     tc_fence_before();
     __syncthreads();
-    FA_T(3, 0, 7);
     if (warp == FA_W_MMA) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(C::TMEM_COLS) : "memory");
@@ -430,30 +415,8 @@ static int launch_tc_d(const AttnParams& p, cudaStream_t st) {
         set = true;
     }
     dim3 grid(((p.L + 255) / 256) * p.n_heads * p.B);
-    long long* dbg = nullptr;
-#ifdef P3_FA_TIMING
-    const bool want_dbg = getenv("P3_FA_DBG") != nullptr;
-    if (want_dbg) { cudaMalloc(&dbg, 4 * 64 * 8 * 8); cudaMemset(dbg, 0, 4 * 64 * 8 * 8); }
-#endif
-    p3_launch_pdl(attn_prefill_tc_kernel<D>, grid, dim3(FA_THREADS), (size_t)C::SMEM, st, tm, p, dbg);
+    p3_launch_pdl(attn_prefill_tc_kernel<D>, grid, dim3(FA_THREADS), (size_t)C::SMEM, st, tm, p);
     P3_CHECK_LAUNCH("attention_prefill_tc");
-#ifdef P3_FA_TIMING
-    if (want_dbg) {
-        static long long h[4 * 64 * 8];
-        cudaStreamSynchronize(st);
-        cudaMemcpy(h, dbg, sizeof(h), cudaMemcpyDeviceToHost);
-        cudaFree(dbg);
-        long long t0 = h[0];
-        auto H = [&](int s, int it, int k) { return h[(s * 64 + it) * 8 + k] - t0; };
-        for (int it = 0; it < 64 && h[(0 * 64 + it) * 8]; it++) {
-            printf("it %2d | smA: sfull %7lld swept %7lld arrived %7lld | smB: %7lld %7lld %7lld | mma top %7lld kfull %7lld | A: woke %7lld vfull %7lld pv %7lld s %7lld commit %7lld | B: %7lld %7lld %7lld %7lld %7lld\n", it,
-                   H(0, it, 0), H(0, it, 2), H(0, it, 3), H(1, it, 0), H(1, it, 2), H(1, it, 3), H(2, it, 5), H(2, it, 6),
-                   H(2, it, 0), H(2, it, 2), H(2, it, 3), H(2, it, 4), H(2, it, 1), H(3, it, 0), H(3, it, 2), H(3, it, 3), H(3, it, 4), H(3, it, 1));
-        }
-        printf("entry %lld setup %lld | softmax A warps done %lld %lld %lld %lld | end %lld\n", H(3, 0, 5), H(3, 0, 6), H(3, 1, 5), H(3, 2, 5), H(3, 3, 5), H(3, 4, 5), H(3, 0, 7));
-        fflush(stdout);
-    }
-#endif
     return 0;
 }
 

@@ -22,7 +22,7 @@
 // A page that belongs to one record of a pass only is multiplied by weights of zero for the other, which a value that is not finite would make something
 // else: the idle half's warps look the page's values over, and where there is one they hold O across the page.
 // Where the passes of a step leave places on the chip empty, two to eight CTAs of a cluster share the pages of each (the caller says how many pages a pass
-// has at most): every CTA sweeps a run of them, and the sums of all are put together through distributed shared memory by the first.
+// has at most): every CTA sweeps a run of them, and each adds up a share of the rows from the sums of all, through distributed shared memory.
 // Bound by the softmax warps: their instructions issue in the order of a page's 64 keys a row, a third of the time a warp waits for the next one from
 // the cache of instructions (so the sweep is two runs of 32 keys, and what a page needs only rarely is a function), and two CTAs share the SM's
 // exponentials; the MMAs keep the tensor cores busy half of the time. 4 x 2048 tokens, 16 heads of 128 over 4, window 1024, penalties: 107.5 us (before

@@ -713,9 +713,6 @@ __device__ __forceinline__ void tc_mma_bf16_2sm(uint32_t d_tmem, uint64_t adesc,
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 struct Tc2Cfg {
     static constexpr int BM = 128, BN_MAX = 256, BK = 64, STAGES = 6;
@@ -777,7 +774,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
-    cluster_sync_all();
+    cluster_sync();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot_ptr;
     // programmatic dependent launch: barrier init / TMEM allocation above overlap the previous kernel's tail; nothing
@@ -948,7 +945,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
     }
     tc_fence_before();
-    cluster_sync_all();
+    cluster_sync();
     if (warp == 2) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(C::TMEM_COLS) : "memory");
@@ -1088,7 +1085,7 @@ static int launch_tc(const void* X, int64_t ldx, const void* W, int64_t ldw, con
     e2.ksplit = 1;
     if (ep.ws && tiles * 2 < num_sms() && (int64_t)BN * K * 2 > (7ll << 18) * BN / 128) {
         // few output tiles AND a long K (each CTA would stream > 1.75 MB of W alone at ~45 KB/us, e.g. down_proj at M <= 320:
-        // 24 tiles x 2 MB): split K so that tiles * ksplit ~ #SM (>= 4 k-blocks each). Measured (tools/gemm_smallm.py): 43 -> 30 us
+        // 24 tiles x 2 MB): split K so that tiles * ksplit ~ #SM (>= 4 k-blocks each). Measured: 43 -> 30 us
         // at M = 80, 40 -> 21 us at M = 16; for K = 3072 shapes the partial round trip costs more than it saves, so they stay unsplit.
         const int kb = (K + C::BK - 1) / C::BK;
         int ks = (int)(num_sms() / tiles);
@@ -1253,7 +1250,7 @@ static int gemm_dispatch(const void* X, int64_t ldx, const void* W, int64_t ldw,
     if (ep.kind == P3_EPI_SWIGLU || !small) return launch_tc<256>(X, ldx, W, ldw, eps, M, N, K, st, wp);
     // one row tile and fewer 128-wide column tiles than SMs (M <= 128 against the 3072..9216-row matrices: constrain steps): the GEMM
     // is a weight stream and a CTA only pulls what its TMA ring turns over per round trip -> 64-row W tiles put twice as many CTAs
-    // on it (tools/gemm_smallm.py, M = 80: qkv 18.9 -> 16.8 us, o_proj 19.3 -> 17.2, down_proj with split-K 28.6 -> 21.8). Not for
+    // on it (M = 80: qkv 18.9 -> 16.8 us, o_proj 19.3 -> 17.2, down_proj with split-K 28.6 -> 21.8). Not for
     // more row tiles: every CTA re-reads its X rows over the whole K, which outweighs the gain (M = 320 down_proj 36.6 -> 39.4 us).
     static int bn64 = -1;
     if (bn64 < 0) { const char* e = getenv("P3_GEMM_BN64"); bn64 = e ? atoi(e) : 1; }

@@ -397,7 +397,7 @@ template <int RS, int N, int MASK> struct ColumnSums {
             }
         }
     }
-    // first column that the lane ends with; -1: another lane writes the same
+    // first column that the lane ends with
     static __device__ __forceinline__ int column(int lane) {
         int n = N, c = 0;
 #pragma unroll
@@ -405,6 +405,7 @@ template <int RS, int N, int MASK> struct ColumnSums {
             if (n > 1) { n /= 2; c += lane & mask ? n : 0; }
         return c;
     }
+    // the same; -1: another lane writes it
     static __device__ __forceinline__ int first(int lane) {
         int n = N;
         bool mine = true;
@@ -861,8 +862,7 @@ __global__ void __launch_bounds__(128) short_conv_kernel(p3_short_conv_args a, i
     }
 }
 
-// ---------------------------------------------------------------- gated delta rule, and the same memory without the correction
-__host__ __device__ inline int64_t delta_head_floats(int dim, int vdim) { return (int64_t)dim * vdim; }
+// ---------------------------------------------------------------- norms of the scans' outputs
 
 // one warp per (token, head)
 template <typename AT>
@@ -1168,7 +1168,7 @@ extern "C" int p3_short_conv(const p3_short_conv_args* a, cudaStream_t st) {
     return 0;
 }
 
-extern "C" int64_t p3_delta_state_floats(int n_heads, int dim, int vdim) { return (int64_t)n_heads * delta_head_floats(dim, vdim); }
+extern "C" int64_t p3_delta_state_floats(int n_heads, int dim, int vdim) { return (int64_t)n_heads * gla_head_floats(dim, vdim); }
 
 namespace {
 int check_scan(const p3_delta_scan_args* a, const char* who) {

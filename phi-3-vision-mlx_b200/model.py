@@ -272,7 +272,7 @@ class Phi3B200:
         self.prefill_chunk = 8192     # long prompts are prefilled in chunks against the paged cache (config 4: 128K)
         import os as _os
         self.pf_chain = _os.environ.get('P3_PF_CHAIN', '1') != '0'
-        self._skip = set(filter(None, _os.environ.get('P3_SKIP', '').split(',')))   # timing ablation only (tools/ablate.py)
+        self._skip = set(filter(None, _os.environ.get('P3_SKIP', '').split(',')))   # timing only: kernel families that a decode step leaves out (its outputs are then garbage)
         # decode: RMSNorm as its own tiny PDL kernel instead of fused into every 32-row CTA of the following skinny GEMM.
         # Neutral for the bf16 weight stream (2.797 vs 2.788 ms/token on the bench), -8 % for the instruction-bound 4-bit one.
         self._opf_in_qkv = _os.environ.get('P3_OPF', 'qkv') != 'attn'
