@@ -419,7 +419,9 @@ typedef struct {
     int32_t chunk;                 /* > 0: a query sees only keys of its own run of `chunk` positions (position / chunk equal,
                                       counted from the sequence's start); 0: no runs. May be combined with a window */
     int32_t max_pages;             /* prefill only: no record of the call sees keys of more pages than about this many; where few rows leave
-                                      the GPU half empty several CTAs then share a record's pages. 0: not known, they do not */
+                                      the GPU half empty several CTAs then share a record's pages, and sum its outputs up in another order: the last
+                                      bits of a record's outputs depend on this number, on n_seqs and on n_tiles. 0: not known, they do not */
+    int32_t n_seqs;                /* with max_pages: sequences that the records belong to, about; 0: not known, each may be one's own */
 } p3_attn_window_args;
 /* query rows per tile that p3_attn_window_prefill takes for these sizes: 64 on its tensor-core path, else 32 */
 int p3_attn_window_tile_rows(const p3_attn_window_args* args);

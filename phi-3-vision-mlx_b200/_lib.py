@@ -264,7 +264,7 @@ class AttnWindowArgs(C.Structure):
                 ('window', C.c_int32), ('act_f32', C.c_int32), ('cache_f32', C.c_int32), ('tiles', _p), ('n_tiles', C.c_int32),
                 ('n_splits', C.c_int32), ('ws', _p), ('v_ld', C.c_int32), ('keep_first', C.c_int32), ('sig_bias', _p),
                 ('out_scale', C.c_float), ('elem_gate', _p), ('ld_elem_gate', _l), ('chunk', C.c_int32),
-                ('max_pages', C.c_int32)]
+                ('max_pages', C.c_int32), ('n_seqs', C.c_int32)]
 
 
 class LatentPostArgs(C.Structure):

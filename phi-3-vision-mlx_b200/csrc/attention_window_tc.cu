@@ -25,8 +25,8 @@
 // has at most): every CTA sweeps a run of them, and each adds up a share of the rows from the sums of all, through distributed shared memory.
 // Bound by the softmax warps: their instructions issue in the order of a page's 64 keys a row, a third of the time a warp waits for the next one from
 // the cache of instructions (so the sweep is two runs of 32 keys, and what a page needs only rarely is a function), and two CTAs share the SM's
-// exponentials; the MMAs keep the tensor cores busy half of the time. 4 x 2048 tokens, 16 heads of 128 over 4, window 1024, penalties: 107.5 us (before
-// the functions 114, mma.sync 298); 333 rows of 32 x 96 behind 704: 33 (one CTA a pass 39, mma.sync 67); 16 prompts of 60 tokens behind 500, 16 heads of
+// exponentials; the MMAs keep the tensor cores busy half of the time. 4 x 2048 tokens, 16 heads of 128 over 4, window 1024, penalties: 110 us (before
+// the functions 113, mma.sync 298); 333 rows of 32 x 96 behind 704: 32 (one CTA a pass 37, mma.sync 67); 16 prompts of 60 tokens behind 500, 16 heads of
 // 96: 0.6 of mma.sync. Not kept: two threads a row and eight warps a CTA (125 for 115: a third more instructions), a loader in warps of its own with
 // the softmax warps' registers raised (130), runs of 16 keys (116).
 //
@@ -878,12 +878,17 @@ int launch_attn_window_tc(const p3_attn_window_args* a, cudaStream_t st) {
     const bool even = (a->n_heads / a->n_kv) % 2 == 0;
     const int64_t full = even ? (int64_t)a->n_tiles * (a->n_heads / 2) : (int64_t)((a->n_tiles + 1) / 2) * a->n_heads;      // passes with both halves in use
     // Passes that leave half of the places (two CTAs an SM) empty share their pages among the CTAs of a cluster, up to eight. A page takes a CTA about 1.6
-    // us, the cluster's launch, exchange and sums about 9 in all, and clusters do not fill an SM's last places (288 CTAs in threes of 333 rows of 32 x 96
-    // behind 704 ran in two rounds: 43 us; in twos 33, unsplit 40). 64 rows of 16 heads of 128 over 4 behind 1500: 44 -> 21 us in eights; 700 rows of 16
-    // over 4: 30.6 -> 27.3 in threes; 500 rows of them stay whole (23.0; in twos 25.6, in fours 24.0).
-    int64_t n_split = 1, least = 16 * (int64_t)a->max_pages;
-    for (int k = 2; k <= 8 && k * full <= 264; k++) {
-        const int64_t cost = 16 * (int64_t)((a->max_pages + k - 1) / k) + 90 + 3 * k;
+    // us (1.2 with sigmoid weights), the cluster's launch, exchange and sums about 11 and 0.6 a CTA, and clusters do not fill an SM's last places (64 passes
+    // in fours took 23 us or 36, as the clusters fell; 96 in threes 37, in twos 25). In groups of odd size a sequence's last record has no partner, nor its first
+    // where it stands second: half a pass more a sequence (records of ten sequences, 8 heads of 128: 24.9 us whole and 40 in threes). 64 rows of 16 heads of
+    // 128 over 4 behind 1500: 44 -> 21 us in eights; 333 rows of 32 x 96 behind 704 37 -> 32 in twos; 500 rows of 16 over 4 stay whole (23.0; in twos
+    // 25.6, in fours 24.0). Over 400 steps of 1 to 16 sequences, each timed with 1 to 8 CTAs a pass, this takes 0.966 of the time of whole passes, 1.07 at the
+    // most, the best of all eight 0.951.
+    const int seqs = a->n_seqs > 0 && a->n_seqs < a->n_tiles ? a->n_seqs : a->n_tiles, page = a->sig_bias ? 12 : 16;
+    const int64_t passes = even ? full : (int64_t)((a->n_tiles + seqs + (seqs > 1)) / 2) * a->n_heads;
+    int64_t n_split = 1, least = page * (int64_t)a->max_pages;
+    for (int k = 2; k <= 8 && k * passes <= 224; k++) {
+        const int64_t cost = page * (((int64_t)a->max_pages + k - 1) / k) + 110 + 6 * k;
         if (cost < least) { least = cost; n_split = k; }
     }
     // Both halves of a CTA in use, unless that would leave half of the SMs without one (a half alone takes about as long as two): 333 rows of

@@ -37,7 +37,7 @@ import torch
 from . import _lib
 from ._lib import call, call_struct, ptr
 from .configs import DugalixConfig, rot_frequencies
-from .lm_base import PagedLM, _max_pages, _page_slices, _stream
+from .lm_base import PagedLM, _page_slices, _shape_of_prompts, _stream
 
 
 class DugalixB200(PagedLM):
@@ -243,7 +243,8 @@ class DugalixB200(PagedLM):
         w.act_f32, w.cache_f32 = self.f32, self.f32
         seen = lambda n: (min(at.window, n) + min(at.keep_first, max(0, n - at.window))) if at.window else n   # keys a query at n - 1 sees
         if b.n_pf:
-            w.tiles, w.n_tiles, w.max_pages = ptr(b.pf_tiles), b.n_pf, _max_pages(b, seen)
+            w.tiles, w.n_tiles = ptr(b.pf_tiles), b.n_pf
+            _shape_of_prompts(w, b, seen)
             ev = self._ev()
             call_struct('p3_attn_window_prefill', w, st)
             span = seen(b.max_pos + 1) if at.window else (b.max_pos + 1) // 2

@@ -79,7 +79,8 @@ class Engine:
             raise ValueError('a request may bring its tokens of a step in one entry only: its recurrent state advances once per step')
         ids, slots, poss, pf, dec, want, seqs = [], [], [], [], [], [], []     # numpy pieces / records, in entry order
         slot_seq = [0] * pool.n_slots                        # slot -> its record in seqs (slots without tokens are never looked up)
-        row = max_pos = pf_pos = 0
+        row = max_pos = 0
+        pf_runs = []                                         # first and last position of every prompt
         for rid, toks, wanted in entries:
             n = len(toks)
             if n == 0:
@@ -97,7 +98,7 @@ class Engine:
             if n == 1:
                 dec.append((row, 1, s, p0))
             else:
-                pf_pos = max(pf_pos, p0 + n - 1)
+                pf_runs.append((p0, p0 + n - 1))
                 r0 = np.arange(0, n, self.q_tile, dtype=np.int32)
                 pf.append(np.stack([row + r0, np.minimum(self.q_tile, n - r0), np.full_like(r0, s), p0 + r0], 1))
             for i in wanted:
@@ -108,7 +109,7 @@ class Engine:
         T = row
         b = StepBatch()
         b.T, b.n_pf, b.n_dec, b.R, b.n_seq, b.n_slots = T, sum(len(p) for p in pf), len(dec), len(want), len(seqs), pool.n_slots
-        b.max_pos, b.pf_pos = max_pos, pf_pos
+        b.max_pos, b.pf_runs = max_pos, pf_runs
         if T == 0:
             return b
         i32 = lambda v: np.asarray(v, np.int32).reshape(-1)

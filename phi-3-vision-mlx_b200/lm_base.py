@@ -34,15 +34,25 @@ def _page_slices(pairs, pages, slots=2 * 148, merge=0.0):
     return best
 
 
-def _max_pages(b, span_of):
-    """pages that a prompt record of 64 rows of the step sees at most; span_of(n) = most keys a query at position n - 1 sees"""
-    last = getattr(b, 'pf_pos', b.max_pos)
-    return min(last // PAGE + 1, (span_of(last + 1) + 2 * PAGE - 2) // PAGE)
+def _shape_of_prompts(w, b, span_of):
+    """what the prefill launch shares its work out by: pages that a record of 64 rows sees at most, sequences of the records; span_of(n) = most keys
+    a query at position n - 1 sees. A batch that does not say where its prompts lie is taken for one sequence's, or for as many as leave their
+    last records half empty where that is more than one can leave"""
+    runs = getattr(b, 'pf_runs', None)
+    rows = b.T - b.n_dec
+    spare = PAGE * b.n_pf - rows
+    w.n_seqs = len(runs) if runs else 1 if spare < PAGE else (spare + PAGE // 4) // (PAGE // 2)
+    w.max_pages = 0
+    for first, last in runs or [(max(0, b.max_pos + 1 - rows), b.max_pos)]:
+        n = last + 1
+        if w.chunk and first // w.chunk == last // w.chunk:
+            n = last % w.chunk + 1
+        w.max_pages = max(w.max_pages, min(last // PAGE + 1, (span_of(n) + 2 * PAGE - 2) // PAGE))
 
 
 class StepBatch:
     """Device-side description of one engine step (built by engine.Engine.step)."""
-    __slots__ = ('T', 'ids', 'tok_slot', 'tok_pos', 'pf_tiles', 'n_pf', 'dec_tiles', 'n_dec', 'want_rows', 'R', 'max_pos', 'pf_pos', 'flat',
+    __slots__ = ('T', 'ids', 'tok_slot', 'tok_pos', 'pf_tiles', 'n_pf', 'dec_tiles', 'n_dec', 'want_rows', 'R', 'max_pos', 'pf_runs', 'flat',
                  'seqs', 'n_seq', 'slot_seq', 'n_slots')
 
 
@@ -184,7 +194,8 @@ class PagedLM:
         st, H = _stream(), w.n_heads
         esz = 4 if self.f32 else 2
         if b.n_pf:
-            w.tiles, w.n_tiles, w.max_pages = ptr(b.pf_tiles), b.n_pf, _max_pages(b, span_of)
+            w.tiles, w.n_tiles = ptr(b.pf_tiles), b.n_pf
+            _shape_of_prompts(w, b, span_of)
             ev = self._ev()
             call_struct('p3_attn_window_prefill', w, st)
             if pf_span is None:

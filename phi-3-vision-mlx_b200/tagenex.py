@@ -23,7 +23,7 @@ else on p3_gemm_any.
 import torch
 from . import _lib
 from ._lib import call, call_struct, ptr
-from .lm_base import PagedLM, StepBatch, _max_pages, _page_slices, _stream  # noqa: F401  (StepBatch is re-exported for engine.py)
+from .lm_base import PagedLM, StepBatch, _page_slices, _shape_of_prompts, _stream  # noqa: F401  (StepBatch is re-exported for engine.py)
 from .configs import TagenexConfig
 from .paged import PAGE
 
@@ -141,7 +141,8 @@ class TagenexB200(PagedLM):
             w.act_f32, w.cache_f32 = self.f32, self.f32
             esz = 4 if self.f32 else 2
             if b.n_pf:
-                w.tiles, w.n_tiles, w.max_pages = ptr(b.pf_tiles), b.n_pf, _max_pages(b, lambda n: m.window or n)
+                w.tiles, w.n_tiles = ptr(b.pf_tiles), b.n_pf
+                _shape_of_prompts(w, b, lambda n: m.window or n)
                 ev = self._ev()
                 call_struct('p3_attn_window_prefill', w, st)
                 span = min(m.window, b.max_pos + 1) if m.window else (b.max_pos + 1) // 2

@@ -31,7 +31,7 @@ import torch
 from . import _lib
 from ._lib import call, call_struct, ptr
 from .configs import TapalixConfig, yarn_frequencies
-from .lm_base import PagedLM, _max_pages, _page_slices, _stream
+from .lm_base import PagedLM, _page_slices, _shape_of_prompts, _stream
 
 
 class TapalixB200(PagedLM):
@@ -216,7 +216,8 @@ class TapalixB200(PagedLM):
         w.act_f32, w.cache_f32 = self.f32, self.f32
         esz = 4 if self.f32 else 2
         if b.n_pf:
-            w.tiles, w.n_tiles, w.max_pages = ptr(b.pf_tiles), b.n_pf, _max_pages(b, lambda n: n)
+            w.tiles, w.n_tiles = ptr(b.pf_tiles), b.n_pf
+            _shape_of_prompts(w, b, lambda n: n)
             ev = self._ev()
             call_struct('p3_attn_window_prefill', w, st)
             self._ev(ev, 'attn_prefill', 2 * (T - b.n_dec) * H * ((b.max_pos + 1) // 2) * (key + R), 0)
