@@ -12,7 +12,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 # kernels) that a fresh checkout compiles when only an engine model is served. The full one wins when both exist.
 FULL_PATH = os.path.join(_HERE, 'libphi3b200.so')
 LM_PATH = os.path.join(_HERE, 'libphi3b200_lm.so')
-LIB_PATH = os.environ.get('P3_LIB') or FULL_PATH                               # P3_LIB: tuning builds (tools/), same ABI
+LIB_PATH = os.environ.get('P3_LIB') or FULL_PATH                               # P3_LIB: another build, same ABI
 
 
 def ensure_built(full=True):

@@ -38,22 +38,30 @@ def _shape_of_prompts(w, b, span_of):
     """what the prefill launch shares its work out by: pages that a record of 64 rows sees at most, sequences of the records; span_of(n) = most keys
     a query at position n - 1 sees. A batch that does not say where its prompts lie is taken for one sequence's, or for as many as leave their
     last records half empty where that is more than one can leave"""
-    runs = getattr(b, 'pf_runs', None)
-    rows = b.T - b.n_dec
-    spare = PAGE * b.n_pf - rows
-    w.n_seqs = len(runs) if runs else 1 if spare < PAGE else (spare + PAGE // 4) // (PAGE // 2)
-    w.max_pages = 0
-    for first, last in runs or [(max(0, b.max_pos + 1 - rows), b.max_pos)]:
-        n = last + 1
-        if w.chunk and first // w.chunk == last // w.chunk:
-            n = last % w.chunk + 1
-        w.max_pages = max(w.max_pages, min(last // PAGE + 1, (span_of(n) + 2 * PAGE - 2) // PAGE))
+    if b.n_pf * w.n_heads > 224:                                 # the launch has passes enough
+        w.max_pages = 0
+        return
+    runs, chunk, pages = b.pf_runs, w.chunk, 0
+    if runs is None:
+        rows = b.T - b.n_dec
+        spare = PAGE * b.n_pf - rows
+        w.n_seqs = 1 if spare < PAGE else (spare + PAGE // 4) // (PAGE // 2)
+        runs = ((max(0, b.max_pos + 1 - rows), b.max_pos),)
+    else:
+        w.n_seqs = len(runs)
+    for first, last in runs:
+        n = last % chunk + 1 if chunk and first // chunk == last // chunk else last + 1
+        pages = max(pages, min(last // PAGE + 1, (span_of(n) + 2 * PAGE - 2) // PAGE))
+    w.max_pages = pages
 
 
 class StepBatch:
     """Device-side description of one engine step (built by engine.Engine.step)."""
     __slots__ = ('T', 'ids', 'tok_slot', 'tok_pos', 'pf_tiles', 'n_pf', 'dec_tiles', 'n_dec', 'want_rows', 'R', 'max_pos', 'pf_runs', 'flat',
                  'seqs', 'n_seq', 'slot_seq', 'n_slots')
+
+    def __init__(self):
+        self.pf_runs = None                                      # (first, last position) of every prompt, where the batch's maker says so
 
 
 class PagedLM:

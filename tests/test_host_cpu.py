@@ -460,7 +460,7 @@ def test_what_a_prefill_launch_is_told_of_its_prompts(runs, rows, n_pf, n_dec, c
     from phi3_b200 import _lib
     from phi3_b200.lm_base import StepBatch, _shape_of_prompts
     w, b = _lib.AttnWindowArgs(), StepBatch()
-    w.chunk = chunk
+    w.chunk, w.n_heads = chunk, 4
     b.T, b.n_pf, b.n_dec, b.max_pos = rows + n_dec, n_pf, n_dec, 1036
     if runs:
         b.pf_runs, b.max_pos = runs, 9999
