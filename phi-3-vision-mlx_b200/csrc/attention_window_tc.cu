@@ -754,6 +754,7 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_split, int*
                 tell(row, sink ? a.sink[now.h0 + row / 64 % n_hc] * LOG2E : -INFINITY, sink ? 1.f : 0.f);
             }
         }
+        __syncwarp();
         cluster_sync();
         if (row < 128 && work) {
             float top = -INFINITY, l = 0.f;
@@ -782,6 +783,7 @@ attn_window_prefill_tc_kernel(p3_attn_window_args a, int n_hc, int n_split, int*
                 }
             }
         }
+        __syncwarp();
         cluster_sync();                                      // nothing is sent to a CTA behind this
         if (work) {
             const int q4 = dv / 4, r_lo = share * rank, n_r = min(share, 128 - r_lo);

@@ -63,10 +63,10 @@ __device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 r; asm("add.rn.f32x2 %0, %1,
 __device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ f2 sub2(f2 a, f2 b) { f2 r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 
-// Barrier of all threads of a cluster (warps whole). Another CTA's shared memory may be touched only behind one that it arrived at, its own left only
+// Barrier of all threads of a cluster; warps come to it whole (a __syncwarp here cost the products 0.2 us a launch). Another CTA's shared memory may be touched only behind one that it arrived at, its own left only
 // behind one that ends the others' use of it.
-__device__ __forceinline__ void cluster_arrive() { __syncwarp(); asm volatile("barrier.cluster.arrive.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { __syncwarp(); asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() { cluster_arrive(); cluster_wait(); }
 
 __device__ __forceinline__ float warp_sum(float v) {
