@@ -586,15 +586,16 @@ __device__ __forceinline__ void move_history(const p3_delta_scan_args& a, int ro
 //   RUNS    prompts: tokens that follow one another, taken by fours, each read ahead of its turn. States are read two rows at a time, beside the tokens on
 //           their way: with all of a tile's reads in a row ptxas gives the loop other registers (one sequence of 1500 tokens, 8 heads of 128 x 256, decays:
 //           148 us, 159 so; 4 x 2048 tokens of the linear attention 418 and 452)
-//   ANY     the same for drafts, and where the caller does not say, with all reads in a row (16 x 3 tokens, delta rule: 19.9 us as RUNS, 11.1)
-//   EITHER  ANY within the registers of five or four CTAs an SM, for more CTAs than that holds two of an SM
+//   ANY     the same for up to 32 tokens a sequence, and where the caller does not say, with all reads in a row and the registers of four CTAs an SM (16 x 3
+//           tokens, delta rule: 19.9 us as RUNS, 11.1; one prompt of 20, 12 heads of 64 x 256, decays: 5.9 and 5.0)
+//   EITHER  ANY within the registers of five or four CTAs an SM, where the caller does not say and there are more CTAs than ANY has places
 //   SINGLE  a token or two per sequence: reads and writes of states, which want to be in flight from many CTAs, six or four an SM, at up to 80 or 128
 //           registers; tokens one by one (states that come from DRAM, 24 sequences of 64 heads of 64 x 128, decays: 19.1 us, 5.2 TB/s, EITHER 19.5)
 //   FEW     the same where four or three CTAs an SM hold all: no number leaves the registers (6 sequences of 8 heads of 128 x 256: 5.5 us as SINGLE, 5.1)
 enum { RUNS, SINGLE, FEW, EITHER, ANY };
 template <int MODE, typename A, int DS, int RS, int NC, int STEP>
 __global__ void __launch_bounds__(GLA_WARPS * 32, STEP == SINGLE ? (DS * NC <= 32 ? 6 : 4) : STEP == FEW ? (DS * NC <= 32 ? 4 : 3) : STEP == EITHER ? (DS * NC <= 32 ? 5 : 4)
-                                                                                                          : MODE == SCAN_DELTA && DS * NC <= 16 ? 1 : 0)
+                                                       : STEP == ANY && DS * NC == 32 ? 4 : MODE == SCAN_DELTA && DS * NC <= 16 ? 1 : 0)
 row_scan_kernel(A a, int tb) {
     pdl_wait();                                              // memory is touched only after the predecessors are done
     constexpr bool DIAG = MODE == SCAN_DIAG, DELTA = MODE == SCAN_DELTA, ONE = STEP == SINGLE || STEP == FEW;
@@ -1046,7 +1047,7 @@ constexpr int MANY_SEQS = 8;
 // Kernel, columns of a lane and tokens of a round for a step of n_rows tokens (0: not known). Row slices by the size of a key alone, so that a sum has one
 // order whatever is chosen (the delta rule closes a sum before every update: fewer slices, 4 x 2048 tokens of 128 x 256 529 us against 626). Over 1430 steps
 // (eight shapes of heads, 1 to 64 sequences, single tokens of states in DRAM, drafts, prompts, one prompt among single tokens) this takes 0.78 of the time of
-// tiles of 16 to 128 rows by one or two columns a lane, 1.12 at the most (0.3 us of 5). Columns, each number of them timed:
+// tiles of 16 to 128 rows by one or two columns a lane, 1.1 at the most (2.1 -> 2.3 us). Columns, each number of them timed:
 //   a token or two   four: states in 16-byte pieces. The delta rule over long keys (its sum S^T k is on the way) fewer while CTAs are few: one up to two CTAs
 //                    an SM (2 sequences of 8 heads of 128 x 256 3.2 us, 3.7 with four), two up to four (6 sequences 5.0 and 5.6; 16: 10.0 and 8.4)
 //   else             by what the busiest SM has to do for a token while CTAs of four columns are two an SM or fewer (2 x 700 tokens of the linear attention 102
@@ -1054,14 +1055,14 @@ constexpr int MANY_SEQS = 8;
 //                    longer than the others (16, one with 500 tokens, decays: 76 us with four, 120 with eight). The delta rule over long keys one or
 //                    two (4 x 1000 tokens 255 us, with four 302; 12 x 300 of 2 heads of 128 x 128 62 and 90), four behind MANY_SEQS that fill the SMs
 //                    (9 x 500 of 8 heads of 128 x 256 235 us, with two 254)
-// Rounds: four tokens for one or two a sequence; eight for drafts of the linear attention (16 x 3 tokens 26.2 -> 19.5 us: 32 leave two CTAs an SM), 32 for
+// Rounds: four tokens for one or two a sequence; 16 for drafts of the linear attention (16 x 3 tokens 26.2 -> 19.7 us: 32 leave two CTAs an SM), 32 for
 // its prompts; else 16, or eight where 16 of long keys would keep EITHER's fourth CTA off an SM (9 single tokens of 8 heads of 256 x 256 15.8 -> 10.2).
 template <int MODE, typename A>
 int launch_row_scan(const A& a, int64_t n_rows, cudaStream_t st) {
     constexpr bool DIAG = MODE == SCAN_DIAG, DELTA = MODE == SCAN_DELTA;
     const int ds = a.dim <= 32 ? 4 : a.dim <= 64 || (!DELTA && a.dim <= 128) ? 8 : a.dim <= 256 ? 16 : 32, rs = a.dim <= (DELTA ? 128 : 64) ? 8 : 16;
     const bool tall = DELTA && ds == 16 && rs == 8, layers = a.n_seqs <= 65535;          // (what a grid's z can number)
-    const bool few = n_rows && n_rows <= 8 * (int64_t)a.n_seqs, single = layers && n_rows && n_rows <= 2 * (int64_t)a.n_seqs;
+    const bool few = n_rows && n_rows <= 32 * (int64_t)a.n_seqs, single = layers && n_rows && n_rows <= 2 * (int64_t)a.n_seqs;
     const int least = tall ? 1 : 2, most = 64 / ds < 8 ? 64 / ds : 8;
     auto ctas = [&](int n) { const int w = GLA_WARPS * 32 / rs * n; return (int64_t)a.n_seqs * a.n_heads * ((a.vdim + w - 1) / w); };
     const int wide = most < 4 ? most : 4;
@@ -1077,8 +1078,8 @@ int launch_row_scan(const A& a, int64_t n_rows, cudaStream_t st) {
             if (!best || cost < best) { nc = n; best = cost; }
         }
     }
-    const int step = single ? ctas(nc) <= (nc * ds <= 32 ? 4 : 3) * 148 ? FEW : SINGLE : (n_rows && !few) || !layers ? RUNS : !DIAG && !n_rows && nc == 4 && ctas(4) > 2 * 148 ? EITHER : ANY;
-    const int many = single ? 4 : DIAG ? few ? 8 : 32 : step == EITHER && a.dim > 128 ? 8 : 16;
+    const int step = single ? ctas(nc) <= (nc * ds <= 32 ? 4 : 3) * 148 ? FEW : SINGLE : (n_rows && !few) || !layers ? RUNS : !DIAG && !n_rows && nc == 4 && ctas(4) > (nc * ds <= 32 ? 4 : 2) * 148 ? EITHER : ANY;
+    const int many = single ? 4 : DIAG ? n_rows <= 8 * (int64_t)a.n_seqs ? 16 : 32 : step == EITHER && a.dim > 128 ? 8 : 16;
     const int cols = GLA_WARPS * 32 / rs * nc;
     const unsigned nvb = (a.vdim + cols - 1) / cols;
     const dim3 grids[3] = {dim3((unsigned)ctas(nc)), dim3(a.n_seqs, a.n_heads, nvb), dim3(nvb, a.n_heads, a.n_seqs)};
