@@ -8,6 +8,7 @@ weight-streaming kernel (p3_gemm_skinny); everything else (fp32 = true 32-bit, o
 on tcgen05; grouped expert products, products per attention head over column blocks, odd shapes) on p3_gemm_any.
 """
 import ctypes as C
+import operator
 import os
 import torch
 from . import _lib
@@ -34,11 +35,14 @@ def _page_slices(pairs, pages, slots=2 * 148, merge=0.0):
     return best
 
 
+_last_of = operator.itemgetter(1)
+
+
 def _shape_of_prompts(w, b, span_of):
     """what the prefill launch shares its work out by: pages that a record of 64 rows sees at most, sequences of the records; span_of(n) = most keys
     a query at position n - 1 sees. A batch that does not say where its prompts lie is taken for one sequence's, or for as many as leave their
     last records half empty where that is more than one can leave"""
-    if b.n_pf * w.n_heads > 224:                                 # the launch has passes enough
+    if b.n_pf * w.n_heads > 224 or b.max_pos < 11 * PAGE:        # passes enough, or pages too few to be worth sharing
         w.max_pages = 0
         return
     runs, chunk, pages = b.pf_runs, w.chunk, 0
@@ -49,6 +53,8 @@ def _shape_of_prompts(w, b, span_of):
         runs = ((max(0, b.max_pos + 1 - rows), b.max_pos),)
     else:
         w.n_seqs = len(runs)
+    if not chunk:
+        runs = (max(runs, key=_last_of),)
     for first, last in runs:
         n = last % chunk + 1 if chunk and first // chunk == last // chunk else last + 1
         pages = max(pages, min(last // PAGE + 1, (span_of(n) + 2 * PAGE - 2) // PAGE))

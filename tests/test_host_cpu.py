@@ -452,7 +452,7 @@ def test_pack_rows16_layout_matches_the_header_formula():
 
 
 @pytest.mark.parametrize('runs,rows,n_pf,n_dec,chunk,window,want', [
-    ([(704, 1036)], 333, 6, 0, 0, 0, (1, 17)), ([(0, 9), (500, 563)], 74, 2, 3, 0, 0, (2, 9)), ([(4336, 4341), (4336, 4519)], 190, 4, 0, 1024, 0, (2, 8)),
+    ([(704, 1036)], 333, 6, 0, 0, 0, (1, 17)), ([(500, 563), (0, 9)], 74, 2, 3, 0, 0, (2, 9)), ([(0, 70)], 71, 200, 0, 0, 0, (0, 0)), ([(0, 703)], 704, 11, 0, 0, 0, (0, 0)), ([(4336, 4341), (4336, 4519)], 190, 4, 0, 1024, 0, (2, 8)),
     ([(1000, 1100)], 101, 2, 0, 1024, 0, (1, 17)), ([(4000, 4400)], 401, 7, 0, 0, 256, (1, 5)),
     (None, 333, 6, 0, 0, 0, (1, 17)), (None, 1092, 18, 2, 0, 0, (1, 17)), (None, 300, 10, 0, 0, 0, (11, 17)), (None, 128, 2, 0, 512, 0, (1, 9))])        # the last: behind a border of chunks, so up to a whole one
 def test_what_a_prefill_launch_is_told_of_its_prompts(runs, rows, n_pf, n_dec, chunk, window, want):
@@ -463,6 +463,6 @@ def test_what_a_prefill_launch_is_told_of_its_prompts(runs, rows, n_pf, n_dec, c
     w.chunk, w.n_heads = chunk, 4
     b.T, b.n_pf, b.n_dec, b.max_pos = rows + n_dec, n_pf, n_dec, 1036
     if runs:
-        b.pf_runs, b.max_pos = runs, 9999
+        b.pf_runs, b.max_pos = runs, 703 if runs == [(0, 703)] else 9999
     _shape_of_prompts(w, b, lambda n: min([n] + [window] * (window > 0) + [chunk] * (chunk > 0)))
     assert (w.n_seqs, w.max_pages) == want
